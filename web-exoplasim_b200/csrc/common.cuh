@@ -50,6 +50,17 @@ inline void pdl_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
   cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Launches a step kernel, by programmatic dependent launch where `pdl` says
+// so (Model::pdl). Every kernel launched through here calls pdl_wait().
+template <typename... KArgs, typename... Args>
+inline void step_launch(int pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                        Args... args) {
+  if (pdl)
+    pdl_launch(kernel, grid, block, smem, st, args...);
+  else
+    kernel<<<grid, block, smem, st>>>(args...);
+}
+
 // Per-planet global budgets (budget.cu): quantities per published step.
 constexpr int kBudgetQuantities = 8;
 constexpr int kBudgetStride = 2 * kBudgetQuantities + 2;  // last[8], sums[8], samples, averaged samples
@@ -199,6 +210,11 @@ struct Model {
   // field after each stage, so there (zero_gdt = 1) the kernels zero and
   // read them as the reference does.
   int zero_gdt;
+  int pdl;    // transform and dynamics kernels start by programmatic dependent launch
+  // Grid and Fourier scratch of mkdheat's first stage (L planes per slot
+  // each; no state field, so a full step can transform both stages' wind
+  // increments in one launch).
+  float *zdu1, *zdv1, *fzdu1, *fzdv1;
   int storm;  // some slot runs the storm-climatology diagnostics (NSTORMDIAG > 0)
 };
 

@@ -26,6 +26,8 @@ __device__ __forceinline__ const float* slot_tabs(const Model& m, int slot) {
 // latency the fourth block hides.
 template <int NL>
 __global__ void __launch_bounds__(kBlock, 4) k_calcgp(Model m) {
+  pdl_wait();
+  pdl_release();
   const Dims& d = m.d;
   // NHOR is a multiple of kBlock at every truncation, so a block lies in one
   // slot and that slot's vertical tables are staged in shared memory once.
@@ -174,6 +176,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_calcgp(Model m) {
 // registers that a looser bound allows measured faster than five blocks.
 template <int NL>
 __global__ void __launch_bounds__(kBlock, 3) k_spectrala(Model m) {
+  pdl_wait();
+  pdl_release();
   const Dims& d = m.d;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= d.S * d.NRSP) return;
@@ -314,6 +318,8 @@ __device__ __forceinline__ void st2(float* p, size_t i, float2 v) { *reinterpret
 // the compiler cannot prove it, and would otherwise order each load after
 // the stores before it.
 __global__ void __launch_bounds__(kBlock) k_spectrald_diffusion(Model m) {
+  pdl_wait();
+  pdl_release();
   const Dims& d = m.d;
   const int c = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   if (c >= d.S * d.NRSP) return;
@@ -376,8 +382,12 @@ constexpr int kCols4 = 4 * kBlock;
 __device__ __forceinline__ float4 ld4(const float* p, size_t i) { return *reinterpret_cast<const float4*>(p + i); }
 __device__ __forceinline__ void st4(float* p, size_t i, float4 v) { *reinterpret_cast<float4*>(p + i) = v; }
 
-// mkdheat's grid-point stages (dynamics/wgsl/mkdheat.wgsl).
-__global__ void __launch_bounds__(kBlock) k_mkdheat(Model m, int stage) {
+// mkdheat's first two grid-point stages (dynamics/wgsl/mkdheat.wgsl): the
+// heating by friction's wind increments (zdu1, zdv1) and the kinetic energy
+// the diffusion's (zdu, zdv) take, in one pass over the winds both read.
+__global__ void __launch_bounds__(kBlock) k_mkdheat_winds(Model m) {
+  pdl_wait();
+  pdl_release();
   const Dims& d = m.d;
   const int slot = blockIdx.x * kCols4 / d.NHOR;
   const int c = blockIdx.x * kCols4 + 4 * threadIdx.x;
@@ -386,60 +396,102 @@ __global__ void __launch_bounds__(kBlock) k_mkdheat(Model m, int stage) {
   const int h = c - slot * d.NHOR;
   const FieldPtrs& F = m.f;
   // inputs first, then the slot's parameters
-  const float4 dq = ld4(F.dq, i);
-  const float4 dp = stage == 1 ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4(F.dp, c);
-  const float4 ek = stage == 3 ? ld4(F.zdekin, i) : make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 zu = ek, zv = ek, zdu = ek, zdv = ek, rc = ek;
-  if (stage != 3) {
-    zu = ld4(F.zu, i);
-    zv = ld4(F.zv, i);
-    zdu = ld4(F.zdu, i);
-    zdv = ld4(F.zdv, i);
-    rc = ld4(m.sh.rcsq, h);
-  }
+  const float4 dq = ld4(F.dq, i), dp = ld4(F.dp, c);
+  const float4 zu = ld4(F.zu, i), zv = ld4(F.zv, i);
+  const float4 du1 = ld4(m.zdu1, i), dv1 = ld4(m.zdv1, i), du2 = ld4(F.zdu, i), dv2 = ld4(F.zdv, i);
+  const float4 rc = ld4(m.sh.rcsq, h);
   const float ds = m.tabs[(size_t)slot * m.to.stride + m.to.dsigma + l];
   const StepParams& P = m.params[slot];
   if (!P.active) return;
   const PlanetConst& K = m.pc[slot];
   const float4 heat = make_float4(1.f + K.ADV * dq.x, 1.f + K.ADV * dq.y, 1.f + K.ADV * dq.z, 1.f + K.ADV * dq.w);
-  if (stage == 3) {
-    // IEEE divisions throughout mkdheat, as in spectrald's diffusion.
-    auto one = [&](float e, float ht, float p) {
-      const float dtdt = __fdiv_rn(__fdiv_rn(__fdiv_rn(__fdiv_rn(-e * 0.5f, K.ACPD), ht), p) * K.GA, ds);
-      return __fdiv_rn(__fdiv_rn(dtdt, K.CT), K.WW);
-    };
-    st4(F.zdtdt, i, make_float4(one(ek.x, heat.x, dp.x), one(ek.y, heat.y, dp.y), one(ek.z, heat.z, dp.z),
-                                one(ek.w, heat.w, dp.w)));
-    return;
-  }
-  auto one = [&](float r, float zu1, float zv1, float zdu1, float zdv1, float ht, float p) {
+  auto change = [&](float r, float zu1, float zv1, float zdu1, float zdv1) {
     const float scale = K.CV * sqrtf(r);
     const float u = zu1 * scale, v = zv1 * scale, du = zdu1 * scale, dv = zdv1 * scale;
-    const float change = du * (2.f * u + du) + dv * (2.f * v + dv);
-    if (stage == 1) {
-      const float dtdt = __fdiv_rn(__fdiv_rn(__fdiv_rn(-change, P.deltsec2) * 0.5f, K.ACPD), ht);
-      return __fdiv_rn(__fdiv_rn(dtdt, K.CT), K.WW);
-    }
-    return __fdiv_rn(__fdiv_rn(change, P.deltsec2) * p, K.GA) * ds;
+    return du * (2.f * u + du) + dv * (2.f * v + dv);
   };
-  const float4 r = make_float4(one(rc.x, zu.x, zv.x, zdu.x, zdv.x, heat.x, dp.x),
-                               one(rc.y, zu.y, zv.y, zdu.y, zdv.y, heat.y, dp.y),
-                               one(rc.z, zu.z, zv.z, zdu.z, zdv.z, heat.z, dp.z),
-                               one(rc.w, zu.w, zv.w, zdu.w, zdv.w, heat.w, dp.w));
-  st4(stage == 1 ? F.zdtdt : F.zdekin, i, r);
+  // IEEE divisions throughout mkdheat, as in spectrald's diffusion.
+  auto friction = [&](float change, float ht) {
+    const float dtdt = __fdiv_rn(__fdiv_rn(__fdiv_rn(-change, P.deltsec2) * 0.5f, K.ACPD), ht);
+    return __fdiv_rn(__fdiv_rn(dtdt, K.CT), K.WW);
+  };
+  auto diffusion = [&](float change, float p) { return __fdiv_rn(__fdiv_rn(change, P.deltsec2) * p, K.GA) * ds; };
+  st4(F.zdtdt, i, make_float4(friction(change(rc.x, zu.x, zv.x, du1.x, dv1.x), heat.x),
+                              friction(change(rc.y, zu.y, zv.y, du1.y, dv1.y), heat.y),
+                              friction(change(rc.z, zu.z, zv.z, du1.z, dv1.z), heat.z),
+                              friction(change(rc.w, zu.w, zv.w, du1.w, dv1.w), heat.w)));
+  st4(F.zdekin, i, make_float4(diffusion(change(rc.x, zu.x, zv.x, du2.x, dv2.x), dp.x),
+                               diffusion(change(rc.y, zu.y, zv.y, du2.y, dv2.y), dp.y),
+                               diffusion(change(rc.z, zu.z, zv.z, du2.z, dv2.z), dp.z),
+                               diffusion(change(rc.w, zu.w, zv.w, du2.w, dv2.w), dp.w)));
 }
 
-// mkdheat's zsdef(2:NESP,:) = 0 (dynamics/wgsl/mean-mode.wgsl).
-// One block row per plane: blockIdx.y = slot, blockIdx.z = level.
-__global__ void k_mean_mode(float* t, int nrsp) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nrsp || r == 0) return;
-  t[((size_t)blockIdx.z * gridDim.y + blockIdx.y) * nrsp + r] = 0.f;
+// mkdheat's third stage. Between the second and the third the shaders
+// transform the kinetic energy to spectral space, keep mode (0, 0) alone
+// (dynamics/wgsl/mean-mode.wgsl) and transform that back. Only fc2sp's sum
+// of mode (0, 0) reaches the result, over the latitude pairs of the Fourier
+// rows' mean (fzdekin, m = 0), and back on the grid a latitude is the
+// constant q(0, 0)[lat] times it, exactly: every other term of sp2fc and
+// fc2gp is a sum with zeros. So each block takes that sum in the shaders'
+// order and no transform runs (fc2sp, the zeroing, sp2gp and this stage's
+// read of zdekin took 20 + 8 + 33 + 8 us at 128 T42 L10 planets, and three
+// of a single planet's launches). The slot's first block also writes the
+// spectral field.
+__global__ void __launch_bounds__(kBlock) k_mkdheat_mean(Model m) {
+  constexpr int kMaxPairs = 48;
+  __shared__ float pair_sum[kMaxPairs], pair_q[kMaxPairs];
+  __shared__ float mean;
+  pdl_wait();
+  pdl_release();
+  const Dims& d = m.d;
+  const int slot = blockIdx.x * kCols4 / d.NHOR;
+  const int c = blockIdx.x * kCols4 + 4 * threadIdx.x;
+  const int l = blockIdx.y;
+  const size_t i = (size_t)l * d.S * d.NHOR + c;
+  const int h = c - slot * d.NHOR, lat = h / d.NLON;
+  const FieldPtrs& F = m.f;
+  const float4 dq = ld4(F.dq, i), dp = ld4(F.dp, c);
+  const size_t plane = (size_t)l * d.S + slot;
+  if (threadIdx.x < 32) {
+    const float* rows = F.fzdekin + plane * d.NLAT * d.NFC;
+    const int step = m.mode >= 1 ? 2 : d.NFC;  // m-major or latitude-major
+    const int half = d.NLAT / 2;
+    for (int j = threadIdx.x; j < half; j += 32) {
+      pair_sum[j] = rows[j * step] + rows[(d.NLAT - 1 - j) * step];
+      pair_q[j] = m.sh.qc[(size_t)j * d.NCSP];
+    }
+    __syncwarp();
+    float s = 0.f;
+#pragma unroll 4
+    for (int j = 0; j < half; ++j) s = fmaf(pair_q[j], pair_sum[j], s);
+    if (threadIdx.x == 0) mean = s;
+  }
+  const float q0 = m.sh.qi[(size_t)lat * d.NCSP];
+  const float ds = m.tabs[(size_t)slot * m.to.stride + m.to.dsigma + l];
+  const StepParams& P = m.params[slot];
+  __syncthreads();
+  if (!P.active) return;
+  const PlanetConst& K = m.pc[slot];
+  const float s00 = mean, ek = q0 * s00;
+  if (c - 4 * (int)threadIdx.x == slot * d.NHOR) {
+    float* out = F.zsdef + plane * d.NRSP;
+    for (int r = threadIdx.x; r < d.NRSP; r += kBlock) out[r] = r == 0 ? s00 : 0.f;
+  }
+  st4(F.zdekin, i, make_float4(ek, ek, ek, ek));
+  const float4 heat = make_float4(1.f + K.ADV * dq.x, 1.f + K.ADV * dq.y, 1.f + K.ADV * dq.z, 1.f + K.ADV * dq.w);
+  // IEEE divisions, as above.
+  auto one = [&](float ht, float p) {
+    const float dtdt = __fdiv_rn(__fdiv_rn(__fdiv_rn(__fdiv_rn(-ek * 0.5f, K.ACPD), ht), p) * K.GA, ds);
+    return __fdiv_rn(__fdiv_rn(dtdt, K.CT), K.WW);
+  };
+  st4(F.zdtdt, i, make_float4(one(heat.x, dp.x), one(heat.y, dp.y), one(heat.z, dp.z), one(heat.w, dp.w)));
 }
 
 // spectrald after mkdheat (dynamics/wgsl/spectrald-update.wgsl), two
 // adjacent real coefficients of one level per thread, inputs read first.
 __global__ void __launch_bounds__(kBlock) k_spectrald_update(Model m) {
+  pdl_wait();
+  pdl_release();
   const Dims& d = m.d;
   const int c = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   if (c >= d.S * d.NRSP) return;
@@ -498,6 +550,8 @@ __global__ void __launch_bounds__(kBlock) k_spectrald_update(Model m) {
 // single-stage replay (Model::zero_gdt).
 template <int NL>
 __global__ void __launch_bounds__(kBlock) k_physics_in(Model m) {
+  pdl_wait();
+  pdl_release();
   const Dims& d = m.d;
   const int slot = blockIdx.x * kBlock / d.NHOR;
   if (!m.params[slot].active) return;
@@ -551,6 +605,8 @@ __global__ void __launch_bounds__(kBlock) k_physics_in(Model m) {
 // Within a full step gudt, gvdt, gtdt hold no earlier increment and are not
 // read (Model::zero_gdt): the sum adds +0 as the zeroed fields would.
 __global__ void __launch_bounds__(kBlock) k_physics_out(Model m) {
+  pdl_wait();
+  pdl_release();
   const Dims& d = m.d;
   const int slot = blockIdx.x * kCols4 / d.NHOR;
   const int c = blockIdx.x * kCols4 + 4 * threadIdx.x;
@@ -587,43 +643,43 @@ void dyn_calcgp(const Model& m, cudaStream_t st) {
   static_assert(2048 % kBlock == 0, "k_calcgp assumes a block lies in one slot");
   const unsigned n = (unsigned)((size_t)m.d.S * m.d.NHOR / kBlock);
   if (m.d.L == 10)
-    k_calcgp<10><<<n, kBlock, 0, st>>>(m);
+    step_launch(m.pdl, k_calcgp<10>, n, kBlock, 0, st, m);
   else
-    k_calcgp<5><<<n, kBlock, 0, st>>>(m);
+    step_launch(m.pdl, k_calcgp<5>, n, kBlock, 0, st, m);
 }
 void dyn_spectrala(const Model& m, cudaStream_t st) {
   const unsigned n = blocks((size_t)m.d.S * m.d.NRSP, kBlock);
   if (m.d.L == 10)
-    k_spectrala<10><<<n, kBlock, 0, st>>>(m);
+    step_launch(m.pdl, k_spectrala<10>, n, kBlock, 0, st, m);
   else
-    k_spectrala<5><<<n, kBlock, 0, st>>>(m);
+    step_launch(m.pdl, k_spectrala<5>, n, kBlock, 0, st, m);
 }
 void dyn_spectrald_diffusion(const Model& m, cudaStream_t st) {
   const dim3 grid(blocks((size_t)m.d.S * m.d.NRSP / 2, kBlock), m.d.NLEV);
-  k_spectrald_diffusion<<<grid, kBlock, 0, st>>>(m);
+  step_launch(m.pdl, k_spectrald_diffusion, grid, kBlock, 0, st, m);
 }
-void dyn_mkdheat(const Model& m, int stage, cudaStream_t st) {
+void dyn_mkdheat_winds(const Model& m, cudaStream_t st) {
   const dim3 grid((unsigned)((size_t)m.d.S * m.d.NHOR / kCols4), m.d.NLEV);
-  k_mkdheat<<<grid, kBlock, 0, st>>>(m, stage);
+  step_launch(m.pdl, k_mkdheat_winds, grid, kBlock, 0, st, m);
 }
-void dyn_mean_mode(const Model& m, float* target, cudaStream_t st) {
-  const dim3 grid(blocks((size_t)m.d.NRSP, 256), m.d.S, m.d.NLEV);
-  k_mean_mode<<<grid, 256, 0, st>>>(target, m.d.NRSP);
+void dyn_mkdheat_mean(const Model& m, cudaStream_t st) {
+  const dim3 grid((unsigned)((size_t)m.d.S * m.d.NHOR / kCols4), m.d.NLEV);
+  step_launch(m.pdl, k_mkdheat_mean, grid, kBlock, 0, st, m);
 }
 void dyn_spectrald_update(const Model& m, cudaStream_t st) {
   const dim3 grid(blocks((size_t)m.d.S * m.d.NRSP / 2, kBlock), m.d.NLEV);
-  k_spectrald_update<<<grid, kBlock, 0, st>>>(m);
+  step_launch(m.pdl, k_spectrald_update, grid, kBlock, 0, st, m);
 }
 void dyn_physics_in(const Model& m, cudaStream_t st) {
   const unsigned n = (unsigned)((size_t)m.d.S * m.d.NHOR / kBlock);
   if (m.d.L == 10)
-    k_physics_in<10><<<n, kBlock, 0, st>>>(m);
+    step_launch(m.pdl, k_physics_in<10>, n, kBlock, 0, st, m);
   else
-    k_physics_in<5><<<n, kBlock, 0, st>>>(m);
+    step_launch(m.pdl, k_physics_in<5>, n, kBlock, 0, st, m);
 }
 void dyn_physics_out(const Model& m, cudaStream_t st) {
   const dim3 grid((unsigned)((size_t)m.d.S * m.d.NHOR / kCols4), m.d.NLEV);
-  k_physics_out<<<grid, kBlock, 0, st>>>(m);
+  step_launch(m.pdl, k_physics_out, grid, kBlock, 0, st, m);
 }
 
 }  // namespace exogcm

@@ -92,6 +92,8 @@ struct exogcm_engine {
   std::map<std::string, size_t> field_index;
   float* arena = nullptr;
   size_t arena_floats = 0;
+  size_t state_floats = 0;    // the fields'
+  size_t scratch_offset = 0;  // mkdheat's scratch
   FieldPtrs fp{};
   // shared tables
   bool shared_ready = false;
@@ -133,6 +135,7 @@ struct exogcm_engine {
   std::map<int, cudaGraphExec_t> graphs;
   std::map<int, cudaGraph_t> graph_templates;  // the captured K-step graphs (child nodes of group graphs)
   Tuning tune{};
+  int pdl = 0;  // Model::pdl
   SharedSetup shared_setup;  // host copy of the shared tables (set-up of later planets)
   // FP64 set-up loops on this device (setup_device.cu), created at the first
   // configure; exogcm_setup_on_device(e, 0) moves them to the host.
@@ -159,6 +162,12 @@ struct exogcm_engine {
     m.tune = tune;
     m.keep_fourier = 0;
     m.zero_gdt = 0;
+    const size_t grid = (size_t)d.L * d.S * d.NHOR, four = (size_t)d.L * d.S * d.NLAT * d.NFC;
+    m.zdu1 = arena + scratch_offset;
+    m.zdv1 = m.zdu1 + grid;
+    m.fzdu1 = m.zdv1 + grid;
+    m.fzdv1 = m.fzdu1 + four;
+    m.pdl = pdl;
     m.storm = 0;
     for (const Slot& s : slots) m.storm |= s.storm ? 1 : 0;
     return m;
@@ -198,6 +207,11 @@ void layout(exogcm_engine* e) {
     EXOGCM_FIELDS(EXOGCM_ADD_FIELD)
   }
 #undef EXOGCM_ADD_FIELD
+  e->state_floats = off;
+  // mkdheat's scratch behind the state fields: two grid, two Fourier fields
+  off = (off + 63) / 64 * 64;
+  e->scratch_offset = off;
+  off += 2 * (size_t)d.L * d.S * (d.NHOR + (size_t)d.NLAT * d.NFC);
   e->arena_floats = off;
 }
 
@@ -384,55 +398,86 @@ void upload_shared(exogcm_engine* e, const SharedSetup& s) {
 }
 
 // ---------------------------------------------------------------- the step
+// One field of a transform launch (TrField): inputs a, b, c, outputs x, y.
+TrField fourier_field(const float* a, float* x, int planes, int opt = 0) {
+  TrField t;
+  t.a = a;
+  t.x = x;
+  t.planes = planes;
+  t.opt = opt;
+  return t;
+}
+TrField grid_field(const float* s, float* f, float* g, int planes, int opt = 0) {
+  TrField t = fourier_field(s, f, planes, opt);
+  t.y = g;
+  return t;
+}
+TrField wind_field(const float* a, const float* b, const float* c, float* x, float* y, int planes, float plavor = 0.f) {
+  TrField t;
+  t.a = a;
+  t.b = b;
+  t.c = c;
+  t.x = x;
+  t.y = y;
+  t.planes = planes;
+  t.plavor = plavor;
+  return t;
+}
+template <typename... T>
+TrSet set_of(const T&... fields) {
+  TrSet s;
+  (s.add(fields), ...);
+  return s;
+}
+
+constexpr float kPlavor = 1.63299310207f;
+
 void stage_gridpointa(const Model& m, cudaStream_t st) {
   const Dims& d = m.d;
   const FieldPtrs& F = m.f;
   const int LP = d.L * d.S, SP = d.S;
-  tr_dv2uv(m, F.sd, F.sz, F.fgu, F.fgv, LP, 1.63299310207f, st);
-  tr_legendre_inverse(m, F.sp, F.fgp, SP, m.sh.qi, st);
-  tr_dlambda(m, F.fgp, F.fgpmt, SP, st);
-  tr_fourier_inverse(m, F.fgu, F.gu, LP, st);
-  tr_fourier_inverse(m, F.fgv, F.gv, LP, st);
-  tr_sp2gp(m, F.st, F.fgt, F.gt, LP, m.sh.qi, st);
-  tr_sp2gp(m, F.sd, F.fgd, F.gd, LP, m.sh.qi, st);
-  tr_sp2gp(m, F.sz, F.fgz, F.gz, LP, m.sh.qi, st);
-  tr_sp2gp(m, F.sp, F.fgpj, F.gpj, SP, m.sh.qj, st);
-  tr_fourier_inverse(m, F.fgpmt, F.gpmt, SP, st);
-  tr_fourier_inverse(m, F.fgp, F.gp, SP, st);
-  tr_sp2gp(m, F.sq, F.fgq, F.gq, LP, m.sh.qi, st);
+  tr_dv2uv(m, set_of(wind_field(F.sd, F.sz, nullptr, F.fgu, F.fgv, LP, kPlavor)), st);
+  tr_to_grid(m,
+             set_of(grid_field(F.st, F.fgt, F.gt, LP), grid_field(F.sd, F.fgd, F.gd, LP),
+                    grid_field(F.sz, F.fgz, F.gz, LP), grid_field(F.sq, F.fgq, F.gq, LP),
+                    grid_field(F.sp, F.fgp, F.gp, SP), grid_field(F.sp, F.fgpmt, F.gpmt, SP, kTrDlambda | kTrKeep),
+                    grid_field(F.sp, F.fgpj, F.gpj, SP, kTrDerivative)),
+             set_of(fourier_field(F.fgu, F.gu, LP), fourier_field(F.fgv, F.gv, LP)), st);
   dyn_calcgp(m, st);
-  tr_fourier_forward(m, F.gtn, F.fgtn, LP, st);
-  tr_fourier_forward(m, F.gqn, F.fgqn, LP, st);
-  tr_fourier_forward(m, F.gut, F.fgut, LP, st);
-  tr_fourier_forward(m, F.gvt, F.fgvt, LP, st);
-  tr_fourier_forward(m, F.guz, F.fguz, LP, st);
-  tr_fourier_forward(m, F.gvz, F.fgvz, LP, st);
-  tr_fourier_forward(m, F.gke, F.fgke, LP, st);
-  tr_fourier_forward(m, F.gvpp, F.fgvpp, SP, st);
-  tr_fourier_forward(m, F.guq, F.fguq, LP, st);
-  tr_fourier_forward(m, F.gvq, F.fgvq, LP, st);
-  tr_legendre_forward(m, F.fgvpp, F.spt, SP, m.sh.qc, st);
-  tr_uv2dv(m, F.fgvz, F.fguz, F.fgke, F.sdt, F.szt, LP, st);
-  tr_qtend(m, F.fgut, F.fgvt, F.fgtn, F.stt, LP, st);
-  tr_qtend(m, F.fguq, F.fgvq, F.fgqn, F.sqt, LP, st);
+  tr_fourier_forward(m,
+                     set_of(fourier_field(F.gtn, F.fgtn, LP), fourier_field(F.gqn, F.fgqn, LP),
+                            fourier_field(F.gut, F.fgut, LP), fourier_field(F.gvt, F.fgvt, LP),
+                            fourier_field(F.guz, F.fguz, LP), fourier_field(F.gvz, F.fgvz, LP),
+                            fourier_field(F.gke, F.fgke, LP), fourier_field(F.guq, F.fguq, LP),
+                            fourier_field(F.gvq, F.fgvq, LP), fourier_field(F.gvpp, F.fgvpp, SP)),
+                     st);
+  tr_legendre_forward(m, set_of(fourier_field(F.fgvpp, F.spt, SP)), st);
+  tr_uv2dv(m, set_of(wind_field(F.fgvz, F.fguz, F.fgke, F.sdt, F.szt, LP)), st);
+  tr_qtend(m,
+           set_of(wind_field(F.fgut, F.fgvt, F.fgtn, F.stt, nullptr, LP),
+                  wind_field(F.fguq, F.fgvq, F.fgqn, F.sqt, nullptr, LP)),
+           st);
 }
 
 void stage_physics_in(const Model& m, cudaStream_t st) {
   const Dims& d = m.d;
   const FieldPtrs& F = m.f;
   const int LP = d.L * d.S, SP = d.S;
-  tr_dv2uv(m, F.sd, F.sz, F.fgu, F.fgv, LP, 1.63299310207f, st);
-  tr_fourier_inverse(m, F.fgu, F.gu, LP, st);
-  tr_fourier_inverse(m, F.fgv, F.gv, LP, st);
-  tr_sp2gp(m, F.st, F.fgt, F.gt, LP, m.sh.qi, st);
-  tr_sp2gp(m, F.sp, F.fgp, F.gp, SP, m.sh.qi, st);
-  tr_sp2gp(m, F.sq, F.fgq, F.gq, LP, m.sh.qi, st);
+  tr_dv2uv(m, set_of(wind_field(F.sd, F.sz, nullptr, F.fgu, F.fgv, LP, kPlavor)), st);
+  tr_to_grid(m,
+             set_of(grid_field(F.st, F.fgt, F.gt, LP), grid_field(F.sq, F.fgq, F.gq, LP),
+                    grid_field(F.sp, F.fgp, F.gp, SP)),
+             set_of(fourier_field(F.fgu, F.gu, LP), fourier_field(F.fgv, F.gv, LP)), st);
   dyn_physics_in(m, st);
 }
 
+// The humidity tendency the precipitation reads.
+void precipitation_dqt(const Model& m, cudaStream_t st) {
+  tr_to_grid(m, set_of(grid_field(m.f.sqt, m.f.fdqt, m.f.dqt, m.d.L * m.d.S)), TrSet{}, st);
+}
+
 void stage_precipitation(const Model& m, cudaStream_t st) {
-  const int LP = m.d.L * m.d.S;
-  tr_sp2gp(m, m.f.sqt, m.f.fdqt, m.f.dqt, LP, m.sh.qi, st);
+  precipitation_dqt(m, st);
   phy_precipitation_columns(m, st);
 }
 
@@ -440,40 +485,40 @@ void stage_physics_out(const Model& m, cudaStream_t st) {
   const int LP = m.d.L * m.d.S;
   const FieldPtrs& F = m.f;
   dyn_physics_out(m, st);
-  tr_fourier_forward(m, F.gtdt, F.fgtdt, LP, st);
-  tr_fourier_forward(m, F.gudt, F.fgudt, LP, st);
-  tr_fourier_forward(m, F.gvdt, F.fgvdt, LP, st);
-  tr_fourier_forward(m, F.gqdt, F.fgqdt, LP, st);
-  tr_legendre_forward(m, F.fgtdt, F.stt, LP, m.sh.qc, st);
-  tr_legendre_forward(m, F.fgqdt, F.sqt, LP, m.sh.qc, st);
-  tr_uv2dv(m, F.fgudt, F.fgvdt, nullptr, F.sdt, F.szt, LP, st);
+  tr_fourier_forward(m,
+                     set_of(fourier_field(F.gtdt, F.fgtdt, LP), fourier_field(F.gudt, F.fgudt, LP),
+                            fourier_field(F.gvdt, F.fgvdt, LP), fourier_field(F.gqdt, F.fgqdt, LP)),
+                     st);
+  tr_legendre_forward(m, set_of(fourier_field(F.fgtdt, F.stt, LP), fourier_field(F.fgqdt, F.sqt, LP)), st);
+  tr_uv2dv(m, set_of(wind_field(F.fgudt, F.fgvdt, nullptr, F.sdt, F.szt, LP)), st);
 }
 
+// mkdheat's two wind increments come from the diffusion's spectral fields
+// alone, so both are transformed with the winds, friction's into scratch of
+// its own; what its second stage passes to the third is a mean per plane
+// (k_mkdheat_mean), for which only m = 0 of the kinetic energy is kept.
 void stage_spectrald(const Model& m, cudaStream_t st) {
   const int LP = m.d.L * m.d.S;
   const FieldPtrs& F = m.f;
-  const float plavor = 1.63299310207f;
   dyn_spectrald_diffusion(m, st);
-  tr_dv2uv(m, F.sdp, F.szp, F.fzu, F.fzv, LP, plavor, st);
-  tr_fourier_inverse(m, F.fzu, F.zu, LP, st);
-  tr_fourier_inverse(m, F.fzv, F.zv, LP, st);
-  tr_dv2uv(m, F.zdsdp1, F.zdszp1, F.fzdu, F.fzdv, LP, 0.f, st);
-  tr_fourier_inverse(m, F.fzdu, F.zdu, LP, st);
-  tr_fourier_inverse(m, F.fzdv, F.zdv, LP, st);
-  dyn_mkdheat(m, 1, st);
-  tr_fourier_forward(m, F.zdtdt, F.fzdtdt, LP, st);
-  tr_legendre_forward(m, F.fzdtdt, F.zstt1, LP, m.sh.qc, st);
-  tr_dv2uv(m, F.zdsdp2, F.zdszp2, F.fzdu, F.fzdv, LP, 0.f, st);
-  tr_fourier_inverse(m, F.fzdu, F.zdu, LP, st);
-  tr_fourier_inverse(m, F.fzdv, F.zdv, LP, st);
-  dyn_mkdheat(m, 2, st);
-  tr_fourier_forward(m, F.zdekin, F.fzdekin, LP, st);
-  tr_legendre_forward(m, F.fzdekin, F.zsdef, LP, m.sh.qc, st);
-  dyn_mean_mode(m, F.zsdef, st);
-  tr_sp2gp(m, F.zsdef, F.fzdekin, F.zdekin, LP, m.sh.qi, st);
-  dyn_mkdheat(m, 3, st);
-  tr_fourier_forward(m, F.zdtdt, F.fzdtdt, LP, st);
-  tr_legendre_forward(m, F.fzdtdt, F.zstt2, LP, m.sh.qc, st);
+  tr_dv2uv(m,
+           set_of(wind_field(F.sdp, F.szp, nullptr, F.fzu, F.fzv, LP, kPlavor),
+                  wind_field(F.zdsdp1, F.zdszp1, nullptr, m.fzdu1, m.fzdv1, LP),
+                  wind_field(F.zdsdp2, F.zdszp2, nullptr, F.fzdu, F.fzdv, LP)),
+           st);
+  tr_fourier_inverse(m,
+                     set_of(fourier_field(F.fzu, F.zu, LP), fourier_field(F.fzv, F.zv, LP),
+                            fourier_field(m.fzdu1, m.zdu1, LP), fourier_field(m.fzdv1, m.zdv1, LP),
+                            fourier_field(F.fzdu, F.zdu, LP), fourier_field(F.fzdv, F.zdv, LP)),
+                     st);
+  dyn_mkdheat_winds(m, st);
+  tr_fourier_forward(m, set_of(fourier_field(F.zdtdt, F.fzdtdt, LP), fourier_field(F.zdekin, F.fzdekin, LP, 1)), st);
+  tr_legendre_forward(m, set_of(fourier_field(F.fzdtdt, F.zstt1, LP)), st);
+  dyn_mkdheat_mean(m, st);
+  // the mean's Fourier field, kept on the plain path and by stage replay
+  if (m.mode == 0 || m.keep_fourier) tr_legendre_inverse(m, set_of(fourier_field(F.zsdef, F.fzdekin, LP)), st);
+  tr_fourier_forward(m, set_of(fourier_field(F.zdtdt, F.fzdtdt, LP)), st);
+  tr_legendre_forward(m, set_of(fourier_field(F.fzdtdt, F.zstt2, LP)), st);
   dyn_spectrald_update(m, st);
 }
 
@@ -503,7 +548,7 @@ void full_step(const Model& m, cudaStream_t st) {
   dyn_spectrala(m, st);
   stage_physics_in(m, st);
   phy_fused_through_radiation(m, st);
-  tr_sp2gp(m, m.f.sqt, m.f.fdqt, m.f.dqt, m.d.L * m.d.S, m.sh.qi, st);  // precipitation's dqt
+  precipitation_dqt(m, st);
   phy_fused_precipitation_to_carbon(m, st);
   phy_storm(m, st);
   stage_physics_out(m, st);
@@ -708,12 +753,20 @@ void autotune(exogcm_engine* e) {
     }
     return total;
   };
+  // launches of as many fields as the step's
+  const TrSet inverse = set_of(fourier_field(F.fgu, F.gu, LP), fourier_field(F.fgv, F.gv, LP),
+                               fourier_field(F.fzu, F.zu, LP), fourier_field(F.fzv, F.zv, LP));
+  const TrSet forward = set_of(fourier_field(F.gtn, F.fgtn, LP), fourier_field(F.gqn, F.fgqn, LP),
+                               fourier_field(F.gut, F.fgut, LP), fourier_field(F.gvt, F.fgvt, LP),
+                               fourier_field(F.guz, F.fguz, LP), fourier_field(F.gvz, F.fgvz, LP));
+  const TrSet to_grid = set_of(grid_field(F.st, F.fgt, F.gt, LP), grid_field(F.sq, F.fgq, F.gq, LP),
+                               grid_field(F.sz, F.fgz, F.gz, LP));
   {
     const Model m = e->model(0);
     auto now = [] { return std::chrono::steady_clock::now(); };
     const auto start = now();
     while (now() - start < std::chrono::milliseconds(50)) {
-      for (int r = 0; r < 20; ++r) tr_fourier_inverse(m, F.fgu, F.gu, LP, e->stream);
+      for (int r = 0; r < 20; ++r) tr_fourier_inverse(m, inverse, e->stream);
       check(cudaStreamSynchronize(e->stream), "autotune warm-up");
     }
   }
@@ -724,8 +777,8 @@ void autotune(exogcm_engine* e) {
       if (!fft_rows_supported(d, rows)) continue;
       t.fft_rows = rows;
       const float ms = time([&](const Model& m) {
-        tr_fourier_inverse(m, F.fgu, F.gu, LP, e->stream);
-        tr_fourier_forward(m, F.gtn, F.fgtn, LP, e->stream);
+        tr_fourier_inverse(m, inverse, e->stream);
+        tr_fourier_forward(m, forward, e->stream);
       });
       if (ms < best) best = ms, pick = rows;
     }
@@ -737,9 +790,9 @@ void autotune(exogcm_engine* e) {
         t.fft_persistent[dir] = form;
         ms[form] = time([&](const Model& m) {
           if (dir == 0)
-            tr_fourier_forward(m, F.gtn, F.fgtn, LP, e->stream);
+            tr_fourier_forward(m, forward, e->stream);
           else
-            tr_fourier_inverse(m, F.fgu, F.gu, LP, e->stream);
+            tr_fourier_inverse(m, inverse, e->stream);
         });
       }
       t.fft_persistent[dir] = ms[1] < ms[0] ? 1 : 0;
@@ -755,9 +808,9 @@ void autotune(exogcm_engine* e) {
         t.inv_tile[k] = tile;
         const float ms = time([&](const Model& m) {
           if (k == 0)
-            tr_legendre_inverse(m, F.st, F.fgt, LP, m.sh.qi, e->stream);
+            tr_legendre_inverse(m, set_of(fourier_field(F.st, F.fgt, LP)), e->stream);
           else
-            tr_dv2uv(m, F.sd, F.sz, F.fgu, F.fgv, LP, 0.f, e->stream);
+            tr_dv2uv(m, set_of(wind_field(F.sd, F.sz, nullptr, F.fgu, F.fgv, LP)), e->stream);
         });
         if (ms < best) best = ms, pg = group, pt = tile;
       }
@@ -774,13 +827,16 @@ void autotune(exogcm_engine* e) {
       t.fwd_buffers[k] = buffers;
       const float ms = time([&](const Model& m) {
         if (k == 0)
-          tr_legendre_forward(m, F.fgtdt, F.zstt1, LP, m.sh.qc, e->stream);
+          tr_legendre_forward(m, set_of(fourier_field(F.fgtdt, F.zstt1, LP)), e->stream);
         else if (k == 1)
-          tr_uv2dv(m, F.fgudt, F.fgvdt, nullptr, F.sdt, F.szt, LP, e->stream);
+          tr_uv2dv(m, set_of(wind_field(F.fgudt, F.fgvdt, nullptr, F.sdt, F.szt, LP)), e->stream);
         else if (k == 2)
-          tr_uv2dv(m, F.fgvz, F.fguz, F.fgke, F.zdsdp1, F.zdszp1, LP, e->stream);
+          tr_uv2dv(m, set_of(wind_field(F.fgvz, F.fguz, F.fgke, F.zdsdp1, F.zdszp1, LP)), e->stream);
         else
-          tr_qtend(m, F.fgut, F.fgvt, F.fgtn, F.zstt2, LP, e->stream);
+          tr_qtend(m,
+                   set_of(wind_field(F.fgut, F.fgvt, F.fgtn, F.zstt2, nullptr, LP),
+                          wind_field(F.fguq, F.fgvq, F.fgqn, F.zstt1, nullptr, LP)),
+                   e->stream);
       });
       if (ms < best) best = ms, pick = tile, pick_buffers = buffers;
     }
@@ -793,7 +849,7 @@ void autotune(exogcm_engine* e) {
     for (int pp : {2, 4}) {
       if (grid_sp2gp_smem(d, pp) > kLegSmemLimit) continue;
       t.sp2gp_planes = pp;
-      const float ms = time([&](const Model& m) { tr_sp2gp(m, F.st, F.fgt, F.gt, LP, m.sh.qi, e->stream); });
+      const float ms = time([&](const Model& m) { tr_to_grid(m, to_grid, TrSet{}, e->stream); });
       if (ms < best) best = ms, pick = pp;
     }
     t.sp2gp_planes = pick;
@@ -1671,10 +1727,10 @@ int exogcm_time_kernel(exogcm_engine* e, const char* kernel, int reps, float* ms
     double b = 0;
     const double L = d.L;
     if (k == "fourier_forward") {
-      launch = [&] { tr_fourier_forward(m, F.gtn, F.fgtn, LP, e->stream); };
+      launch = [&] { tr_fourier_forward(m, set_of(fourier_field(F.gtn, F.fgtn, LP)), e->stream); };
       b = LP * (grid + four);
     } else if (k == "fourier_inverse") {
-      launch = [&] { tr_fourier_inverse(m, F.fgu, F.gu, LP, e->stream); };
+      launch = [&] { tr_fourier_inverse(m, set_of(fourier_field(F.fgu, F.gu, LP)), e->stream); };
       b = LP * (four + grid);
     } else if (k == "fourier_forward_per_chunk" || k == "fourier_forward_persistent" ||
                k == "fourier_inverse_per_chunk" || k == "fourier_inverse_persistent") {
@@ -1685,17 +1741,17 @@ int exogcm_time_kernel(exogcm_engine* e, const char* kernel, int reps, float* ms
         Model mp = m;
         mp.tune.fft_persistent[forward ? 0 : 1] = form;
         if (forward)
-          tr_fourier_forward(mp, F.gtn, F.fgtn, LP, e->stream);
+          tr_fourier_forward(mp, set_of(fourier_field(F.gtn, F.fgtn, LP)), e->stream);
         else
-          tr_fourier_inverse(mp, F.fgu, F.gu, LP, e->stream);
+          tr_fourier_inverse(mp, set_of(fourier_field(F.fgu, F.gu, LP)), e->stream);
       };
       b = LP * (grid + four);
     } else if (k == "legendre_forward") {
-      launch = [&] { tr_legendre_forward(m, F.fgtdt, F.zstt1, LP, m.sh.qc, e->stream); };
+      launch = [&] { tr_legendre_forward(m, set_of(fourier_field(F.fgtdt, F.zstt1, LP)), e->stream); };
       b = LP * (four + spec);
     } else if (k == "sp2gp") {
       // fused sp2fc + fc2gp: the spectral plane in, the grid plane out
-      launch = [&] { tr_sp2gp(m, F.st, F.fgt, F.gt, LP, m.sh.qi, e->stream); };
+      launch = [&] { tr_to_grid(m, set_of(grid_field(F.st, F.fgt, F.gt, LP)), TrSet{}, e->stream); };
       b = LP * (spec + grid);
     } else if (k == "sp2gp_planes2" || k == "sp2gp_planes4") {
       // the fused transform at a fixed number of planes per pass
@@ -1704,20 +1760,20 @@ int exogcm_time_kernel(exogcm_engine* e, const char* kernel, int reps, float* ms
       launch = [&, pp] {
         Model mp = m;
         mp.tune.sp2gp_planes = pp;
-        tr_sp2gp(mp, F.st, F.fgt, F.gt, LP, mp.sh.qi, e->stream);
+        tr_to_grid(mp, set_of(grid_field(F.st, F.fgt, F.gt, LP)), TrSet{}, e->stream);
       };
       b = LP * (spec + grid);
     } else if (k == "legendre_inverse") {
-      launch = [&] { tr_legendre_inverse(m, F.st, F.fgt, LP, m.sh.qi, e->stream); };
+      launch = [&] { tr_legendre_inverse(m, set_of(fourier_field(F.st, F.fgt, LP)), e->stream); };
       b = LP * (spec + four);
     } else if (k == "dv2uv") {
-      launch = [&] { tr_dv2uv(m, F.sd, F.sz, F.fgu, F.fgv, LP, 1.63299310207f, e->stream); };
+      launch = [&] { tr_dv2uv(m, set_of(wind_field(F.sd, F.sz, nullptr, F.fgu, F.fgv, LP, kPlavor)), e->stream); };
       b = LP * 2 * (spec + four);
     } else if (k == "uv2dv") {
-      launch = [&] { tr_uv2dv(m, F.fgvz, F.fguz, F.fgke, F.zdsdp1, F.zdszp1, LP, e->stream); };
+      launch = [&] { tr_uv2dv(m, set_of(wind_field(F.fgvz, F.fguz, F.fgke, F.zdsdp1, F.zdszp1, LP)), e->stream); };
       b = LP * (3 * four + 2 * spec);
     } else if (k == "qtend") {
-      launch = [&] { tr_qtend(m, F.fgut, F.fgvt, F.fgtn, F.zstt2, LP, e->stream); };
+      launch = [&] { tr_qtend(m, set_of(wind_field(F.fgut, F.fgvt, F.fgtn, F.zstt2, nullptr, LP)), e->stream); };
       b = LP * (3 * four + spec);
     } else if (k == "calcgp") {
       launch = [&] { dyn_calcgp(m, e->stream); };
@@ -1726,9 +1782,9 @@ int exogcm_time_kernel(exogcm_engine* e, const char* kernel, int reps, float* ms
       launch = [&] { dyn_spectrala(m, e->stream); };
       b = (double)S * d.NRSP * 4 * (6.0 * d.L + 3 + 14.0 * d.L + 3);
     } else if (k == "mkdheat") {
-      // stage 1: dq, u, v, du, dv per level and dp in; dtdt out
-      launch = [&] { dyn_mkdheat(m, 1, e->stream); };
-      b = cols * 4 * (6.0 * d.L + 1);
+      // its first two stages: dq, u, v and two du, dv per level and dp in; dtdt and the kinetic energy out
+      launch = [&] { dyn_mkdheat_winds(m, e->stream); };
+      b = cols * 4 * (9.0 * d.L + 1);
     } else if (k == "physics_in") {
       // gp, u, v, t, q in; dp, the dimensional u, v, t, q and the surface
       // level of the zeroed dimensional tendencies out

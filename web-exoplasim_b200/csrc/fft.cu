@@ -27,6 +27,7 @@
 
 #include <algorithm>
 
+#include "async_copy.cuh"
 #include "common.cuh"
 #include "fft_core.cuh"
 #include "launch.h"
@@ -41,7 +42,7 @@ constexpr int kMaxThreads = 512;
 
 // gp2fc: rows of N grid values -> m-major coefficients.
 template <int Q>
-__global__ void __launch_bounds__(kMaxThreads) k_fft_forward(const float* __restrict__ g, float* __restrict__ c,
+__global__ void __launch_bounds__(kMaxThreads) k_fft_forward(const __grid_constant__ TrSet set,
                                                              const float2* __restrict__ twg, int nlat, int rows) {
   using Sh = Shape<Q>;
   constexpr int T = Sh::T, N = Sh::N, NTP1 = Sh::NTP1;
@@ -52,17 +53,21 @@ __global__ void __launch_bounds__(kMaxThreads) k_fft_forward(const float* __rest
   float2* fc = xb + rows * Sh::XP;
   const int pitch = fc_pitch(rows, T);
   const int chunks = nlat / rows;
-  const size_t plane = blockIdx.x / chunks;
+  const int tile = blockIdx.x / chunks, fi = tr_find(set, tile);
+  const size_t plane = tile - set.at[fi];
   const int lat0 = (blockIdx.x % chunks) * rows;
   const int r = threadIdx.x / T, t = threadIdx.x % T;
+  copy_twiddles<Q>(twg, tw, twq);
+  pdl_wait();
+  pdl_release();
   // z_n = g_2n + i g_2n+1 for n = Q p + q
-  const float2* in = reinterpret_cast<const float2*>(g + (plane * nlat + lat0 + r) * N);
+  const float2* in = reinterpret_cast<const float2*>(set.f[fi].a + (plane * nlat + lat0 + r) * N);
   float2 a[Sh::QT][8];
 #pragma unroll
   for (int i = 0; i < Sh::QT; ++i)
 #pragma unroll
-    for (int p = 0; p < 8; ++p) a[i][p] = in[Q * p + t + T * i];
-  load_twiddles<Q>(twg, tw, twq);
+    for (int p = 0; p < 8; ++p) a[i][p] = __ldg(in + Q * p + t + T * i);
+  cp_async_wait_all();
   __syncthreads();
   float2* xr = xb + r * Sh::XP;
   float2 b[Sh::KT][Q];
@@ -96,14 +101,15 @@ __global__ void __launch_bounds__(kMaxThreads) k_fft_forward(const float* __rest
   __syncthreads();
   // rows * T threads: thread (m0, lat) writes m = m0, m0 + T, ...
   const int lat = threadIdx.x % rows, m0 = threadIdx.x / rows;
-  float2* out = reinterpret_cast<float2*>(c) + plane * nlat * NTP1 + lat0 + lat;
+  float2* out = reinterpret_cast<float2*>(set.f[fi].x) + plane * nlat * NTP1 + lat0 + lat;
+  const int mend = set.f[fi].opt ? set.f[fi].opt : NTP1;
 #pragma unroll 4
-  for (int m = m0; m < NTP1; m += T) out[(size_t)m * nlat] = fc[m * pitch + lat];
+  for (int m = m0; m < mend; m += T) out[(size_t)m * nlat] = fc[m * pitch + lat];
 }
 
 // fc2gp: m-major coefficients -> rows of N grid values.
 template <int Q>
-__global__ void __launch_bounds__(kMaxThreads) k_fft_inverse(const float* __restrict__ c, float* __restrict__ g,
+__global__ void __launch_bounds__(kMaxThreads) k_fft_inverse(const __grid_constant__ TrSet set,
                                                              const float2* __restrict__ twg, int nlat, int rows) {
   using Sh = Shape<Q>;
   constexpr int T = Sh::T, M = Sh::M, N = Sh::N, NTP1 = Sh::NTP1;
@@ -114,21 +120,25 @@ __global__ void __launch_bounds__(kMaxThreads) k_fft_inverse(const float* __rest
   float2* fc = xb + rows * Sh::XP;
   const int pitch = fc_pitch(rows, T);
   const int chunks = nlat / rows;
-  const size_t plane = blockIdx.x / chunks;
+  const int tile = blockIdx.x / chunks, fi = tr_find(set, tile);
+  const size_t plane = tile - set.at[fi];
   const int lat0 = (blockIdx.x % chunks) * rows;
+  copy_twiddles<Q>(twg, tw, twq);
+  pdl_wait();
+  pdl_release();
   {
     // rows * T threads: thread (m0, lat) stages m = m0, m0 + T, ... < NTP1;
     // Im c_0 is ignored.
     const int lat = threadIdx.x % rows, m0 = threadIdx.x / rows;
-    const float2* src = reinterpret_cast<const float2*>(c) + plane * nlat * NTP1 + lat0 + lat;
+    const float2* src = reinterpret_cast<const float2*>(set.f[fi].a) + plane * nlat * NTP1 + lat0 + lat;
 #pragma unroll 4
     for (int m = m0; m < NTP1; m += T) {
-      float2 v = src[(size_t)m * nlat];
+      float2 v = __ldg(src + (size_t)m * nlat);
       if (m == 0) v.y = 0.f;
       fc[m * pitch + lat] = v;
     }
   }
-  load_twiddles<Q>(twg, tw, twq);
+  cp_async_wait_all();
   __syncthreads();
   const int r = threadIdx.x / T, t = threadIdx.x % T;
   float2 a[Sh::QT][8];
@@ -148,7 +158,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_fft_inverse(const float* __rest
   float2* xr = xb + r * Sh::XP;
   float2 b[Sh::KT][Q];
   four_step<Q, 1>(a, b, twq, xr, t);
-  float2* out = reinterpret_cast<float2*>(g + (plane * nlat + lat0 + r) * N);
+  float2* out = reinterpret_cast<float2*>(set.f[fi].x + (plane * nlat + lat0 + r) * N);
 #pragma unroll
   for (int j = 0; j < Sh::KT; ++j)
 #pragma unroll
@@ -161,8 +171,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_fft_inverse(const float* __rest
 // registers while it finishes the current one. Each row's arithmetic is the
 // per-chunk kernels', so the results are the same bit for bit.
 template <int Q>
-__global__ void __launch_bounds__(kMaxThreads) k_fft_forward_persistent(const float* __restrict__ g,
-                                                                        float* __restrict__ c,
+__global__ void __launch_bounds__(kMaxThreads) k_fft_forward_persistent(const __grid_constant__ TrSet set,
                                                                         const float2* __restrict__ twg, int nlat,
                                                                         int rows, int items) {
   using Sh = Shape<Q>;
@@ -177,24 +186,29 @@ __global__ void __launch_bounds__(kMaxThreads) k_fft_forward_persistent(const fl
   const int r = threadIdx.x / T, t = threadIdx.x % T;
   float2 a[Sh::QT][8];
   auto load = [&](int item) {
-    const size_t plane = item / chunks;
+    const int tile = item / chunks, fi = tr_find(set, tile);
+    const size_t plane = tile - set.at[fi];
     const int lat0 = (item % chunks) * rows;
-    const float2* in = reinterpret_cast<const float2*>(g + (plane * nlat + lat0 + r) * N);
+    const float2* in = reinterpret_cast<const float2*>(set.f[fi].a + (plane * nlat + lat0 + r) * N);
 #pragma unroll
     for (int i = 0; i < Sh::QT; ++i)
 #pragma unroll
-      for (int p = 0; p < 8; ++p) a[i][p] = in[Q * p + t + T * i];
+      for (int p = 0; p < 8; ++p) a[i][p] = __ldg(in + Q * p + t + T * i);
   };
   int item = blockIdx.x;
+  copy_twiddles<Q>(twg, tw, twq);
+  pdl_wait();
+  pdl_release();
   if (item >= items) return;
   load(item);
-  load_twiddles<Q>(twg, tw, twq);
+  cp_async_wait_all();
   __syncthreads();
   float2* xr = xb + r * Sh::XP;
   const float inv_n = 1.f / (float)N;
   const int lane = threadIdx.x & 31, src = lane - t + (T - t) % T;
   for (; item < items; item += gridDim.x) {
-    const size_t plane = item / chunks;
+    const int tile = item / chunks, fi = tr_find(set, tile);
+    const size_t plane = tile - set.at[fi];
     const int lat0 = (item % chunks) * rows;
     float2 b[Sh::KT][Q];
     four_step<Q, -1>(a, b, twq, xr, t);
@@ -221,16 +235,16 @@ __global__ void __launch_bounds__(kMaxThreads) k_fft_forward_persistent(const fl
     }
     __syncthreads();
     const int lat = threadIdx.x % rows, m0 = threadIdx.x / rows;
-    float2* out = reinterpret_cast<float2*>(c) + plane * nlat * NTP1 + lat0 + lat;
+    float2* out = reinterpret_cast<float2*>(set.f[fi].x) + plane * nlat * NTP1 + lat0 + lat;
+    const int mend = set.f[fi].opt ? set.f[fi].opt : NTP1;
 #pragma unroll 4
-    for (int m = m0; m < NTP1; m += T) out[(size_t)m * nlat] = fc[m * pitch + lat];
+    for (int m = m0; m < mend; m += T) out[(size_t)m * nlat] = fc[m * pitch + lat];
     __syncthreads();  // the next chunk's split rewrites fc
   }
 }
 
 template <int Q>
-__global__ void __launch_bounds__(kMaxThreads) k_fft_inverse_persistent(const float* __restrict__ c,
-                                                                        float* __restrict__ g,
+__global__ void __launch_bounds__(kMaxThreads) k_fft_inverse_persistent(const __grid_constant__ TrSet set,
                                                                         const float2* __restrict__ twg, int nlat,
                                                                         int rows, int items) {
   using Sh = Shape<Q>;
@@ -247,23 +261,28 @@ __global__ void __launch_bounds__(kMaxThreads) k_fft_inverse_persistent(const fl
   const int lat = threadIdx.x % rows, m0 = threadIdx.x / rows;
   float2 v[KS];
   auto load = [&](int item) {
-    const size_t plane = item / chunks;
+    const int tile = item / chunks, fi = tr_find(set, tile);
+    const size_t plane = tile - set.at[fi];
     const int lat0 = (item % chunks) * rows;
-    const float2* src = reinterpret_cast<const float2*>(c) + plane * nlat * NTP1 + lat0 + lat;
+    const float2* src = reinterpret_cast<const float2*>(set.f[fi].a) + plane * nlat * NTP1 + lat0 + lat;
 #pragma unroll
     for (int k = 0; k < KS; ++k) {
       const int m = m0 + T * k;
-      v[k] = m < NTP1 ? src[(size_t)m * nlat] : make_float2(0.f, 0.f);
+      v[k] = m < NTP1 ? __ldg(src + (size_t)m * nlat) : make_float2(0.f, 0.f);
     }
   };
   int item = blockIdx.x;
+  copy_twiddles<Q>(twg, tw, twq);
+  pdl_wait();
+  pdl_release();
   if (item >= items) return;
   load(item);
-  load_twiddles<Q>(twg, tw, twq);
+  cp_async_wait_all();
   const int r = threadIdx.x / T, t = threadIdx.x % T;
   float2* xr = xb + r * Sh::XP;
   for (; item < items; item += gridDim.x) {
-    const size_t plane = item / chunks;
+    const int tile = item / chunks, fi = tr_find(set, tile);
+    const size_t plane = tile - set.at[fi];
     const int lat0 = (item % chunks) * rows;
 #pragma unroll
     for (int k = 0; k < KS; ++k) {
@@ -287,7 +306,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_fft_inverse_persistent(const fl
       }
     float2 b[Sh::KT][Q];
     four_step<Q, 1>(a, b, twq, xr, t);
-    float2* out = reinterpret_cast<float2*>(g + (plane * nlat + lat0 + r) * N);
+    float2* out = reinterpret_cast<float2*>(set.f[fi].x + (plane * nlat + lat0 + r) * N);
 #pragma unroll
     for (int j = 0; j < Sh::KT; ++j)
 #pragma unroll
@@ -304,13 +323,21 @@ void allow_plane_smem(K kernel) {
 int q_of(const Dims& d) { return d.NLON / 16; }
 int t_of(const Dims& d) { return q_of(d) == 8 ? 8 : 4; }
 
+template <typename K>
+void launch_fft(const Model& m, K per_chunk, const TrSet& s, unsigned items, int threads, size_t smem,
+                cudaStream_t st) {
+  step_launch(m.pdl, per_chunk, items, threads, smem, st, s, reinterpret_cast<const float2*>(m.sh.tw), m.d.NLAT,
+              m.tune.fft_rows);
+}
+
 // One block per resident slot (at most one per chunk), each looping over
 // the `items` chunks.
 template <typename K>
-void launch_persistent(K kernel, const float* in, float* out, const float2* tw, int nlat, int rows, unsigned items,
-                       int threads, size_t smem, cudaStream_t st) {
+void launch_persistent(const Model& m, K kernel, const TrSet& s, unsigned items, int threads, size_t smem,
+                       cudaStream_t st) {
   const unsigned grid = std::min<unsigned>(items, persistent_grid((const void*)kernel, threads, smem));
-  kernel<<<grid, threads, smem, st>>>(in, out, tw, nlat, rows, (int)items);
+  step_launch(m.pdl, kernel, grid, threads, smem, st, s, reinterpret_cast<const float2*>(m.sh.tw), m.d.NLAT,
+              m.tune.fft_rows, (int)items);
 }
 
 }  // namespace
@@ -339,46 +366,26 @@ bool fft_rows_supported(const Dims& d, int rows) {
          fft_chunk_smem(d, rows) <= kLegSmemLimit;
 }
 
-void fft_forward(const Model& m, const float* g, float* c, int planes, cudaStream_t st) {
-  const float2* tw = reinterpret_cast<const float2*>(m.sh.tw);
-  const int rows = m.tune.fft_rows;
-  const size_t smem = fft_chunk_smem(m.d, rows);
-  const unsigned blocks = planes * (m.d.NLAT / rows);
-  const int threads = rows * t_of(m.d);
-  if (m.tune.fft_persistent[0]) {
-    switch (q_of(m.d)) {
-      case 4: return launch_persistent(k_fft_forward_persistent<4>, g, c, tw, m.d.NLAT, rows, blocks, threads, smem, st);
-      case 8: return launch_persistent(k_fft_forward_persistent<8>, g, c, tw, m.d.NLAT, rows, blocks, threads, smem, st);
-      default:
-        return launch_persistent(k_fft_forward_persistent<12>, g, c, tw, m.d.NLAT, rows, blocks, threads, smem, st);
-    }
+#define EXOGCM_FFT(name, persistent)                                                                     \
+  void name(const Model& m, const TrSet& set, cudaStream_t st) {                                         \
+    TrSet s = set;                                                                                       \
+    const int rows = m.tune.fft_rows, threads = rows * t_of(m.d);                                        \
+    const size_t smem = fft_chunk_smem(m.d, rows);                                                       \
+    const unsigned items = tr_tiles(s, 1) * (m.d.NLAT / rows);                                           \
+    switch (q_of(m.d)) {                                                                                 \
+      case 4:                                                                                            \
+        return persistent ? launch_persistent(m, k_##name##_persistent<4>, s, items, threads, smem, st)  \
+                          : launch_fft(m, k_##name<4>, s, items, threads, smem, st);                     \
+      case 8:                                                                                            \
+        return persistent ? launch_persistent(m, k_##name##_persistent<8>, s, items, threads, smem, st)  \
+                          : launch_fft(m, k_##name<8>, s, items, threads, smem, st);                     \
+      default:                                                                                           \
+        return persistent ? launch_persistent(m, k_##name##_persistent<12>, s, items, threads, smem, st) \
+                          : launch_fft(m, k_##name<12>, s, items, threads, smem, st);                    \
+    }                                                                                                    \
   }
-  switch (q_of(m.d)) {
-    case 4: k_fft_forward<4><<<blocks, threads, smem, st>>>(g, c, tw, m.d.NLAT, rows); break;
-    case 8: k_fft_forward<8><<<blocks, threads, smem, st>>>(g, c, tw, m.d.NLAT, rows); break;
-    default: k_fft_forward<12><<<blocks, threads, smem, st>>>(g, c, tw, m.d.NLAT, rows); break;
-  }
-}
-
-void fft_inverse(const Model& m, const float* c, float* g, int planes, cudaStream_t st) {
-  const float2* tw = reinterpret_cast<const float2*>(m.sh.tw);
-  const int rows = m.tune.fft_rows;
-  const size_t smem = fft_chunk_smem(m.d, rows);
-  const unsigned blocks = planes * (m.d.NLAT / rows);
-  const int threads = rows * t_of(m.d);
-  if (m.tune.fft_persistent[1]) {
-    switch (q_of(m.d)) {
-      case 4: return launch_persistent(k_fft_inverse_persistent<4>, c, g, tw, m.d.NLAT, rows, blocks, threads, smem, st);
-      case 8: return launch_persistent(k_fft_inverse_persistent<8>, c, g, tw, m.d.NLAT, rows, blocks, threads, smem, st);
-      default:
-        return launch_persistent(k_fft_inverse_persistent<12>, c, g, tw, m.d.NLAT, rows, blocks, threads, smem, st);
-    }
-  }
-  switch (q_of(m.d)) {
-    case 4: k_fft_inverse<4><<<blocks, threads, smem, st>>>(c, g, tw, m.d.NLAT, rows); break;
-    case 8: k_fft_inverse<8><<<blocks, threads, smem, st>>>(c, g, tw, m.d.NLAT, rows); break;
-    default: k_fft_inverse<12><<<blocks, threads, smem, st>>>(c, g, tw, m.d.NLAT, rows); break;
-  }
-}
+EXOGCM_FFT(fft_forward, m.tune.fft_persistent[0])
+EXOGCM_FFT(fft_inverse, m.tune.fft_persistent[1])
+#undef EXOGCM_FFT
 
 }  // namespace exogcm

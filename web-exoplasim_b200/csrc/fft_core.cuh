@@ -6,6 +6,8 @@
 
 #include <cuda_runtime.h>
 
+#include "async_copy.cuh"
+
 namespace exogcm {
 namespace fftcore {
 
@@ -144,15 +146,16 @@ inline size_t chunk_smem(int Q, int T, int rows) {
   return ((size_t)2 * 8 * Q + 9 * Q + (size_t)rows * 9 * Q + (size_t)ntp1 * fc_pitch(rows, T)) * sizeof(float2);
 }
 
-// Twiddle tables into shared memory: tw[j] = e^{2 pi i j / N};
+// Twiddle tables into shared memory by asynchronous copies (the caller waits
+// for them and meets at a barrier): tw[j] = e^{2 pi i j / N};
 // twq[9 q + k1] = w_M^{q k1}.
 template <int Q>
-__device__ __forceinline__ void load_twiddles(const float2* __restrict__ twg, float2* tw, float2* twq) {
+__device__ __forceinline__ void copy_twiddles(const float2* __restrict__ twg, float2* tw, float2* twq) {
   using Sh = Shape<Q>;
-  for (int i = threadIdx.x; i < Sh::N; i += blockDim.x) tw[i] = twg[i];
+  for (int i = threadIdx.x; i < Sh::N; i += blockDim.x) cp_async8(tw + i, twg + i);
   for (int i = threadIdx.x; i < 9 * Q; i += blockDim.x) {
     const int q = i / 9, k1 = i - 9 * q;
-    twq[i] = k1 < 8 ? twg[(2 * q * k1) % Sh::N] : make_float2(0.f, 0.f);
+    if (k1 < 8) cp_async8(twq + i, twg + (2 * q * k1) % Sh::N);
   }
 }
 

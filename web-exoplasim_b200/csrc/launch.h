@@ -10,22 +10,68 @@
 
 namespace exogcm {
 
+// A set of fields one transform launch works through: independent planes of
+// several fields in one grid, so that a step pays one launch, one ramp and
+// one tail for all of them. What the pointers mean is each transform's own.
+struct TrField {
+  const float* a = nullptr;
+  const float* b = nullptr;
+  const float* c = nullptr;
+  float* x = nullptr;
+  float* y = nullptr;
+  int planes = 0;
+  int opt = 0;
+  float plavor = 0.f;
+};
+constexpr int kMaxTr = 12;
+struct TrSet {
+  int n = 0;
+  int at[kMaxTr + 1] = {};  // first tile of each field (tr_tiles)
+  TrField f[kMaxTr];
+  void add(const TrField& t) { f[n++] = t; }
+};
+// Numbers the tiles of `tile` planes of the set's fields one after another
+// (no tile spans two fields); returns their count.
+inline int tr_tiles(TrSet& s, int tile) {
+  s.at[0] = 0;
+  for (int i = 0; i < s.n; ++i) s.at[i + 1] = s.at[i] + (s.f[i].planes + tile - 1) / tile;
+  return s.at[s.n];
+}
+#ifdef __CUDACC__
+// The field of a tile; tile - s.at[field] is the tile's number in it.
+__device__ __forceinline__ int tr_find(const TrSet& s, int tile) {
+  int f = 0;
+  while (f + 1 < s.n && tile >= s.at[f + 1]) ++f;
+  return f;
+}
+#endif
+
+// Options of a spectral -> grid field (TrField::opt).
+constexpr int kTrDerivative = 1;  // sp2fcdmu: the d/dmu table
+constexpr int kTrDlambda = 2;     // d/dlambda of the Fourier coefficients before fc2gp
+constexpr int kTrKeep = 4;        // the Fourier field is written whatever Model::keep_fourier
+
 // transforms.cu
 void tr_init();
-void tr_fourier_forward(const Model& m, const float* g, float* c, int planes, cudaStream_t st);
-void tr_fourier_inverse(const Model& m, const float* c, float* g, int planes, cudaStream_t st);
-void tr_dlambda(const Model& m, const float* a, float* b, int planes, cudaStream_t st);
-void tr_legendre_inverse(const Model& m, const float* s, float* f, int planes, const float* q, cudaStream_t st);
-// sp2fc then fc2gp of one field: f is the Fourier field between them (on the
-// optimized path written only when m.keep_fourier), g the grid field.
-void tr_sp2gp(const Model& m, const float* s, float* f, float* g, int planes, const float* q, cudaStream_t st);
-void tr_dv2uv(const Model& m, const float* D, const float* Z, float* U, float* V, int planes, float plavor,
-              cudaStream_t st);
-void tr_legendre_forward(const Model& m, const float* f, float* s, int planes, const float* q, cudaStream_t st);
-void tr_uv2dv(const Model& m, const float* u, const float* v, const float* ke, float* D, float* Z, int planes,
-              cudaStream_t st);
-void tr_qtend(const Model& m, const float* u, const float* v, const float* src, float* out, int planes,
-              cudaStream_t st);
+// gp2fc: a grid, x Fourier; opt: wavenumbers written (0: all).
+void tr_fourier_forward(const Model& m, TrSet s, cudaStream_t st);
+// fc2gp: a Fourier, x grid.
+void tr_fourier_inverse(const Model& m, TrSet s, cudaStream_t st);
+// sp2fc (a spectral, x Fourier; opt: kTrDerivative).
+void tr_legendre_inverse(const Model& m, TrSet s, cudaStream_t st);
+// sp2fc then fc2gp of each field of `s` (a spectral, x the Fourier field
+// between them - on the optimized path written only when m.keep_fourier or
+// kTrKeep - and y the grid field; opt: kTr*), and fc2gp of each field of
+// `fourier` (a Fourier, x grid).
+void tr_to_grid(const Model& m, TrSet s, TrSet fourier, cudaStream_t st);
+// dv2uv: a D, b zeta, x u, y v (Fourier), plavor.
+void tr_dv2uv(const Model& m, TrSet s, cudaStream_t st);
+// fc2sp: a Fourier, x spectral.
+void tr_legendre_forward(const Model& m, TrSet s, cudaStream_t st);
+// uv2dv / mktend: a u, b v, c kinetic energy (every field or none), x D, y zeta.
+void tr_uv2dv(const Model& m, TrSet s, cudaStream_t st);
+// qtend: a u, b v, c source, x out.
+void tr_qtend(const Model& m, TrSet s, cudaStream_t st);
 
 // legendre.cu (optimized path)
 constexpr size_t kLegSmemLimit = 200 * 1024;  // dynamic shared memory the transform kernels may ask
@@ -35,27 +81,23 @@ int persistent_grid(const void* kernel, int threads, size_t smem);
 size_t leg_inverse_smem(const Dims& d, int kind, int group, int tile);
 size_t leg_forward_smem(const Dims& d, int kind, int tile);
 Tuning default_tuning(const Dims& d);
-void leg_inverse(const Model& m, const float* s, float* f, int planes, bool derivative, cudaStream_t st);
-void leg_dv2uv(const Model& m, const float* D, const float* Z, float* U, float* V, int planes, float plavor,
-               cudaStream_t st);
-void leg_forward(const Model& m, const float* f, float* s, int planes, const float* q, cudaStream_t st);
-void leg_uv2dv(const Model& m, const float* u, const float* v, const float* ke, float* D, float* Z, int planes,
-               cudaStream_t st);
-void leg_qtend(const Model& m, const float* u, const float* v, const float* src, float* out, int planes,
-               cudaStream_t st);
+void leg_inverse(const Model& m, const TrSet& s, cudaStream_t st);
+void leg_dv2uv(const Model& m, const TrSet& s, cudaStream_t st);
+// The forward transforms of every mode but the tensor cores': the plain path
+// (mode 0) runs them on its own Fourier layout.
+void leg_forward(const Model& m, const TrSet& s, cudaStream_t st);
+void leg_uv2dv(const Model& m, const TrSet& s, cudaStream_t st);
+void leg_qtend(const Model& m, const TrSet& s, cudaStream_t st);
 
 // legendre_tc.cu (mode 2: the Legendre transforms on the tensor cores, split precision)
 void tc_init();
 std::vector<float> tc_table_images(const Dims& d, const std::map<std::string, std::vector<double>>& q,
                                    std::vector<int>& at);
-void tc_inverse(const Model& m, const float* s, float* f, int planes, bool derivative, cudaStream_t st);
-void tc_dv2uv(const Model& m, const float* D, const float* Z, float* U, float* V, int planes, float plavor,
-              cudaStream_t st);
-void tc_forward(const Model& m, const float* f, float* s, int planes, cudaStream_t st);
-void tc_uv2dv(const Model& m, const float* u, const float* v, const float* ke, float* D, float* Z, int planes,
-              cudaStream_t st);
-void tc_qtend(const Model& m, const float* u, const float* v, const float* src, float* out, int planes,
-              cudaStream_t st);
+void tc_inverse(const Model& m, const TrSet& s, cudaStream_t st);
+void tc_dv2uv(const Model& m, const TrSet& s, cudaStream_t st);
+void tc_forward(const Model& m, const TrSet& s, cudaStream_t st);
+void tc_uv2dv(const Model& m, const TrSet& s, cudaStream_t st);
+void tc_qtend(const Model& m, const TrSet& s, cudaStream_t st);
 
 // fft.cu (optimized path; Fourier planes m-major)
 void fft_init();
@@ -66,18 +108,18 @@ std::vector<float> grid_table_layout(const Dims& d, const std::vector<double>& q
 // Shared memory of the fused inverse transform at 2 or 4 planes per pass.
 size_t grid_sp2gp_smem(const Dims& d, int planes_per_pass);
 void grid_init();
-void grid_sp2gp(const Model& m, const float* s, float* f, float* g, int planes, bool derivative, cudaStream_t st);
+void grid_sp2gp(const Model& m, const TrSet& s, cudaStream_t st);
 size_t fft_chunk_smem(const Dims& d, int rows);
 bool fft_rows_supported(const Dims& d, int rows);
-void fft_forward(const Model& m, const float* g, float* c, int planes, cudaStream_t st);
-void fft_inverse(const Model& m, const float* c, float* g, int planes, cudaStream_t st);
+void fft_forward(const Model& m, const TrSet& s, cudaStream_t st);
+void fft_inverse(const Model& m, const TrSet& s, cudaStream_t st);
 
 // dynamics.cu
 void dyn_calcgp(const Model& m, cudaStream_t st);
 void dyn_spectrala(const Model& m, cudaStream_t st);
 void dyn_spectrald_diffusion(const Model& m, cudaStream_t st);
-void dyn_mkdheat(const Model& m, int stage, cudaStream_t st);
-void dyn_mean_mode(const Model& m, float* target, cudaStream_t st);
+void dyn_mkdheat_winds(const Model& m, cudaStream_t st);
+void dyn_mkdheat_mean(const Model& m, cudaStream_t st);
 void dyn_spectrald_update(const Model& m, cudaStream_t st);
 void dyn_physics_in(const Model& m, cudaStream_t st);
 void dyn_physics_out(const Model& m, cudaStream_t st);

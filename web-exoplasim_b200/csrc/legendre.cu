@@ -61,30 +61,34 @@ inline int group_terms(const Dims& d, int group) {
 // latency overlaps arithmetic. Each thread owns latitude pair j and two
 // planes of the tile.
 template <int KIND>
-__global__ void k_sym_inverse(const float* __restrict__ s0, const float* __restrict__ s1, float* __restrict__ f0,
-                              float* __restrict__ f1, int planes, int tile, int group, int ntmax, int buf_floats,
-                              const float* __restrict__ qa, const float* __restrict__ qb, int odd, float plavor,
-                              Dims d) {
+__global__ void k_sym_inverse(const __grid_constant__ TrSet set, int tile, int group, int ntmax, int buf_floats,
+                              const float* __restrict__ qa, const float* __restrict__ qb, int odd, Dims d) {
   constexpr int NIN = KIND == 0 ? 1 : 2;
   extern __shared__ float4 smem4[];
   float* smem = reinterpret_cast<float*>(smem4);
   const int JH = d.NLAT / 2;
   const int ngroups = (d.NTP1 + group - 1) / group;
-  const int items = ngroups * ((planes + tile - 1) / tile);
+  const int items = ngroups * set.at[set.n];
   const size_t plane_floats = (size_t)d.NLAT * d.NFC;
   // One buffer: [NIN][nt][tile] (re, im) term-major coefficients, then the
   // [NIN tables][nt][JH] table slice at a fixed 16-byte aligned offset.
   const int qs_at = 2 * NIN * ntmax * tile;
-  auto stage = [&](int item, float* buf) {
-    const int m0 = (item % ngroups) * group, p0 = (item / ngroups) * tile;
-    const int m1 = min(m0 + group, d.NTP1);
+  auto stage_tables = [&](int item, float* buf) {
+    const int m0 = (item % ngroups) * group, m1 = min(m0 + group, d.NTP1);
     const int w0 = first_mode(m0, d.NTP1), nt = first_mode(m1, d.NTP1) - w0;
-    const int np = min(tile, planes - p0);
     float* qs = buf + qs_at;
     for (int i = threadIdx.x; i < nt * JH / 4; i += blockDim.x) {
       cp_async16(qs + 4 * i, qa + (size_t)w0 * JH + 4 * i);
       if (KIND == 1) cp_async16(qs + nt * JH + 4 * i, qb + (size_t)w0 * JH + 4 * i);
     }
+  };
+  auto stage_spectral = [&](int item, float* buf) {
+    const int m0 = (item % ngroups) * group, m1 = min(m0 + group, d.NTP1);
+    const int w0 = first_mode(m0, d.NTP1), nt = first_mode(m1, d.NTP1) - w0;
+    const int at = item / ngroups, fi = tr_find(set, at);
+    const int p0 = (at - set.at[fi]) * tile;
+    const int np = min(tile, set.f[fi].planes - p0);
+    const float *s0 = set.f[fi].a, *s1 = set.f[fi].b;
     float2* ss = reinterpret_cast<float2*>(buf);
     for (int k = 0; k < NIN; ++k) {
       const float* src = k == 0 ? s0 : s1;
@@ -95,24 +99,34 @@ __global__ void k_sym_inverse(const float* __restrict__ s0, const float* __restr
     }
   };
   int item = blockIdx.x;
-  if (item < items) stage(item, smem);
+  if (item < items) stage_tables(item, smem);
+  pdl_wait();
+  pdl_release();
+  if (item < items) stage_spectral(item, smem);
   cp_async_commit();
   for (int it = 0; item < items; ++it) {
     float* buf = smem + (size_t)(it & 1) * buf_floats;
     const int next = item + gridDim.x;
-    if (next < items) stage(next, smem + (size_t)((it + 1) & 1) * buf_floats);
+    if (next < items) {
+      float* other = smem + (size_t)((it + 1) & 1) * buf_floats;
+      stage_tables(next, other);
+      stage_spectral(next, other);
+    }
     cp_async_commit();
     cp_async_wait_one();  // this item's copies have landed (the next item's may be in flight)
     __syncthreads();
-    const int m0 = (item % ngroups) * group, p0 = (item / ngroups) * tile;
+    const int m0 = (item % ngroups) * group;
     const int m1 = min(m0 + group, d.NTP1);
     const int w0 = first_mode(m0, d.NTP1), nt = first_mode(m1, d.NTP1) - w0;
-    const int np = min(tile, planes - p0);
+    const int at = item / ngroups, fi = tr_find(set, at);
+    const int p0 = (at - set.at[fi]) * tile;
+    const int np = min(tile, set.f[fi].planes - p0);
+    float *f0 = set.f[fi].x, *f1 = set.f[fi].y;
     float2* ss = reinterpret_cast<float2*>(buf);
     const float* qs = buf + qs_at;
     if (KIND == 1 && w0 <= 1 && 1 < w0 + nt) {
       // vorticity mode w = 1 (real part) without plavor
-      for (int p = threadIdx.x; p < np; p += blockDim.x) ss[((size_t)nt + (1 - w0)) * tile + p].x -= plavor;
+      for (int p = threadIdx.x; p < np; p += blockDim.x) ss[((size_t)nt + (1 - w0)) * tile + p].x -= set.f[fi].plavor;
       __syncthreads();
     }
     // A thread owns pair j and PPT consecutive planes of the tile (2 for
@@ -218,11 +232,6 @@ __global__ void k_sym_inverse(const float* __restrict__ s0, const float* __restr
 }
 
 // ---------------------------------------------------------------- forward
-template <int NIN>
-struct SymIn {
-  const float* p[NIN];
-};
-
 // KIND 0: fc2sp with table q (forward.wgsl).
 // KIND 1: uv2dv, in = {u, v}, outputs D, Z (uv2dv.wgsl without the KE term).
 // KIND 2: mktend's uv2dv, in = {u, v, ke} (uv2dv.wgsl with HAS_KINETIC).
@@ -240,6 +249,7 @@ struct SymIn {
 // table value it loads serves all of them. Every mode's sum runs over the
 // pairs in the shaders' order and expression, so the results equal the
 // plain path's bit for bit, whatever the tiling.
+// One launch takes the tiles of several fields (none spans two).
 template <int KIND>
 struct FwdTables {
   static constexpr int N = KIND == 0 ? 1 : KIND == 3 ? 3 : KIND == 2 ? 3 : 2;
@@ -259,10 +269,10 @@ struct FwdShape {
 // NB staging buffers: with two, the next tile is stored while the current
 // one is read; with one, a barrier separates them and the block needs about
 // half the shared memory, so more blocks share an SM (the autotuner picks).
+// `plain`: Fourier planes in the plain path's layout, [latitude][m].
 template <int KIND, int NIN, int JH, int TP, int NB>
 __global__ void __launch_bounds__(FwdShape<JH, TP>::THREADS)
-    k_sym_forward(SymIn<NIN> in, float* __restrict__ out0, float* __restrict__ out1, int planes, int per_block,
-                  SharedTabs sh, const float* __restrict__ q, int ncsp) {
+    k_sym_forward(const __grid_constant__ TrSet set, int per_block, SharedTabs sh, int ncsp, int plain) {
   using S = FwdShape<JH, TP>;
   constexpr int NTAB = FwdTables<KIND>::N;
   constexpr int NLAT = S::NLAT, NTP1 = S::NTP1, NT = S::NT, PP = S::PP, ROW = S::ROW;
@@ -272,8 +282,9 @@ __global__ void __launch_bounds__(FwdShape<JH, TP>::THREADS)
   float* tab = reinterpret_cast<float*>(fsm);           // [NTAB][JH][NT]
   float4* conv = fsm + (NTAB * JH * NT + 3) / 4;        // [NB][NIN][TP][2][ROW]
   const int g = blockIdx.x % S::GROUPS;
-  const int pbeg = (blockIdx.x / S::GROUPS) * per_block;
-  const int pend = min(planes, pbeg + per_block);
+  const int tbeg = (blockIdx.x / S::GROUPS) * per_block;
+  const int tend = min(set.at[set.n], tbeg + per_block);
+  const int row_m = plain ? 1 : NLAT, row_l = plain ? NTP1 : 1;  // (re, im) strides of m and latitude
   const int ma = g, mb = NTP1 - 1 - g;
   const bool pair = mb != ma;
   const int Ka = NTP1 - ma;
@@ -285,7 +296,10 @@ __global__ void __launch_bounds__(FwdShape<JH, TP>::THREADS)
   constexpr int E = NIN * TP * 2 * JH;
   constexpr int R = (E + S::THREADS - 1) / S::THREADS;
   float2 rn[R], rs[R];
-  auto fetch = [&](int tile) {
+  auto fetch = [&](int at) {
+    const int fi = tr_find(set, at);
+    const int tile = (at - set.at[fi]) * TP, pend = set.f[fi].planes;
+    const float *in0 = set.f[fi].a, *in1 = set.f[fi].b, *in2 = set.f[fi].c;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
       const int e = threadIdx.x + i * S::THREADS;
@@ -293,11 +307,10 @@ __global__ void __launch_bounds__(FwdShape<JH, TP>::THREADS)
       const int plane = tile + p;
       float2 a = make_float2(0.f, 0.f), b = a;
       if (e < E && plane < pend && (mi == 0 || pair)) {
-        const float* base = k == 0 ? in.p[0] : k == 1 ? in.p[NIN > 1 ? 1 : 0] : in.p[NIN > 2 ? 2 : 0];
-        const float2* row =
-            reinterpret_cast<const float2*>(base + (size_t)plane * PLANE) + (size_t)(mi ? mb : ma) * NLAT;
-        a = row[l];
-        b = row[NLAT - 1 - l];
+        const float* base = k == 0 ? in0 : k == 1 ? in1 : in2;
+        const float2* row = reinterpret_cast<const float2*>(base + (size_t)plane * PLANE) + (mi ? mb : ma) * row_m;
+        a = __ldg(row + l * row_l);
+        b = __ldg(row + (NLAT - 1 - l) * row_l);
       }
       rn[i] = a;
       rs[i] = b;
@@ -315,19 +328,22 @@ __global__ void __launch_bounds__(FwdShape<JH, TP>::THREADS)
     }
   };
 
-  fetch(pbeg);
-  // Tables in KIND order: 0: q; 1: qe, qm; 2: qe, qm, qq; 3: qe, qc, qm.
+  // Tables in KIND order: 0: qc; 1: qe, qm; 2: qe, qm, qq; 3: qe, qc, qm.
 #pragma unroll
   for (int k = 0; k < NTAB; ++k) {
-    const float* src = k == 0 ? (KIND == 0 ? q : sh.qe) : k == 1 ? (KIND == 3 ? sh.qc : sh.qm)
+    const float* src = k == 0 ? (KIND == 0 ? sh.qc : sh.qe) : k == 1 ? (KIND == 3 ? sh.qc : sh.qm)
                                                                  : (KIND == 2 ? sh.qq : sh.qm);
     for (int i = threadIdx.x; i < JH * NT; i += S::THREADS) {
       const int t = i % NT, l = i / NT;
       const int w = t < Ka ? wa + t : wb + (t - Ka);
-      tab[k * JH * NT + i] = t < nt ? __ldg(src + (size_t)l * ncsp + w) : 0.f;
+      if (t < nt) cp_async4(tab + k * JH * NT + i, src + (size_t)l * ncsp + w);
     }
   }
+  pdl_wait();
+  pdl_release();
+  fetch(tbeg);
   store(conv);
+  cp_async_wait_all();
   __syncthreads();
 
   // This thread's task: mode t of the block, planes pq * PP .. of each tile.
@@ -339,10 +355,12 @@ __global__ void __launch_bounds__(FwdShape<JH, TP>::THREADS)
   const bool even = (toff & 1) == 0;
   const float* tq = tab + t;
   int it = 0;
-  for (int tile = pbeg; tile < pend; tile += TP, ++it) {
+  for (int at = tbeg; at < tend; ++at, ++it) {
+    const int fi = tr_find(set, at);
+    const int tile = (at - set.at[fi]) * TP, pend = set.f[fi].planes;
     const float4* cur = conv + (NB == 2 ? (it & 1) * CONV : 0);
-    const int next = tile + TP;
-    if (next < pend) fetch(next);
+    const bool more = at + 1 < tend;
+    if (more) fetch(at + 1);
     if (active) {
       // staged row of input k, plane pp of this thread's planes, at pair l: pin(k, pp)[l]
       auto pin = [&](int k, int pp) { return cur + ((k * TP + pq * PP + pp) * 2 + mi) * ROW; };
@@ -391,15 +409,15 @@ __global__ void __launch_bounds__(FwdShape<JH, TP>::THREADS)
       for (int pp = 0; pp < PP; ++pp) {
         const int plane = tile + pq * PP + pp;
         if (plane < pend) {
-          const size_t at = (size_t)plane * (2 * ncsp) + 2 * w;
-          *reinterpret_cast<float2*>(out0 + at) = make_float2(r0[pp], r1[pp]);
-          if (KIND == 1 || KIND == 2) *reinterpret_cast<float2*>(out1 + at) = make_float2(r2[pp], r3[pp]);
+          const size_t o = (size_t)plane * (2 * ncsp) + 2 * w;
+          *reinterpret_cast<float2*>(set.f[fi].x + o) = make_float2(r0[pp], r1[pp]);
+          if (KIND == 1 || KIND == 2) *reinterpret_cast<float2*>(set.f[fi].y + o) = make_float2(r2[pp], r3[pp]);
         }
       }
     }
     if (NB == 2) {
-      if (next < pend) store(conv + ((it + 1) & 1) * CONV);
-    } else if (next < pend) {
+      if (more) store(conv + ((it + 1) & 1) * CONV);
+    } else if (more) {
       __syncthreads();
       store(conv);
     }
@@ -432,30 +450,28 @@ void allow_smem(K kernel) {
 }
 
 template <int KIND, int NIN, int JH, int TP, int NB>
-void launch_forward_shape(const Model& m, SymIn<NIN> in, float* out0, float* out1, int planes, const float* q,
-                          cudaStream_t st) {
+void launch_forward_shape(const Model& m, TrSet set, cudaStream_t st) {
   using S = FwdShape<JH, TP>;
   const auto kernel = k_sym_forward<KIND, NIN, JH, TP, NB>;
   const size_t smem = forward_smem<KIND, NIN, JH, TP, NB>();
   // Blocks per wavenumber pair: enough for every SM's resident blocks, in
   // whole tiles of planes.
-  const int tiles = (planes + TP - 1) / TP;
+  const int tiles = tr_tiles(set, TP);
   const int target = persistent_grid((const void*)kernel, S::THREADS, smem);
   const int splits = std::max(1, std::min(tiles, (target + S::GROUPS - 1) / S::GROUPS));
   const int per_tiles = (tiles + splits - 1) / splits;
   const int blocks = S::GROUPS * ((tiles + per_tiles - 1) / per_tiles);
-  kernel<<<blocks, S::THREADS, smem, st>>>(in, out0, out1, planes, per_tiles * TP, m.sh, q, m.d.NCSP);
+  step_launch(m.pdl, kernel, blocks, S::THREADS, smem, st, set, per_tiles, m.sh, m.d.NCSP, m.mode == 0 ? 1 : 0);
 }
 
 template <int KIND, int NIN>
-void launch_sym_forward(const Model& m, SymIn<NIN> in, float* out0, float* out1, int planes, const float* q,
-                        cudaStream_t st) {
+void launch_sym_forward(const Model& m, const TrSet& set, cudaStream_t st) {
   const bool big = m.tune.fwd_tile[KIND] == 16, one = m.tune.fwd_buffers[KIND] == 1;
-#define EXOGCM_FWD(JH)                                                                         \
-  (big ? (one ? launch_forward_shape<KIND, NIN, JH, 16, 1>(m, in, out0, out1, planes, q, st)  \
-              : launch_forward_shape<KIND, NIN, JH, 16, 2>(m, in, out0, out1, planes, q, st)) \
-       : (one ? launch_forward_shape<KIND, NIN, JH, 8, 1>(m, in, out0, out1, planes, q, st)   \
-              : launch_forward_shape<KIND, NIN, JH, 8, 2>(m, in, out0, out1, planes, q, st)))
+#define EXOGCM_FWD(JH)                                                    \
+  (big ? (one ? launch_forward_shape<KIND, NIN, JH, 16, 1>(m, set, st)   \
+              : launch_forward_shape<KIND, NIN, JH, 16, 2>(m, set, st))  \
+       : (one ? launch_forward_shape<KIND, NIN, JH, 8, 1>(m, set, st)    \
+              : launch_forward_shape<KIND, NIN, JH, 8, 2>(m, set, st)))
   switch (m.d.NLAT) {
     case 32: EXOGCM_FWD(16); break;
     case 64: EXOGCM_FWD(32); break;
@@ -516,27 +532,25 @@ void leg_init() {
 }
 
 template <int KIND>
-void launch_inverse(const Model& m, const float* s0, const float* s1, float* f0, float* f1, int planes,
-                    const float* qa, const float* qb, int odd, float plavor, cudaStream_t st) {
+void launch_inverse(const Model& m, TrSet set, const float* qa, const float* qb, int odd, cudaStream_t st) {
   const int nin = KIND == 0 ? 1 : 2;
   const int group = m.tune.inv_group[KIND], tile = m.tune.inv_tile[KIND];
   const int threads = (m.d.NLAT / 2) * tile / (KIND == 0 ? 2 : 4);
   const size_t smem = inverse_smem(m.d, nin, group, tile);
-  const int items = ((m.d.NTP1 + group - 1) / group) * ((planes + tile - 1) / tile);
+  const int items = ((m.d.NTP1 + group - 1) / group) * tr_tiles(set, tile);
   const int grid = std::min(items, persistent_grid((const void*)k_sym_inverse<KIND>, threads, smem));
-  k_sym_inverse<KIND><<<grid, threads, smem, st>>>(s0, s1, f0, f1, planes, tile, group, group_terms(m.d, group),
-                                                   (int)inverse_buffer_floats(m.d, nin, group, tile), qa, qb, odd,
-                                                   plavor, m.d);
+  step_launch(m.pdl, k_sym_inverse<KIND>, grid, threads, smem, st, set, tile, group, group_terms(m.d, group),
+              (int)inverse_buffer_floats(m.d, nin, group, tile), qa, qb, odd, m.d);
 }
 
-void leg_inverse(const Model& m, const float* s, float* f, int planes, bool derivative, cudaStream_t st) {
-  launch_inverse<0>(m, s, nullptr, f, nullptr, planes, derivative ? m.sh.qjT : m.sh.qiT, nullptr,
-                    derivative ? 1 : 0, 0.f, st);
+// sp2fc of fields of one table (opt: kTrDerivative, the same for all).
+void leg_inverse(const Model& m, const TrSet& s, cudaStream_t st) {
+  const bool derivative = (s.f[0].opt & kTrDerivative) != 0;
+  launch_inverse<0>(m, s, derivative ? m.sh.qjT : m.sh.qiT, nullptr, derivative ? 1 : 0, st);
 }
 
-void leg_dv2uv(const Model& m, const float* D, const float* Z, float* U, float* V, int planes, float plavor,
-               cudaStream_t st) {
-  launch_inverse<1>(m, D, Z, U, V, planes, m.sh.quT, m.sh.qvT, 0, plavor, st);
+void leg_dv2uv(const Model& m, const TrSet& s, cudaStream_t st) {
+  launch_inverse<1>(m, s, m.sh.quT, m.sh.qvT, 0, st);
 }
 
 // Shared memory a tuning asks of each transform kernel, and the default
@@ -577,26 +591,15 @@ Tuning default_tuning(const Dims& d) {
   return t;
 }
 
-void leg_forward(const Model& m, const float* f, float* s, int planes, const float* q, cudaStream_t st) {
-  SymIn<1> in{{f}};
-  launch_sym_forward<0, 1>(m, in, s, nullptr, planes, q, st);
+void leg_forward(const Model& m, const TrSet& s, cudaStream_t st) { launch_sym_forward<0, 1>(m, s, st); }
+
+void leg_uv2dv(const Model& m, const TrSet& s, cudaStream_t st) {
+  if (s.f[0].c)
+    launch_sym_forward<2, 3>(m, s, st);
+  else
+    launch_sym_forward<1, 2>(m, s, st);
 }
 
-void leg_uv2dv(const Model& m, const float* u, const float* v, const float* ke, float* D, float* Z, int planes,
-               cudaStream_t st) {
-  if (ke) {
-    SymIn<3> in{{u, v, ke}};
-    launch_sym_forward<2, 3>(m, in, D, Z, planes, nullptr, st);
-  } else {
-    SymIn<2> in{{u, v}};
-    launch_sym_forward<1, 2>(m, in, D, Z, planes, nullptr, st);
-  }
-}
-
-void leg_qtend(const Model& m, const float* u, const float* v, const float* src, float* out, int planes,
-               cudaStream_t st) {
-  SymIn<3> in{{u, v, src}};
-  launch_sym_forward<3, 3>(m, in, out, nullptr, planes, nullptr, st);
-}
+void leg_qtend(const Model& m, const TrSet& s, cudaStream_t st) { launch_sym_forward<3, 3>(m, s, st); }
 
 }  // namespace exogcm

@@ -44,6 +44,8 @@
 //           table and data stages are full, commits them to the stages'
 //           "empty" barriers and, after an item's last chunk, to the
 //           accumulator's "full" barrier; TMEM holds two accumulators.
+// One launch takes the (m, plane tile) items of several fields, each with its
+// tensor maps, outputs and table set.
 // Every tensor map covers this GPU's own memory, and no load uses cluster
 // multicast. Every wait on an mbarrier is bounded: a role that gives up sets
 // the engine's fault word and an abort flag the other roles poll, the
@@ -260,27 +262,34 @@ __device__ __forceinline__ float tf32_round(float x) {
 
 // Per-launch geometry, computed on the host.
 struct TcGeom {
-  int planes;       // planes of each field
-  int tiles;        // plane tiles (TP planes each)
-  int items;        // NTP1 * tiles
+  int items;        // NTP1 * plane tiles (TP planes each) of all fields
   int npad_max;     // table rows of the largest m (the table stage's size)
   int raw_floats;   // floats of one raw stage
   int raw_row;      // inverse: floats per staged plane row (a multiple of 32)
   int box;          // inverse: TMA box width in floats (a multiple of 4)
   int out_plane;    // floats per output plane
-  float plavor;     // dv2uv: planetary vorticity removed from mode (0, 1)
   int n_tab;        // table stages in the ring (as many as shared memory holds, 2..kMaxTab)
   int raw2d;        // inverse: the planes' rows arrive as one 2-D box (NRSP * 4 a multiple of 16)
 };
 
+constexpr int kTcFields = 6;  // fields of one launch at most
+
 struct TcMaps {
-  CUtensorMap in[3];
+  CUtensorMap in[kTcFields][3];
+};
+
+struct TcField {
+  float* out[2];
+  const int* at;  // float offset of m's images in this field's table set, [NTP1 + 1]
+  int planes;
+  float plavor;   // dv2uv: planetary vorticity removed from mode (0, 1)
 };
 
 struct TcOut {
-  float* out[2];
-  const float* images;  // this kind's table images
-  const int* at;        // float offset of m's images, [NTP1 + 1]
+  TcField f[kTcFields];
+  int tile0[kTcFields + 1];  // first plane tile of each field
+  int n;
+  const float* images;  // every table set's images
 };
 
 // Shared memory carve-up (byte offsets from a 128-byte aligned base).
@@ -305,7 +314,8 @@ __host__ __device__ inline TcSmem tc_smem(int npad_max, int raw_floats, int n_ta
 
 template <int KIND>
 __global__ void __launch_bounds__(kThreads, 1)
-    k_tc_legendre(const __grid_constant__ TcMaps maps, TcOut io, TcGeom g, int* __restrict__ fault, Dims d) {
+    k_tc_legendre(const __grid_constant__ TcMaps maps, const __grid_constant__ TcOut io, TcGeom g,
+                  int* __restrict__ fault, Dims d) {
   using S = Shape<KIND>;
   extern __shared__ unsigned char smem_raw_base[];
   unsigned char* base =
@@ -360,6 +370,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  pdl_wait();
+  pdl_release();
 
   // Bounded wait: gives up after kWaitLimit polls or when another role
   // aborted, recording the fault once.
@@ -380,7 +392,12 @@ __global__ void __launch_bounds__(kThreads, 1)
   // K steps of item m: inverse NA * ceil(K_m / 8) in chunks of 4; forward
   // units * NA chunks of 4.
   auto item_m = [&](int item) { return item % ntp1; };
-  auto item_p0 = [&](int item) { return (item / ntp1) * S::TP; };
+  auto item_f = [&](int item) {
+    int f = 0;
+    while (f + 1 < io.n && item / ntp1 >= io.tile0[f + 1]) ++f;
+    return f;
+  };
+  auto item_p0 = [&](int item, int f) { return (item / ntp1 - io.tile0[f]) * S::TP; };
   auto ks_block = [&](int m) { return (ntp1 - m + kStepK - 1) / kStepK; };
   auto chunks_of = [&](int m) {
     return S::fwd ? units * S::NA : (S::NA * ks_block(m) + kChunkSteps - 1) / kChunkSteps;
@@ -393,11 +410,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (lane == 0) {
       bool ok = true;
       for (int item = blockIdx.x; item < g.items && ok; item += gridDim.x) {
-        const int m = item_m(item), p0 = item_p0(item);
-        const int np = min(S::TP, g.planes - p0);
+        const int m = item_m(item), fi = item_f(item), p0 = item_p0(item, fi);
+        const int np = min(S::TP, io.f[fi].planes - p0);
+        const CUtensorMap* in = maps.in[fi];
         const int nchunks = chunks_of(m), npad = npad_of(m);
         const int total_steps = S::fwd ? nchunks * kChunkSteps : S::NA * ks_block(m);
-        const float* img = io.images + io.at[m];
+        const float* img = io.images + io.f[fi].at[m];
         int chunk = 0;
         for (int u = 0; u < units && ok; ++u) {
           const int rb = ri & 1;
@@ -416,8 +434,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             mbar_expect_tx(raw_full + rb, bytes);
             for (int f = 0; f < S::NR; ++f) {
-              tma_load_2d(r + (size_t)(2 * f) * S::TP * 32, &maps.in[f], xn, p0, raw_full + rb);
-              tma_load_2d(r + (size_t)(2 * f + 1) * S::TP * 32, &maps.in[f], xs, p0, raw_full + rb);
+              tma_load_2d(r + (size_t)(2 * f) * S::TP * 32, &in[f], xn, p0, raw_full + rb);
+              tma_load_2d(r + (size_t)(2 * f + 1) * S::TP * 32, &in[f], xs, p0, raw_full + rb);
             }
           } else {
             // per field and plane: the modes of m, from the 16-byte boundary
@@ -428,13 +446,13 @@ __global__ void __launch_bounds__(kThreads, 1)
               // at the same 16-byte boundary below its first coefficient
               mbar_expect_tx(raw_full + rb, (uint32_t)(S::NR * S::TP * g.box * 4));
               for (int f = 0; f < S::NR; ++f)
-                tma_load_2d(r + (size_t)f * S::TP * g.raw_row, &maps.in[f], (2 * w0) & ~3, p0, raw_full + rb);
+                tma_load_2d(r + (size_t)f * S::TP * g.raw_row, &in[f], (2 * w0) & ~3, p0, raw_full + rb);
             } else {
               mbar_expect_tx(raw_full + rb, (uint32_t)(S::NR * np * g.box * 4));
               for (int f = 0; f < S::NR; ++f)
                 for (int p = 0; p < np; ++p) {
                   const int x = ((p0 + p) * d.NRSP + 2 * w0) & ~3;
-                  tma_load_1d(r + ((size_t)f * S::TP + p) * g.raw_row, &maps.in[f], x, raw_full + rb);
+                  tma_load_1d(r + ((size_t)f * S::TP + p) * g.raw_row, &in[f], x, raw_full + rb);
                 }
             }
           }
@@ -538,7 +556,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int ab = iidx & 1;
       if (!wait(acc_full + ab, (iidx >> 1) & 1)) return false;
       fence_after_sync();
-      const int m = item_m(it), p0 = item_p0(it);
+      const int m = item_m(it), fi = item_f(it), p0 = item_p0(it, fi);
       const int w0 = first_mode(m, ntp1);
       const int ncols = S::fwd ? ntp1 - m : d.NLAT;
       const size_t out_base = S::fwd ? (size_t)2 * w0 : (size_t)2 * m * d.NLAT;
@@ -552,10 +570,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int nvalid = 2 * min(32, ncols - c0);
         for (int pp = 0; pp < PPW; ++pp) {
           const int plane = p0 + q * PPW + pp;
-          if (plane >= g.planes) break;
+          if (plane >= io.f[fi].planes) break;
 #pragma unroll
           for (int o = 0; o < S::NOUT; ++o) {
-            float* dst = io.out[o] + (size_t)plane * g.out_plane + out_base + 2 * c0;
+            float* dst = io.f[fi].out[o] + (size_t)plane * g.out_plane + out_base + 2 * c0;
             const int row = pp * S::NC + 2 * o;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -571,8 +589,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       return true;
     };
     for (int item = blockIdx.x; item < g.items && ok; item += gridDim.x, ++ii) {
-      const int m = item_m(item), p0 = item_p0(item);
-      const int np = min(S::TP, g.planes - p0);
+      const int m = item_m(item), fi = item_f(item), p0 = item_p0(item, fi);
+      const int np = min(S::TP, io.f[fi].planes - p0);
+      const float plavor = io.f[fi].plavor;
       const int nchunks = chunks_of(m);
       const int K = ntp1 - m, ksb = ks_block(m);
       const int total_steps = S::fwd ? nchunks * kChunkSteps : S::NA * ksb;
@@ -624,7 +643,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int j = 0; j < 4; ++j) {
                   const int tmode = t0 + j;
                   float v = tmode < K ? rr[2 * tmode] : 0.f;
-                  if (KIND == DV2UV && tm.field == 1 && tm.comp == 0 && m == 0 && tmode == 1) v -= g.plavor;
+                  if (KIND == DV2UV && tm.field == 1 && tm.comp == 0 && m == 0 && tmode == 1) v -= plavor;
                   x[j] = tm.sign * v;
                 }
               }
@@ -725,12 +744,10 @@ int sm_count() {
 }
 
 template <int KIND>
-TcGeom geometry(const Dims& d, int planes, float plavor) {
+TcGeom geometry(const Dims& d, int tiles) {
   using S = Shape<KIND>;
   TcGeom g{};
-  g.planes = planes;
-  g.tiles = (planes + S::TP - 1) / S::TP;
-  g.items = d.NTP1 * g.tiles;
+  g.items = d.NTP1 * tiles;
   g.npad_max = S::fwd ? (d.NTP1 + 15) / 16 * 16 : d.NLAT;
   g.box = (2 * d.NTP1 + 4 + 3) / 4 * 4;
   // a 2-D box lands as TP rows of `box` floats; per-plane 1-D boxes land on
@@ -740,7 +757,6 @@ TcGeom geometry(const Dims& d, int planes, float plavor) {
   g.raw_floats = S::fwd ? S::NR * 2 * S::TP * 32 : S::NR * S::TP * g.raw_row;
   g.raw_floats = (g.raw_floats + 31) / 32 * 32;
   g.out_plane = S::fwd ? d.NRSP : d.NLAT * d.NFC;
-  g.plavor = plavor;
   // as many table stages as shared memory holds
   g.n_tab = 2;
   while (g.n_tab < kMaxTab && tc_smem(g.npad_max, g.raw_floats, g.n_tab + 1).total + 1024 <= kTcSmemLimit) ++g.n_tab;
@@ -752,30 +768,35 @@ size_t smem_bytes(const TcGeom& g) {
   return tc_smem(g.npad_max, g.raw_floats, g.n_tab).total + 1024;
 }
 
+// Table image sets, in the order of the at[] rows.
+enum ImageSet : int { SET_QI = 0, SET_QJ, SET_DV2UV, SET_FC2SP, SET_UV2DV, SET_MKTEND, SET_QTEND, SET_COUNT };
+
 template <int KIND>
-void launch(const Model& m, const float* const* in, float* out0, float* out1, int planes, int set, float plavor,
-            cudaStream_t st) {
+void launch(const Model& m, TrSet set, int table_set, cudaStream_t st) {
   using S = Shape<KIND>;
   const Dims& d = m.d;
-  const TcGeom g = geometry<KIND>(d, planes, plavor);
+  if (set.n > kTcFields) throw std::runtime_error("tensor-core transform: too many fields in one launch");
+  const TcGeom g = geometry<KIND>(d, tr_tiles(set, S::TP));
   TcMaps maps{};
-  for (int f = 0; f < S::NR; ++f)
-    maps.in[f] = S::fwd    ? map_2d(in[f], d.NLAT * d.NFC, planes, 32, S::TP, true)
-                 : g.raw2d ? map_2d(in[f], d.NRSP, planes, g.box, S::TP)
-                           : map_1d(in[f], (size_t)planes * d.NRSP, g.box);
   TcOut io{};
-  io.out[0] = out0;
-  io.out[1] = out1;
+  io.n = set.n;
+  for (int i = 0; i <= set.n; ++i) io.tile0[i] = set.at[i];
+  for (int i = 0; i < set.n; ++i) {
+    const TrField& t = set.f[i];
+    const float* const in[3] = {t.a, t.b, t.c};
+    for (int f = 0; f < S::NR; ++f)
+      maps.in[i][f] = S::fwd    ? map_2d(in[f], d.NLAT * d.NFC, t.planes, 32, S::TP, true)
+                      : g.raw2d ? map_2d(in[f], d.NRSP, t.planes, g.box, S::TP)
+                                : map_1d(in[f], (size_t)t.planes * d.NRSP, g.box);
+    const int tables = KIND == INV && (t.opt & kTrDerivative) ? (int)SET_QJ : table_set;
+    io.f[i] = {{t.x, t.y}, m.sh.tc_at + (size_t)tables * (d.NTP1 + 1), t.planes, t.plavor};
+  }
   io.images = m.sh.tc_img;
-  io.at = m.sh.tc_at + (size_t)set * (d.NTP1 + 1);
   const size_t smem = smem_bytes<KIND>(g);
   if (smem > kTcSmemLimit) throw std::runtime_error("tensor-core transform: shared memory over budget");
   const int grid = std::min(g.items, sm_count());
-  k_tc_legendre<KIND><<<grid, kThreads, smem, st>>>(maps, io, g, m.fault, d);
+  step_launch(m.pdl, k_tc_legendre<KIND>, grid, kThreads, smem, st, maps, io, g, m.fault, d);
 }
-
-// Table image sets, in the order of the at[] rows.
-enum ImageSet : int { SET_QI = 0, SET_QJ, SET_DV2UV, SET_FC2SP, SET_UV2DV, SET_MKTEND, SET_QTEND, SET_COUNT };
 
 }  // namespace
 
@@ -876,37 +897,19 @@ std::vector<float> tc_table_images(const Dims& d, const std::map<std::string, st
   return out;
 }
 
-void tc_inverse(const Model& m, const float* s, float* f, int planes, bool derivative, cudaStream_t st) {
-  const float* in[1] = {s};
-  launch<INV>(m, in, f, nullptr, planes, derivative ? SET_QJ : SET_QI, 0.f, st);
+void tc_inverse(const Model& m, const TrSet& s, cudaStream_t st) { launch<INV>(m, s, SET_QI, st); }
+
+void tc_dv2uv(const Model& m, const TrSet& s, cudaStream_t st) { launch<DV2UV>(m, s, SET_DV2UV, st); }
+
+void tc_forward(const Model& m, const TrSet& s, cudaStream_t st) { launch<FWD>(m, s, SET_FC2SP, st); }
+
+void tc_uv2dv(const Model& m, const TrSet& s, cudaStream_t st) {
+  if (s.f[0].c)
+    launch<MKTEND>(m, s, SET_MKTEND, st);
+  else
+    launch<UV2DV>(m, s, SET_UV2DV, st);
 }
 
-void tc_dv2uv(const Model& m, const float* D, const float* Z, float* U, float* V, int planes, float plavor,
-              cudaStream_t st) {
-  const float* in[2] = {D, Z};
-  launch<DV2UV>(m, in, U, V, planes, SET_DV2UV, plavor, st);
-}
-
-void tc_forward(const Model& m, const float* f, float* s, int planes, cudaStream_t st) {
-  const float* in[1] = {f};
-  launch<FWD>(m, in, s, nullptr, planes, SET_FC2SP, 0.f, st);
-}
-
-void tc_uv2dv(const Model& m, const float* u, const float* v, const float* ke, float* D, float* Z, int planes,
-              cudaStream_t st) {
-  if (ke) {
-    const float* in[3] = {u, v, ke};
-    launch<MKTEND>(m, in, D, Z, planes, SET_MKTEND, 0.f, st);
-  } else {
-    const float* in[2] = {u, v};
-    launch<UV2DV>(m, in, D, Z, planes, SET_UV2DV, 0.f, st);
-  }
-}
-
-void tc_qtend(const Model& m, const float* u, const float* v, const float* src, float* out, int planes,
-              cudaStream_t st) {
-  const float* in[3] = {u, v, src};
-  launch<QTEND>(m, in, out, nullptr, planes, SET_QTEND, 0.f, st);
-}
+void tc_qtend(const Model& m, const TrSet& s, cudaStream_t st) { launch<QTEND>(m, s, SET_QTEND, st); }
 
 }  // namespace exogcm

@@ -22,8 +22,15 @@
 // The next pair's spectral coefficients are fetched into registers during
 // step 2, and the spectral stage shares its memory with the FFT's exchange
 // rows. Results equal the unfused kernels' bit for bit. When the model asks
-// to keep the Fourier fields (stage replay), step 1 also writes them in the
-// path's m-major layout.
+// to keep the Fourier fields (stage replay), or a field asks for it, step 1
+// also writes them in the path's m-major layout.
+//
+// One launch takes the planes of several fields: passes of a block go from
+// field to field (none spans two), the fields with the d/dmu table in blocks
+// of their own. gp's d/dlambda is the coefficients times i m between the
+// steps (fourier/wgsl/dlambda.wgsl). One launch for gridpointa's seven
+// fields in place of nine kernels (sp2fc and d/dlambda, two FFTs, and a
+// fused transform for each other field).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -123,9 +130,8 @@ __device__ __forceinline__ int stage_lat(int rr, int j0) {
 // table slice and the barriers shared by twice the planes; the autotuner picks).
 template <int Q, int PP>
 __global__ void __launch_bounds__(GridShape<Q, PP>::THREADS)
-    k_sp2gp(const float* __restrict__ s, float* __restrict__ f, float* __restrict__ g, int planes, int per_block,
-            const float* __restrict__ qT, const float2* __restrict__ twg, int odd,
-            int keep) {
+    k_sp2gp(const __grid_constant__ TrSet set, int per_block, int passes0, int ranges0,
+            const float* __restrict__ qi, const float* __restrict__ qj, const float2* __restrict__ twg, int keep_all) {
   using G = GridShape<Q, PP>;
   constexpr int T = G::T, M = G::M, N = G::N, NTP1 = G::NTP1, JR = G::JR, JH = G::JH, TP = G::TP;
   constexpr int NLAT = G::NLAT, ROWS = G::ROWS, PITCH = G::PITCH, NCSP = G::NCSP, R = G::R;
@@ -143,13 +149,20 @@ __global__ void __launch_bounds__(GridShape<Q, PP>::THREADS)
   int* tpos = reinterpret_cast<int*>(tab + JR * TP);           // [NTP1] first position of m's modes
   const int chunks = JH / JR;
   const int j0 = (blockIdx.x % chunks) * JR;
-  const int pbeg = (blockIdx.x / chunks) * per_block;
-  const int pend = min(planes, pbeg + per_block);
+  // The block's range of passes: the first ranges0 ranges cover the passes
+  // below passes0 (the fields with the plain table), the others the rest.
+  const int range = blockIdx.x / chunks;
+  const bool odd = range >= ranges0;
+  const int beg = odd ? passes0 + (range - ranges0) * per_block : range * per_block;
+  const int end = min(odd ? set.at[set.n] : passes0, beg + per_block);
 
   // Spectral coefficients of the pass's plane pairs (p + 2k, p + 2k + 1)
   // as (re a, im a, re b, im b), pair-major.
   float4 rs[R];
-  auto fetch = [&](int p) {
+  auto fetch = [&](int pass) {
+    const int fi = tr_find(set, pass);
+    const int p = (pass - set.at[fi]) * G::PP, pend = set.f[fi].planes;
+    const float* s = set.f[fi].a;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
       const int e = threadIdx.x + i * G::THREADS;
@@ -157,8 +170,8 @@ __global__ void __launch_bounds__(GridShape<Q, PP>::THREADS)
       const int pa = p + 2 * pair;
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
       if (e < G::SPEC && pa < pend) {
-        const float2 x = reinterpret_cast<const float2*>(s + (size_t)pa * SPLANE)[w];
-        const float2 y = pa + 1 < pend ? reinterpret_cast<const float2*>(s + (size_t)(pa + 1) * SPLANE)[w]
+        const float2 x = __ldg(reinterpret_cast<const float2*>(s + (size_t)pa * SPLANE) + w);
+        const float2 y = pa + 1 < pend ? __ldg(reinterpret_cast<const float2*>(s + (size_t)(pa + 1) * SPLANE) + w)
                                        : make_float2(0.f, 0.f);
         v = make_float4(x.x, x.y, y.x, y.y);
       }
@@ -175,14 +188,15 @@ __global__ void __launch_bounds__(GridShape<Q, PP>::THREADS)
 
   {
     // the block's table slice, laid out in HBM as it sits here
-    const float4* src = reinterpret_cast<const float4*>(qT + (size_t)(j0 / JR) * JR * TP);
+    const float4* src = reinterpret_cast<const float4*>((odd ? qj : qi) + (size_t)(j0 / JR) * JR * TP);
     float4* dst = reinterpret_cast<float4*>(tab);
     for (int i = threadIdx.x; i < JR * TP / 4; i += G::THREADS) cp_async16(dst + i, src + i);
-    cp_async_commit();
   }
-  if (pbeg < pend) fetch(pbeg);
-  load_twiddles<Q>(twg, tw, twq);
+  copy_twiddles<Q>(twg, tw, twq);
   if (threadIdx.x == 0) grid_table_positions(NTP1, tpos);
+  pdl_wait();
+  pdl_release();
+  if (beg < end) fetch(beg);
   store();
   cp_async_wait_all();
   __syncthreads();
@@ -191,7 +205,10 @@ __global__ void __launch_bounds__(GridShape<Q, PP>::THREADS)
   const int r = threadIdx.x / T, t = threadIdx.x % T;  // FFT row and lane
   const int pr = r / ROWS, rr = r - pr * ROWS;         // plane of the pass, stage row
   const int lat = stage_lat<G>(rr, j0);
-  for (int p = pbeg; p < pend; p += G::PP) {
+  for (int pass = beg; pass < end; ++pass) {
+    const int fi = tr_find(set, pass);
+    const int p = (pass - set.at[fi]) * G::PP, pend = set.f[fi].planes, opt = set.f[fi].opt;
+    const bool dlambda = (opt & kTrDlambda) != 0;
     // 1. Legendre sums into the coefficient stage.
     for (int task = threadIdx.x; task < G::TASKS; task += G::THREADS) {
       const int pair = task / (G::GROUPS * JR), rest = task - pair * (G::GROUPS * JR);
@@ -229,14 +246,17 @@ __global__ void __launch_bounds__(GridShape<Q, PP>::THREADS)
         float2* fa = fc + (2 * pair) * G::FC + m * PITCH;
         float2* fb = fa + G::FC;
         const int rn = jj, rsouth = ROWS - 1 - jj;
-        fa[rn] = make_float2(e.x + o.x, e.y + o.y);
-        fa[rsouth] = make_float2(sg * (e.x - o.x), sg * (e.y - o.y));
-        fb[rn] = make_float2(e.z + o.z, e.w + o.w);
-        fb[rsouth] = make_float2(sg * (e.z - o.z), sg * (e.w - o.w));
+        const float fm = (float)m;
+        auto put = [&](float re, float im) { return dlambda ? make_float2(-im * fm, re * fm) : make_float2(re, im); };
+        fa[rn] = put(e.x + o.x, e.y + o.y);
+        fa[rsouth] = put(sg * (e.x - o.x), sg * (e.y - o.y));
+        fb[rn] = put(e.z + o.z, e.w + o.w);
+        fb[rsouth] = put(sg * (e.z - o.z), sg * (e.w - o.w));
       }
     }
     __syncthreads();
-    if (keep) {
+    if (keep_all || (opt & kTrKeep)) {
+      float* f = set.f[fi].x;
       for (int i = threadIdx.x; i < G::PP * NTP1 * ROWS; i += G::THREADS) {
         const int q = i / (NTP1 * ROWS), rem = i - q * NTP1 * ROWS, m = rem / ROWS, row = rem - m * ROWS;
         if (p + q < pend)
@@ -244,8 +264,7 @@ __global__ void __launch_bounds__(GridShape<Q, PP>::THREADS)
               fc[q * G::FC + m * PITCH + row];
       }
     }
-    const int next = p + G::PP;
-    if (next < pend) fetch(next);
+    if (pass + 1 < end) fetch(pass + 1);
     // 2. FFT of the pass's rows (the exchange rows reuse the spectral stage).
     const float2* fr = fc + pr * G::FC;
     float2 a[G::F::QT][8];
@@ -264,14 +283,14 @@ __global__ void __launch_bounds__(GridShape<Q, PP>::THREADS)
     float2 b[G::F::KT][Q];
     four_step<Q, 1>(a, b, twq, xb + r * G::F::XP, t);
     if (p + pr < pend) {
-      float2* out = reinterpret_cast<float2*>(g + (size_t)(p + pr) * GPLANE + (size_t)lat * N);
+      float2* out = reinterpret_cast<float2*>(set.f[fi].y + (size_t)(p + pr) * GPLANE + (size_t)lat * N);
 #pragma unroll
       for (int j = 0; j < G::F::KT; ++j)
 #pragma unroll
         for (int k2 = 0; k2 < Q; ++k2) out[t + T * j + 8 * k2] = b[j][k2];
     }
     __syncthreads();
-    if (next < pend) {
+    if (pass + 1 < end) {
       store();
       __syncthreads();
     }
@@ -279,18 +298,24 @@ __global__ void __launch_bounds__(GridShape<Q, PP>::THREADS)
 }
 
 template <int Q, int PP>
-void launch_sp2gp(const Model& m, const float* s, float* f, float* g, int planes, const float* qT, int odd,
-                  cudaStream_t st) {
+void launch_sp2gp(const Model& m, const TrSet& set, cudaStream_t st) {
   using G = GridShape<Q, PP>;
+  // the fields with the plain table first
+  TrSet s;
+  for (int odd = 0; odd < 2; ++odd)
+    for (int i = 0; i < set.n; ++i)
+      if (((set.f[i].opt & kTrDerivative) != 0) == (odd != 0)) s.add(set.f[i]);
+  const int passes = tr_tiles(s, PP);
+  int passes0 = passes;
+  for (int i = s.n - 1; i >= 0 && (s.f[i].opt & kTrDerivative); --i) passes0 = s.at[i];
   const size_t smem = G::smem();
   const int chunks = G::JH / G::JR;
-  const int passes = (planes + PP - 1) / PP;
   const int target = persistent_grid((const void*)k_sp2gp<Q, PP>, G::THREADS, smem);
   const int splits = std::max(1, std::min(passes, (target + chunks - 1) / chunks));
-  const int per_passes = (passes + splits - 1) / splits;
-  const int blocks = chunks * ((passes + per_passes - 1) / per_passes);
-  k_sp2gp<Q, PP><<<blocks, G::THREADS, smem, st>>>(s, f, g, planes, PP * per_passes, qT,
-                                                    reinterpret_cast<const float2*>(m.sh.tw), odd, m.keep_fourier);
+  const int per = (passes + splits - 1) / splits;
+  const int ranges0 = (passes0 + per - 1) / per, ranges1 = (passes - passes0 + per - 1) / per;
+  step_launch(m.pdl, k_sp2gp<Q, PP>, chunks * (ranges0 + ranges1), G::THREADS, smem, st, s, per, passes0, ranges0,
+              m.sh.qiG, m.sh.qjG, reinterpret_cast<const float2*>(m.sh.tw), m.keep_fourier);
 }
 
 template <int Q, int PP>
@@ -318,21 +343,12 @@ size_t grid_sp2gp_smem(const Dims& d, int planes_per_pass) {
   }
 }
 
-void grid_sp2gp(const Model& m, const float* s, float* f, float* g, int planes, bool derivative, cudaStream_t st) {
-  const float* qT = derivative ? m.sh.qjG : m.sh.qiG;
-  const int odd = derivative ? 1 : 0;
+void grid_sp2gp(const Model& m, const TrSet& s, cudaStream_t st) {
   const bool four = m.tune.sp2gp_planes == 4;
   switch (m.d.NLON) {
-    case 64:
-      four ? launch_sp2gp<4, 4>(m, s, f, g, planes, qT, odd, st) : launch_sp2gp<4, 2>(m, s, f, g, planes, qT, odd, st);
-      break;
-    case 128:
-      four ? launch_sp2gp<8, 4>(m, s, f, g, planes, qT, odd, st) : launch_sp2gp<8, 2>(m, s, f, g, planes, qT, odd, st);
-      break;
-    default:
-      four ? launch_sp2gp<12, 4>(m, s, f, g, planes, qT, odd, st)
-           : launch_sp2gp<12, 2>(m, s, f, g, planes, qT, odd, st);
-      break;
+    case 64: return four ? launch_sp2gp<4, 4>(m, s, st) : launch_sp2gp<4, 2>(m, s, st);
+    case 128: return four ? launch_sp2gp<8, 4>(m, s, st) : launch_sp2gp<8, 2>(m, s, st);
+    default: return four ? launch_sp2gp<12, 4>(m, s, st) : launch_sp2gp<12, 2>(m, s, st);
   }
 }
 

@@ -12,6 +12,9 @@
 // planes, so each table element read from L2 serves a whole tile.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
+#include "async_copy.cuh"
 #include "common.cuh"
 #include "launch.h"
 
@@ -19,55 +22,76 @@ namespace exogcm {
 
 namespace {
 
-constexpr int kThreads = 256;
-
 // ---------------------------------------------------------------- DFTs
-// gp2fc: rows of NLON grid values -> rows of NFC (re, im) coefficients.
-__global__ void __launch_bounds__(kThreads) k_dft_forward(const float* __restrict__ g,
-                                                          float* __restrict__ c, int rows,
-                                                          const float* __restrict__ tab, int nlon,
-                                                          int nfc, int rows_per_block) {
-  extern __shared__ float smem[];
-  float* ts = smem;               // [nlon][nfc]
-  float* gs = smem + nlon * nfc;  // [rows_per_block][nlon]
-  const int row0 = blockIdx.x * rows_per_block;
-  const int nrows = min(rows_per_block, rows - row0);
-  for (int i = threadIdx.x; i < nlon * nfc; i += blockDim.x) ts[i] = tab[i];
-  for (int i = threadIdx.x; i < nrows * nlon; i += blockDim.x) gs[i] = g[(size_t)row0 * nlon + i];
-  __syncthreads();
-  for (int o = threadIdx.x; o < nrows * nfc; o += blockDim.x) {
-    const int r = o / nfc, k = o % nfc;
-    const float* gr = gs + r * nlon;
-    float s = 0.f;
-    for (int j = 0; j < nlon; ++j) s = fmaf(ts[j * nfc + k], gr[j], s);
-    c[(size_t)(row0 + r) * nfc + k] = s;
-  }
-}
+// gp2fc and fc2gp of the plain path as one dense product: row r of `in` (K
+// values) times the table [K][N], N columns out, summed over K in order as
+// the shaders do. A block stages the table once and walks chunks of R rows;
+// a thread owns two adjacent columns of four rows, so a table pair and a
+// row's four K values loaded from shared memory serve 8 and 2 multiply-adds.
+// What bounds it is the shared-memory loads (12 wavefronts per 32 warp-wide
+// multiply-adds). One thread per output with the table staged by each of 20
+// blocks took 39 us for one T42 L10 planet's field, whatever its number of
+// rows: a chain of 128 loads and multiply-adds behind a 44 KB staging on 20
+// SMs. A launch now takes every field of a stage.
+constexpr int kDftRows = 4;  // rows per thread
 
-// fc2gp: rows of NFC coefficients -> rows of NLON grid values.
-__global__ void __launch_bounds__(kThreads) k_dft_inverse(const float* __restrict__ c,
-                                                          float* __restrict__ g, int rows,
-                                                          const float* __restrict__ tab, int nlon,
-                                                          int nfc, int rows_per_block) {
-  extern __shared__ float smem[];
-  float* ts = smem;               // [nfc][nlon]
-  float* cs = smem + nlon * nfc;  // [rows_per_block][nfc]
-  const int row0 = blockIdx.x * rows_per_block;
-  const int nrows = min(rows_per_block, rows - row0);
-  for (int i = threadIdx.x; i < nlon * nfc; i += blockDim.x) ts[i] = tab[i];
-  for (int i = threadIdx.x; i < nrows * nfc; i += blockDim.x) cs[i] = c[(size_t)row0 * nfc + i];
-  __syncthreads();
-  for (int o = threadIdx.x; o < nrows * nlon; o += blockDim.x) {
-    const int r = o / nlon, j = o % nlon;
-    const float* cr = cs + r * nfc;
-    float s = 0.f;
-    for (int k = 0; k < nfc; ++k) s = fmaf(ts[k * nlon + j], cr[k], s);
-    g[(size_t)(row0 + r) * nlon + j] = s;
+__global__ void __launch_bounds__(768) k_dft(const __grid_constant__ TrSet set, const float* __restrict__ tab, int K,
+                                             int N, int nlat, int R, int items) {
+  extern __shared__ float4 dft_smem[];
+  const int KP = (K + 3) / 4 * 4;  // row pitch: rows start 16-byte aligned
+  float* ts = reinterpret_cast<float*>(dft_smem);  // [K][N]
+  float* rs = ts + (K * N + 3) / 4 * 4;            // [R][KP]
+  for (int i = threadIdx.x; i < K * N / 4; i += blockDim.x) cp_async16(ts + 4 * i, tab + 4 * i);
+  pdl_wait();
+  pdl_release();
+  const int pairs = N / 2, chunks = nlat / R;
+  const int col = 2 * (threadIdx.x % pairs), r0 = kDftRows * (threadIdx.x / pairs);
+  for (int item = blockIdx.x; item < items; item += gridDim.x) {
+    const int tile = item / chunks, fi = tr_find(set, tile);
+    const size_t row0 = (size_t)(tile - set.at[fi]) * nlat + (item % chunks) * R;
+    const float* in = set.f[fi].a + row0 * K;
+    for (int i = threadIdx.x; i < R * (K / 2); i += blockDim.x) {
+      const int r = i / (K / 2), k = 2 * (i - r * (K / 2));
+      cp_async8(rs + r * KP + k, in + (size_t)r * K + k);
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    const int ncol = set.f[fi].opt ? 2 * set.f[fi].opt : N;  // gp2fc: wavenumbers written
+    if (r0 < R && col < ncol) {
+      float2 s[kDftRows] = {};
+      const float* tc = ts + col;
+      const float* rr = rs + r0 * KP;
+      auto add = [&](int k, float x0, float x1, float x2, float x3) {
+        const float2 t = *reinterpret_cast<const float2*>(tc + k * N);
+        s[0] = make_float2(fmaf(t.x, x0, s[0].x), fmaf(t.y, x0, s[0].y));
+        s[1] = make_float2(fmaf(t.x, x1, s[1].x), fmaf(t.y, x1, s[1].y));
+        s[2] = make_float2(fmaf(t.x, x2, s[2].x), fmaf(t.y, x2, s[2].y));
+        s[3] = make_float2(fmaf(t.x, x3, s[3].x), fmaf(t.y, x3, s[3].y));
+      };
+      int k = 0;
+#pragma unroll 2
+      for (; k + 3 < K; k += 4) {
+        float4 x[kDftRows];
+#pragma unroll
+        for (int i = 0; i < kDftRows; ++i) x[i] = *reinterpret_cast<const float4*>(rr + i * KP + k);
+        add(k, x[0].x, x[1].x, x[2].x, x[3].x);
+        add(k + 1, x[0].y, x[1].y, x[2].y, x[3].y);
+        add(k + 2, x[0].z, x[1].z, x[2].z, x[3].z);
+        add(k + 3, x[0].w, x[1].w, x[2].w, x[3].w);
+      }
+      for (; k < K; ++k) add(k, rr[k], rr[KP + k], rr[2 * KP + k], rr[3 * KP + k]);
+      float* out = set.f[fi].x + (row0 + r0) * N + col;
+#pragma unroll
+      for (int i = 0; i < kDftRows; ++i) *reinterpret_cast<float2*>(out + (size_t)i * N) = s[i];
+    }
+    __syncthreads();  // the next chunk restages the rows
   }
 }
 
 // gpmt: d/dlambda in Fourier space, (re, im) * i m (fourier/wgsl/dlambda.wgsl).
 __global__ void k_dlambda(const float* __restrict__ a, float* __restrict__ b, int n, int ntp1, int nfc) {
+  pdl_wait();
+  pdl_release();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int m = i % ntp1;
@@ -80,6 +104,8 @@ __global__ void k_dlambda(const float* __restrict__ a, float* __restrict__ b, in
 // The same on the optimized path's m-major Fourier planes (coefficient
 // (m, lat) at 2 * (m * NLAT + lat)).
 __global__ void k_dlambda_m_major(const float* __restrict__ a, float* __restrict__ b, int n, int nlat, int ntp1) {
+  pdl_wait();
+  pdl_release();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int m = (i / nlat) % ntp1;
@@ -92,96 +118,94 @@ __global__ void k_dlambda_m_major(const float* __restrict__ a, float* __restrict
 // ---------------------------------------------------------------- Legendre
 // Inverse transforms (sp2fc, sp2fcdmu, dv2uv): output (plane, lat, m) sums
 // modes n = m..NTRU of its plane. A block stages a tile of spectral planes
-// and the table rows of a tile of latitudes in shared memory (coalesced
-// loads, reused by every plane), and each thread computes wavenumbers j and
-// NTRU - j together so every thread sums NTRU + 2 terms.
-constexpr int kInvPlanes = 4;
-
-struct InvTile {
-  int lats;    // latitudes per block
-  size_t smem; // bytes
-};
-
-InvTile inverse_tile(const Dims& d, int tables, int inputs) {
-  const size_t budget = 160 * 1024;
-  for (int lats = 16; lats >= 2; lats /= 2) {
-    const size_t smem = (size_t)inputs * kInvPlanes * d.NRSP * 4 + (size_t)tables * lats * d.NCSP * 4;
-    if (smem <= budget && d.NLAT % lats == 0) return {lats, smem};
-  }
-  return {1, (size_t)inputs * kInvPlanes * d.NRSP * 4 + (size_t)tables * d.NCSP * 4};
-}
+// and the table rows of a tile of latitudes in shared memory, and each
+// thread computes wavenumbers j and NTRU - j of one (plane, latitude)
+// together, so every thread sums NTRU + 2 terms. The tiles are small (two
+// planes by four or eight latitudes) because the path steps single planets:
+// four planes by sixteen latitudes left one planet's field 12 blocks (49 us
+// at T42 L10), and a launch takes every field of a stage.
+constexpr int kInvPlanes = 2;
+constexpr int kInvLats = 8, kDvLats = 4;  // latitudes per block: sp2fc, dv2uv (divide every NLAT)
 
 __device__ __forceinline__ int mode_first(int m, int ntp1) { return m * (2 * ntp1 - m + 1) / 2; }
 
-__global__ void __launch_bounds__(kThreads) k_leg_inverse(const float* __restrict__ s, float* __restrict__ f,
-                                                          int planes, const float* __restrict__ q, Dims d,
-                                                          int lats) {
-  extern __shared__ float smem[];
-  float* sp = smem;                        // [kInvPlanes][NRSP]
-  float* qs = smem + kInvPlanes * d.NRSP;  // [lats][NCSP]
-  const int p0 = blockIdx.x * kInvPlanes;
-  const int np = min(kInvPlanes, planes - p0);
-  const int lat0 = blockIdx.y * lats;
-  for (int i = threadIdx.x; i < np * d.NRSP; i += blockDim.x) sp[i] = s[(size_t)p0 * d.NRSP + i];
-  for (int i = threadIdx.x; i < lats * d.NCSP; i += blockDim.x) qs[i] = q[(size_t)lat0 * d.NCSP + i];
+// Copies `n` floats (both 8-byte aligned, n even).
+__device__ __forceinline__ void copy_floats(float* dst, const float* src, int n) {
+  for (int i = threadIdx.x; i < n / 2; i += blockDim.x) cp_async8(dst + 2 * i, src + 2 * i);
+}
+
+__global__ void k_leg_inverse(const __grid_constant__ TrSet set, const float* __restrict__ qi,
+                              const float* __restrict__ qj, Dims d) {
+  extern __shared__ float4 inv_smem[];
+  float* sp = reinterpret_cast<float*>(inv_smem);  // [kInvPlanes][NRSP]
+  float* qs = sp + kInvPlanes * d.NRSP;            // [kInvLats][NCSP]
+  const int fi = tr_find(set, blockIdx.x);
+  const int p0 = (blockIdx.x - set.at[fi]) * kInvPlanes;
+  const int np = min(kInvPlanes, set.f[fi].planes - p0);
+  const int lat0 = blockIdx.y * kInvLats;
+  const float* q = set.f[fi].opt & kTrDerivative ? qj : qi;
+  copy_floats(qs, q + (size_t)lat0 * d.NCSP, kInvLats * d.NCSP);
+  pdl_wait();
+  pdl_release();
+  copy_floats(sp, set.f[fi].a + (size_t)p0 * d.NRSP, np * d.NRSP);
+  cp_async_wait_all();
   __syncthreads();
   const int pairs = (d.NTP1 + 1) / 2;
-  for (int o = threadIdx.x; o < np * lats * pairs; o += blockDim.x) {
+  for (int o = threadIdx.x; o < np * kInvLats * pairs; o += blockDim.x) {
     const int j = o % pairs;
-    const int lat = (o / pairs) % lats;
-    const int p = o / (pairs * lats);
+    const int lat = (o / pairs) % kInvLats;
+    const int p = o / (pairs * kInvLats);
     const float* spp = sp + p * d.NRSP;
     const float* qr = qs + lat * d.NCSP;
-    float* out = f + ((size_t)(p0 + p) * d.NLAT + lat0 + lat) * d.NFC;
+    float* out = set.f[fi].x + ((size_t)(p0 + p) * d.NLAT + lat0 + lat) * d.NFC;
 #pragma unroll 1
     for (int half = 0; half < 2; ++half) {
       const int m = half == 0 ? j : d.T - j;
       if (half == 1 && m == j) break;
       const int first = mode_first(m, d.NTP1);
       float re = 0.f, im = 0.f;
+#pragma unroll 4
       for (int w = first; w < first + d.NTP1 - m; ++w) {
         const float qq = qr[w];
-        re = fmaf(qq, spp[2 * w], re);
-        im = fmaf(qq, spp[2 * w + 1], im);
+        const float2 v = *reinterpret_cast<const float2*>(spp + 2 * w);
+        re = fmaf(qq, v.x, re);
+        im = fmaf(qq, v.y, im);
       }
-      out[2 * m] = re;
-      out[2 * m + 1] = im;
+      *reinterpret_cast<float2*>(out + 2 * m) = make_float2(re, im);
     }
   }
 }
 
 // dv2uv: winds at every latitude from spectral divergence and vorticity,
 // with plavor removed from vorticity mode w = 1 (legendre/wgsl/dv2uv.wgsl).
-__global__ void __launch_bounds__(kThreads) k_dv2uv(const float* __restrict__ D, const float* __restrict__ Z,
-                                                    float* __restrict__ U, float* __restrict__ V, int planes,
-                                                    const float* __restrict__ qu, const float* __restrict__ qv,
-                                                    float plavor, Dims d, int lats) {
-  extern __shared__ float smem[];
-  float* sp = smem;                                 // [kInvPlanes][2][NRSP]
-  float* qus = smem + 2 * kInvPlanes * d.NRSP;      // [lats][NCSP]
-  float* qvs = qus + (size_t)lats * d.NCSP;         // [lats][NCSP]
-  const int p0 = blockIdx.x * kInvPlanes;
-  const int np = min(kInvPlanes, planes - p0);
-  const int lat0 = blockIdx.y * lats;
-  for (int i = threadIdx.x; i < np * d.NRSP; i += blockDim.x) {
-    const int p = i / d.NRSP, k = i % d.NRSP;
-    sp[(2 * p) * d.NRSP + k] = D[(size_t)p0 * d.NRSP + i];
-    float z = Z[(size_t)p0 * d.NRSP + i];
-    if (k == 2) z -= plavor;  // w == 1, real part
-    sp[(2 * p + 1) * d.NRSP + k] = z;
-  }
-  for (int i = threadIdx.x; i < lats * d.NCSP; i += blockDim.x) {
-    qus[i] = qu[(size_t)lat0 * d.NCSP + i];
-    qvs[i] = qv[(size_t)lat0 * d.NCSP + i];
-  }
+__global__ void k_dv2uv(const __grid_constant__ TrSet set, const float* __restrict__ qu,
+                        const float* __restrict__ qv, Dims d) {
+  extern __shared__ float4 inv_smem[];
+  float* dd0 = reinterpret_cast<float*>(inv_smem);    // [kInvPlanes][NRSP]
+  float* zz0 = dd0 + kInvPlanes * d.NRSP;             // [kInvPlanes][NRSP]
+  float* qus = zz0 + kInvPlanes * d.NRSP;             // [kDvLats][NCSP]
+  float* qvs = qus + kDvLats * d.NCSP;                // [kDvLats][NCSP]
+  const int fi = tr_find(set, blockIdx.x);
+  const int p0 = (blockIdx.x - set.at[fi]) * kInvPlanes;
+  const int np = min(kInvPlanes, set.f[fi].planes - p0);
+  const int lat0 = blockIdx.y * kDvLats;
+  copy_floats(qus, qu + (size_t)lat0 * d.NCSP, kDvLats * d.NCSP);
+  copy_floats(qvs, qv + (size_t)lat0 * d.NCSP, kDvLats * d.NCSP);
+  pdl_wait();
+  pdl_release();
+  copy_floats(dd0, set.f[fi].a + (size_t)p0 * d.NRSP, np * d.NRSP);
+  copy_floats(zz0, set.f[fi].b + (size_t)p0 * d.NRSP, np * d.NRSP);
+  cp_async_wait_all();
+  __syncthreads();
+  if (threadIdx.x < np) zz0[threadIdx.x * d.NRSP + 2] -= set.f[fi].plavor;  // w == 1, real part
   __syncthreads();
   const int pairs = (d.NTP1 + 1) / 2;
-  for (int o = threadIdx.x; o < np * lats * pairs; o += blockDim.x) {
+  for (int o = threadIdx.x; o < np * kDvLats * pairs; o += blockDim.x) {
     const int j = o % pairs;
-    const int lat = (o / pairs) % lats;
-    const int p = o / (pairs * lats);
-    const float* dd = sp + (2 * p) * d.NRSP;
-    const float* zz = sp + (2 * p + 1) * d.NRSP;
+    const int lat = (o / pairs) % kDvLats;
+    const int p = o / (pairs * kDvLats);
+    const float* dd = dd0 + p * d.NRSP;
+    const float* zz = zz0 + p * d.NRSP;
     const float* qur = qus + lat * d.NCSP;
     const float* qvr = qvs + lat * d.NCSP;
     const size_t row = ((size_t)(p0 + p) * d.NLAT + lat0 + lat) * d.NFC;
@@ -191,6 +215,7 @@ __global__ void __launch_bounds__(kThreads) k_dv2uv(const float* __restrict__ D,
       if (half == 1 && m == j) break;
       const int first = mode_first(m, d.NTP1);
       float ure = 0.f, uim = 0.f, vre = 0.f, vim = 0.f;
+#pragma unroll 4
       for (int w = first; w < first + d.NTP1 - m; ++w) {
         const float a = qur[w], b = qvr[w];
         const float zre = zz[2 * w], zim = zz[2 * w + 1], dre = dd[2 * w], dim = dd[2 * w + 1];
@@ -199,108 +224,10 @@ __global__ void __launch_bounds__(kThreads) k_dv2uv(const float* __restrict__ D,
         vre = vre + a * zim - b * dre;
         vim = vim - a * zre - b * dim;
       }
-      U[row + 2 * m] = ure;
-      U[row + 2 * m + 1] = uim;
-      V[row + 2 * m] = vre;
-      V[row + 2 * m + 1] = vim;
+      *reinterpret_cast<float2*>(set.f[fi].x + row + 2 * m) = make_float2(ure, uim);
+      *reinterpret_cast<float2*>(set.f[fi].y + row + 2 * m) = make_float2(vre, vim);
     }
   }
-}
-
-// Forward transforms: each output (plane, mode w) sums latitude pairs of its
-// plane's Fourier coefficients at wavenumber m; a block stages kFwdPlanes
-// Fourier planes of each input.
-template <int NIN>
-struct FwdIn {
-  const float* p[NIN];
-};
-
-// kind 0: fc2sp with table q (legendre/wgsl/forward.wgsl).
-// kind 1: uv2dv, in = {u, v}, outputs D, Z (uv2dv.wgsl without the KE term).
-// kind 2: mktend's uv2dv, in = {u, v, ke} (uv2dv.wgsl with HAS_KINETIC).
-// kind 3: qtend, in = {u, v, source} (qtend.wgsl).
-template <int KIND, int NIN>
-__global__ void __launch_bounds__(kThreads) k_leg_forward(FwdIn<NIN> in, float* __restrict__ out0,
-                                                          float* __restrict__ out1, int planes,
-                                                          int planes_per_block, SharedTabs sh,
-                                                          const float* __restrict__ q, Dims d) {
-  extern __shared__ float fs[];  // [NIN][planes_per_block][NLAT * NFC]
-  const int plane_floats = d.NLAT * d.NFC;
-  const int p0 = blockIdx.x * planes_per_block;
-  const int np = min(planes_per_block, planes - p0);
-  for (int k = 0; k < NIN; ++k)
-    for (int i = threadIdx.x; i < np * plane_floats; i += blockDim.x)
-      fs[(size_t)k * planes_per_block * plane_floats + i] = in.p[k][(size_t)p0 * plane_floats + i];
-  __syncthreads();
-  const int half = d.NLAT / 2;
-  for (int o = threadIdx.x; o < np * d.NCSP; o += blockDim.x) {
-    const int w = o % d.NCSP;
-    const int p = o / d.NCSP;
-    const int m = sh.mode_m[w], n = sh.mode_n[w];
-    const float s = ((m + n) & 1) == 0 ? 1.f : -1.f;
-    const size_t at = (size_t)(p0 + p) * d.NRSP + 2 * w;
-    if (KIND == 0) {
-      const float* fp = fs + p * plane_floats + 2 * m;
-      float re = 0.f, im = 0.f;
-      for (int l = 0; l < half; ++l) {
-        const float qq = q[l * d.NCSP + w];
-        const float* north = fp + l * d.NFC;
-        const float* south = fp + (d.NLAT - 1 - l) * d.NFC;
-        re = fmaf(qq, north[0] + s * south[0], re);
-        im = fmaf(qq, north[1] + s * south[1], im);
-      }
-      out0[at] = re;
-      out0[at + 1] = im;
-    } else if (KIND == 1 || KIND == 2) {
-      const float* U = fs + p * plane_floats + 2 * m;
-      const float* V = U + (size_t)planes_per_block * plane_floats;
-      const float* K = V + (size_t)planes_per_block * plane_floats;
-      float dre = 0.f, dim = 0.f, zre = 0.f, zim = 0.f;
-      for (int l = 0; l < half; ++l) {
-        const int north = l * d.NFC, south = (d.NLAT - 1 - l) * d.NFC;
-        const float e = sh.qe[l * d.NCSP + w], mq = sh.qm[l * d.NCSP + w];
-        const float dure = U[north] - s * U[south], duim = U[north + 1] - s * U[south + 1];
-        const float dvre = V[north] - s * V[south], dvim = V[north + 1] - s * V[south + 1];
-        const float sure = U[north] + s * U[south], suim = U[north + 1] + s * U[south + 1];
-        const float svre = V[north] + s * V[south], svim = V[north + 1] + s * V[south + 1];
-        if (KIND == 2) {
-          const float q2 = sh.qq[l * d.NCSP + w];
-          dre = dre + q2 * (K[north] + s * K[south]);
-          dim = dim + q2 * (K[north + 1] + s * K[south + 1]);
-        }
-        dre = dre - e * dvre - mq * suim;
-        dim = dim - e * dvim + mq * sure;
-        zre = zre + e * dure - mq * svim;
-        zim = zim + e * duim + mq * svre;
-      }
-      out0[at] = dre;
-      out0[at + 1] = dim;
-      out1[at] = zre;
-      out1[at + 1] = zim;
-    } else {
-      const float* U = fs + p * plane_floats + 2 * m;
-      const float* V = U + (size_t)planes_per_block * plane_floats;
-      const float* X = V + (size_t)planes_per_block * plane_floats;
-      float re = 0.f, im = 0.f;
-      for (int l = 0; l < half; ++l) {
-        const int north = l * d.NFC, south = (d.NLAT - 1 - l) * d.NFC;
-        const float e = sh.qe[l * d.NCSP + w], c = sh.qc[l * d.NCSP + w], mq = sh.qm[l * d.NCSP + w];
-        re = re + e * (V[north] - s * V[south]) + c * (X[north] + s * X[south]) +
-             mq * (U[north + 1] + s * U[south + 1]);
-        im = im + e * (V[north + 1] - s * V[south + 1]) + c * (X[north + 1] + s * X[south + 1]) -
-             mq * (U[north] + s * U[south]);
-      }
-      out0[at] = re;
-      out0[at + 1] = im;
-    }
-  }
-}
-
-int forward_planes_per_block(const Dims& d, int nin) {
-  const int plane_bytes = d.NLAT * d.NFC * 4;
-  const int budget = 96 * 1024;
-  int ppb = budget / (plane_bytes * nin);
-  return ppb < 1 ? 1 : (ppb > 8 ? 8 : ppb);
 }
 
 // Dynamic shared memory above 48 KB needs an opt-in per kernel; tr_init sets
@@ -311,17 +238,24 @@ void allow_smem(K kernel) {
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
 }
 
-template <int KIND, int NIN>
-void launch_forward(const Model& m, FwdIn<NIN> in, float* out0, float* out1, int planes, const float* q,
-                    cudaStream_t st) {
-  const int ppb = forward_planes_per_block(m.d, NIN);
-  const size_t smem = (size_t)NIN * ppb * m.d.NLAT * m.d.NFC * sizeof(float);
-  auto kernel = k_leg_forward<KIND, NIN>;
-  const int blocks = (planes + ppb - 1) / ppb;
-  kernel<<<blocks, kThreads, smem, st>>>(in, out0, out1, planes, ppb, m.sh, q, m.d);
+// Rows per DFT chunk (dividing every NLAT): the most that still gives every
+// SM a chunk, so that one planet's few rows spread over the chip and a
+// batch's many rows reuse a staged table pair 8 times.
+int dft_rows(const Dims& d, int planes) {
+  for (int r : {32, 16})
+    if (planes * (d.NLAT / r) >= 148) return r;
+  return 8;
 }
 
-int dft_rows_per_block(const Dims& d) { return d.NLAT == 96 ? 24 : 32; }
+void launch_dft(const Model& m, TrSet set, const float* tab, int K, int N, cudaStream_t st) {
+  const int planes = tr_tiles(set, 1);
+  const int R = dft_rows(m.d, planes);
+  const int items = planes * (m.d.NLAT / R);
+  const size_t smem = ((size_t)(K * N + 3) / 4 * 4 + (size_t)R * ((K + 3) / 4 * 4)) * sizeof(float);
+  const int threads = N / 2 * (R / kDftRows);
+  const int grid = std::min(items, persistent_grid((const void*)k_dft, threads, smem));
+  step_launch(m.pdl, k_dft, grid, threads, smem, st, set, tab, K, N, m.d.NLAT, R, items);
+}
 
 }  // namespace
 
@@ -330,94 +264,84 @@ void tr_init() {
   tc_init();
   fft_init();
   grid_init();
-  allow_smem(k_dft_forward);
-  allow_smem(k_dft_inverse);
+  allow_smem(k_dft);
   allow_smem(k_leg_inverse);
   allow_smem(k_dv2uv);
-  allow_smem(k_leg_forward<0, 1>);
-  allow_smem(k_leg_forward<1, 2>);
-  allow_smem(k_leg_forward<2, 3>);
-  allow_smem(k_leg_forward<3, 3>);
 }
 
-void tr_fourier_forward(const Model& m, const float* g, float* c, int planes, cudaStream_t st) {
-  if (m.mode >= 1) return fft_forward(m, g, c, planes, st);
-  const int rows = planes * m.d.NLAT;
-  const int rpb = dft_rows_per_block(m.d);
-  const size_t smem = ((size_t)m.d.NLON * m.d.NFC + (size_t)rpb * m.d.NLON) * sizeof(float);
-  k_dft_forward<<<(rows + rpb - 1) / rpb, kThreads, smem, st>>>(g, c, rows, m.sh.fwd, m.d.NLON, m.d.NFC, rpb);
+void tr_fourier_forward(const Model& m, TrSet s, cudaStream_t st) {
+  if (m.mode >= 1) return fft_forward(m, s, st);
+  launch_dft(m, s, m.sh.fwd, m.d.NLON, m.d.NFC, st);
 }
 
-void tr_fourier_inverse(const Model& m, const float* c, float* g, int planes, cudaStream_t st) {
-  if (m.mode >= 1) return fft_inverse(m, c, g, planes, st);
-  const int rows = planes * m.d.NLAT;
-  const int rpb = dft_rows_per_block(m.d);
-  const size_t smem = ((size_t)m.d.NLON * m.d.NFC + (size_t)rpb * m.d.NFC) * sizeof(float);
-  k_dft_inverse<<<(rows + rpb - 1) / rpb, kThreads, smem, st>>>(c, g, rows, m.sh.inv, m.d.NLON, m.d.NFC, rpb);
+void tr_fourier_inverse(const Model& m, TrSet s, cudaStream_t st) {
+  if (m.mode >= 1) return fft_inverse(m, s, st);
+  launch_dft(m, s, m.sh.inv, m.d.NFC, m.d.NLON, st);
 }
 
-void tr_dlambda(const Model& m, const float* a, float* b, int planes, cudaStream_t st) {
+static void dlambda(const Model& m, const float* a, float* b, int planes, cudaStream_t st) {
   const int n = planes * m.d.NLAT * m.d.NTP1;
-  if (m.mode >= 1) {
-    k_dlambda_m_major<<<(n + 255) / 256, 256, 0, st>>>(a, b, n, m.d.NLAT, m.d.NTP1);
-    return;
+  const unsigned grid = (n + 255) / 256;
+  if (m.mode >= 1)
+    step_launch(m.pdl, k_dlambda_m_major, grid, 256, 0, st, a, b, n, m.d.NLAT, m.d.NTP1);
+  else
+    step_launch(m.pdl, k_dlambda, grid, 256, 0, st, a, b, n, m.d.NTP1, m.d.NFC);
+}
+
+void tr_to_grid(const Model& m, TrSet s, TrSet fourier, cudaStream_t st) {
+  if (m.mode == 1) {
+    if (fourier.n) fft_inverse(m, fourier, st);
+    return grid_sp2gp(m, s, st);
   }
-  k_dlambda<<<(n + 255) / 256, 256, 0, st>>>(a, b, n, m.d.NTP1, m.d.NFC);
-}
-
-void tr_sp2gp(const Model& m, const float* s, float* f, float* g, int planes, const float* q, cudaStream_t st) {
-  if (m.mode == 1 && (q == m.sh.qi || q == m.sh.qj)) return grid_sp2gp(m, s, f, g, planes, q == m.sh.qj, st);
-  tr_legendre_inverse(m, s, f, planes, q, st);
-  tr_fourier_inverse(m, f, g, planes, st);
-}
-
-void tr_legendre_inverse(const Model& m, const float* s, float* f, int planes, const float* q,
-                         cudaStream_t st) {
-  if (m.mode >= 1 && (q == m.sh.qi || q == m.sh.qj)) {
-    if (m.mode == 2) return tc_inverse(m, s, f, planes, q == m.sh.qj, st);
-    return leg_inverse(m, s, f, planes, q == m.sh.qj, st);
+  // sp2fc of every field that is not another's d/dlambda, then d/dlambda
+  // from the field sharing its spectral input, then fc2gp of everything.
+  TrSet inv;
+  for (int i = 0; i < s.n; ++i)
+    if (!(s.f[i].opt & kTrDlambda)) inv.add(s.f[i]);
+  tr_legendre_inverse(m, inv, st);
+  for (int i = 0; i < s.n; ++i) {
+    if (!(s.f[i].opt & kTrDlambda)) continue;
+    const float* from = nullptr;
+    for (int k = 0; k < s.n; ++k)
+      if (s.f[k].a == s.f[i].a && !(s.f[k].opt & (kTrDlambda | kTrDerivative))) from = s.f[k].x;
+    dlambda(m, from, s.f[i].x, s.f[i].planes, st);
   }
-  const InvTile t = inverse_tile(m.d, 1, 1);
-  dim3 grid((planes + kInvPlanes - 1) / kInvPlanes, m.d.NLAT / t.lats);
-  k_leg_inverse<<<grid, kThreads, t.smem, st>>>(s, f, planes, q, m.d, t.lats);
-}
-
-void tr_dv2uv(const Model& m, const float* D, const float* Z, float* U, float* V, int planes, float plavor,
-              cudaStream_t st) {
-  if (m.mode == 2) return tc_dv2uv(m, D, Z, U, V, planes, plavor, st);
-  if (m.mode >= 1) return leg_dv2uv(m, D, Z, U, V, planes, plavor, st);
-  const InvTile t = inverse_tile(m.d, 2, 2);
-  dim3 grid((planes + kInvPlanes - 1) / kInvPlanes, m.d.NLAT / t.lats);
-  k_dv2uv<<<grid, kThreads, t.smem, st>>>(D, Z, U, V, planes, m.sh.qu, m.sh.qv, plavor, m.d, t.lats);
-}
-
-void tr_legendre_forward(const Model& m, const float* f, float* s, int planes, const float* q,
-                         cudaStream_t st) {
-  if (m.mode == 2 && q == m.sh.qc) return tc_forward(m, f, s, planes, st);
-  if (m.mode >= 1) return leg_forward(m, f, s, planes, q, st);
-  FwdIn<1> in{{f}};
-  launch_forward<0, 1>(m, in, s, nullptr, planes, q, st);
-}
-
-void tr_uv2dv(const Model& m, const float* u, const float* v, const float* ke, float* D, float* Z, int planes,
-              cudaStream_t st) {
-  if (m.mode == 2) return tc_uv2dv(m, u, v, ke, D, Z, planes, st);
-  if (m.mode >= 1) return leg_uv2dv(m, u, v, ke, D, Z, planes, st);
-  if (ke) {
-    FwdIn<3> in{{u, v, ke}};
-    launch_forward<2, 3>(m, in, D, Z, planes, nullptr, st);
-  } else {
-    FwdIn<2> in{{u, v}};
-    launch_forward<1, 2>(m, in, D, Z, planes, nullptr, st);
+  for (int i = 0; i < s.n; ++i) {
+    TrField t;
+    t.a = s.f[i].x;
+    t.x = s.f[i].y;
+    t.planes = s.f[i].planes;
+    fourier.add(t);
   }
+  tr_fourier_inverse(m, fourier, st);
 }
 
-void tr_qtend(const Model& m, const float* u, const float* v, const float* src, float* out, int planes,
-              cudaStream_t st) {
-  if (m.mode == 2) return tc_qtend(m, u, v, src, out, planes, st);
-  if (m.mode >= 1) return leg_qtend(m, u, v, src, out, planes, st);
-  FwdIn<3> in{{u, v, src}};
-  launch_forward<3, 3>(m, in, out, nullptr, planes, nullptr, st);
+void tr_legendre_inverse(const Model& m, TrSet s, cudaStream_t st) {
+  if (m.mode == 2) return tc_inverse(m, s, st);
+  if (m.mode == 1) return leg_inverse(m, s, st);
+  const dim3 grid(tr_tiles(s, kInvPlanes), m.d.NLAT / kInvLats);
+  const int threads = (kInvPlanes * kInvLats * ((m.d.NTP1 + 1) / 2) + 31) / 32 * 32;
+  const size_t smem = ((size_t)kInvPlanes * m.d.NRSP + (size_t)kInvLats * m.d.NCSP) * sizeof(float);
+  step_launch(m.pdl, k_leg_inverse, grid, threads, smem, st, s, m.sh.qi, m.sh.qj, m.d);
 }
+
+void tr_dv2uv(const Model& m, TrSet s, cudaStream_t st) {
+  if (m.mode == 2) return tc_dv2uv(m, s, st);
+  if (m.mode == 1) return leg_dv2uv(m, s, st);
+  const dim3 grid(tr_tiles(s, kInvPlanes), m.d.NLAT / kDvLats);
+  const int threads = (kInvPlanes * kDvLats * ((m.d.NTP1 + 1) / 2) + 31) / 32 * 32;
+  const size_t smem = ((size_t)2 * kInvPlanes * m.d.NRSP + (size_t)2 * kDvLats * m.d.NCSP) * sizeof(float);
+  step_launch(m.pdl, k_dv2uv, grid, threads, smem, st, s, m.sh.qu, m.sh.qv, m.d);
+}
+
+// The latitude-pair kernels sum in the shaders' order, so the plain path's
+// forward transforms run on them too (on its own Fourier layout).
+void tr_legendre_forward(const Model& m, TrSet s, cudaStream_t st) {
+  m.mode == 2 ? tc_forward(m, s, st) : leg_forward(m, s, st);
+}
+
+void tr_uv2dv(const Model& m, TrSet s, cudaStream_t st) { m.mode == 2 ? tc_uv2dv(m, s, st) : leg_uv2dv(m, s, st); }
+
+void tr_qtend(const Model& m, TrSet s, cudaStream_t st) { m.mode == 2 ? tc_qtend(m, s, st) : leg_qtend(m, s, st); }
 
 }  // namespace exogcm
