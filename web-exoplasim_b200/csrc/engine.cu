@@ -939,6 +939,14 @@ int exogcm_create(int truncation, int levels, int slots, int mode, exogcm_engine
     e->d = make_dims(truncation, levels, slots);
     e->mode = mode;
     e->tune = default_tuning(e->d);
+    // Programmatic dependent launch of the transform, dynamics and reduction
+    // kernels while the batch's columns fit the chip about once (148 SMs x 4
+    // blocks x 128 columns): there the launch gap is a good part of a kernel.
+    // Above that a waiting block takes the place of a running one. us a step,
+    // without -> with: 8,192 columns (T42 L10, 1 planet) 236 -> 219, 57,344
+    // (T42 L5, 7) 254 -> 236, 65,536 (T42 L10, 8) 386 -> 384, 131,072 (16)
+    // 577 -> 586, 1,048,576 (128) 3494 -> 3677.
+    e->pdl = (long)slots * e->d.NHOR <= 65536 ? 1 : 0;
     check(cudaGetDevice(&e->device), "device");
     layout(e.get());
     table_layout(e.get());

@@ -11,6 +11,12 @@
 // The fixer's apply step, the surface fluxes, vertical diffusion, solar
 // angle and ozone are in physics_flux.cu (IEEE division).
 #include "physics_common.cuh"
+#ifndef RAIN_B
+#define RAIN_B 1
+#endif
+#ifndef RAIN_U
+#define RAIN_U 1
+#endif
 
 namespace exogcm {
 
@@ -57,6 +63,8 @@ constexpr int kMaxNlon = 192;  // NLON at T63, the largest truncation an engine 
 
 template <int NL>
 __global__ void __launch_bounds__(32 * kRowWarps) k_fixer_row(Model m) {
+  pdl_wait();
+  pdl_release();
   __shared__ float stage[kRowWarps][kMaxNlon];
   const Dims& d = m.d;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -101,16 +109,32 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_fixer_row(Model m) {
 // and as doubles to sums[slot * 4 + which * 2 + 0|1].
 __global__ void __launch_bounds__(kSumThreads) k_slot_sums(Model m, const float* a, const float* b, float* target,
                                                            int which) {
+  pdl_wait();
+  pdl_release();
   const Dims& d = m.d;
   const int slot = blockIdx.x;
   if (!m.params[slot].active) return;
   if (which == 1 && m.params[slot].coupled == 0.f) return;  // getiflx runs with icestep only
   __shared__ double sa[kSumThreads], sb[kSumThreads];
   double x = 0.0, y = 0.0;
-  const size_t base = (size_t)slot * d.NHOR;
-  for (int h = threadIdx.x; h < d.NHOR; h += kSumThreads) {
-    x += (double)a[base + h];
-    y += (double)b[base + h];
+  // Eight points of each field in flight, added in order: one at a time, the
+  // block waited for memory 32 times in a row at T42 (11 us for two 32 KB
+  // sums). NHOR is a multiple of 8 kSumThreads.
+  constexpr int kAhead = 8;
+  const float* pa = a + (size_t)slot * d.NHOR + threadIdx.x;
+  const float* pb = b + (size_t)slot * d.NHOR + threadIdx.x;
+  for (int h = 0; h < d.NHOR; h += kAhead * kSumThreads) {
+    float va[kAhead], vb[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      va[k] = pa[h + k * kSumThreads];
+      vb[k] = pb[h + k * kSumThreads];
+    }
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      x += (double)va[k];
+      y += (double)vb[k];
+    }
   }
   sa[threadIdx.x] = x;
   sb[threadIdx.x] = y;
@@ -331,6 +355,8 @@ __device__ __forceinline__ void swr_band(const Model& m, const PlanetConst& K, c
 // shader's order (band 1 + band 2).
 template <int NL>
 __global__ void __launch_bounds__(kBlock) k_swr(Model m) {
+  pdl_wait();
+  pdl_release();
   static_assert(NL <= SwrLevels::MAXLEV, "swr level state holds at most MAXLEV levels");
   constexpr int NP = NL + 1;
   constexpr int kCols = kBlock / 2;
@@ -912,11 +938,14 @@ __global__ void __launch_bounds__(kBlock) k_mkdca(Model m, const PlanetConst* __
 // mkdca-limit (physics/precipitation/wgsl/mkdca-limit.wgsl): per slot, skip
 // every adjustment when any column needed more than 2 NL passes.
 __global__ void __launch_bounds__(kSumThreads) k_mkdca_limit(Model m) {
+  pdl_wait();
+  pdl_release();
   const Dims& d = m.d;
   const int slot = blockIdx.x;
   if (!m.params[slot].active) return;
   __shared__ float part[kSumThreads];
   float flag = 0.f;
+#pragma unroll 8
   for (int h = threadIdx.x; h < d.NHOR; h += kSumThreads) flag = fmaxf(flag, m.f.dca_limited[slot * d.NHOR + h]);
   part[threadIdx.x] = flag;
   __syncthreads();
@@ -927,95 +956,98 @@ __global__ void __launch_bounds__(kSumThreads) k_mkdca_limit(Model m) {
   if (threadIdx.x == 0) m.f.dca_skip[slot] = part[0];
 }
 
-// column.wgsl: mkdca's adjustment (unless skipped), mklsp, mkrain, mkclouds.
-// Its parameters carry no __restrict__: with it the compiler keeps more
-// values in registers (165), and the lower occupancy measured slower. The
-// planet's constants, read again after the stores of each level loop, sit
-// in shared memory (259 -> 252 us per launch at 128 T42 L10 planets).
+// column.wgsl: mkdca's adjustment (unless skipped), mklsp, mkrain, mkclouds,
+// one thread per column. The level loops stay rolled: the condensation and
+// mkrain's falling fluxes go down the column together, each level's loads one
+// level ahead, and what the later loops need of a level (its relative
+// humidity, temperature, and humidity or height) waits in this thread's
+// column of shared memory. Unrolled, with the level columns in registers, the
+// kernel was 126 registers (16 warps per SM) and mostly waited for
+// instruction fetch at one planet and for memory and fetch at 128.
 template <int NL>
-__device__ __forceinline__ void b_rain_column(const Model& m, const PlanetConst* pcr, const float* tabr) {
+__global__ void __launch_bounds__(kBlock, RAIN_B)
+    k_rain_column(Model m, const PlanetConst* __restrict__ pcr, const float* __restrict__ tabr) {
   COLUMN_PROLOGUE_STAGED
+  __shared__ float s_rh[NL][kBlock], s_t[NL][kBlock], s_q[NL][kBlock];
+  const int tx = threadIdx.x;
   const float* ds = tb + m.to.dsigma;
   const float* sg = tb + m.to.sigma;
   const float D2 = P.deltsec2;
   const bool skip = F.dca_skip[slot] != 0.f;
   const float dp = F.dp[c];
-  // mkrain's and mkclouds' inputs are read after mklsp's stores; registers
-  // cannot hold them from here, so they are fetched into L2 now.
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    const size_t at = l * SN + c;
-    prefetch_l2(F.dprscl + at);
-    prefetch_l2(F.dprcl + at);
-    prefetch_l2(F.icclev + at);
-    if (K.CLWFAC > 0.f) prefetch_l2(F.dw + at);
-  }
-  prefetch_l2(F.icctot + c);
-  prefetch_l2(F.dt + NL * SN + c);
-  float dq_[NL], dt_[NL], dtdt_[NL], dqdt_[NL];
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    const size_t at = l * SN + c;
-    dq_[l] = F.dq[at];
-    dt_[l] = F.dt[at];
-    dtdt_[l] = F.dtdt[at];
-    dqdt_[l] = F.dqdt[at];
-    if (!skip) {
-      dtdt_[l] = dtdt_[l] + F.dca_dtdt[at];
-      dqdt_[l] = dqdt_[l] + F.dca_dqdt[at];
-    }
-  }
-  // mklsp
-  float dprll[NL];
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    dprll[l] = 0.f;
-    const float dq = dq_[l];
-    const float zq = dq + dqdt_[l] * D2;
-    const float zt = dt_[l] + dtdt_[l] * D2;
-    // IEEE divisions here (the file otherwise divides to 2 ulp): the
-    // large-scale precipitation is the difference of two iterated states.
-    const float zlcpe = __fdiv_rn(K.ALV, K.ACPD * (1.f + K.ADV * dq));
-    const float p = dp * sg[l];
-    float zqsat = sat_capped_rn(K, zt, p);
-    float zcor = __fdiv_rn(1.f, 1.f - K.MOIST * zqsat);
-    zqsat = zqsat * zcor;
-    if (zqsat < 0.f) zqsat = 0.f;
-    if (zq > zqsat) {
-      float zdqdt = __fdiv_rn(zqsat - zq, 1.f + __fdiv_rn(zlcpe * K.RA2 * (K.TMELT - K.RA4) * zqsat * zcor,
-                                                          (zt - K.RA4) * (zt - K.RA4)));
-      float ztn = zt - zdqdt * zlcpe;
-      float zqn = zq + zdqdt;
-      zqsat = sat_capped_rn(K, ztn, p);
-      zcor = __fdiv_rn(1.f, 1.f - K.MOIST * zqsat);
-      zqsat = zqsat * zcor;
-      zdqdt = __fdiv_rn(zqsat - zqn, 1.f + __fdiv_rn(zlcpe * K.RA2 * (K.TMELT - K.RA4) * zqsat * zcor,
-                                                     (ztn - K.RA4) * (ztn - K.RA4)));
-      ztn = ztn - zdqdt * zlcpe;
-      zqn = zqn + zdqdt;
-      const float dqdt = __fdiv_rn(zqn - zq, D2), dtdt = __fdiv_rn(ztn - zt, D2);
-      dqdt_[l] = dqdt_[l] + dqdt;
-      dtdt_[l] = dtdt_[l] + dtdt;
-      dprll[l] = -fminf(dqdt, 0.f) * ds[l];
-    }
-    F.dprsll[l * SN + c] = 0.f;
-    F.dprll[l * SN + c] = dprll[l];
-  }
-  // mkrain
+  const float tsurf = F.dt[NL * SN + c], convective = F.icctot[c];
   float zprc = 0.f, zprl = 0.f, zprsc = 0.f, zprsl = 0.f;
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
+  struct Level {
+    float dq, dt, dtdt, dqdt, adt, adq, scl, cl;
+  };
+  auto load = [&](int l) {
     const size_t at = l * SN + c;
-    const float dsl = ds[l], dq = dq_[l];
+    Level v;
+    v.dq = F.dq[at];
+    v.dt = F.dt[at];
+    v.dtdt = F.dtdt[at];
+    v.dqdt = F.dqdt[at];
+    v.adt = skip ? 0.f : F.dca_dtdt[at];
+    v.adq = skip ? 0.f : F.dca_dqdt[at];
+    v.scl = F.dprscl[at];
+    v.cl = F.dprcl[at];
+    return v;
+  };
+  Level next = load(0);
+  constexpr int kUnroll = RAIN_U;
+#pragma unroll kUnroll
+  for (int l = 0; l < NL; ++l) {
+    const Level in = next;
+    if (l + 1 < NL) next = load(l + 1);
+    const size_t at = l * SN + c;
+    const float dsl = ds[l], dq = in.dq, dt = in.dt, p = dp * sg[l];
+    float dtdt_ = in.dtdt, dqdt_ = in.dqdt;
+    if (!skip) {
+      dtdt_ = dtdt_ + in.adt;
+      dqdt_ = dqdt_ + in.adq;
+    }
+    // mklsp
+    float dprll = 0.f;
+    {
+      const float zq = dq + dqdt_ * D2;
+      const float zt = dt + dtdt_ * D2;
+      // IEEE divisions here (the file otherwise divides to 2 ulp): the
+      // large-scale precipitation is the difference of two iterated states.
+      const float zlcpe = __fdiv_rn(K.ALV, K.ACPD * (1.f + K.ADV * dq));
+      float zqsat = sat_capped_rn(K, zt, p);
+      float zcor = __fdiv_rn(1.f, 1.f - K.MOIST * zqsat);
+      zqsat = zqsat * zcor;
+      if (zqsat < 0.f) zqsat = 0.f;
+      if (zq > zqsat) {
+        float zdqdt = __fdiv_rn(zqsat - zq, 1.f + __fdiv_rn(zlcpe * K.RA2 * (K.TMELT - K.RA4) * zqsat * zcor,
+                                                            (zt - K.RA4) * (zt - K.RA4)));
+        float ztn = zt - zdqdt * zlcpe;
+        float zqn = zq + zdqdt;
+        zqsat = sat_capped_rn(K, ztn, p);
+        zcor = __fdiv_rn(1.f, 1.f - K.MOIST * zqsat);
+        zqsat = zqsat * zcor;
+        zdqdt = __fdiv_rn(zqsat - zqn, 1.f + __fdiv_rn(zlcpe * K.RA2 * (K.TMELT - K.RA4) * zqsat * zcor,
+                                                       (ztn - K.RA4) * (ztn - K.RA4)));
+        ztn = ztn - zdqdt * zlcpe;
+        zqn = zqn + zdqdt;
+        const float dqdt = __fdiv_rn(zqn - zq, D2), dtdt = __fdiv_rn(ztn - zt, D2);
+        dqdt_ = dqdt_ + dqdt;
+        dtdt_ = dtdt_ + dtdt;
+        dprll = -fminf(dqdt, 0.f) * dsl;
+      }
+      F.dprsll[at] = 0.f;
+      F.dprll[at] = dprll;
+    }
+    // mkrain
     float zdtdt = 0.f, zdqdtl = 0.f, zdqdts = 0.f;
-    const float dprscl = F.dprscl[at];
-    zprc = zprc + F.dprcl[at] - dprscl;
-    zprl = zprl + dprll[l] - 0.f;
-    zprsc = zprsc + dprscl;
+    zprc = zprc + in.cl - in.scl;
+    zprl = zprl + dprll - 0.f;
+    zprsc = zprsc + in.scl;
     zprsl = zprsl + 0.f;
     const int surface = l == NL - 1 ? 2 : 1;
+#pragma unroll 1
     for (int below = 0; below < surface; ++below) {
-      const float temperature = F.dt[(l + below) * SN + c];
+      const float temperature = below == 0 ? dt : tsurf;
       const float zlcp = (K.ALS - K.ALV) / (K.ACPD * (1.f + K.ADV * dq));
       if (zprsc + zprsl > 0.f && temperature > K.TMELT) {
         zdtdt = -(zprsc + zprsl) / dsl * zlcp + zdtdt;
@@ -1031,45 +1063,56 @@ __device__ __forceinline__ void b_rain_column(const Model& m, const PlanetConst*
         zprl = 0.f;
       }
     }
-    const float zq = dq + dqdt_[l] * D2;
-    const float zt = dt_[l] + dtdt_[l] * D2;
-    float zqsat = sat_capped(K, zt, dp * sg[l]);
-    const float zcor = 1.f / (1.f - K.MOIST * zqsat);
-    zqsat = zqsat * zcor;
-    if (zqsat < 0.f) zqsat = 0.f;
-    if (zq < zqsat) {
-      const float deficit = zqsat - zq;
-      const float water = K.ALV / (K.ACPD * (1.f + K.ADV * dq));
-      const float ice = K.ALS / (K.ACPD * (1.f + K.ADV * dq));
-      const float curve = K.RA2 * (K.TMELT - K.RA4) * zqsat * zcor / ((zt - K.RA4) * (zt - K.RA4));
-      auto evap = [&](float& flux, float zlcpe) {
-        const float zd = fminf(K.GAMMA * deficit * dsl / D2 / (1.f + zlcpe * curve), flux);
-        flux = flux - zd;
-        return zd / dsl;
-      };
-      if (zprl > 0.f) {
-        const float e = evap(zprl, water);
-        zdtdt = zdtdt - e * water;
-        zdqdtl = zdqdtl + e;
-      }
-      if (zprc > 0.f) {
-        const float e = evap(zprc, water);
-        zdtdt = zdtdt - e * water;
-        zdqdtl = zdqdtl + e;
-      }
-      if (zprsl > 0.f) {
-        const float e = evap(zprsl, ice);
-        zdtdt = zdtdt - e * ice;
-        zdqdts = zdqdts + e;
-      }
-      if (zprsc > 0.f) {
-        const float e = evap(zprsc, ice);
-        zdtdt = zdtdt - e * ice;
-        zdqdts = zdqdts + e;
+    {
+      const float zq = dq + dqdt_ * D2;
+      const float zt = dt + dtdt_ * D2;
+      float zqsat = sat_capped(K, zt, p);
+      const float zcor = 1.f / (1.f - K.MOIST * zqsat);
+      zqsat = zqsat * zcor;
+      if (zqsat < 0.f) zqsat = 0.f;
+      if (zq < zqsat) {
+        const float deficit = zqsat - zq;
+        const float water = K.ALV / (K.ACPD * (1.f + K.ADV * dq));
+        const float ice = K.ALS / (K.ACPD * (1.f + K.ADV * dq));
+        const float curve = K.RA2 * (K.TMELT - K.RA4) * zqsat * zcor / ((zt - K.RA4) * (zt - K.RA4));
+        auto evap = [&](float& flux, float zlcpe) {
+          const float zd = fminf(K.GAMMA * deficit * dsl / D2 / (1.f + zlcpe * curve), flux);
+          flux = flux - zd;
+          return zd / dsl;
+        };
+        if (zprl > 0.f) {
+          const float e = evap(zprl, water);
+          zdtdt = zdtdt - e * water;
+          zdqdtl = zdqdtl + e;
+        }
+        if (zprc > 0.f) {
+          const float e = evap(zprc, water);
+          zdtdt = zdtdt - e * water;
+          zdqdtl = zdqdtl + e;
+        }
+        if (zprsl > 0.f) {
+          const float e = evap(zprsl, ice);
+          zdtdt = zdtdt - e * ice;
+          zdqdts = zdqdts + e;
+        }
+        if (zprsc > 0.f) {
+          const float e = evap(zprsc, ice);
+          zdtdt = zdtdt - e * ice;
+          zdqdts = zdqdts + e;
+        }
       }
     }
-    dqdt_[l] = dqdt_[l] + zdqdtl + zdqdts;
-    dtdt_[l] = dtdt_[l] + zdtdt;
+    dqdt_ = dqdt_ + zdqdtl + zdqdts;
+    dtdt_ = dtdt_ + zdtdt;
+    F.dtdt[at] = dtdt_;
+    F.dqdt[at] = dqdt_;
+    // mkclouds' relative humidity
+    const float zt = dt + dtdt_ * D2;
+    const float zq = dq + dqdt_ * D2;
+    const float zqsat = sat_divided(K, zt, p);
+    s_rh[l][tx] = zq / zqsat;
+    s_t[l][tx] = dt;
+    s_q[l][tx] = dq;
   }
   const float dprc = (zprc + zprsc) * dp / K.GA / 1000.f;
   F.dprc[c] = dprc;
@@ -1081,67 +1124,57 @@ __device__ __forceinline__ void b_rain_column(const Model& m, const PlanetConst*
   if (dprc > 0.f) {
     zcctot = ZCCA + ZCCB * logf(dprc * K.ZRFAC);
     zcctot = fminf(ZCCMAX, fmaxf(ZCCMIN, zcctot));
-    const float levels = F.icctot[c];
-    zccconv = levels == 0.f ? 1.f : 1.f - fpow(1.f - zcctot, 1.f / levels);
+    zccconv = convective == 0.f ? 1.f : 1.f - fpow(1.f - zcctot, 1.f / convective);
   }
-  float cover[NL];
-#pragma unroll
+  // up the column: the water vapour and the heights (over the spent humidity)
+  const float* lnsig = tb + m.to.rad_lnsig;
+  float dqvi = 0.f, zzh = 0.f;
+#pragma unroll 2
+  for (int l = NL - 1; l >= 1; --l) {
+    dqvi = s_q[l][tx] * ds[l] + dqvi;
+    const float zdh = -s_t[l][tx] * K.GASCON / K.GA * lnsig[l];
+    s_q[l][tx] = zzh + zdh * 0.5f;
+    zzh = zzh + zdh;
+  }
+  dqvi = s_q[0][tx] * ds[0] + dqvi;
+  s_q[0][tx] = zzh - s_t[0][tx] * K.GASCON / K.GA * lnsig[0];
+  dqvi = dqvi * dp / K.GA;
+  F.dqvi[c] = dqvi;
+  zzh = 700.f * logf(1.f + dqvi);
+  float clear = 1.f;
+  float icc_n = F.icclev[c], dw_n = K.CLWFAC > 0.f ? F.dw[c] : 0.f;
+#pragma unroll 1
   for (int l = 0; l < NL; ++l) {
     const size_t at = l * SN + c;
-    const float zt = dt_[l] + dtdt_[l] * D2;
-    const float zq = dq_[l] + dqdt_[l] * D2;
-    const float zqsat = sat_divided(K, zt, dp * sg[l]);
-    float zrh = zq / zqsat;
-    const float icclev = F.icclev[at];
+    const float icclev = icc_n, dw = dw_n, sgl = sg[l];
+    if (l + 1 < NL) {
+      icc_n = F.icclev[at + SN];
+      if (K.CLWFAC > 0.f) dw_n = F.dw[at + SN];
+    }
+    float zrh = s_rh[l][tx];
     float dcc = icclev > 0.f ? zccconv : 0.f;
     if (icclev == 2.f && zcctot >= 0.3f) dcc = fminf(dcc + 2.f * (zcctot - 0.3f), ZCLMAX);
     zrh = zrh * (1.f - dcc);
     const float zrcrit = tb[m.to.rcrit + l];
     float zwfac = 1.f;
-    if (sg[l] > 0.8f && K.CLWFAC > 0.f) {
-      const float dw = F.dw[at];
+    if (sgl > 0.8f && K.CLWFAC > 0.f) {
       zwfac = K.CLWFAC * fmaxf(0.f, K.CLWCRIT1 - dw);
       if (K.CLWCRIT2 > dw) zwfac = 1.f;
     }
     const float excess = fmaxf(0.f, (zrh - zrcrit) / (1.f - zrcrit));
-    cover[l] = fminf(dcc + zwfac * (excess * excess), ZCLMAX);
-  }
-  const float* lnsig = tb + m.to.rad_lnsig;
-  float zzf[NL];
-  float dqvi = 0.f, zzh = 0.f;
-#pragma unroll
-  for (int l = NL - 1; l >= 1; --l) {
-    dqvi = dq_[l] * ds[l] + dqvi;
-    const float zdh = -dt_[l] * K.GASCON / K.GA * lnsig[l];
-    zzf[l] = zzh + zdh * 0.5f;
-    zzh = zzh + zdh;
-  }
-  dqvi = dq_[0] * ds[0] + dqvi;
-  zzf[0] = zzh - dt_[0] * K.GASCON / K.GA * lnsig[0];
-  dqvi = dqvi * dp / K.GA;
-  F.dqvi[c] = dqvi;
-  zzh = 700.f * logf(1.f + dqvi);
-  float clear = 1.f;
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    const size_t at = l * SN + c;
+    const float cover = fminf(dcc + zwfac * (excess * excess), ZCLMAX);
     float dql = 0.f;
-    if (zzh > 0.f && cover[l] > 0.f) {
-      dql = 0.00021f * expf(-zzf[l] / zzh) * K.GASCON * dt_[l] / (sg[l] * dp);
+    if (zzh > 0.f && cover > 0.f) {
+      dql = 0.00021f * expf(-s_q[l][tx] / zzh) * K.GASCON * s_t[l][tx] / (sgl * dp);
       dql = fmaxf(dql, 1.0e-9f);
     }
     F.dql[at] = dql;
-    F.dcc[at] = cover[l];
-    F.dtdt[at] = dtdt_[l];
-    F.dqdt[at] = dqdt_[l];
-    clear = clear * (1.f - cover[l]);
+    F.dcc[at] = cover;
+    const float open = 1.f - cover;
+    if (l == NL - 1) F.dcc[at + SN] = 1.f - clear * open;
+    clear = clear * open;
   }
   F.dql[NL * SN + c] = 0.f;
-  F.dcc[NL * SN + c] = 1.f - clear;
-}
-template <int NL>
-__global__ void __launch_bounds__(kBlock) k_rain_column(Model m, const PlanetConst* pcr, const float* tabr) {
-  b_rain_column<NL>(m, pcr, tabr);
 }
 
 
@@ -1289,6 +1322,8 @@ __global__ void __launch_bounds__(kBlock) k_soil(Model m, const PlanetConst* __r
 __device__ __forceinline__ float river(const FieldPtrs& F, int c) { return F.driver[c] * F.darea[c] * F.dls[c]; }
 
 __global__ void __launch_bounds__(kBlock) k_mkradv(Model m) {
+  pdl_wait();
+  pdl_release();
   const Dims& d = m.d;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= d.S * d.NHOR) return;
@@ -1914,71 +1949,75 @@ __global__ void __launch_bounds__(kBlock) k_pack(Model m, const PlanetConst* __r
     F.carbon_step[slot] = P.carbon;
   }
   if (snapflag == 0.f) return;
+  // Nothing below but the snapshot and its tracking is written here, so the
+  // fields are read as read-only data: the compiler may then hold many loads in
+  // flight past the stores, which it cannot prove distinct from the fields (33
+  // us for 7 T42 L5 planets when each of 76 loads waited for the store before it).
   const int jet = (int)K.JET;
-  put(0, F.dt[NL * SN + c]);
-  put(1, F.dtsa[c]);
-  put(2, F.du[(NL - 1) * SN + c]);
-  put(3, F.dv[(NL - 1) * SN + c]);
-  put(4, F.dcc[NL * SN + c]);
-  put(5, F.dprc[c] + F.dprl[c]);
-  put(6, F.dp[c]);
-  put(7, F.dqvi[c]);
-  put(8, F.dicec[c]);
-  put(9, F.dsnow[c]);
-  put(10, F.dwatc[c]);
-  put(11, F.dalb[c]);
-  put(12, F.du[jet * SN + c]);
-  put(13, F.dv[jet * SN + c]);
-  put(14, -F.dlwfl[c]);
-  put(15, F.dls[c]);
-  put(16, F.dswfl[c] + F.dlwfl[c]);
-  put(17, F.dsmelt[c] * -333700000.f + F.dswfl[NL * SN + c] + F.dlwfl[NL * SN + c] + F.dshfl[c] + F.dlhfl[c]);
-  put(18, -F.devap[c]);
-  put(19, F.drunoff[c]);
-  put(20, F.dforest[c]);
-  put(21, F.dlai[c]);
-  put(22, F.dprs[c]);
-  put(23, F.dsmelt[c]);
-  put(24, F.diced[c]);
-  put(25, F.dglac[c]);
-  put(27, F.dswfl[NL * SN + c]);
-  put(28, F.dlwfl[NL * SN + c]);
-  put(29, F.dshfl[c]);
-  put(30, F.dlhfl[c]);
-  put(31, F.dprc[c]);
-  put(32, F.dprl[c]);
-  put(33, F.dswfl[c]);
-  put(34, F.dlwfl[c]);
+  put(0, __ldg(F.dt + NL * SN + c));
+  put(1, __ldg(F.dtsa + c));
+  put(2, __ldg(F.du + (NL - 1) * SN + c));
+  put(3, __ldg(F.dv + (NL - 1) * SN + c));
+  put(4, __ldg(F.dcc + NL * SN + c));
+  put(5, __ldg(F.dprc + c) + __ldg(F.dprl + c));
+  put(6, __ldg(F.dp + c));
+  put(7, __ldg(F.dqvi + c));
+  put(8, __ldg(F.dicec + c));
+  put(9, __ldg(F.dsnow + c));
+  put(10, __ldg(F.dwatc + c));
+  put(11, __ldg(F.dalb + c));
+  put(12, __ldg(F.du + jet * SN + c));
+  put(13, __ldg(F.dv + jet * SN + c));
+  put(14, -__ldg(F.dlwfl + c));
+  put(15, __ldg(F.dls + c));
+  put(16, __ldg(F.dswfl + c) + __ldg(F.dlwfl + c));
+  put(17, __ldg(F.dsmelt + c) * -333700000.f + __ldg(F.dswfl + NL * SN + c) + __ldg(F.dlwfl + NL * SN + c) + __ldg(F.dshfl + c) + __ldg(F.dlhfl + c));
+  put(18, -__ldg(F.devap + c));
+  put(19, __ldg(F.drunoff + c));
+  put(20, __ldg(F.dforest + c));
+  put(21, __ldg(F.dlai + c));
+  put(22, __ldg(F.dprs + c));
+  put(23, __ldg(F.dsmelt + c));
+  put(24, __ldg(F.diced + c));
+  put(25, __ldg(F.dglac + c));
+  put(27, __ldg(F.dswfl + NL * SN + c));
+  put(28, __ldg(F.dlwfl + NL * SN + c));
+  put(29, __ldg(F.dshfl + c));
+  put(30, __ldg(F.dlhfl + c));
+  put(31, __ldg(F.dprc + c));
+  put(32, __ldg(F.dprl + c));
+  put(33, __ldg(F.dswfl + c));
+  put(34, __ldg(F.dlwfl + c));
   const bool windowed = tr[8 * SN] != 0.f;
   put(35, windowed ? tr[2 * SN] : tr[0]);
   put(36, windowed ? tr[3 * SN] : tr[SN]);
   put(37, windowed ? tr[4 * SN] : tr[SN] - tr[0]);
   put(38, tr[5 * SN]);
   put(39, tr[6 * SN]);
-  put(40, F.dnpp[c]);
-  put(41, F.gmu0[c]);
+  put(40, __ldg(F.dnpp + c));
+  put(41, __ldg(F.gmu0 + c));
   tr[5 * SN] = 0.f;
   tr[6 * SN] = 0.f;
 #pragma unroll
   for (int l = 0; l < NL; ++l) {
     const int f = 51 + 5 * l;
-    put(f, F.dt[l * SN + c]);
-    put(f + 1, F.du[l * SN + c]);
-    put(f + 2, F.dv[l * SN + c]);
-    put(f + 4, F.dcc[l * SN + c]);
+    put(f, __ldg(F.dt + l * SN + c));
+    put(f + 1, __ldg(F.du + l * SN + c));
+    put(f + 2, __ldg(F.dv + l * SN + c));
+    put(f + 4, __ldg(F.dcc + l * SN + c));
   }
-  put(42, F.capen[c]);
-  put(43, F.lnb[c]);
-  put(44, F.mpoti[c]);
-  put(45, F.chim[c]);
-  put(46, F.laav[c]);
-  put(47, F.venti[c]);
-  put(48, F.vrmpi[c]);
-  put(49, F.gpi[c]);
-  put(50, F.shear[c]);
+  put(42, __ldg(F.capen + c));
+  put(43, __ldg(F.lnb + c));
+  put(44, __ldg(F.mpoti + c));
+  put(45, __ldg(F.chim + c));
+  put(46, __ldg(F.laav + c));
+  put(47, __ldg(F.venti + c));
+  put(48, __ldg(F.vrmpi + c));
+  put(49, __ldg(F.gpi + c));
+  put(50, __ldg(F.shear + c));
   const int lowest = NL - 1;
-  const float qsat = sat_divided(K, F.dt[lowest * SN + c], F.dp[c] * K.SIGMA_LOW);
-  put(51 + 5 * lowest + 3, fmaxf(0.f, F.dq[lowest * SN + c]) / fmaxf(1.17549435e-38f, qsat));
+  const float qsat = sat_divided(K, __ldg(F.dt + lowest * SN + c), __ldg(F.dp + c) * K.SIGMA_LOW);
+  put(51 + 5 * lowest + 3, fmaxf(0.f, __ldg(F.dq + lowest * SN + c)) / fmaxf(1.17549435e-38f, qsat));
 }
 
 // Non-finite check per slot over the prognostic spectral state: sets
@@ -2012,11 +2051,6 @@ __global__ void __launch_bounds__(kBlock, 4) k_fused_kuo_mkdca(Model m, const Pl
   b_mkdca<NL>(m, pcr, tabr);
 }
 template <int NL>
-__global__ void __launch_bounds__(kBlock) k_fused_rain_soil(Model m, const PlanetConst* pcr, const float* tabr) {
-  b_rain_column<NL>(m, pcr, tabr);
-  b_soil<NL>(m, pcr, tabr);
-}
-template <int NL>
 __global__ void __launch_bounds__(kBlock) k_fused_land_seaice(Model m, const PlanetConst* __restrict__ pcr,
                                                               const float* __restrict__ tabr) {
   b_land_surface<NL>(m, pcr, tabr);
@@ -2032,13 +2066,12 @@ __global__ void __launch_bounds__(kBlock) k_fused_sea_carbon(Model m, const Plan
 
 COLUMN_LAUNCHER(FixerColumn, k_fixer_column)
 COLUMN_LAUNCHER(FusedKuoMkdca, k_fused_kuo_mkdca)
-COLUMN_LAUNCHER(FusedRainSoil, k_fused_rain_soil)
 COLUMN_LAUNCHER(FusedLandSeaice, k_fused_land_seaice)
 COLUMN_LAUNCHER(FusedSeaCarbon, k_fused_sea_carbon)
 template <int NL>
 struct Swr {
   static void run(const Model& m, cudaStream_t st) {
-    k_swr<NL><<<nblocks((size_t)m.d.S * m.d.NHOR, kBlock / 2), kBlock, 0, st>>>(m);
+    step_launch(m.pdl, k_swr<NL>, nblocks((size_t)m.d.S * m.d.NHOR, kBlock / 2), kBlock, 0, st, m);
   }
 };
 COLUMN_LAUNCHER(LwrRadstep, k_lwr_radstep)
@@ -2055,7 +2088,7 @@ COLUMN_LAUNCHER(Pack, k_pack)
 template <int NL>
 struct FixerRow {
   static void run(const Model& m, cudaStream_t st) {
-    k_fixer_row<NL><<<nblocks((size_t)m.d.S * m.d.NLAT, kRowWarps), 32 * kRowWarps, 0, st>>>(m);
+    step_launch(m.pdl, k_fixer_row<NL>, nblocks((size_t)m.d.S * m.d.NLAT, kRowWarps), 32 * kRowWarps, 0, st, m);
   }
 };
 
@@ -2064,7 +2097,7 @@ struct FixerRow {
 void phy_fixer(const Model& m, cudaStream_t st) {
   by_levels<FixerColumn>(m.d.L, m, st);
   by_levels<FixerRow>(m.d.L, m, st);
-  k_slot_sums<<<m.d.S, kSumThreads, 0, st>>>(m, m.f.fixneg, m.f.fixpos, m.f.fixsum, 0);
+  step_launch(m.pdl, k_slot_sums, m.d.S, kSumThreads, 0, st, m, m.f.fixneg, m.f.fixpos, m.f.fixsum, 0);
   phy_fixer_apply(m, st);
 }
 
@@ -2077,16 +2110,16 @@ void phy_radiation(const Model& m, cudaStream_t st) {
 void phy_precipitation_columns(const Model& m, cudaStream_t st) {
   by_levels<Kuo>(m.d.L, m, st);
   by_levels<Mkdca>(m.d.L, m, st);
-  k_mkdca_limit<<<m.d.S, kSumThreads, 0, st>>>(m);
+  step_launch(m.pdl, k_mkdca_limit, m.d.S, kSumThreads, 0, st, m);
   by_levels<RainColumn>(m.d.L, m, st);
 }
 
 void phy_surface(const Model& m, cudaStream_t st) {
   by_levels<Soil>(m.d.L, m, st);
-  k_mkradv<<<nblocks((size_t)m.d.S * m.d.NHOR, kBlock), kBlock, 0, st>>>(m);
+  step_launch(m.pdl, k_mkradv, nblocks((size_t)m.d.S * m.d.NHOR, kBlock), kBlock, 0, st, m);
   by_levels<LandSurface>(m.d.L, m, st);
   by_levels<SeaIce>(m.d.L, m, st);
-  k_slot_sums<<<m.d.S, kSumThreads, 0, st>>>(m, m.f.ice_part1, m.f.ice_part2, m.f.ice_sums, 1);
+  step_launch(m.pdl, k_slot_sums, m.d.S, kSumThreads, 0, st, m, m.f.ice_part1, m.f.ice_part2, m.f.ice_sums, 1);
   by_levels<Sea>(m.d.L, m, st);
 }
 
@@ -2109,9 +2142,9 @@ void phy_fused_through_radiation(const Model& m, cudaStream_t st) {
 void phy_fused_precipitation_to_carbon(const Model& m, cudaStream_t st) {
   phy_precipitation_columns(m, st);
   by_levels<Soil>(m.d.L, m, st);
-  k_mkradv<<<nblocks((size_t)m.d.S * m.d.NHOR, kBlock), kBlock, 0, st>>>(m);
+  step_launch(m.pdl, k_mkradv, nblocks((size_t)m.d.S * m.d.NHOR, kBlock), kBlock, 0, st, m);
   by_levels<FusedLandSeaice>(m.d.L, m, st);
-  k_slot_sums<<<m.d.S, kSumThreads, 0, st>>>(m, m.f.ice_part1, m.f.ice_part2, m.f.ice_sums, 1);
+  step_launch(m.pdl, k_slot_sums, m.d.S, kSumThreads, 0, st, m, m.f.ice_part1, m.f.ice_part2, m.f.ice_sums, 1);
   by_levels<FusedSeaCarbon>(m.d.L, m, st);
 }
 
@@ -2152,9 +2185,10 @@ bool phy_launch_one(const Model& m, const std::string& kernel, cudaStream_t st) 
     by_levels<Carbon>(L, m, st);
   else if (kernel == "fused_kuo_mkdca")
     by_levels<FusedKuoMkdca>(L, m, st);
-  else if (kernel == "fused_rain_soil")
-    by_levels<FusedRainSoil>(L, m, st);
-  else if (kernel == "fused_land_seaice")
+  else if (kernel == "fused_rain_soil") {  // the pair as a step runs it
+    by_levels<RainColumn>(L, m, st);
+    by_levels<Soil>(L, m, st);
+  } else if (kernel == "fused_land_seaice")
     by_levels<FusedLandSeaice>(L, m, st);
   else if (kernel == "fused_sea_carbon")
     by_levels<FusedSeaCarbon>(L, m, st);
