@@ -210,7 +210,8 @@ struct Model {
   // field after each stage, so there (zero_gdt = 1) the kernels zero and
   // read them as the reference does.
   int zero_gdt;
-  int pdl;    // transform and dynamics kernels start by programmatic dependent launch
+  int pdl;         // transform, dynamics and reduction kernels start by programmatic dependent launch
+  int column_pdl;  // column-physics kernels do
   // Grid and Fourier scratch of mkdheat's first stage (L planes per slot
   // each; no state field, so a full step can transform both stages' wind
   // increments in one launch).

@@ -86,6 +86,8 @@ struct exogcm_engine {
   int mode = 0;
   int device = 0;
   cudaStream_t stream = nullptr;
+  cudaStream_t side[2] = {};      // side streams a step is captured on (Lanes)
+  cudaEvent_t side_event[2] = {};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float last_ms = 0.f;
   std::vector<FieldInfo> fields;
@@ -168,6 +170,7 @@ struct exogcm_engine {
     m.fzdu1 = m.zdv1 + grid;
     m.fzdv1 = m.fzdu1 + four;
     m.pdl = pdl;
+    m.column_pdl = 1;
     m.storm = 0;
     for (const Slot& s : slots) m.storm |= s.storm ? 1 : 0;
     return m;
@@ -432,18 +435,62 @@ TrSet set_of(const T&... fields) {
 
 constexpr float kPlavor = 1.63299310207f;
 
-void stage_gridpointa(const Model& m, cudaStream_t st) {
+// The streams a step is captured on. Work whose inputs are ready before the
+// main chain needs its results is captured on a side stream between a fork
+// (the side follows what the main stream holds) and a join, so that in the
+// batch graph it runs beside the main chain: a planet's kernels fill a small
+// part of the chip and wait mostly on latency, and a batch's leave it idle in
+// their last waves. Without sides (stage replay) everything runs in order on
+// the main stream. The first kernel after a fork or join has edges from two
+// streams and is launched with full dependencies (`whole`).
+struct Lanes {
+  cudaStream_t main = nullptr;
+  cudaStream_t sides[2] = {};
+  cudaEvent_t events[2] = {};
+  cudaStream_t side(int k) const { return sides[k] ? sides[k] : main; }
+  void fork(int k) const {
+    if (!sides[k]) return;
+    check(cudaEventRecord(events[k], main), "fork");
+    check(cudaStreamWaitEvent(sides[k], events[k], 0), "fork");
+  }
+  void join(int k) const {
+    if (!sides[k]) return;
+    check(cudaEventRecord(events[k], sides[k]), "join");
+    check(cudaStreamWaitEvent(main, events[k], 0), "join");
+  }
+};
+Model whole(Model m) {
+  m.pdl = m.column_pdl = 0;
+  return m;
+}
+
+// `spectral` fields to the grid, beside the winds u, v of sd, sz (launched
+// as `first` says).
+void winds_and_fields(const Model& m, const Model& first, const TrSet& spectral, const Lanes& on) {
+  const FieldPtrs& F = m.f;
+  const int LP = m.d.L * m.d.S;
+  on.fork(0);
+  tr_spectral_part(whole(m), spectral, on.side(0));
+  tr_dv2uv(first, set_of(wind_field(F.sd, F.sz, nullptr, F.fgu, F.fgv, LP, kPlavor)), on.main);
+  if (m.mode != 1) on.join(0);
+  tr_grid_part(m.mode != 1 ? whole(m) : m, spectral, set_of(fourier_field(F.fgu, F.gu, LP), fourier_field(F.fgv, F.gv, LP)),
+               on.main);
+  if (m.mode == 1) on.join(0);
+}
+
+void stage_gridpointa(const Model& m, const Lanes& on) {
+  const cudaStream_t st = on.main;
   const Dims& d = m.d;
   const FieldPtrs& F = m.f;
   const int LP = d.L * d.S, SP = d.S;
-  tr_dv2uv(m, set_of(wind_field(F.sd, F.sz, nullptr, F.fgu, F.fgv, LP, kPlavor)), st);
-  tr_to_grid(m,
-             set_of(grid_field(F.st, F.fgt, F.gt, LP), grid_field(F.sd, F.fgd, F.gd, LP),
-                    grid_field(F.sz, F.fgz, F.gz, LP), grid_field(F.sq, F.fgq, F.gq, LP),
-                    grid_field(F.sp, F.fgp, F.gp, SP), grid_field(F.sp, F.fgpmt, F.gpmt, SP, kTrDlambda | kTrKeep),
-                    grid_field(F.sp, F.fgpj, F.gpj, SP, kTrDerivative)),
-             set_of(fourier_field(F.fgu, F.gu, LP), fourier_field(F.fgv, F.gv, LP)), st);
-  dyn_calcgp(m, st);
+  winds_and_fields(m, whole(m),  // the step before ends in a join
+                   set_of(grid_field(F.st, F.fgt, F.gt, LP), grid_field(F.sd, F.fgd, F.gd, LP),
+                          grid_field(F.sz, F.fgz, F.gz, LP), grid_field(F.sq, F.fgq, F.gq, LP),
+                          grid_field(F.sp, F.fgp, F.gp, SP),
+                          grid_field(F.sp, F.fgpmt, F.gpmt, SP, kTrDlambda | kTrKeep),
+                          grid_field(F.sp, F.fgpj, F.gpj, SP, kTrDerivative)),
+                   on);
+  dyn_calcgp(whole(m), st);
   tr_fourier_forward(m,
                      set_of(fourier_field(F.gtn, F.fgtn, LP), fourier_field(F.gqn, F.fgqn, LP),
                             fourier_field(F.gut, F.fgut, LP), fourier_field(F.gvt, F.fgvt, LP),
@@ -451,37 +498,44 @@ void stage_gridpointa(const Model& m, cudaStream_t st) {
                             fourier_field(F.gke, F.fgke, LP), fourier_field(F.guq, F.fguq, LP),
                             fourier_field(F.gvq, F.fgvq, LP), fourier_field(F.gvpp, F.fgvpp, SP)),
                      st);
-  tr_legendre_forward(m, set_of(fourier_field(F.fgvpp, F.spt, SP)), st);
+  on.fork(0);
+  on.fork(1);
   tr_uv2dv(m, set_of(wind_field(F.fgvz, F.fguz, F.fgke, F.sdt, F.szt, LP)), st);
-  tr_qtend(m,
+  tr_qtend(whole(m),
            set_of(wind_field(F.fgut, F.fgvt, F.fgtn, F.stt, nullptr, LP),
                   wind_field(F.fguq, F.fgvq, F.fgqn, F.sqt, nullptr, LP)),
-           st);
+           on.side(0));
+  tr_legendre_forward(whole(m), set_of(fourier_field(F.fgvpp, F.spt, SP)), on.side(1));
+  on.join(0);
+  on.join(1);
 }
 
-void stage_physics_in(const Model& m, cudaStream_t st) {
+void stage_physics_in(const Model& m, const Lanes& on) {
   const Dims& d = m.d;
   const FieldPtrs& F = m.f;
   const int LP = d.L * d.S, SP = d.S;
-  tr_dv2uv(m, set_of(wind_field(F.sd, F.sz, nullptr, F.fgu, F.fgv, LP, kPlavor)), st);
-  tr_to_grid(m,
-             set_of(grid_field(F.st, F.fgt, F.gt, LP), grid_field(F.sq, F.fgq, F.gq, LP),
-                    grid_field(F.sp, F.fgp, F.gp, SP)),
-             set_of(fourier_field(F.fgu, F.gu, LP), fourier_field(F.fgv, F.gv, LP)), st);
-  dyn_physics_in(m, st);
+  winds_and_fields(m, m,
+                   set_of(grid_field(F.st, F.fgt, F.gt, LP), grid_field(F.sq, F.fgq, F.gq, LP),
+                          grid_field(F.sp, F.fgp, F.gp, SP)),
+                   on);
+  dyn_physics_in(whole(m), on.main);
 }
 
 // The humidity tendency the precipitation reads.
 void precipitation_dqt(const Model& m, cudaStream_t st) {
-  tr_to_grid(m, set_of(grid_field(m.f.sqt, m.f.fdqt, m.f.dqt, m.d.L * m.d.S)), TrSet{}, st);
+  const TrSet s = set_of(grid_field(m.f.sqt, m.f.fdqt, m.f.dqt, m.d.L * m.d.S));
+  tr_spectral_part(m, s, st);
+  tr_grid_part(m, s, TrSet{}, st);
 }
 
 void stage_precipitation(const Model& m, cudaStream_t st) {
   precipitation_dqt(m, st);
-  phy_precipitation_columns(m, st);
+  phy_kuo(m, st);
+  phy_dca_rain(m, st);
 }
 
-void stage_physics_out(const Model& m, cudaStream_t st) {
+void stage_physics_out(const Model& m, const Lanes& on) {
+  const cudaStream_t st = on.main;
   const int LP = m.d.L * m.d.S;
   const FieldPtrs& F = m.f;
   dyn_physics_out(m, st);
@@ -489,18 +543,21 @@ void stage_physics_out(const Model& m, cudaStream_t st) {
                      set_of(fourier_field(F.gtdt, F.fgtdt, LP), fourier_field(F.gudt, F.fgudt, LP),
                             fourier_field(F.gvdt, F.fgvdt, LP), fourier_field(F.gqdt, F.fgqdt, LP)),
                      st);
-  tr_legendre_forward(m, set_of(fourier_field(F.fgtdt, F.stt, LP), fourier_field(F.fgqdt, F.sqt, LP)), st);
+  on.fork(0);
   tr_uv2dv(m, set_of(wind_field(F.fgudt, F.fgvdt, nullptr, F.sdt, F.szt, LP)), st);
+  tr_legendre_forward(whole(m), set_of(fourier_field(F.fgtdt, F.stt, LP), fourier_field(F.fgqdt, F.sqt, LP)), on.side(0));
+  on.join(0);
 }
 
 // mkdheat's two wind increments come from the diffusion's spectral fields
 // alone, so both are transformed with the winds, friction's into scratch of
 // its own; what its second stage passes to the third is a mean per plane
 // (k_mkdheat_mean), for which only m = 0 of the kinetic energy is kept.
-void stage_spectrald(const Model& m, cudaStream_t st) {
+void stage_spectrald(const Model& m, const Lanes& on) {
+  const cudaStream_t st = on.main;
   const int LP = m.d.L * m.d.S;
   const FieldPtrs& F = m.f;
-  dyn_spectrald_diffusion(m, st);
+  dyn_spectrald_diffusion(whole(m), st);
   tr_dv2uv(m,
            set_of(wind_field(F.sdp, F.szp, nullptr, F.fzu, F.fzv, LP, kPlavor),
                   wind_field(F.zdsdp1, F.zdszp1, nullptr, m.fzdu1, m.fzdv1, LP),
@@ -512,20 +569,26 @@ void stage_spectrald(const Model& m, cudaStream_t st) {
                             fourier_field(F.fzdu, F.zdu, LP), fourier_field(F.fzdv, F.zdv, LP)),
                      st);
   dyn_mkdheat_winds(m, st);
-  tr_fourier_forward(m, set_of(fourier_field(F.zdtdt, F.fzdtdt, LP), fourier_field(F.zdekin, F.fzdekin, LP, 1)), st);
-  tr_legendre_forward(m, set_of(fourier_field(F.fzdtdt, F.zstt1, LP)), st);
+  // friction's heating goes through the scratch fzdu1, spent by now: its
+  // forward Legendre sums run beside the third stage's transforms
+  tr_fourier_forward(m, set_of(fourier_field(F.zdtdt, m.fzdu1, LP), fourier_field(F.zdekin, F.fzdekin, LP, 1)), st);
+  on.fork(0);
+  tr_legendre_forward(whole(m), set_of(fourier_field(m.fzdu1, F.zstt1, LP)), on.side(0));
   dyn_mkdheat_mean(m, st);
   // the mean's Fourier field, kept on the plain path and by stage replay
   if (m.mode == 0 || m.keep_fourier) tr_legendre_inverse(m, set_of(fourier_field(F.zsdef, F.fzdekin, LP)), st);
   tr_fourier_forward(m, set_of(fourier_field(F.zdtdt, F.fzdtdt, LP)), st);
   tr_legendre_forward(m, set_of(fourier_field(F.fzdtdt, F.zstt2, LP)), st);
-  dyn_spectrald_update(m, st);
+  on.join(0);
+  dyn_spectrald_update(whole(m), st);
 }
 
 void run_stage(const Model& m, const std::string& s, cudaStream_t st) {
-  if (s == "gridpointa") stage_gridpointa(m, st);
+  Lanes on;
+  on.main = st;
+  if (s == "gridpointa") stage_gridpointa(m, on);
   else if (s == "spectrala") dyn_spectrala(m, st);
-  else if (s == "physics_in") stage_physics_in(m, st);
+  else if (s == "physics_in") stage_physics_in(m, on);
   else if (s == "fixer") phy_fixer(m, st);
   else if (s == "surface_flux") phy_surface_flux(m, st);
   else if (s == "radiation") phy_radiation(m, st);
@@ -533,28 +596,49 @@ void run_stage(const Model& m, const std::string& s, cudaStream_t st) {
   else if (s == "surface") phy_surface(m, st);
   else if (s == "carbon") phy_carbon(m, st);
   else if (s == "storm") phy_storm(m, st);
-  else if (s == "physics_out") stage_physics_out(m, st);
-  else if (s == "spectrald") stage_spectrald(m, st);
+  else if (s == "physics_out") stage_physics_out(m, on);
+  else if (s == "spectrald") stage_spectrald(m, on);
   else if (s == "pack") phy_pack(m, st);
   else throw Error(EXOGCM_EINVAL, "unknown stage " + s);
 }
 
-// master's step order (stepper/index.ts:148-161).
-// The physics between the per-planet reductions runs as column kernels,
-// fused where that measured faster (physics.cu); exogcm_run_stage runs the
-// same routines stage by stage, unfused.
-void full_step(const Model& m, cudaStream_t st) {
-  stage_gridpointa(m, st);
-  dyn_spectrala(m, st);
-  stage_physics_in(m, st);
-  phy_fused_through_radiation(m, st);
-  precipitation_dqt(m, st);
-  phy_fused_precipitation_to_carbon(m, st);
-  phy_storm(m, st);
-  stage_physics_out(m, st);
-  stage_spectrald(m, st);
-  phy_pack(m, st);
-  phy_budget(m, m.d.P, st);
+// master's step order (stepper/index.ts:148-161), as far as it orders what
+// depends on one another: the humidity tendency's transform runs beside the
+// physics up to kuo, the shortwave beside the surface fluxes and the vertical
+// diffusion (each reads the fixed humidity and writes fields of its own; the
+// longwave's radstep adds to the diffusion's dtdt), and the surface routines,
+// storm diagnostics, snapshot and budgets (which write surface fields and
+// levels only) beside the frame out and the spectral diffusion.
+// The column routines are fused where that measured faster (physics.cu);
+// exogcm_run_stage runs the same routines stage by stage, unfused.
+void full_step(const Model& m, const Lanes& on) {
+  const cudaStream_t st = on.main;
+  stage_gridpointa(m, on);
+  dyn_spectrala(whole(m), st);
+  on.fork(1);
+  precipitation_dqt(whole(m), on.side(1));
+  stage_physics_in(m, on);
+  phy_fixer(m, st);
+  on.fork(0);
+  phy_solang_mko3(whole(m), on.side(0));
+  phy_swr(m, on.side(0));
+  phy_surface_flux(m, st);
+  on.join(0);
+  phy_lwr(whole(m), st);
+  on.join(1);
+  phy_kuo(whole(m), st);
+  phy_dca_rain(m, st);
+  on.fork(1);
+  {
+    const Model side = whole(m);
+    phy_fused_surface_to_carbon(side, on.side(1));
+    phy_storm(side, on.side(1));
+    phy_pack(side, on.side(1));
+    phy_budget(side, m.d.P, on.side(1));
+  }
+  stage_physics_out(m, on);
+  stage_spectrald(m, on);
+  on.join(1);
 }
 
 // The host values of one slot's next step; advances the slot's counters when
@@ -593,12 +677,22 @@ StepParams next_params(Slot& s, int publish_every, bool advance) {
   return p;
 }
 
+Lanes lanes(const exogcm_engine* e) {
+  Lanes on;
+  on.main = e->stream;
+  for (int k = 0; k < 2; ++k) {
+    on.sides[k] = e->side[k];
+    on.events[k] = e->side_event[k];
+  }
+  return on;
+}
+
 cudaGraphExec_t batch_graph(exogcm_engine* e, int K) {
   auto it = e->graphs.find(K);
   if (it != e->graphs.end()) return it->second;
   cudaGraph_t graph;
   check(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed), "capture");
-  for (int k = 0; k < K; ++k) full_step(e->model(k), e->stream);
+  for (int k = 0; k < K; ++k) full_step(e->model(k), lanes(e));
   check(cudaStreamEndCapture(e->stream, &graph), "capture end");
   cudaGraphExec_t exec;
   check(cudaGraphInstantiate(&exec, graph, 0), "graph instantiate");
@@ -849,7 +943,7 @@ void autotune(exogcm_engine* e) {
     for (int pp : {2, 4}) {
       if (grid_sp2gp_smem(d, pp) > kLegSmemLimit) continue;
       t.sp2gp_planes = pp;
-      const float ms = time([&](const Model& m) { tr_to_grid(m, to_grid, TrSet{}, e->stream); });
+      const float ms = time([&](const Model& m) { tr_spectral_part(m, to_grid, e->stream); });
       if (ms < best) best = ms, pick = pp;
     }
     t.sp2gp_planes = pick;
@@ -981,6 +1075,10 @@ int exogcm_create(int truncation, int levels, int slots, int mode, exogcm_engine
     check(cudaMalloc(&e->fault, sizeof(int)), "fault word");
     check(cudaMemset(e->fault, 0, sizeof(int)), "fault word");
     check(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking), "stream");
+    for (int k = 0; k < 2; ++k) {
+      check(cudaStreamCreateWithFlags(&e->side[k], cudaStreamNonBlocking), "stream");
+      check(cudaEventCreateWithFlags(&e->side_event[k], cudaEventDisableTiming), "event");
+    }
     check(cudaEventCreate(&e->ev0), "event");
     check(cudaEventCreate(&e->ev1), "event");
     tr_init();
@@ -1015,6 +1113,10 @@ void exogcm_destroy(exogcm_engine* e) {
   cudaFree(e->wlat64);
   cudaFree(e->flags);
   cudaFree(e->fault);
+  for (int k = 0; k < 2; ++k) {
+    if (e->side_event[k]) cudaEventDestroy(e->side_event[k]);
+    if (e->side[k]) cudaStreamDestroy(e->side[k]);
+  }
   if (e->ev0) cudaEventDestroy(e->ev0);
   if (e->ev1) cudaEventDestroy(e->ev1);
   for (auto& b : e->batch) {
@@ -1759,7 +1861,11 @@ int exogcm_time_kernel(exogcm_engine* e, const char* kernel, int reps, float* ms
       b = LP * (four + spec);
     } else if (k == "sp2gp") {
       // fused sp2fc + fc2gp: the spectral plane in, the grid plane out
-      launch = [&] { tr_to_grid(m, set_of(grid_field(F.st, F.fgt, F.gt, LP)), TrSet{}, e->stream); };
+      launch = [&] {
+        const TrSet s = set_of(grid_field(F.st, F.fgt, F.gt, LP));
+        tr_spectral_part(m, s, e->stream);
+        tr_grid_part(m, s, TrSet{}, e->stream);
+      };
       b = LP * (spec + grid);
     } else if (k == "sp2gp_planes2" || k == "sp2gp_planes4") {
       // the fused transform at a fixed number of planes per pass
@@ -1768,7 +1874,9 @@ int exogcm_time_kernel(exogcm_engine* e, const char* kernel, int reps, float* ms
       launch = [&, pp] {
         Model mp = m;
         mp.tune.sp2gp_planes = pp;
-        tr_to_grid(mp, set_of(grid_field(F.st, F.fgt, F.gt, LP)), TrSet{}, e->stream);
+        const TrSet s = set_of(grid_field(F.st, F.fgt, F.gt, LP));
+        tr_spectral_part(mp, s, e->stream);
+        tr_grid_part(mp, s, TrSet{}, e->stream);
       };
       b = LP * (spec + grid);
     } else if (k == "legendre_inverse") {
@@ -1853,7 +1961,7 @@ int exogcm_graph_launches(exogcm_engine* e, int steps, size_t* launches) {
     if (!e || !launches || steps < 1 || steps > kMaxBatch) throw Error(EXOGCM_EINVAL, "bad argument");
     cudaGraph_t graph;
     check(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed), "capture");
-    for (int k = 0; k < steps; ++k) full_step(e->model(k), e->stream);
+    for (int k = 0; k < steps; ++k) full_step(e->model(k), lanes(e));
     check(cudaStreamEndCapture(e->stream, &graph), "capture end");
     size_t n = 0;
     check(cudaGraphGetNodes(graph, nullptr, &n), "graph nodes");

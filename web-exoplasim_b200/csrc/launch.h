@@ -62,8 +62,11 @@ void tr_legendre_inverse(const Model& m, TrSet s, cudaStream_t st);
 // sp2fc then fc2gp of each field of `s` (a spectral, x the Fourier field
 // between them - on the optimized path written only when m.keep_fourier or
 // kTrKeep - and y the grid field; opt: kTr*), and fc2gp of each field of
-// `fourier` (a Fourier, x grid).
-void tr_to_grid(const Model& m, TrSet s, TrSet fourier, cudaStream_t st);
+// `fourier` (a Fourier, x grid), in two parts: the first takes the spectral
+// fields as far as they go alone (mode 1: to the grid; else to Fourier
+// space), the second the rest.
+void tr_spectral_part(const Model& m, const TrSet& s, cudaStream_t st);
+void tr_grid_part(const Model& m, const TrSet& s, TrSet fourier, cudaStream_t st);
 // dv2uv: a D, b zeta, x u, y v (Fourier), plavor.
 void tr_dv2uv(const Model& m, TrSet s, cudaStream_t st);
 // fc2sp: a Fourier, x spectral.
@@ -134,15 +137,17 @@ bool phy_flux_launch_one(const Model& m, const std::string& kernel, cudaStream_t
 void phy_fixer(const Model& m, cudaStream_t st);
 void phy_surface_flux(const Model& m, cudaStream_t st);
 void phy_radiation(const Model& m, cudaStream_t st);
-void phy_precipitation_columns(const Model& m, cudaStream_t st);
+void phy_kuo(const Model& m, cudaStream_t st);
+void phy_dca_rain(const Model& m, cudaStream_t st);  // mkdca, its limit, rain and clouds
 void phy_surface(const Model& m, cudaStream_t st);
 void phy_carbon(const Model& m, cudaStream_t st);
 // hurricanestep (physics/storm/wgsl/storm.wgsl), for slots with NSTORMDIAG > 0.
 void phy_storm(const Model& m, cudaStream_t st);
-// The full step's fused physics (see physics.cu): fixer through radiation,
-// and (after the precipitation transform) precipitation through carbon.
-void phy_fused_through_radiation(const Model& m, cudaStream_t st);
-void phy_fused_precipitation_to_carbon(const Model& m, cudaStream_t st);
+// The full step's radiation in two parts, and its surface routines, fused
+// where that measured faster (see physics.cu).
+void phy_swr(const Model& m, cudaStream_t st);
+void phy_lwr(const Model& m, cudaStream_t st);
+void phy_fused_surface_to_carbon(const Model& m, cudaStream_t st);
 void phy_pack(const Model& m, cudaStream_t st);
 
 // budget.cu: per-slot FP64 global budgets and the snapshot's running sums

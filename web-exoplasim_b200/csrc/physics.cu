@@ -2103,12 +2103,13 @@ void phy_fixer(const Model& m, cudaStream_t st) {
 
 void phy_radiation(const Model& m, cudaStream_t st) {
   phy_solang_mko3(m, st);
-  by_levels<Swr>(m.d.L, m, st);
-  by_levels<LwrRadstep>(m.d.L, m, st);
+  phy_swr(m, st);
+  phy_lwr(m, st);
 }
 
-void phy_precipitation_columns(const Model& m, cudaStream_t st) {
-  by_levels<Kuo>(m.d.L, m, st);
+void phy_kuo(const Model& m, cudaStream_t st) { by_levels<Kuo>(m.d.L, m, st); }
+
+void phy_dca_rain(const Model& m, cudaStream_t st) {
   by_levels<Mkdca>(m.d.L, m, st);
   step_launch(m.pdl, k_mkdca_limit, m.d.S, kSumThreads, 0, st, m);
   by_levels<RainColumn>(m.d.L, m, st);
@@ -2125,7 +2126,7 @@ void phy_surface(const Model& m, cudaStream_t st) {
 
 void phy_carbon(const Model& m, cudaStream_t st) { by_levels<Carbon>(m.d.L, m, st); }
 
-// The full step's physics between physics_in and physics_out. Fusing
+// The full step's physics. Fusing
 // consecutive per-column routines into one kernel was measured per pair at
 // 128 T42 L10 planets (CUDA events): land surface + sea ice (86.5 against
 // 88.7 us) and sea + carbon (57.7 against 60.2 us) pay and run fused; fixer
@@ -2133,14 +2134,11 @@ void phy_carbon(const Model& m, cudaStream_t st) { by_levels<Carbon>(m.d.L, m, s
 // (199.7 against 180.6 us) and rain + soil (274.0 against 259.5 us) lost more
 // to the fused kernels' register pressure and lower occupancy than they saved
 // in re-reads, and run as separate kernels.
-void phy_fused_through_radiation(const Model& m, cudaStream_t st) {
-  phy_fixer(m, st);
-  phy_surface_flux(m, st);
-  phy_radiation(m, st);
-}
+void phy_swr(const Model& m, cudaStream_t st) { by_levels<Swr>(m.d.L, m, st); }
 
-void phy_fused_precipitation_to_carbon(const Model& m, cudaStream_t st) {
-  phy_precipitation_columns(m, st);
+void phy_lwr(const Model& m, cudaStream_t st) { by_levels<LwrRadstep>(m.d.L, m, st); }
+
+void phy_fused_surface_to_carbon(const Model& m, cudaStream_t st) {
   by_levels<Soil>(m.d.L, m, st);
   step_launch(m.pdl, k_mkradv, nblocks((size_t)m.d.S * m.d.NHOR, kBlock), kBlock, 0, st, m);
   by_levels<FusedLandSeaice>(m.d.L, m, st);

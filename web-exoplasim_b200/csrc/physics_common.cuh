@@ -196,7 +196,7 @@ void by_levels(int L, A&&... a) {
   template <int NL>                                                                                 \
   struct name {                                                                                     \
     static void run(const Model& m, cudaStream_t st) {                                              \
-      pdl_launch(kernel<NL>, nblocks((size_t)m.d.S * m.d.NHOR, kBlock), kBlock, 0, st, m, m.pc, m.tabs); \
+      step_launch(m.column_pdl, kernel<NL>, nblocks((size_t)m.d.S * m.d.NHOR, kBlock), kBlock, 0, st, m, m.pc, m.tabs); \
     }                                                                                               \
   };
 

@@ -288,13 +288,10 @@ static void dlambda(const Model& m, const float* a, float* b, int planes, cudaSt
     step_launch(m.pdl, k_dlambda, grid, 256, 0, st, a, b, n, m.d.NTP1, m.d.NFC);
 }
 
-void tr_to_grid(const Model& m, TrSet s, TrSet fourier, cudaStream_t st) {
-  if (m.mode == 1) {
-    if (fourier.n) fft_inverse(m, fourier, st);
-    return grid_sp2gp(m, s, st);
-  }
+void tr_spectral_part(const Model& m, const TrSet& s, cudaStream_t st) {
+  if (m.mode == 1) return grid_sp2gp(m, s, st);
   // sp2fc of every field that is not another's d/dlambda, then d/dlambda
-  // from the field sharing its spectral input, then fc2gp of everything.
+  // from the field sharing its spectral input
   TrSet inv;
   for (int i = 0; i < s.n; ++i)
     if (!(s.f[i].opt & kTrDlambda)) inv.add(s.f[i]);
@@ -306,14 +303,18 @@ void tr_to_grid(const Model& m, TrSet s, TrSet fourier, cudaStream_t st) {
       if (s.f[k].a == s.f[i].a && !(s.f[k].opt & (kTrDlambda | kTrDerivative))) from = s.f[k].x;
     dlambda(m, from, s.f[i].x, s.f[i].planes, st);
   }
-  for (int i = 0; i < s.n; ++i) {
-    TrField t;
-    t.a = s.f[i].x;
-    t.x = s.f[i].y;
-    t.planes = s.f[i].planes;
-    fourier.add(t);
-  }
-  tr_fourier_inverse(m, fourier, st);
+}
+
+void tr_grid_part(const Model& m, const TrSet& s, TrSet fourier, cudaStream_t st) {
+  if (m.mode != 1)
+    for (int i = 0; i < s.n; ++i) {
+      TrField t;
+      t.a = s.f[i].x;
+      t.x = s.f[i].y;
+      t.planes = s.f[i].planes;
+      fourier.add(t);
+    }
+  if (fourier.n) tr_fourier_inverse(m, fourier, st);
 }
 
 void tr_legendre_inverse(const Model& m, TrSet s, cudaStream_t st) {
