@@ -86,8 +86,6 @@ struct exogcm_engine {
   int mode = 0;
   int device = 0;
   cudaStream_t stream = nullptr;
-  cudaStream_t side[2] = {};      // side streams a step is captured on (Lanes)
-  cudaEvent_t side_event[2] = {};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float last_ms = 0.f;
   std::vector<FieldInfo> fields;
@@ -435,28 +433,50 @@ TrSet set_of(const T&... fields) {
 
 constexpr float kPlavor = 1.63299310207f;
 
-// The streams a step is captured on. Work whose inputs are ready before the
-// main chain needs its results is captured on a side stream between a fork
-// (the side follows what the main stream holds) and a join, so that in the
-// batch graph it runs beside the main chain: a planet's kernels fill a small
-// part of the chip and wait mostly on latency, and a batch's leave it idle in
-// their last waves. Without sides (stage replay) everything runs in order on
-// the main stream. The first kernel after a fork or join has edges from two
-// streams and is launched with full dependencies (`whole`).
-struct Lanes {
-  cudaStream_t main = nullptr;
-  cudaStream_t sides[2] = {};
-  cudaEvent_t events[2] = {};
-  cudaStream_t side(int k) const { return sides[k] ? sides[k] : main; }
-  void fork(int k) const {
-    if (!sides[k]) return;
-    check(cudaEventRecord(events[k], main), "fork");
-    check(cudaStreamWaitEvent(sides[k], events[k], 0), "fork");
+// The chains of a step. Work whose inputs are ready before the main chain
+// needs its results is captured beside it, between a fork (the side follows
+// what the main chain holds then) and a join, so that in the batch graph it
+// runs beside the main chain: a planet's kernels fill a small part of the
+// chip and wait mostly on latency, and a batch's leave it idle in their last
+// waves. The sides need no streams: what the next captured launch depends on
+// is set on the one stream being captured. Without sides (stage replay)
+// everything runs in order. The first kernel after a fork or join depends on
+// another chain than the launch before it and is launched with full
+// dependencies (`whole`).
+class Lanes {
+ public:
+  Lanes(cudaStream_t stream, bool sides) : main(stream), sides_(sides) {}
+  const cudaStream_t main;
+  void fork(int k) {
+    if (sides_) side_[k] = held();
   }
-  void join(int k) const {
-    if (!sides[k]) return;
-    check(cudaEventRecord(events[k], sides[k]), "join");
-    check(cudaStreamWaitEvent(main, events[k], 0), "join");
+  // Launches `work` on side k.
+  template <typename F>
+  void beside(int k, F&& work) {
+    if (!sides_) return work(main);
+    const std::vector<cudaGraphNode_t> here = held();
+    hold(side_[k], cudaStreamSetCaptureDependencies);
+    work(main);
+    side_[k] = held();
+    hold(here, cudaStreamSetCaptureDependencies);
+  }
+  void join(int k) {
+    if (sides_) hold(side_[k], cudaStreamAddCaptureDependencies);
+  }
+
+ private:
+  const bool sides_;
+  std::vector<cudaGraphNode_t> side_[2];
+  // What the next launch captured depends on.
+  std::vector<cudaGraphNode_t> held() const {
+    cudaStreamCaptureStatus status;
+    const cudaGraphNode_t* nodes = nullptr;
+    size_t n = 0;
+    check(cudaStreamGetCaptureInfo_v2(main, &status, nullptr, nullptr, &nodes, &n), "capture");
+    return std::vector<cudaGraphNode_t>(nodes, nodes + n);
+  }
+  void hold(std::vector<cudaGraphNode_t> nodes, unsigned how) const {
+    check(cudaStreamUpdateCaptureDependencies(main, nodes.data(), nodes.size(), how), "capture");
   }
 };
 Model whole(Model m) {
@@ -466,11 +486,11 @@ Model whole(Model m) {
 
 // `spectral` fields to the grid, beside the winds u, v of sd, sz (launched
 // as `first` says).
-void winds_and_fields(const Model& m, const Model& first, const TrSet& spectral, const Lanes& on) {
+void winds_and_fields(const Model& m, const Model& first, const TrSet& spectral, Lanes& on) {
   const FieldPtrs& F = m.f;
   const int LP = m.d.L * m.d.S;
   on.fork(0);
-  tr_spectral_part(whole(m), spectral, on.side(0));
+  on.beside(0, [&](cudaStream_t st) { tr_spectral_part(whole(m), spectral, st); });
   tr_dv2uv(first, set_of(wind_field(F.sd, F.sz, nullptr, F.fgu, F.fgv, LP, kPlavor)), on.main);
   if (m.mode != 1) on.join(0);
   tr_grid_part(m.mode != 1 ? whole(m) : m, spectral, set_of(fourier_field(F.fgu, F.gu, LP), fourier_field(F.fgv, F.gv, LP)),
@@ -478,7 +498,7 @@ void winds_and_fields(const Model& m, const Model& first, const TrSet& spectral,
   if (m.mode == 1) on.join(0);
 }
 
-void stage_gridpointa(const Model& m, const Lanes& on) {
+void stage_gridpointa(const Model& m, Lanes& on) {
   const cudaStream_t st = on.main;
   const Dims& d = m.d;
   const FieldPtrs& F = m.f;
@@ -501,16 +521,20 @@ void stage_gridpointa(const Model& m, const Lanes& on) {
   on.fork(0);
   on.fork(1);
   tr_uv2dv(m, set_of(wind_field(F.fgvz, F.fguz, F.fgke, F.sdt, F.szt, LP)), st);
-  tr_qtend(whole(m),
-           set_of(wind_field(F.fgut, F.fgvt, F.fgtn, F.stt, nullptr, LP),
-                  wind_field(F.fguq, F.fgvq, F.fgqn, F.sqt, nullptr, LP)),
-           on.side(0));
-  tr_legendre_forward(whole(m), set_of(fourier_field(F.fgvpp, F.spt, SP)), on.side(1));
+  on.beside(0, [&](cudaStream_t side) {
+    tr_qtend(whole(m),
+             set_of(wind_field(F.fgut, F.fgvt, F.fgtn, F.stt, nullptr, LP),
+                    wind_field(F.fguq, F.fgvq, F.fgqn, F.sqt, nullptr, LP)),
+             side);
+  });
+  on.beside(1, [&](cudaStream_t side) {
+    tr_legendre_forward(whole(m), set_of(fourier_field(F.fgvpp, F.spt, SP)), side);
+  });
   on.join(0);
   on.join(1);
 }
 
-void stage_physics_in(const Model& m, const Lanes& on) {
+void stage_physics_in(const Model& m, Lanes& on) {
   const Dims& d = m.d;
   const FieldPtrs& F = m.f;
   const int LP = d.L * d.S, SP = d.S;
@@ -534,7 +558,7 @@ void stage_precipitation(const Model& m, cudaStream_t st) {
   phy_dca_rain(m, st);
 }
 
-void stage_physics_out(const Model& m, const Lanes& on) {
+void stage_physics_out(const Model& m, Lanes& on) {
   const cudaStream_t st = on.main;
   const int LP = m.d.L * m.d.S;
   const FieldPtrs& F = m.f;
@@ -545,7 +569,9 @@ void stage_physics_out(const Model& m, const Lanes& on) {
                      st);
   on.fork(0);
   tr_uv2dv(m, set_of(wind_field(F.fgudt, F.fgvdt, nullptr, F.sdt, F.szt, LP)), st);
-  tr_legendre_forward(whole(m), set_of(fourier_field(F.fgtdt, F.stt, LP), fourier_field(F.fgqdt, F.sqt, LP)), on.side(0));
+  on.beside(0, [&](cudaStream_t side) {
+    tr_legendre_forward(whole(m), set_of(fourier_field(F.fgtdt, F.stt, LP), fourier_field(F.fgqdt, F.sqt, LP)), side);
+  });
   on.join(0);
 }
 
@@ -553,7 +579,7 @@ void stage_physics_out(const Model& m, const Lanes& on) {
 // alone, so both are transformed with the winds, friction's into scratch of
 // its own; what its second stage passes to the third is a mean per plane
 // (k_mkdheat_mean), for which only m = 0 of the kinetic energy is kept.
-void stage_spectrald(const Model& m, const Lanes& on) {
+void stage_spectrald(const Model& m, Lanes& on) {
   const cudaStream_t st = on.main;
   const int LP = m.d.L * m.d.S;
   const FieldPtrs& F = m.f;
@@ -573,7 +599,9 @@ void stage_spectrald(const Model& m, const Lanes& on) {
   // forward Legendre sums run beside the third stage's transforms
   tr_fourier_forward(m, set_of(fourier_field(F.zdtdt, m.fzdu1, LP), fourier_field(F.zdekin, F.fzdekin, LP, 1)), st);
   on.fork(0);
-  tr_legendre_forward(whole(m), set_of(fourier_field(m.fzdu1, F.zstt1, LP)), on.side(0));
+  on.beside(0, [&](cudaStream_t side) {
+    tr_legendre_forward(whole(m), set_of(fourier_field(m.fzdu1, F.zstt1, LP)), side);
+  });
   dyn_mkdheat_mean(m, st);
   // the mean's Fourier field, kept on the plain path and by stage replay
   if (m.mode == 0 || m.keep_fourier) tr_legendre_inverse(m, set_of(fourier_field(F.zsdef, F.fzdekin, LP)), st);
@@ -584,8 +612,7 @@ void stage_spectrald(const Model& m, const Lanes& on) {
 }
 
 void run_stage(const Model& m, const std::string& s, cudaStream_t st) {
-  Lanes on;
-  on.main = st;
+  Lanes on(st, false);
   if (s == "gridpointa") stage_gridpointa(m, on);
   else if (s == "spectrala") dyn_spectrala(m, st);
   else if (s == "physics_in") stage_physics_in(m, on);
@@ -611,17 +638,19 @@ void run_stage(const Model& m, const std::string& s, cudaStream_t st) {
 // levels only) beside the frame out and the spectral diffusion.
 // The column routines are fused where that measured faster (physics.cu);
 // exogcm_run_stage runs the same routines stage by stage, unfused.
-void full_step(const Model& m, const Lanes& on) {
+void full_step(const Model& m, Lanes& on) {
   const cudaStream_t st = on.main;
   stage_gridpointa(m, on);
   dyn_spectrala(whole(m), st);
   on.fork(1);
-  precipitation_dqt(whole(m), on.side(1));
+  on.beside(1, [&](cudaStream_t side) { precipitation_dqt(whole(m), side); });
   stage_physics_in(m, on);
   phy_fixer(m, st);
   on.fork(0);
-  phy_solang_mko3(whole(m), on.side(0));
-  phy_swr(m, on.side(0));
+  on.beside(0, [&](cudaStream_t side) {
+    phy_solang_mko3(whole(m), side);
+    phy_swr(m, side);
+  });
   phy_surface_flux(m, st);
   on.join(0);
   phy_lwr(whole(m), st);
@@ -629,13 +658,13 @@ void full_step(const Model& m, const Lanes& on) {
   phy_kuo(whole(m), st);
   phy_dca_rain(m, st);
   on.fork(1);
-  {
-    const Model side = whole(m);
-    phy_fused_surface_to_carbon(side, on.side(1));
-    phy_storm(side, on.side(1));
-    phy_pack(side, on.side(1));
-    phy_budget(side, m.d.P, on.side(1));
-  }
+  on.beside(1, [&](cudaStream_t side) {
+    const Model off = whole(m);
+    phy_fused_surface_to_carbon(off, side);
+    phy_storm(off, side);
+    phy_pack(off, side);
+    phy_budget(off, m.d.P, side);
+  });
   stage_physics_out(m, on);
   stage_spectrald(m, on);
   on.join(1);
@@ -677,22 +706,13 @@ StepParams next_params(Slot& s, int publish_every, bool advance) {
   return p;
 }
 
-Lanes lanes(const exogcm_engine* e) {
-  Lanes on;
-  on.main = e->stream;
-  for (int k = 0; k < 2; ++k) {
-    on.sides[k] = e->side[k];
-    on.events[k] = e->side_event[k];
-  }
-  return on;
-}
-
 cudaGraphExec_t batch_graph(exogcm_engine* e, int K) {
   auto it = e->graphs.find(K);
   if (it != e->graphs.end()) return it->second;
   cudaGraph_t graph;
   check(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed), "capture");
-  for (int k = 0; k < K; ++k) full_step(e->model(k), lanes(e));
+  Lanes on(e->stream, true);
+  for (int k = 0; k < K; ++k) full_step(e->model(k), on);
   check(cudaStreamEndCapture(e->stream, &graph), "capture end");
   cudaGraphExec_t exec;
   check(cudaGraphInstantiate(&exec, graph, 0), "graph instantiate");
@@ -1075,10 +1095,6 @@ int exogcm_create(int truncation, int levels, int slots, int mode, exogcm_engine
     check(cudaMalloc(&e->fault, sizeof(int)), "fault word");
     check(cudaMemset(e->fault, 0, sizeof(int)), "fault word");
     check(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking), "stream");
-    for (int k = 0; k < 2; ++k) {
-      check(cudaStreamCreateWithFlags(&e->side[k], cudaStreamNonBlocking), "stream");
-      check(cudaEventCreateWithFlags(&e->side_event[k], cudaEventDisableTiming), "event");
-    }
     check(cudaEventCreate(&e->ev0), "event");
     check(cudaEventCreate(&e->ev1), "event");
     tr_init();
@@ -1113,10 +1129,6 @@ void exogcm_destroy(exogcm_engine* e) {
   cudaFree(e->wlat64);
   cudaFree(e->flags);
   cudaFree(e->fault);
-  for (int k = 0; k < 2; ++k) {
-    if (e->side_event[k]) cudaEventDestroy(e->side_event[k]);
-    if (e->side[k]) cudaStreamDestroy(e->side[k]);
-  }
   if (e->ev0) cudaEventDestroy(e->ev0);
   if (e->ev1) cudaEventDestroy(e->ev1);
   for (auto& b : e->batch) {
@@ -1961,7 +1973,8 @@ int exogcm_graph_launches(exogcm_engine* e, int steps, size_t* launches) {
     if (!e || !launches || steps < 1 || steps > kMaxBatch) throw Error(EXOGCM_EINVAL, "bad argument");
     cudaGraph_t graph;
     check(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed), "capture");
-    for (int k = 0; k < steps; ++k) full_step(e->model(k), lanes(e));
+    Lanes on(e->stream, true);
+    for (int k = 0; k < steps; ++k) full_step(e->model(k), on);
     check(cudaStreamEndCapture(e->stream, &graph), "capture end");
     size_t n = 0;
     check(cudaGraphGetNodes(graph, nullptr, &n), "graph nodes");
