@@ -170,142 +170,141 @@ __global__ void __launch_bounds__(kBlock, 4) k_calcgp(Model m) {
   F.dp0[c] = K.PSURF * ps;
 }
 
-// spectrala for one real spectral coefficient (dynamics/wgsl/spectrala.wgsl):
-// the Hoskins-Simmons semi-implicit scheme with this slot's bm1 for its phase.
-// At least three resident blocks per SM: with its last pass read ahead, the
-// registers that a looser bound allows measured faster than five blocks.
+// spectrala (dynamics/wgsl/spectrala.wgsl): the Hoskins-Simmons semi-implicit
+// scheme with this slot's bm1 for its phase. A block takes 32 real
+// coefficients, a thread per (coefficient, level): what couples the levels -
+// the g, bm1 and tau products - reads the other levels' values from shared
+// memory and sums them in level order. One thread per coefficient gathered
+// NL^2 values of bm1 by itself with the level columns in 168 registers: one
+// T42 planet's 15 blocks waited for those loads (10 us), 128 planets' ran at
+// three blocks per SM.
+constexpr int kSpecCols = 32;
+
 template <int NL>
-__global__ void __launch_bounds__(kBlock, 3) k_spectrala(Model m) {
+__global__ void __launch_bounds__(kSpecCols* NL) k_spectrala(Model m) {
+  __shared__ float s_stt[NL][kSpecCols], s_atm[NL][kSpecCols], s_adt[NL][kSpecCols], s_adm[NL][kSpecCols];
+  __shared__ float s_zz[NL][kSpecCols], s_sdt[NL][kSpecCols];
   pdl_wait();
   pdl_release();
   const Dims& d = m.d;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.S * d.NRSP) return;
-  const int slot = c / d.NRSP, s = c % d.NRSP;
+  const int lane = threadIdx.x % kSpecCols, l = threadIdx.x / kSpecCols;
+  const int c = blockIdx.x * kSpecCols + lane;
+  const bool inside = c < d.S * d.NRSP;
+  const int slot = inside ? c / d.NRSP : 0, s = inside ? c % d.NRSP : 0;
   const StepParams& P = m.params[slot];
-  if (!P.active) return;
+  const bool run = inside && P.active;
   const PlanetConst& K = m.pc[slot];
   const float* tb = slot_tabs(m, slot);
-  const float* G = tb + m.to.g;
-  const float* t0T = tb + m.to.t0;
-  const float* ds = tb + m.to.dsigma;
-  const float* tau = tb + m.to.tau;
-  const float* bm1 = tb + m.to.bm1 + (size_t)P.phase * d.T * NL * NL;
-  const size_t SR = (size_t)d.S * d.NRSP;
+  const size_t SR = (size_t)d.S * d.NRSP, at = l * SR + c;
   const FieldPtrs& F = m.f;
   const bool filter = P.filter != 0.f;
   const float DELT = P.delt, DELT2 = P.delt2;
-  const float apm = F.spm[c];
-  float adm[NL], azm[NL], atm[NL], aqm[NL], adt[NL], stt[NL];
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    const size_t at = l * SR + c;
-    adm[l] = F.sdm[at];
-    azm[l] = F.szm[at];
-    atm[l] = F.stm[at];
-    aqm[l] = F.sqm[at];
-    adt[l] = F.sdt[at];
-    stt[l] = F.stt[at];
+  float adm = 0.f, azm = 0.f, atm = 0.f, aqm = 0.f, adt = 0.f, stt = 0.f, szt = 0.f, sqt = 0.f;
+  float sdp0 = 0.f, szp0 = 0.f, stp0 = 0.f, sqp0 = 0.f, apm = 0.f, spt = 0.f, spp = 0.f;
+  if (run) {
+    adm = F.sdm[at];
+    azm = F.szm[at];
+    atm = F.stm[at];
+    aqm = F.sqm[at];
+    adt = F.sdt[at];
+    stt = F.stt[at];
+    szt = F.szt[at];
+    sqt = F.sqt[at];
+    if (filter) {
+      sdp0 = F.sdp[at];
+      szp0 = F.szp[at];
+      stp0 = F.stp[at];
+      sqp0 = F.sqp[at];
+    }
+    apm = F.spm[c];
+    spt = F.spt[c];
+    if (l == 0) spp = F.spp[c];
   }
-  float zgt[NL], zgm[NL];
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    float gt = 0.f, gm = 0.f;
+  s_stt[l][lane] = stt;
+  s_atm[l][lane] = atm;
+  s_adt[l][lane] = adt;
+  s_adm[l][lane] = adm;
+  __syncthreads();
+  const int jn = run ? (int)m.sh.nindex[s] : 0;
+  float zz = 0.f;
+  if (run) {
+    const float* G = tb + m.to.g + l * NL;
+    float zgt = 0.f, zgm = 0.f;
 #pragma unroll
     for (int k = 0; k < NL; ++k) {
-      gt = gt + G[l * NL + k] * stt[k];
-      gm = gm + G[l * NL + k] * atm[k];
+      zgt = zgt + G[k] * s_stt[k][lane];
+      zgm = zgm + G[k] * s_atm[k][lane];
     }
-    zgt[l] = gt;
-    zgm[l] = gm;
-  }
-  float spt = F.spt[c];
-  const float spm = apm;
-  const float sop = tb[m.to.sop + s];
-  const int jn = (int)m.sh.nindex[s];
-  float sdt[NL];
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    float zsum = 0.f;
     if (jn > 0) {
       const float zq = 1.f / (float)(jn * (jn + 1));
-#pragma unroll
-      for (int l2 = 0; l2 < NL; ++l2) {
-        const float z0 = t0T[l2];
-        const float zt = zgt[l2] - z0 * spt;
-        const float zm = zgm[l2] + z0 * spm;
-        const float za = adt[l2] * zq + sop;
-        const float zb = adm[l2] * zq;
-        const float zz = zb + DELT * (zm + za + DELT * zt);
-        zsum = zsum + zz * bm1[((jn - 1) * NL + l) * NL + l2];
-      }
+      const float z0 = tb[m.to.t0 + l];
+      const float zt = zgt - z0 * spt;
+      const float zm = zgm + z0 * apm;
+      const float za = adt * zq + tb[m.to.sop + s];
+      const float zb = adm * zq;
+      zz = zb + DELT * (zm + za + DELT * zt);
     }
-    sdt[l] = s < 2 ? 0.f : zsum;
   }
+  s_zz[l][lane] = zz;
+  __syncthreads();
+  float sdt = 0.f;
+  if (run && jn > 0 && s >= 2) {
+    const float* bm1 = tb + m.to.bm1 + (size_t)P.phase * d.T * NL * NL + ((jn - 1) * NL + l) * NL;
+    if constexpr (NL % 2 == 0) {  // every table before bm1 holds an even count then: rows start 8-byte aligned
+      float2 b[NL / 2];
 #pragma unroll
-  for (int l = 0; l < NL; ++l) spt = spt + ds[l] * sdt[l];
+      for (int k = 0; k < NL / 2; ++k) b[k] = __ldg(reinterpret_cast<const float2*>(bm1) + k);
 #pragma unroll
-  for (int l = 0; l < NL; ++l) {
+      for (int k = 0; k < NL / 2; ++k) {
+        sdt = sdt + s_zz[2 * k][lane] * b[k].x;
+        sdt = sdt + s_zz[2 * k + 1][lane] * b[k].y;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < NL; ++k) sdt = sdt + s_zz[k][lane] * __ldg(bm1 + k);
+    }
+  }
+  s_sdt[l][lane] = sdt;
+  __syncthreads();
+  if (!run) return;
+  {
+    const float* tau = tb + m.to.tau + l * NL;
     float t = 0.f;
 #pragma unroll
-    for (int k = 0; k < NL; ++k) t = t + tau[l * NL + k] * sdt[k];
-    stt[l] = stt[l] - t;
+    for (int k = 0; k < NL; ++k) t = t + tau[k] * s_sdt[k][lane];
+    stt = stt - t;
   }
-  const float spp = F.spp[c];
-  if (filter) F.spm[c] = K.PNU21 * spp + K.PNU * apm;
-  const float sppNew = s < 2 ? 0.f : apm - DELT2 * spt;
-  F.spp[c] = sppNew;
-  F.sp[c] = sppNew;
-  F.spt[c] = spt;
-  // The last pass runs in two halves of levels, each reading all its inputs
-  // before its stores: the fields are distinct arrays, but the compiler
-  // cannot prove it and would otherwise wait for each level's loads in turn.
-  constexpr int H = (NL + 1) / 2;
+  if (l == 0) {
+    const float* ds = tb + m.to.dsigma;
+#pragma unroll
+    for (int k = 0; k < NL; ++k) spt = spt + ds[k] * s_sdt[k][lane];
+    if (filter) F.spm[c] = K.PNU21 * spp + K.PNU * apm;
+    const float sppNew = s < 2 ? 0.f : apm - DELT2 * spt;
+    F.spp[c] = sppNew;
+    F.sp[c] = sppNew;
+    F.spt[c] = spt;
+  }
   const float PNU21 = K.PNU21, PNU = K.PNU;
-#pragma unroll
-  for (int h0 = 0; h0 < NL; h0 += H) {
-    float szt_[H], sqt_[H], sdp_[H], szp_[H], stp_[H], sqp_[H];
-#pragma unroll
-    for (int i = 0; i < H; ++i) {
-      const int l = h0 + i;
-      if (l >= NL) break;
-      const size_t at = l * SR + c;
-      szt_[i] = F.szt[at];
-      sqt_[i] = F.sqt[at];
-      if (filter) {
-        sdp_[i] = F.sdp[at];
-        szp_[i] = F.szp[at];
-        stp_[i] = F.stp[at];
-        sqp_[i] = F.sqp[at];
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < H; ++i) {
-      const int l = h0 + i;
-      if (l >= NL) break;
-      const size_t at = l * SR + c;
-      if (filter) {
-        F.sdm[at] = PNU21 * sdp_[i] + PNU * adm[l];
-        F.szm[at] = PNU21 * szp_[i] + PNU * azm[l];
-        F.stm[at] = PNU21 * stp_[i] + PNU * atm[l];
-        F.sqm[at] = PNU21 * sqp_[i] + PNU * aqm[l];
-      }
-      const float sdp = 2.f * sdt[l] - adm[l];
-      const float stp = DELT2 * stt[l] + atm[l];
-      const float szp = DELT2 * szt_[i] + azm[l];
-      const float sqp = DELT2 * sqt_[i] + aqm[l];
-      F.sdt[at] = sdt[l];
-      F.stt[at] = stt[l];
-      F.sdp[at] = sdp;
-      F.stp[at] = stp;
-      F.szp[at] = szp;
-      F.sqp[at] = sqp;
-      F.sd[at] = sdp;
-      F.st[at] = stp;
-      F.sz[at] = szp;
-      F.sq[at] = sqp;
-    }
+  if (filter) {
+    F.sdm[at] = __fmaf_rn(PNU21, sdp0, PNU * adm);
+    F.szm[at] = __fmaf_rn(PNU21, szp0, PNU * azm);
+    F.stm[at] = __fmaf_rn(PNU21, stp0, PNU * atm);
+    F.sqm[at] = __fmaf_rn(PNU21, sqp0, PNU * aqm);
   }
+  const float sdp = 2.f * sdt - adm;
+  const float stp = DELT2 * stt + atm;
+  const float szp = DELT2 * szt + azm;
+  const float sqp = DELT2 * sqt + aqm;
+  F.sdt[at] = sdt;
+  F.stt[at] = stt;
+  F.sdp[at] = sdp;
+  F.stp[at] = stp;
+  F.szp[at] = szp;
+  F.sqp[at] = sqp;
+  F.sd[at] = sdp;
+  F.st[at] = stp;
+  F.sz[at] = szp;
+  F.sq[at] = sqp;
 }
 
 __device__ __forceinline__ float2 ld2(const float* p, size_t i) { return *reinterpret_cast<const float2*>(p + i); }
@@ -648,11 +647,11 @@ void dyn_calcgp(const Model& m, cudaStream_t st) {
     step_launch(m.pdl, k_calcgp<5>, n, kBlock, 0, st, m);
 }
 void dyn_spectrala(const Model& m, cudaStream_t st) {
-  const unsigned n = blocks((size_t)m.d.S * m.d.NRSP, kBlock);
+  const unsigned n = blocks((size_t)m.d.S * m.d.NRSP, kSpecCols);
   if (m.d.L == 10)
-    step_launch(m.pdl, k_spectrala<10>, n, kBlock, 0, st, m);
+    step_launch(m.pdl, k_spectrala<10>, n, kSpecCols * 10, 0, st, m);
   else
-    step_launch(m.pdl, k_spectrala<5>, n, kBlock, 0, st, m);
+    step_launch(m.pdl, k_spectrala<5>, n, kSpecCols * 5, 0, st, m);
 }
 void dyn_spectrald_diffusion(const Model& m, cudaStream_t st) {
   const dim3 grid(blocks((size_t)m.d.S * m.d.NRSP / 2, kBlock), m.d.NLEV);

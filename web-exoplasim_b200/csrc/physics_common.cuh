@@ -182,6 +182,62 @@ __device__ __forceinline__ void diffuse_potential(const float* ds, float* x, con
 }
 
 
+// Clear-sky longwave transmissivity for absorber sums (lwr.wgsl's band fits).
+// Each fit is a power law below its threshold and a logarithm above; both
+// sides are written through one base-2 logarithm of the side's argument,
+// x^y = 2^(y log2 x) and log10 x = log10(2) log2 x, so that the columns of
+// a warp, whichever side they take, share one instruction stream (no
+// divergent branches) and two special-function operations per fit. All
+// power-law arguments are positive.
+__device__ __forceinline__ float lwr_clear_sky(const PlanetConst& K, float sumwv, float sumo3, float sumco2) {
+  const float ZERO = 1.0e-6f, LOG10_2 = 0.30102999566398120f, LN_2 = 0.69314718055994531f;
+  const bool wv1 = sumwv <= 0.01f, wv2 = sumwv <= 2.f, co2 = sumco2 <= 1.f, o3 = sumo3 <= 0.01f;
+  const float lah = fit_log2(sumwv + (wv1 ? 3.59e-5f : 0.01f));
+  const float lth = fit_log2(wv2 ? sumwv + 0.0286f : sumwv - 0.6931f);
+  const float lco = fit_log2(co2 ? sumco2 + 0.01022f : sumco2);
+  const float lo3 = fit_log2(o3 ? sumo3 + 7.0e-5f : sumo3);
+  float ah2o = wv1 ? 0.846f * fit_exp2(0.243f * lah) - K.ZH2O0A : 0.24f * (LOG10_2 * lah) + K.ZAH2OC;
+  if (K.TH2OC > 0.f) ah2o = fminf(ah2o + (1.f - expf(-K.TH2OC * sumwv)), 1.f);
+  const float aco2 = co2 ? 0.0676f * fit_exp2(0.421f * lco) - K.ZCO20 : 0.0546f * (LOG10_2 * lco) + K.ZACO2C;
+  const float th2o = wv2 ? 1.f - (0.832f * fit_exp2(0.26f * lth) - K.ZH2O0)
+                         : fmaxf(0.f, K.ZTH2OC - 0.1196f * (LN_2 * lth));
+  const float ao3 = o3 ? 0.209f * fit_exp2(0.436f * lo3) - K.ZAO30 : 0.0212f * (LOG10_2 * lo3) + K.ZAO3C;
+  return fminf(1.f - ZERO, fmaxf(ZERO, 1.f - ah2o - ao3 - aco2 * th2o));
+}
+
+struct Parcel {
+  float t, q, cor;
+  bool saturated;
+};
+
+// kuo.wgsl's condense: a lifted parcel's two Newton condensation steps.
+__device__ __forceinline__ Parcel condense(const PlanetConst& K, float t0, float q0, float p) {
+  float s = sat_capped(K, t0, p);
+  float cor = 1.f / (1.f - K.MOIST * s);
+  s = s * cor;
+  if (!(s < q0)) return {t0, q0, cor, false};
+  float t = t0, q = q0;
+  const float lcp = (t0 < K.TMELT ? K.ALS : K.ALV) / (K.ACPD * (1.f + K.ADV * q0));
+  for (int i = 0; i < 2; ++i) {
+    if (i == 1) {
+      s = sat_capped(K, t, p);
+      cor = 1.f / (1.f - K.MOIST * s);
+      s = s * cor;
+    }
+    const float dqsdt = K.RA2 * (K.TMELT - K.RA4) * s * cor / ((t - K.RA4) * (t - K.RA4));
+    const float rain = (q - s) / (1.f + lcp * dqsdt);
+    t = t + lcp * rain;
+    q = q - rain;
+  }
+  return {t, q, cor, true};
+}
+
+// |(u, v)| with both squares rounded before the sum (no contraction), the
+// same wherever the speed is formed.
+__device__ __forceinline__ float wind_speed(float u, float v) {
+  return sqrtf(__fadd_rn(__fmul_rn(u, u), __fmul_rn(v, v)));
+}
+
 template <template <int> class Launch, typename... A>
 void by_levels(int L, A&&... a) {
   if (L == 10)

@@ -145,12 +145,6 @@ __global__ void __launch_bounds__(kBlock) k_surflx(Model m, const PlanetConst* _
 // surflx raised the lowest level), -1 decided at run time from zero_gdt.
 // With HOLD = 0 the other levels' tendencies are the constant 0 and need no
 // registers.
-// |(u, v)| with both squares rounded before the sum (no contraction), the
-// same wherever the speed is formed.
-__device__ __forceinline__ float wind_speed(float u, float v) {
-  return sqrtf(__fadd_rn(__fmul_rn(u, u), __fmul_rn(v, v)));
-}
-
 template <int NL, int HOLD = -1>
 __device__ __forceinline__ void b_vdiff(const Model& m, const PlanetConst* __restrict__ pcr, const float* __restrict__ tabr) {
   COLUMN_PROLOGUE
