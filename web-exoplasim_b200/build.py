@@ -9,7 +9,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libexogcm.so")
 SOURCES = ["engine.cu", "transforms.cu", "legendre.cu", "legendre_tc.cu", "fft.cu", "spectral_grid.cu", "dynamics.cu",
-           "physics.cu", "physics_flux.cu", "physics_storm.cu", "budget.cu", "noalloc.cu", "setup_device.cu", "setup.cpp", "server.cpp"]
+           "physics.cu", "physics_levels.cu", "physics_flux.cu", "physics_storm.cu", "budget.cu", "noalloc.cu", "setup_device.cu", "setup.cpp", "server.cpp"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
          "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
@@ -29,6 +29,7 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std
 # the IEEE division sequence.
 PHYSICS_FLAGS = ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"]
 FILE_FLAGS = {"physics.cu": PHYSICS_FLAGS + ["-DEXOGCM_LWR_FAST_EXP2", "-DEXOGCM_LWR_FAST_LOG2"],
+              "physics_levels.cu": PHYSICS_FLAGS,
               "physics_flux.cu": PHYSICS_FLAGS, "dynamics.cu": ["-prec-div=false"],
               # The FP64 set-up kernels follow the host loops operation for
               # operation and must not contract a*b+c into one rounding.

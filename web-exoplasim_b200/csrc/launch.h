@@ -127,6 +127,12 @@ void dyn_spectrald_update(const Model& m, cudaStream_t st);
 void dyn_physics_in(const Model& m, cudaStream_t st);
 void dyn_physics_out(const Model& m, cudaStream_t st);
 
+// physics_levels.cu: convection and rain with a thread per (column, level),
+// used where phy_levels says so.
+bool phy_levels(const Model& m);
+void lev_rain(const Model& m, cudaStream_t st);
+void lev_kuo(const Model& m, cudaStream_t st);
+
 // physics_flux.cu (IEEE division): fixer apply, surface fluxes, vdiff, solang/mko3
 void phy_fixer_apply(const Model& m, cudaStream_t st);
 void phy_solang_mko3(const Model& m, cudaStream_t st);

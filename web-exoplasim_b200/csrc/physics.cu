@@ -11,12 +11,6 @@
 // The fixer's apply step, the surface fluxes, vertical diffusion, solar
 // angle and ozone are in physics_flux.cu (IEEE division).
 #include "physics_common.cuh"
-#ifndef RAIN_B
-#define RAIN_B 1
-#endif
-#ifndef RAIN_U
-#define RAIN_U 1
-#endif
 
 namespace exogcm {
 
@@ -913,11 +907,13 @@ __global__ void __launch_bounds__(kSumThreads) k_mkdca_limit(Model m) {
 // mkrain's falling fluxes go down the column together, each level's loads one
 // level ahead, and what the later loops need of a level (its relative
 // humidity, temperature, and humidity or height) waits in this thread's
-// column of shared memory. Unrolled, with the level columns in registers, the
-// kernel was 126 registers (16 warps per SM) and mostly waited for
-// instruction fetch at one planet and for memory and fetch at 128.
+// column of shared memory. Fully unrolled, with the level columns in
+// registers, the kernel took 126 registers (16 warps per SM) and waited for
+// memory and instruction fetch; two levels at a time at eight blocks per SM
+// measured fastest (us at 128 T42 L10 planets: 264 -> 193; one level at a time
+// 254, five 245, two at six blocks 197).
 template <int NL>
-__global__ void __launch_bounds__(kBlock, RAIN_B)
+__global__ void __launch_bounds__(kBlock, 8)
     k_rain_column(Model m, const PlanetConst* __restrict__ pcr, const float* __restrict__ tabr) {
   COLUMN_PROLOGUE_STAGED
   __shared__ float s_rh[NL][kBlock], s_t[NL][kBlock], s_q[NL][kBlock];
@@ -946,8 +942,7 @@ __global__ void __launch_bounds__(kBlock, RAIN_B)
     return v;
   };
   Level next = load(0);
-  constexpr int kUnroll = RAIN_U;
-#pragma unroll kUnroll
+#pragma unroll 2
   for (int l = 0; l < NL; ++l) {
     const Level in = next;
     if (l + 1 < NL) next = load(l + 1);
@@ -2027,9 +2022,22 @@ struct Swr {
   }
 };
 COLUMN_LAUNCHER(LwrRadstep, k_lwr_radstep)
-COLUMN_LAUNCHER(Kuo, k_kuo)
+template <int NL>
+struct Kuo {
+  static void run(const Model& m, cudaStream_t st) {
+    if (phy_levels(m)) return lev_kuo(m, st);
+    step_launch(m.column_pdl, k_kuo<NL>, nblocks((size_t)m.d.S * m.d.NHOR, kBlock), kBlock, 0, st, m, m.pc, m.tabs);
+  }
+};
 COLUMN_LAUNCHER(Mkdca, k_mkdca)
-COLUMN_LAUNCHER(RainColumn, k_rain_column)
+template <int NL>
+struct RainColumn {
+  static void run(const Model& m, cudaStream_t st) {
+    if (phy_levels(m)) return lev_rain(m, st);
+    step_launch(m.column_pdl, k_rain_column<NL>, nblocks((size_t)m.d.S * m.d.NHOR, kBlock), kBlock, 0, st, m, m.pc,
+                m.tabs);
+  }
+};
 COLUMN_LAUNCHER(Soil, k_soil)
 COLUMN_LAUNCHER(LandSurface, k_land_surface)
 COLUMN_LAUNCHER(SeaIce, k_sea_ice)
