@@ -580,143 +580,138 @@ __global__ void __launch_bounds__(kBlock, 5) k_lwr_radstep(Model m, const Planet
 }
 
 // ---------------------------------------------------------------- precipitation
-// mkdqtgp scaling, kuo and mkshallow (physics/precipitation/wgsl/kuo.wgsl).
-// Four resident blocks per SM: with the restrict parameters the compiler
-// keeps more values in registers, and four blocks measured faster than six
-// or three.
+// mkdqtgp scaling, kuo and mkshallow (physics/precipitation/wgsl/kuo.wgsl),
+// one thread per column. The level loops stay rolled, the level columns in
+// this thread's column of shared memory ([level][thread], conflict-free), so
+// the code is small - unrolled with 128 registers of level columns the kernel
+// mostly waited for instruction fetch - and a parcel's ascent ends where it
+// stops being buoyant. The incoming tendencies are read again by the columns
+// that change them. A step of 128 T42 L10 planets 3284 -> 3108 us, of 32 T63
+// L10 2063 -> 1987; six blocks per SM measured as seven or eight do, five 25 us
+// slower.
 template <int NL>
-__device__ __forceinline__ void b_kuo(const Model& m, const PlanetConst* __restrict__ pcr, const float* __restrict__ tabr) {
-  COLUMN_PROLOGUE
-  const int NM = NL - 1;
+__global__ void __launch_bounds__(kBlock, 6)
+    k_kuo(Model m, const PlanetConst* __restrict__ pcr, const float* __restrict__ tabr) {
+  COLUMN_PROLOGUE_STAGED
+  __shared__ float s_tot[NL][kBlock], s_qe[NL][kBlock], s_te[NL][kBlock], s_acpe[NL][kBlock];
+  __shared__ float s_dq[NL][kBlock], s_dt[NL][kBlock];  // zdqdt, zdtdt of the cloud's levels
+  constexpr int NM = NL - 1;
+  const int tx = threadIdx.x;
   const float* ds = tb + m.to.dsigma;
   const float* sg = tb + m.to.sigma;
   const float D2 = P.deltsec2;
   const float dp = F.dp[c];
-  float zdqt[NL], zqe[NL], zte[NL], zdqtot[NL], zalcpe[NL], zacpe[NL], zdqdt[NL], zdtdt[NL];
-  // Every field this column reads is loaded before its first store (the
-  // compiler cannot prove the fields distinct, and would otherwise wait for
-  // each later load in turn); dtdt and dqdt stay in registers.
-  float dqt_in[NL], dq_in[NL], dqdt_in[NL], dt_in[NL], dtdt_in[NL];
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    const size_t at = l * SN + c;
-    dqt_in[l] = F.dqt[at];
-    dq_in[l] = F.dq[at];
-    dqdt_in[l] = F.dqdt[at];
-    dt_in[l] = F.dt[at];
-    dtdt_in[l] = F.dtdt[at];
-  }
   const float dt_surface = F.dt[NL * SN + c], dq_surface = F.dq[NL * SN + c];
+  {
+    // every load before the first store (the compiler cannot prove the
+    // fields distinct)
+    float dqt[NL], dq[NL], dqdt[NL], dt[NL], dtdt[NL];
 #pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    const size_t at = l * SN + c;
-    zdqt[l] = dqt_in[l] * K.PSURF * K.WW / dp;
-    F.dqt[at] = zdqt[l];
-    const float dq = dq_in[l], dqdt = dqdt_in[l];
-    zdqtot[l] = (zdqt[l] + dqdt) * D2;
-    zqe[l] = dq + dqdt * D2;
-    zte[l] = dt_in[l] + dtdt_in[l] * D2;
-    zacpe[l] = K.ACPD * (1.f + K.ADV * dq);
-    zalcpe[l] = K.ALV / zacpe[l];
-    zdqdt[l] = 0.f;
-    zdtdt[l] = 0.f;
+    for (int l = 0; l < NL; ++l) {
+      const size_t at = l * SN + c;
+      dqt[l] = F.dqt[at];
+      dq[l] = F.dq[at];
+      dqdt[l] = F.dqdt[at];
+      dt[l] = F.dt[at];
+      dtdt[l] = F.dtdt[at];
+    }
+#pragma unroll
+    for (int l = 0; l < NL; ++l) {
+      const float zdqt = dqt[l] * K.PSURF * K.WW / dp;
+      F.dqt[l * SN + c] = zdqt;
+      s_tot[l][tx] = (zdqt + dqdt[l]) * D2;
+      s_qe[l][tx] = dq[l] + dqdt[l] * D2;
+      s_te[l][tx] = dt[l] + dtdt[l] * D2;
+      s_acpe[l][tx] = K.ACPD * (1.f + K.ADV * dq[l]);
+    }
+  }
+  // The lowest level whose parcel is buoyant: the surface's, then each
+  // level's lifted to the one above.
+  int from = -1;
+  Parcel parcel{0.f, 0.f, 0.f, false};
+  {
+    const float ztsurf = dt_surface * tb[m.to.vdiff_skap + NM];
+    if (s_tot[NM][tx] > 0.f && ztsurf > s_te[NM][tx]) {
+      const float pn = dp * sg[NM];
+      const float zqsnl = sat_divided(K, s_te[NM][tx], pn);
+      const float zqnew = dq_surface * fminf(1.f, s_qe[NM][tx] / zqsnl);
+      parcel = condense(K, ztsurf, zqnew, pn);
+      if (parcel.saturated) from = NM;
+    }
+  }
+#pragma unroll 1
+  for (int l = NM - 1; l >= 0 && from < 0; --l) {
+    if (s_tot[l + 1][tx] > 0.f) {
+      parcel = condense(K, s_te[l + 1][tx] * tb[m.to.kuo_zfac + l], s_qe[l + 1][tx], dp * sg[l]);
+      if (parcel.saturated && parcel.t > s_te[l][tx]) from = l;
+    }
   }
   int ilift = -1, itop = -1;
   float zi = 0.f, zpt = 0.f, zpq = 0.f, zbeta = 0.f, zpbeta = 0.f, ztp = 0.f, zqp = 0.f;
-  {
-    const int n = NL - 1;
-    const float dsn = ds[n];
-    const float ztsurf = dt_surface * tb[m.to.vdiff_skap + n];
-    if (zdqtot[n] > 0.f && ztsurf > zte[n]) {
-      const float p = dp * sg[n];
-      const float zqsnl = sat_divided(K, zte[n], p);
-      const float zqnew = dq_surface * fminf(1.f, zqe[n] / zqsnl);
-      const Parcel parcel = condense(K, ztsurf, zqnew, p);
-      if (parcel.saturated) {
-        ilift = NL + 1;
-        itop = NL;
-        ztp = parcel.t;
-        zqp = parcel.q;
-        const float zqsa = sat_divided(K, zte[n], p);
-        zdqdt[n] = fmaxf(zqsa - zqe[n], 0.f);
-        zdtdt[n] = ztp - zte[n];
-        zpt = zdtdt[n] * dsn * zacpe[n];
-        zpq = zdqdt[n] * dsn * K.ALV;
-        zbeta = fminf(1.f, zqe[n] / zqsa) * dsn;
-        zpbeta = dsn;
-        zi = zdqtot[n] * dsn * K.ALV;
-      }
-    }
-  }
-  // Both level loops are unrolled: a rolled loop would index the per-level
-  // arrays at run time and keep them in local memory.
-#pragma unroll
-  for (int l = NM - 1; l >= 0; --l) {
-    const int lp = l + 1;
-    if (ilift == -1 && zdqtot[lp] > 0.f) {
-      const float p = dp * sg[l];
-      const Parcel parcel = condense(K, zte[lp] * tb[m.to.kuo_zfac + l], zqe[lp], p);
-      if (parcel.saturated && parcel.t > zte[l]) {
-        const float dsl = ds[l], dsp = ds[lp];
-        ilift = l + 2;
-        itop = l + 1;
-        ztp = parcel.t;
-        zqp = parcel.q;
-        const float zqsa = sat_divided(K, zte[l], p);
-        zdqdt[l] = fmaxf(zqsa - zqe[l], 0.f);
-        zdtdt[l] = ztp - zte[l];
-        zpt = zdtdt[l] * dsl * zacpe[l];
-        zpq = zdqdt[l] * dsl * K.ALV;
-        zbeta = fminf(1.f, zqe[l] / zqsa) * dsl;
-        zpbeta = dsl;
-        const float pp = dp * sg[lp];
-        float zqsnl = sat_divided(K, zte[lp], pp);
-        if (zqe[lp] > zqsnl) {
-          float t = zte[lp], q = zqe[lp];
-          const float lcp = (t < K.TMELT ? K.ALS : K.ALV) / (K.ACPD * (1.f + K.ADV * q));
-          float cor = parcel.cor;
-          for (int i = 0; i < 2; ++i) {
-            if (i == 1) {
-              zqsnl = sat_capped(K, t, pp);
-              cor = 1.f / (1.f - K.MOIST * zqsnl);
-              zqsnl = zqsnl * cor;
-            }
-            const float dqsdt = K.RA2 * (K.TMELT - K.RA4) * zqsnl * cor / ((t - K.RA4) * (t - K.RA4));
-            const float rain = (q - zqsnl) / (1.f + lcp * dqsdt);
-            t = t + lcp * rain;
-            q = q - rain;
+  if (from >= 0) {
+    ztp = parcel.t;
+    zqp = parcel.q;
+    const float dsf = ds[from], zqsa = sat_divided(K, s_te[from][tx], dp * sg[from]);
+    ilift = from + 2;
+    itop = from + 1;
+    const float ddq = fmaxf(zqsa - s_qe[from][tx], 0.f), ddt = ztp - s_te[from][tx];
+    s_dq[from][tx] = ddq;
+    s_dt[from][tx] = ddt;
+    zpt = ddt * dsf * s_acpe[from][tx];
+    zpq = ddq * dsf * K.ALV;
+    zbeta = fminf(1.f, s_qe[from][tx] / zqsa) * dsf;
+    zpbeta = dsf;
+    if (from == NM) {
+      zi = s_tot[from][tx] * dsf * K.ALV;
+    } else {
+      const int lp = from + 1;
+      const float dsp = ds[lp], pp = dp * sg[lp];
+      float zqsnl = sat_divided(K, s_te[lp][tx], pp);
+      float pdq = 0.f, pdt = 0.f;
+      if (s_qe[lp][tx] > zqsnl) {
+        float t = s_te[lp][tx], q = s_qe[lp][tx];
+        const float lcp = (t < K.TMELT ? K.ALS : K.ALV) / (K.ACPD * (1.f + K.ADV * q));
+        float cor = parcel.cor;
+        for (int i = 0; i < 2; ++i) {
+          if (i == 1) {
+            zqsnl = sat_capped(K, t, pp);
+            cor = 1.f / (1.f - K.MOIST * zqsnl);
+            zqsnl = zqsnl * cor;
           }
-          zdqdt[lp] = fmaxf(q - zqe[lp], 0.f);
-          zdtdt[lp] = t - zte[lp];
-          zpt = zdtdt[lp] * dsp * zacpe[lp] + zpt;
-          zpq = zdqdt[lp] * dsp * K.ALV + zpq;
-          zbeta = fminf(1.f, zqe[lp] / zqsnl) * dsp + zbeta;
-          zpbeta = dsp + zpbeta;
+          const float dqsdt = K.RA2 * (K.TMELT - K.RA4) * zqsnl * cor / ((t - K.RA4) * (t - K.RA4));
+          const float rain = (q - zqsnl) / (1.f + lcp * dqsdt);
+          t = t + lcp * rain;
+          q = q - rain;
         }
-        zi = zdqtot[l] * dsl * K.ALV + zdqtot[lp] * dsp * K.ALV;
+        pdq = fmaxf(q - s_qe[lp][tx], 0.f);
+        pdt = t - s_te[lp][tx];
+        zpt = pdt * dsp * s_acpe[lp][tx] + zpt;
+        zpq = pdq * dsp * K.ALV + zpq;
+        zbeta = fminf(1.f, s_qe[lp][tx] / zqsnl) * dsp + zbeta;
+        zpbeta = dsp + zpbeta;
       }
+      s_dq[lp][tx] = pdq;
+      s_dt[lp][tx] = pdt;
+      zi = s_tot[from][tx] * dsf * K.ALV + s_tot[lp][tx] * dsp * K.ALV;
     }
   }
-#pragma unroll
-  for (int l = NM - 1; l >= 0; --l) {
-    if (itop == l + 2) {
-      const float p = dp * sg[l];
-      const Parcel parcel = condense(K, ztp * tb[m.to.kuo_zfac + l], zqp, p);
-      if (parcel.saturated && parcel.t > zte[l]) {
-        const float dsl = ds[l];
-        itop = l + 1;
-        ztp = parcel.t;
-        zqp = parcel.q;
-        const float zqsa = sat_divided(K, zte[l], p);
-        zdqdt[l] = fmaxf(zqsa - zqe[l], 0.f);
-        zdtdt[l] = ztp - zte[l];
-        zpt = zdtdt[l] * dsl * zacpe[l] + zpt;
-        zpq = zdqdt[l] * dsl * K.ALV + zpq;
-        zbeta = fminf(1.f, zqe[l] / zqsa) * dsl + zbeta;
-        zpbeta = zpbeta + dsl;
-        zi = zdqtot[l] * dsl * K.ALV + zi;
-      }
-    }
+#pragma unroll 1
+  for (int k = from - 1; k >= 0; --k) {
+    const float p = dp * sg[k];
+    const Parcel up = condense(K, ztp * tb[m.to.kuo_zfac + k], zqp, p);
+    if (!(up.saturated && up.t > s_te[k][tx])) break;
+    const float dsk = ds[k], zqsa = sat_divided(K, s_te[k][tx], p);
+    itop = k + 1;
+    ztp = up.t;
+    zqp = up.q;
+    const float ddq = fmaxf(zqsa - s_qe[k][tx], 0.f), ddt = ztp - s_te[k][tx];
+    s_dq[k][tx] = ddq;
+    s_dt[k][tx] = ddt;
+    zpt = ddt * dsk * s_acpe[k][tx] + zpt;
+    zpq = ddq * dsk * K.ALV + zpq;
+    zbeta = fminf(1.f, s_qe[k][tx] / zqsa) * dsk + zbeta;
+    zpbeta = zpbeta + dsk;
+    zi = s_tot[k][tx] * dsk * K.ALV + zi;
   }
   zi = fmaxf(0.f, zi);
   const float zrhm = zpbeta > 0.f ? zbeta / zpbeta : 0.f;
@@ -726,15 +721,17 @@ __device__ __forceinline__ void b_kuo(const Model& m, const PlanetConst* __restr
   const float zaq = zpq > 0.f ? zi * beta / zpq : 0.f;
   const bool shallow = itop > 0 && (dp * sg[itop - 1] > K.PDEEP || zi <= 0.f);
   float icctot = 0.f;
-#pragma unroll
+#pragma unroll 2
   for (int l = 0; l < NL; ++l) {
     const int level = l + 1;
     const size_t at = l * SN + c;
     float dprcl = 0.f, icclev = 0.f;
     if (ilift >= level && itop <= level && zi > 0.f && !shallow) {
-      F.dqdt[at] = zaq * zdqdt[l] / D2 - zdqt[l];
-      F.dtdt[at] = zat * zdtdt[l] / D2 + dtdt_in[l];
-      dprcl = zat * zdtdt[l] * ds[l] / zalcpe[l] / D2;
+      const float zdqt = F.dqt[at], dtdt_in = F.dtdt[at];
+      const float zalcpe = K.ALV / s_acpe[l][tx];
+      F.dqdt[at] = zaq * s_dq[l][tx] / D2 - zdqt;
+      F.dtdt[at] = zat * s_dt[l][tx] / D2 + dtdt_in;
+      dprcl = zat * s_dt[l][tx] * ds[l] / zalcpe / D2;
     }
     if (dprcl > 0.f) {
       icclev = 1.f;
@@ -747,57 +744,47 @@ __device__ __forceinline__ void b_kuo(const Model& m, const PlanetConst* __restr
   }
   F.icctot[c] = icctot;
   if (!shallow) return;
+  // mkshallow: the exchange coefficients take the place of s_tot (humidity)
+  // and s_acpe (temperature), the solves' scratch that of s_dq.
   const float zkonst1 = K.GA * D2 / K.GASCON;
   const float zkonst2 = K.RKSHALLOW * zkonst1 * K.GA / K.GASCON;
   int kktop = 1;
   for (int level = 2; level <= NM; ++level)
     if (dp * sg[level - 1] < K.PDEEPTH) kktop = level;
   const int ktop = max(itop, kktop);
-  float zkdiff[NL], skap[NL];
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    zkdiff[l] = 0.f;
-    skap[l] = tb[m.to.vdiff_skap + l];
-  }
-#pragma unroll
+#pragma unroll 1
   for (int l = 0; l < NM; ++l) {
     const int lp = l + 1, level = l + 1;
+    const float zte = s_te[l][tx], ztep = s_te[lp][tx];
     const float sigmah = tb[m.to.sigmah + l];
     const float zfac = zkonst2 * sigmah * sigmah * tb[m.to.vdiff_rdsig + l];
     const float dsl = ds[l], dsp = ds[lp];
-    const float zrthl = (dsp + dsl) / (zte[l] * dsp + zte[lp] * dsl);
-    if (level >= ktop && level < ilift) zkdiff[l] = zfac * zrthl * zrthl;
+    const float zrthl = (dsp + dsl) / sum_products(zte, dsp, ztep, dsl);
+    float zkdiff = 0.f;
+    if (level >= ktop && level < ilift) zkdiff = zfac * zrthl * zrthl;
     if (level + 1 == ktop) {
-      float zzqs = sat_capped(K, zte[l], dp * sg[l]);
+      float zzqs = sat_capped(K, zte, dp * sg[l]);
       zzqs = zzqs * (1.f / (1.f - K.MOIST * zzqs));
-      float zzqsp = sat_capped(K, zte[lp], dp * sg[lp]);
+      float zzqsp = sat_capped(K, ztep, dp * sg[lp]);
       zzqsp = zzqsp * (1.f / (1.f - K.MOIST * zzqsp));
-      const float zrh = zqe[l] / zzqs, zrhp = zqe[lp] / zzqsp;
+      const float zrh = s_qe[l][tx] / zzqs, zrhp = s_qe[lp][tx] / zzqsp;
       const float zzf = fabsf((zrh - 0.8f) / 0.2f * (zrhp - zrh));
-      zkdiff[l] = zfac * zrthl * zrthl * zzf;
+      zkdiff = zfac * zrthl * zrthl * zzf;
     }
+    s_tot[l][tx] = zkdiff;
+    s_acpe[l][tx] = zkdiff * tb[m.to.vdiff_skaph + l];
   }
-  float zqn[NL], ztn[NL];
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    zqn[l] = zqe[l];
-    ztn[l] = zte[l];
-  }
-  diffuse<NL>(ds, zqn, zkdiff);
-#pragma unroll
-  for (int l = 0; l < NM; ++l) zkdiff[l] = zkdiff[l] * tb[m.to.vdiff_skaph + l];
-  diffuse_potential<NL>(ds, ztn, zkdiff, skap);
-#pragma unroll
+  diffuse_column<NL, kBlock>(ds, &s_qe[0][tx], &s_tot[0][tx], &s_dq[0][tx]);
+  diffuse_potential_column<NL, kBlock>(ds, &s_te[0][tx], &s_acpe[0][tx], tb + m.to.vdiff_skap, &s_dq[0][tx]);
+#pragma unroll 2
   for (int l = 0; l < NL; ++l) {
     // a shallow column's deep-convection writes above did not run
     const size_t at = l * SN + c;
-    F.dtdt[at] = dtdt_in[l] + (ztn[l] - zte[l]) / D2;
-    F.dqdt[at] = dqdt_in[l] + (zqn[l] - zqe[l]) / D2;
+    const float dtdt_in = F.dtdt[at], dqdt_in = F.dqdt[at];
+    const float zte = F.dt[at] + dtdt_in * D2, zqe = F.dq[at] + dqdt_in * D2;
+    F.dtdt[at] = dtdt_in + (s_te[l][tx] - zte) / D2;
+    F.dqdt[at] = dqdt_in + (s_qe[l][tx] - zqe) / D2;
   }
-}
-template <int NL>
-__global__ void __launch_bounds__(kBlock, 4) k_kuo(Model m, const PlanetConst* __restrict__ pcr, const float* __restrict__ tabr) {
-  b_kuo<NL>(m, pcr, tabr);
 }
 
 
@@ -1992,12 +1979,6 @@ __global__ void k_finite(Model m) {
 // (see phy_fused_precipitation_to_carbon); stage replay (exogcm_run_stage)
 // runs the separate kernels, and a full step equals its stages bit for bit.
 template <int NL>
-__global__ void __launch_bounds__(kBlock, 4) k_fused_kuo_mkdca(Model m, const PlanetConst* __restrict__ pcr,
-                                                               const float* __restrict__ tabr) {
-  b_kuo<NL>(m, pcr, tabr);
-  b_mkdca<NL>(m, pcr, tabr);
-}
-template <int NL>
 __global__ void __launch_bounds__(kBlock) k_fused_land_seaice(Model m, const PlanetConst* __restrict__ pcr,
                                                               const float* __restrict__ tabr) {
   b_land_surface<NL>(m, pcr, tabr);
@@ -2012,7 +1993,6 @@ __global__ void __launch_bounds__(kBlock) k_fused_sea_carbon(Model m, const Plan
 
 
 COLUMN_LAUNCHER(FixerColumn, k_fixer_column)
-COLUMN_LAUNCHER(FusedKuoMkdca, k_fused_kuo_mkdca)
 COLUMN_LAUNCHER(FusedLandSeaice, k_fused_land_seaice)
 COLUMN_LAUNCHER(FusedSeaCarbon, k_fused_sea_carbon)
 template <int NL>
@@ -2141,9 +2121,10 @@ bool phy_launch_one(const Model& m, const std::string& kernel, cudaStream_t st) 
     by_levels<Sea>(L, m, st);
   else if (kernel == "carbon")
     by_levels<Carbon>(L, m, st);
-  else if (kernel == "fused_kuo_mkdca")
-    by_levels<FusedKuoMkdca>(L, m, st);
-  else if (kernel == "fused_rain_soil") {  // the pair as a step runs it
+  else if (kernel == "fused_kuo_mkdca") {  // the pair as a step runs it
+    by_levels<Kuo>(L, m, st);
+    by_levels<Mkdca>(L, m, st);
+  } else if (kernel == "fused_rain_soil") {  // the pair as a step runs it
     by_levels<RainColumn>(L, m, st);
     by_levels<Soil>(L, m, st);
   } else if (kernel == "fused_land_seaice")

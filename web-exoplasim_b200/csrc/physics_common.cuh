@@ -182,6 +182,71 @@ __device__ __forceinline__ void diffuse_potential(const float* ds, float* x, con
 }
 
 
+// a b + c d with the first product fused, as the compiler forms the sums of
+// diffuse and k_kuo that have two products to choose from.
+__device__ __forceinline__ float sum_products(float a, float b, float c, float d) {
+  return __fmaf_rn(a, b, __fmul_rn(c, d));
+}
+
+// The implicit vertical diffusion of one column in shared memory (diffuse,
+// diffuse_potential above): the same solves, the level loop rolled. x and k
+// are the column's levels, STRIDE apart; ebs is scratch.
+template <int NL, int STRIDE>
+__device__ __forceinline__ void diffuse_column(const float* __restrict__ ds, float* x, const float* k, float* ebs) {
+  const float ds0 = ds[0], k0 = k[0];
+  float e = __fdiv_rn(k0, ds0 + k0), v = __fdiv_rn(ds0 * x[0], ds0 + k0), kp = k0;
+  ebs[0] = e;
+  x[0] = v;
+#pragma unroll 1
+  for (int l = 1; l < NL - 1; ++l) {
+    const float kl = k[l * STRIDE];
+    const float den = ds[l] + kl + kp * (1.f - e);
+    e = __fdiv_rn(kl, den);
+    v = __fdiv_rn(sum_products(x[l * STRIDE], ds[l], kp, v), den);
+    ebs[l * STRIDE] = e;
+    x[l * STRIDE] = v;
+    kp = kl;
+  }
+  const float dsn = ds[NL - 1];
+  v = __fdiv_rn(sum_products(x[(NL - 1) * STRIDE], dsn, kp, v), dsn + kp * (1.f - e));
+  x[(NL - 1) * STRIDE] = v;
+#pragma unroll 1
+  for (int l = NL - 2; l >= 0; --l) {
+    v = x[l * STRIDE] + ebs[l * STRIDE] * v;
+    x[l * STRIDE] = v;
+  }
+}
+
+template <int NL, int STRIDE>
+__device__ __forceinline__ void diffuse_potential_column(const float* __restrict__ ds, float* x, const float* k,
+                                                         const float* __restrict__ skap, float* ebs) {
+  const float ds0 = ds[0], k0 = k[0];
+  float e = __fdiv_rn(k0, ds0 + __fdiv_rn(k0, skap[0]));
+  float v = __fdiv_rn(ds0 * x[0], ds0 + __fdiv_rn(k0, skap[0]));
+  float kp = k0;
+  ebs[0] = e;
+  x[0] = v;
+#pragma unroll 1
+  for (int l = 1; l < NL - 1; ++l) {
+    const float kl = k[l * STRIDE], sp = skap[l - 1];
+    const float den = ds[l] + __fdiv_rn(kl + kp * (1.f - __fdiv_rn(e, sp)), skap[l]);
+    e = __fdiv_rn(kl, den);
+    v = __fdiv_rn(sum_products(x[l * STRIDE], ds[l], __fdiv_rn(kp, sp), v), den);
+    ebs[l * STRIDE] = e;
+    x[l * STRIDE] = v;
+    kp = kl;
+  }
+  const int last = NL - 1;
+  const float dsn = ds[last], sp = skap[NL - 2];
+  v = __fdiv_rn(x[last * STRIDE] * dsn + __fdiv_rn(kp * v, sp), dsn + __fdiv_rn(kp, skap[last]) * (1.f - __fdiv_rn(e, sp)));
+  x[last * STRIDE] = v;
+#pragma unroll 1
+  for (int l = NL - 2; l >= 0; --l) {
+    v = x[l * STRIDE] + __fdiv_rn(ebs[l * STRIDE] * v, skap[l + 1]);
+    x[l * STRIDE] = v;
+  }
+}
+
 // Clear-sky longwave transmissivity for absorber sums (lwr.wgsl's band fits).
 // Each fit is a power law below its threshold and a logarithm above; both
 // sides are written through one base-2 logarithm of the side's argument,

@@ -17,12 +17,6 @@ namespace exogcm {
 
 namespace {
 
-// a b + c d with the first product fused, as the compiler forms the sums of
-// diffuse and k_kuo that have two products to choose from.
-__device__ __forceinline__ float sum_products(float a, float b, float c, float d) {
-  return __fmaf_rn(a, b, __fmul_rn(c, d));
-}
-
 constexpr int kCols = 32;  // columns of a block; kCols divides NHOR, so they are of one slot
 
 #define LEVEL_PROLOGUE                                               \
@@ -268,66 +262,7 @@ __global__ void __launch_bounds__(32 * NL)
 }
 
 // ---------------------------------------------------------------- kuo
-// The implicit vertical diffusion of one column in shared memory (diffuse,
-// diffuse_potential in physics_common.cuh): the same solves, the level loop
-// rolled. x and k are the columns' levels, kCols apart; ebs is scratch.
-template <int NL>
-__device__ __forceinline__ void diffuse_column(const float* __restrict__ ds, float* x, const float* k, float* ebs) {
-  const float ds0 = ds[0], k0 = k[0];
-  float e = __fdiv_rn(k0, ds0 + k0), v = __fdiv_rn(ds0 * x[0], ds0 + k0), kp = k0;
-  ebs[0] = e;
-  x[0] = v;
-#pragma unroll 1
-  for (int l = 1; l < NL - 1; ++l) {
-    const float kl = k[l * kCols];
-    const float den = ds[l] + kl + kp * (1.f - e);
-    e = __fdiv_rn(kl, den);
-    v = __fdiv_rn(sum_products(x[l * kCols], ds[l], kp, v), den);
-    ebs[l * kCols] = e;
-    x[l * kCols] = v;
-    kp = kl;
-  }
-  const float dsn = ds[NL - 1];
-  v = __fdiv_rn(sum_products(x[(NL - 1) * kCols], dsn, kp, v), dsn + kp * (1.f - e));
-  x[(NL - 1) * kCols] = v;
-#pragma unroll 1
-  for (int l = NL - 2; l >= 0; --l) {
-    v = x[l * kCols] + ebs[l * kCols] * v;
-    x[l * kCols] = v;
-  }
-}
-
-template <int NL>
-__device__ __forceinline__ void diffuse_potential_column(const float* __restrict__ ds, float* x, const float* k,
-                                                         const float* __restrict__ skap, float* ebs) {
-  const float ds0 = ds[0], k0 = k[0];
-  float e = __fdiv_rn(k0, ds0 + __fdiv_rn(k0, skap[0]));
-  float v = __fdiv_rn(ds0 * x[0], ds0 + __fdiv_rn(k0, skap[0]));
-  float kp = k0;
-  ebs[0] = e;
-  x[0] = v;
-#pragma unroll 1
-  for (int l = 1; l < NL - 1; ++l) {
-    const float kl = k[l * kCols], sp = skap[l - 1];
-    const float den = ds[l] + __fdiv_rn(kl + kp * (1.f - __fdiv_rn(e, sp)), skap[l]);
-    e = __fdiv_rn(kl, den);
-    v = __fdiv_rn(sum_products(x[l * kCols], ds[l], __fdiv_rn(kp, sp), v), den);
-    ebs[l * kCols] = e;
-    x[l * kCols] = v;
-    kp = kl;
-  }
-  const int last = NL - 1;
-  const float dsn = ds[last], sp = skap[NL - 2];
-  v = __fdiv_rn(x[last * kCols] * dsn + __fdiv_rn(kp * v, sp), dsn + __fdiv_rn(kp, skap[last]) * (1.f - __fdiv_rn(e, sp)));
-  x[last * kCols] = v;
-#pragma unroll 1
-  for (int l = NL - 2; l >= 0; --l) {
-    v = x[l * kCols] + __fdiv_rn(ebs[l * kCols] * v, skap[l + 1]);
-    x[l * kCols] = v;
-  }
-}
-
-// b_kuo's routine: every level lifts its own parcel (the surface's in the
+// k_kuo's routine: every level lifts its own parcel (the surface's in the
 // lowest); the first level from below whose parcel is buoyant starts the
 // cloud, which one warp follows up the column; the shallow convection's
 // humidity and temperature are diffused by a warp each.
@@ -527,9 +462,9 @@ __global__ void __launch_bounds__(32 * NL)
   s_kt[l][lane] = l < NM ? zkdiff * tb[m.to.vdiff_skaph + l] : zkdiff;
   __syncthreads();
   if (l == 0 && shallow)
-    diffuse_column<NL>(ds, &s_qe[0][lane], &s_kq[0][lane], &s_pt[0][lane]);
+    diffuse_column<NL, kCols>(ds, &s_qe[0][lane], &s_kq[0][lane], &s_pt[0][lane]);
   else if (l == 1 && shallow)
-    diffuse_potential_column<NL>(ds, &s_te[0][lane], &s_kt[0][lane], tb + m.to.vdiff_skap, &s_pq[0][lane]);
+    diffuse_potential_column<NL, kCols>(ds, &s_te[0][lane], &s_kt[0][lane], tb + m.to.vdiff_skap, &s_pq[0][lane]);
   __syncthreads();
   if (!shallow) return;
   F.dtdt[at] = dtdt_in + (s_te[l][lane] - zte) / D2;
