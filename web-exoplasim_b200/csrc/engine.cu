@@ -113,7 +113,7 @@ struct exogcm_engine {
   // runner/webgpu/gcm.worker.ts:215-225). Batch b uploads its step values
   // from its own pinned row 1 + b, so the host never overwrites values a
   // queued copy has yet to read, and copies the device fault word into its
-  // own pinned int before recording its end event.
+  // own pinned int (k_finite) before recording its end event.
   struct Batch {
     cudaEvent_t start = nullptr, end = nullptr, done = nullptr;
     int* fault_host = nullptr;
@@ -1399,9 +1399,7 @@ int exogcm_step_async(exogcm_engine* e, int steps, int publish_every) {
     check(cudaEventRecord(B.start, e->stream), "event");
     check(cudaGraphLaunch(g, e->stream), "graph launch");
     check(cudaEventRecord(B.end, e->stream), "event");
-    phy_finite_check(e->model(steps - 1), e->stream);
-    check(cudaMemcpyAsync(B.fault_host, e->fault, sizeof(int), cudaMemcpyDeviceToHost, e->stream), "fault word");
-    check(cudaMemsetAsync(e->fault, 0, sizeof(int), e->stream), "fault word");
+    phy_finite_check(e->model(steps - 1), B.fault_host, e->stream);
     // start/end bracket the graph alone (the step time); done marks the
     // fault word's arrival in host memory, after which the batch retires.
     check(cudaEventRecord(B.done, e->stream), "event");
@@ -1485,7 +1483,7 @@ int exogcm_group_step(exogcm_engine** engines, int count, const int* steps, int 
     check(cudaEventRecord(lead->ev0, st), "event");
     check(cudaGraphLaunch(exec, st), "group graph launch");
     check(cudaEventRecord(lead->ev1, st), "event");
-    for (int i = 0; i < count; ++i) phy_finite_check(engines[i]->model(steps[i] - 1), st);
+    for (int i = 0; i < count; ++i) phy_finite_check(engines[i]->model(steps[i] - 1), nullptr, st);
     check(cudaStreamSynchronize(st), "group step");
     float t = 0.f;
     check(cudaEventElapsedTime(&t, lead->ev0, lead->ev1), "event time");

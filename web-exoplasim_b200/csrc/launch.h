@@ -158,7 +158,8 @@ void phy_pack(const Model& m, cudaStream_t st);
 
 // budget.cu: per-slot FP64 global budgets and the snapshot's running sums
 void phy_budget(const Model& m, int snapshot_planes, cudaStream_t st);
-void phy_finite_check(const Model& m, cudaStream_t st);
+// The batch's last check (k_finite); fault_host may be null.
+void phy_finite_check(const Model& m, int* fault_host, cudaStream_t st);
 // One named column kernel of the physics (for timing); false if unknown.
 bool phy_launch_one(const Model& m, const std::string& kernel, cudaStream_t st);
 

@@ -1956,7 +1956,14 @@ __global__ void __launch_bounds__(kBlock) k_pack(Model m, const PlanetConst* __r
 
 // Non-finite check per slot over the prognostic spectral state: sets
 // flags[slot] = 1 when any coefficient of sp, st, sz, sd or sq is NaN or Inf.
-__global__ void k_finite(Model m) {
+// With `fault_host` (pinned host memory) it also hands the batch's fault word
+// over and clears it for the next batch, in place of a copy and a clear behind
+// the batch.
+__global__ void k_finite(Model m, int* fault_host) {
+  if (fault_host && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+    *fault_host = *m.fault;
+    *m.fault = 0;
+  }
   const Dims& d = m.d;
   const int SR = d.S * d.NRSP;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2088,9 +2095,9 @@ void phy_fused_surface_to_carbon(const Model& m, cudaStream_t st) {
 
 void phy_pack(const Model& m, cudaStream_t st) { by_levels<Pack>(m.d.L, m, st); }
 
-void phy_finite_check(const Model& m, cudaStream_t st) {
+void phy_finite_check(const Model& m, int* fault_host, cudaStream_t st) {
   const dim3 grid(nblocks((size_t)m.d.S * m.d.NRSP, 256), m.d.NLEV);
-  k_finite<<<grid, 256, 0, st>>>(m);
+  k_finite<<<grid, 256, 0, st>>>(m, fault_host);
 }
 
 bool phy_launch_one(const Model& m, const std::string& kernel, cudaStream_t st) {
