@@ -51,7 +51,7 @@ inline void pdl_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
 }
 
 // Launches a step kernel, by programmatic dependent launch where `pdl` says
-// so (Model::pdl). Every kernel launched through here calls pdl_wait().
+// so (Model::pdl, Model::column_pdl). Every kernel launched through here calls pdl_wait().
 template <typename... KArgs, typename... Args>
 inline void step_launch(int pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                         Args... args) {

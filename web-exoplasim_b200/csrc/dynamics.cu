@@ -435,21 +435,20 @@ __global__ void __launch_bounds__(kBlock) k_mkdheat_winds(Model m) {
 // order and no transform runs (fc2sp, the zeroing, sp2gp and this stage's
 // read of zdekin took 20 + 8 + 33 + 8 us at 128 T42 L10 planets, and three
 // of a single planet's launches). The slot's first block also writes the
-// spectral field.
-__global__ void __launch_bounds__(kBlock) k_mkdheat_mean(Model m) {
+// spectral field. A block takes `chunks` runs of kCols4 columns of its plane,
+// so that the sum, a chain of NLAT / 2 multiply-adds in one warp, is taken
+// once for all of them.
+__global__ void __launch_bounds__(kBlock) k_mkdheat_mean(Model m, int chunks) {
   constexpr int kMaxPairs = 48;
   __shared__ float pair_sum[kMaxPairs], pair_q[kMaxPairs];
   __shared__ float mean;
   pdl_wait();
   pdl_release();
   const Dims& d = m.d;
-  const int slot = blockIdx.x * kCols4 / d.NHOR;
-  const int c = blockIdx.x * kCols4 + 4 * threadIdx.x;
+  const int first = blockIdx.x * chunks * kCols4;  // the block's columns, all of one slot
+  const int slot = first / d.NHOR;
   const int l = blockIdx.y;
-  const size_t i = (size_t)l * d.S * d.NHOR + c;
-  const int h = c - slot * d.NHOR, lat = h / d.NLON;
   const FieldPtrs& F = m.f;
-  const float4 dq = ld4(F.dq, i), dp = ld4(F.dp, c);
   const size_t plane = (size_t)l * d.S + slot;
   if (threadIdx.x < 32) {
     const float* rows = F.fzdekin + plane * d.NLAT * d.NFC;
@@ -465,25 +464,30 @@ __global__ void __launch_bounds__(kBlock) k_mkdheat_mean(Model m) {
     for (int j = 0; j < half; ++j) s = fmaf(pair_q[j], pair_sum[j], s);
     if (threadIdx.x == 0) mean = s;
   }
-  const float q0 = m.sh.qi[(size_t)lat * d.NCSP];
   const float ds = m.tabs[(size_t)slot * m.to.stride + m.to.dsigma + l];
   const StepParams& P = m.params[slot];
   __syncthreads();
   if (!P.active) return;
   const PlanetConst& K = m.pc[slot];
-  const float s00 = mean, ek = q0 * s00;
-  if (c - 4 * (int)threadIdx.x == slot * d.NHOR) {
+  const float s00 = mean;
+  if (first == slot * d.NHOR) {
     float* out = F.zsdef + plane * d.NRSP;
     for (int r = threadIdx.x; r < d.NRSP; r += kBlock) out[r] = r == 0 ? s00 : 0.f;
   }
-  st4(F.zdekin, i, make_float4(ek, ek, ek, ek));
-  const float4 heat = make_float4(1.f + K.ADV * dq.x, 1.f + K.ADV * dq.y, 1.f + K.ADV * dq.z, 1.f + K.ADV * dq.w);
-  // IEEE divisions, as above.
-  auto one = [&](float ht, float p) {
-    const float dtdt = __fdiv_rn(__fdiv_rn(__fdiv_rn(__fdiv_rn(-ek * 0.5f, K.ACPD), ht), p) * K.GA, ds);
-    return __fdiv_rn(__fdiv_rn(dtdt, K.CT), K.WW);
-  };
-  st4(F.zdtdt, i, make_float4(one(heat.x, dp.x), one(heat.y, dp.y), one(heat.z, dp.z), one(heat.w, dp.w)));
+  for (int k = 0; k < chunks; ++k) {
+    const int c = first + k * kCols4 + 4 * threadIdx.x;
+    const size_t i = (size_t)l * d.S * d.NHOR + c;
+    const float4 dq = ld4(F.dq, i), dp = ld4(F.dp, c);
+    const float ek = m.sh.qi[(size_t)((c - slot * d.NHOR) / d.NLON) * d.NCSP] * s00;
+    st4(F.zdekin, i, make_float4(ek, ek, ek, ek));
+    const float4 heat = make_float4(1.f + K.ADV * dq.x, 1.f + K.ADV * dq.y, 1.f + K.ADV * dq.z, 1.f + K.ADV * dq.w);
+    // IEEE divisions, as above.
+    auto one = [&](float ht, float p) {
+      const float dtdt = __fdiv_rn(__fdiv_rn(__fdiv_rn(__fdiv_rn(-ek * 0.5f, K.ACPD), ht), p) * K.GA, ds);
+      return __fdiv_rn(__fdiv_rn(dtdt, K.CT), K.WW);
+    };
+    st4(F.zdtdt, i, make_float4(one(heat.x, dp.x), one(heat.y, dp.y), one(heat.z, dp.z), one(heat.w, dp.w)));
+  }
 }
 
 // spectrald after mkdheat (dynamics/wgsl/spectrald-update.wgsl), two
@@ -662,8 +666,12 @@ void dyn_mkdheat_winds(const Model& m, cudaStream_t st) {
   step_launch(m.pdl, k_mkdheat_winds, grid, kBlock, 0, st, m);
 }
 void dyn_mkdheat_mean(const Model& m, cudaStream_t st) {
-  const dim3 grid((unsigned)((size_t)m.d.S * m.d.NHOR / kCols4), m.d.NLEV);
-  step_launch(m.pdl, k_mkdheat_mean, grid, kBlock, 0, st, m);
+  // 4 kCols4 = 2,048 divides NHOR; four runs a block once that leaves several
+  // blocks per SM
+  const size_t runs = (size_t)m.d.S * m.d.NHOR / kCols4;
+  const int chunks = runs * m.d.NLEV >= 148 * 32 ? 4 : 1;
+  const dim3 grid((unsigned)(runs / chunks), m.d.NLEV);
+  step_launch(m.pdl, k_mkdheat_mean, grid, kBlock, 0, st, m, chunks);
 }
 void dyn_spectrald_update(const Model& m, cudaStream_t st) {
   const dim3 grid(blocks((size_t)m.d.S * m.d.NRSP / 2, kBlock), m.d.NLEV);

@@ -135,7 +135,6 @@ struct exogcm_engine {
   std::map<int, cudaGraphExec_t> graphs;
   std::map<int, cudaGraph_t> graph_templates;  // the captured K-step graphs (child nodes of group graphs)
   Tuning tune{};
-  int pdl = 0;  // Model::pdl
   SharedSetup shared_setup;  // host copy of the shared tables (set-up of later planets)
   // FP64 set-up loops on this device (setup_device.cu), created at the first
   // configure; exogcm_setup_on_device(e, 0) moves them to the host.
@@ -167,8 +166,17 @@ struct exogcm_engine {
     m.zdv1 = m.zdu1 + grid;
     m.fzdu1 = m.zdv1 + grid;
     m.fzdv1 = m.fzdu1 + four;
-    m.pdl = pdl;
-    m.column_pdl = 1;
+    // Programmatic dependent launch. A dependent's waiting blocks are placed
+    // where there is room while its predecessor drains: that hides the launch,
+    // but packs a grid of one to three blocks per SM unevenly. us a step, column
+    // kernels without / with it, at columns: 8,192 (one T42 L10 planet)
+    // 150.5 / 149.3, 16,384 190 / 196, 18,432 288 / 299, 40,960 260 / 272,
+    // 49,152 266 / 276, 57,344 209 / 202, 131,072 487 / 483, 1,048,576 3109 /
+    // 3090. Everything else has it at every size (75,776 columns 342 -> 319,
+    // 196,608 392 -> 372, 1,048,576 3108 -> 3090).
+    const long columns = (long)d.S * d.NHOR;
+    m.pdl = 1;
+    m.column_pdl = columns <= 8192 || columns > 53248 ? 1 : 0;
     m.storm = 0;
     for (const Slot& s : slots) m.storm |= s.storm ? 1 : 0;
     return m;
@@ -1053,14 +1061,6 @@ int exogcm_create(int truncation, int levels, int slots, int mode, exogcm_engine
     e->d = make_dims(truncation, levels, slots);
     e->mode = mode;
     e->tune = default_tuning(e->d);
-    // Programmatic dependent launch of the transform, dynamics and reduction
-    // kernels while the batch's columns fit the chip about once (148 SMs x 4
-    // blocks x 128 columns): there the launch gap is a good part of a kernel.
-    // Above that a waiting block takes the place of a running one. us a step,
-    // without -> with: 8,192 columns (T42 L10, 1 planet) 236 -> 219, 57,344
-    // (T42 L5, 7) 254 -> 236, 65,536 (T42 L10, 8) 386 -> 384, 131,072 (16)
-    // 577 -> 586, 1,048,576 (128) 3494 -> 3677.
-    e->pdl = (long)slots * e->d.NHOR <= 65536 ? 1 : 0;
     check(cudaGetDevice(&e->device), "device");
     layout(e.get());
     table_layout(e.get());
