@@ -160,12 +160,14 @@ __device__ __forceinline__ float vapour_absorption(float wv, float zsolar2) {
 
 // Per-level state of one swr band for the block's threads, [level][thread]
 // in shared memory: the level loops stay rolled, so both bands' code fits
-// the instruction cache, and the accesses are conflict-free.
+// the instruction cache, and the accesses are conflict-free. Sized by the
+// level count (96 T21 L5 planets 33.9 -> 30.2 us against room for ten levels).
+template <int NL>
 struct SwrLevels {
   float* p;
-  __device__ float& at(int array, int level) const { return p[(array * (MAXLEV + 1) + level) * kBlock + threadIdx.x]; }
-  static constexpr int MAXLEV = 10;
+  __device__ float& at(int array, int level) const { return p[(array * (NL + 1) + level) * kBlock + threadIdx.x]; }
   static constexpr int kArrays = 6;  // tl, rls (NL + 1 levels), tbd, tbu, rb, rbs
+  static constexpr int kFloats = kArrays * (NL + 1) * kBlock;
 };
 
 // One band of swr (physics/radiation/wgsl/swr.wgsl) for one column: ozone
@@ -177,7 +179,7 @@ struct SwrLevels {
 // nalb2, albedo) the column writes.
 template <int NL, int BAND>
 __device__ __forceinline__ void swr_band(const Model& m, const PlanetConst& K, const float* tb, size_t SN, int c,
-                                         float mu0, float ftop, SwrLevels lv, float* fu, float* fd, int stride,
+                                         float mu0, float ftop, SwrLevels<NL> lv, float* fu, float* fd, int stride,
                                          float* alb) {
   enum { TL = 0, RLS = 1, TBD = 2, TBU = 3, RB = 4, RBS = 5 };
   const FieldPtrs& F = m.f;
@@ -351,11 +353,10 @@ template <int NL>
 __global__ void __launch_bounds__(kBlock) k_swr(Model m) {
   pdl_wait();
   pdl_release();
-  static_assert(NL <= SwrLevels::MAXLEV, "swr level state holds at most MAXLEV levels");
   constexpr int NP = NL + 1;
   constexpr int kCols = kBlock / 2;
   __shared__ float sfu[2][NP][kCols], sfd[2][NP][kCols];
-  __shared__ float levels[SwrLevels::kArrays * (SwrLevels::MAXLEV + 1) * kBlock];
+  __shared__ float levels[SwrLevels<NL>::kFloats];
   const Dims& d = m.d;
   const int warp = threadIdx.x >> 5;
   const int band = warp & 1;
@@ -377,7 +378,7 @@ __global__ void __launch_bounds__(kBlock) k_swr(Model m) {
     const float ftop2 = K.ZSOLAR2 * K.GSOL0 * gdist2 * mu0;
     lit = ftop1 + ftop2 > 1.0e-6f;
     if (lit) {
-      const SwrLevels lv{levels};
+      const SwrLevels<NL> lv{levels};
       if (band == 0)
         swr_band<NL, 0>(m, K, tb, SN, c, mu0, ftop1, lv, &sfu[0][0][lc], &sfd[0][0][lc], kCols, alb);
       else
@@ -405,9 +406,10 @@ __global__ void __launch_bounds__(kBlock) k_swr(Model m) {
 
 // lwr (physics/radiation/wgsl/lwr.wgsl) then radstep (radstep.wgsl).
 template <int NL>
-// Five blocks per SM (at most 102 registers): the kernel is latency-bound;
-// five measured faster than six (239 -> 224 us at 128 planets) or seven.
-__global__ void __launch_bounds__(kBlock, 5) k_lwr_radstep(Model m, const PlanetConst* __restrict__ pcr, const float* __restrict__ tabr) {
+// Four blocks per SM, no spills: us at 128, 16 T42 L10 and 32 T63 L10 planets
+// 255, 35.4, 147 against 254, 36.9, 151 at five (48 bytes spilled); two levels
+// of the rolled loop at a time 257, 34.7, 149.
+__global__ void __launch_bounds__(kBlock, 4) k_lwr_radstep(Model m, const PlanetConst* __restrict__ pcr, const float* __restrict__ tabr) {
   COLUMN_PROLOGUE_STAGED
   const int NP = NL + 1;
   const float ZERO = 1.0e-6f, ZFH2O = 0.1f, ZFO3 = 100.f / 2.14f;
