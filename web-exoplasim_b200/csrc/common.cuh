@@ -219,4 +219,36 @@ struct Model {
   int storm;  // some slot runs the storm-climatology diagnostics (NSTORMDIAG > 0)
 };
 
+// physics/fixer/wgsl/column.wgsl: fix0d of one column, whose humidity dq and
+// surface pressure dp the caller holds. dq stays in registers for the stores
+// (a reload after each store would wait for it: the compiler cannot prove the
+// fields distinct).
+#ifdef __CUDACC__
+template <int NL>
+__device__ __forceinline__ void fixer_column(const Model& m, const float* ds, size_t SN, int c, int h,
+                                             const float (&dq)[NL], float dp) {
+  float negative = 0.f, positive = 0.f;
+#pragma unroll
+  for (int l = 0; l < NL; ++l) {
+    const float q = dq[l] * ds[l];
+    if (dq[l] < 0.f) negative = negative + q;
+    if (dq[l] > 0.f) positive = positive + q;
+  }
+  const float zgw = m.sh.zgw[h];
+  float zneg = -negative * dp * zgw;
+  float zpos = positive * dp * zgw;
+  float factor = 1.f;
+  const bool fixed = zneg > 0.f && zpos >= zneg;
+  if (fixed) {
+    factor = (zpos - zneg) / zpos;
+    zneg = 0.f;
+    zpos = zpos * factor;
+  }
+#pragma unroll
+  for (int l = 0; l < NL; ++l) m.f.fixq[l * SN + c] = fixed ? fmaxf(dq[l] * factor, 0.f) : dq[l];
+  m.f.fixneg[c] = zneg;
+  m.f.fixpos[c] = zpos;
+}
+#endif
+
 }  // namespace exogcm

@@ -550,7 +550,9 @@ __global__ void __launch_bounds__(kBlock) k_spectrald_update(Model m) {
 // one thread per column, every input read before the first store. A block's
 // columns share one slot: kBlock divides NHOR. The grid tendencies, and the
 // dimensional ones below the surface level, are zeroed only under
-// single-stage replay (Model::zero_gdt).
+// single-stage replay (Model::zero_gdt); within a full step the fixer's column
+// stage follows here, from the humidity in registers (a kernel of its own read
+// it back: 15 us at 128 T42 L10 planets, and a launch).
 template <int NL>
 __global__ void __launch_bounds__(kBlock) k_physics_in(Model m) {
   pdl_wait();
@@ -566,7 +568,7 @@ __global__ void __launch_bounds__(kBlock) k_physics_in(Model m) {
   const size_t SN = (size_t)d.S * d.NHOR;
   const FieldPtrs& F = m.f;
   const float gp = F.gp[c], rcsq = m.sh.rcsq[h];
-  float gu[NL], gv[NL], gt[NL], gq[NL], t0l[NL];
+  float gu[NL], gv[NL], gt[NL], gq[NL], t0l[NL], dsl[NL], dq[NL];
 #pragma unroll
   for (int l = 0; l < NL; ++l) {
     const size_t at = l * SN + c;
@@ -575,6 +577,7 @@ __global__ void __launch_bounds__(kBlock) k_physics_in(Model m) {
     gt[l] = F.gt[at];
     gq[l] = F.gq[at];
     t0l[l] = t0[l];
+    dsl[l] = m.tabs[(size_t)slot * m.to.stride + m.to.dsigma + l];
   }
   const float dp = PSURF * expf(gp);
   F.dp[c] = dp;
@@ -598,9 +601,11 @@ __global__ void __launch_bounds__(kBlock) k_physics_in(Model m) {
       F.du[at] = CV * gu[l] * scale;
       F.dv[at] = CV * gv[l] * scale;
       F.dt[at] = CT * (gt[l] + t0l[l]);
-      F.dq[at] = gq[l] * PSURF / dp;
+      dq[l] = gq[l] * PSURF / dp;
+      F.dq[at] = dq[l];
     }
   }
+  if (!m.zero_gdt) fixer_column<NL>(m, dsl, SN, c, h, dq, dp);
 }
 
 // gridpointd after the parameterizations (dynamics/wgsl/physics-out.wgsl),

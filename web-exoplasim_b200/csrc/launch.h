@@ -144,7 +144,7 @@ void phy_fixer(const Model& m, cudaStream_t st);
 void phy_surface_flux(const Model& m, cudaStream_t st);
 void phy_radiation(const Model& m, cudaStream_t st);
 void phy_kuo(const Model& m, cudaStream_t st);
-void phy_dca_rain(const Model& m, cudaStream_t st);  // mkdca, its limit, rain and clouds
+void phy_dca_rain(const Model& m, cudaStream_t st);  // mkdca with its limit, rain and clouds
 void phy_surface(const Model& m, cudaStream_t st);
 void phy_carbon(const Model& m, cudaStream_t st);
 // hurricanestep (physics/storm/wgsl/storm.wgsl), for slots with NSTORMDIAG > 0.

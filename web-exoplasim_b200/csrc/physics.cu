@@ -17,134 +17,129 @@ namespace exogcm {
 namespace {
 
 // ---------------------------------------------------------------- fixer
-// physics/fixer/wgsl/column.wgsl: fix0d per column.
+// physics/fixer/wgsl/column.wgsl: fix0d per column (fixer_column in
+// physics_common.cuh). Stage replay's; within a full step physics_in takes it
+// with the humidity it has just formed.
 template <int NL>
 __global__ void __launch_bounds__(kBlock) k_fixer_column(Model m, const PlanetConst* __restrict__ pcr, const float* __restrict__ tabr) {
   COLUMN_PROLOGUE
-  const float* ds = tb + m.to.dsigma;
-  // dq stays in registers for the stores below (a reload after each store
-  // would wait for it: the compiler cannot prove the fields distinct)
-  float dq[NL], negative = 0.f, positive = 0.f;
+  float dq[NL];
 #pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    dq[l] = F.dq[l * SN + c];
-    const float q = dq[l] * ds[l];
-    if (dq[l] < 0.f) negative = negative + q;
-    if (dq[l] > 0.f) positive = positive + q;
-  }
-  const float zgw = m.sh.zgw[h];
-  float zneg = -negative * F.dp[c] * zgw;
-  float zpos = positive * F.dp[c] * zgw;
-  float factor = 1.f;
-  const bool fixed = zneg > 0.f && zpos >= zneg;
-  if (fixed) {
-    factor = (zpos - zneg) / zpos;
-    zneg = 0.f;
-    zpos = zpos * factor;
-  }
-#pragma unroll
-  for (int l = 0; l < NL; ++l) F.fixq[l * SN + c] = fixed ? fmaxf(dq[l] * factor, 0.f) : dq[l];
-  F.fixneg[c] = zneg;
-  F.fixpos[c] = zpos;
+  for (int l = 0; l < NL; ++l) dq[l] = F.dq[l * SN + c];
+  fixer_column<NL>(m, tb + m.to.dsigma, SN, c, h, dq, F.dp[c]);
 }
 
-// physics/fixer/wgsl/row.wgsl: fix1d per latitude row, summed in longitude
-// order. One warp per row: its lanes stage the row in shared memory with
-// coalesced loads, lane 0 adds the values in longitude order (the shader's
-// sums, bit for bit), and the update of a fixed row runs over all lanes.
-constexpr int kRowWarps = 4;
-constexpr int kMaxNlon = 192;  // NLON at T63, the largest truncation an engine accepts
+// The sum of `n` floats at src, src + kSumThreads, ... in FP64, eight in
+// flight, added in order: one at a time, the block waited for memory 32 times
+// in a row at T42 (11 us for two 32 KB sums). n is a multiple of 8 (NHOR is
+// one of 8 kSumThreads).
+__device__ __forceinline__ double strided_sum(const float* src, int n) {
+  constexpr int kAhead = 8;
+  double x = 0.0;
+  for (int k0 = 0; k0 < n; k0 += kAhead) {
+    float v[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) v[k] = src[(k0 + k) * kSumThreads];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) x += (double)v[k];
+  }
+  return x;
+}
 
-template <int NL>
-__global__ void __launch_bounds__(32 * kRowWarps) k_fixer_row(Model m) {
-  pdl_wait();
-  pdl_release();
-  __shared__ float stage[kRowWarps][kMaxNlon];
-  const Dims& d = m.d;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r = blockIdx.x * kRowWarps + warp;
-  if (r >= d.S * d.NLAT) return;  // the whole warp
-  const int slot = r / d.NLAT;
-  if (!m.params[slot].active) return;
-  const size_t SN = (size_t)d.S * d.NHOR;
-  const FieldPtrs& F = m.f;
-  const int first = r * d.NLON;  // slot * NHOR + lat * NLON
-  float* row = stage[warp];
-  auto ordered_sum = [&](const float* src) {
-    for (int j = lane; j < d.NLON; j += 32) row[j] = src[first + j];
-    __syncwarp();
-    float sum = 0.f;
-    if (lane == 0)
-      for (int j = 0; j < d.NLON; ++j) sum = sum + row[j];
-    sum = __shfl_sync(0xffffffffu, sum, 0);
-    __syncwarp();  // the row buffer is staged again next
-    return sum;
-  };
-  const float zneg = ordered_sum(F.fixneg);
-  if (zneg <= 0.f) return;
-  const float zpos = ordered_sum(F.fixpos);
-  if (zpos < zneg) return;
-  const float factor = (zpos - zneg) / zpos;
-  for (int j = lane; j < d.NLON; j += 32) {
-    float q[NL];
-#pragma unroll
-    for (int l = 0; l < NL; ++l) q[l] = F.fixq[l * SN + first + j];
-    const float pos = F.fixpos[first + j];
-#pragma unroll
-    for (int l = 0; l < NL; ++l) F.fixq[l * SN + first + j] = fmaxf(q[l] * factor, 0.f);
-    F.fixneg[first + j] = 0.f;
-    F.fixpos[first + j] = pos * factor;
+// The tree over the block's two halves of kSumThreads partial sums, s[2]:
+// both sums' totals end in s[0][0] and s[1][0].
+__device__ __forceinline__ void tree_sums(double (*s)[kSumThreads], int half, int t, bool in) {
+  __syncthreads();
+  for (int stride = kSumThreads / 2; stride > 0; stride /= 2) {
+    if (in && t < stride) s[half][t] += s[half][t + stride];
+    __syncthreads();
   }
 }
 
 // Per-slot global sums of two grid fields in FP64 with a fixed order (the
 // reference's reduction/wgsl/sum.wgsl, kept in double as the build asks of
-// global budget reductions). Writes the sums as floats to target[0|1 * S + slot]
-// and as doubles to sums[slot * 4 + which * 2 + 0|1].
-__global__ void __launch_bounds__(kSumThreads) k_slot_sums(Model m, const float* a, const float* b, float* target,
-                                                           int which) {
+// global budget reductions), a half of the block each. Writes the sums as
+// floats to target[0|1 * S + slot] and as doubles to sums[slot * 4 + which * 2
+// + 0|1].
+__global__ void __launch_bounds__(2 * kSumThreads) k_slot_sums(Model m, const float* a, const float* b, float* target,
+                                                               int which) {
+  __shared__ double s[2][kSumThreads];
   pdl_wait();
   pdl_release();
   const Dims& d = m.d;
   const int slot = blockIdx.x;
   if (!m.params[slot].active) return;
   if (which == 1 && m.params[slot].coupled == 0.f) return;  // getiflx runs with icestep only
-  __shared__ double sa[kSumThreads], sb[kSumThreads];
-  double x = 0.0, y = 0.0;
-  // Eight points of each field in flight, added in order: one at a time, the
-  // block waited for memory 32 times in a row at T42 (11 us for two 32 KB
-  // sums). NHOR is a multiple of 8 kSumThreads.
-  constexpr int kAhead = 8;
-  const float* pa = a + (size_t)slot * d.NHOR + threadIdx.x;
-  const float* pb = b + (size_t)slot * d.NHOR + threadIdx.x;
-  for (int h = 0; h < d.NHOR; h += kAhead * kSumThreads) {
-    float va[kAhead], vb[kAhead];
+  const int half = threadIdx.x / kSumThreads, t = threadIdx.x % kSumThreads;
+  s[half][t] = strided_sum((half ? b : a) + (size_t)slot * d.NHOR + t, d.NHOR / kSumThreads);
+  tree_sums(s, half, t, true);
+  if (t == 0) {
+    target[half * d.S + slot] = (float)s[half][0];
+    m.sums[slot * 4 + which * 2 + half] = s[half][0];
+  }
+}
+
+// physics/fixer/wgsl/row.wgsl: fix1d per latitude row, summed in longitude
+// order, then the planet's sums. A block takes a planet, a warp a row at a
+// time: its lanes stage the row in shared memory with coalesced loads, lane 0
+// adds the values in longitude order (the shader's sums, bit for bit), and the
+// update of a fixed row runs over all lanes.
+constexpr int kRowWarps = 32;
+constexpr int kMaxNlon = 192;  // NLON at T63, the largest truncation an engine accepts
+
+template <int NL>
+__global__ void __launch_bounds__(32 * kRowWarps) k_fixer_rows(Model m) {
+  __shared__ float stage[kRowWarps][kMaxNlon];
+  __shared__ double s[2][kSumThreads];
+  pdl_wait();
+  pdl_release();
+  const Dims& d = m.d;
+  const int slot = blockIdx.x;
+  if (!m.params[slot].active) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t SN = (size_t)d.S * d.NHOR;
+  const FieldPtrs& F = m.f;
+  float* row = stage[warp];
+  for (int lat = warp; lat < d.NLAT; lat += kRowWarps) {
+    const int first = slot * d.NHOR + lat * d.NLON;
+    auto ordered_sum = [&](const float* src) {
+      for (int j = lane; j < d.NLON; j += 32) row[j] = src[first + j];
+      __syncwarp();
+      float sum = 0.f;
+      if (lane == 0)
+        for (int j = 0; j < d.NLON; ++j) sum = sum + row[j];
+      sum = __shfl_sync(0xffffffffu, sum, 0);
+      __syncwarp();  // the row buffer is staged again next
+      return sum;
+    };
+    // a row without negatives needs no sum: fixneg is zero or positive
+    bool any = false;
+    for (int j = lane; j < d.NLON; j += 32) any = any || !(F.fixneg[first + j] == 0.f);
+    if (!__any_sync(0xffffffffu, any)) continue;
+    const float zneg = ordered_sum(F.fixneg);
+    if (zneg <= 0.f) continue;
+    const float zpos = ordered_sum(F.fixpos);
+    if (zpos < zneg) continue;
+    const float factor = (zpos - zneg) / zpos;
+    for (int j = lane; j < d.NLON; j += 32) {
+      float q[NL];
 #pragma unroll
-    for (int k = 0; k < kAhead; ++k) {
-      va[k] = pa[h + k * kSumThreads];
-      vb[k] = pb[h + k * kSumThreads];
-    }
+      for (int l = 0; l < NL; ++l) q[l] = F.fixq[l * SN + first + j];
+      const float pos = F.fixpos[first + j];
 #pragma unroll
-    for (int k = 0; k < kAhead; ++k) {
-      x += (double)va[k];
-      y += (double)vb[k];
+      for (int l = 0; l < NL; ++l) F.fixq[l * SN + first + j] = fmaxf(q[l] * factor, 0.f);
+      F.fixneg[first + j] = 0.f;
+      F.fixpos[first + j] = pos * factor;
     }
   }
-  sa[threadIdx.x] = x;
-  sb[threadIdx.x] = y;
   __syncthreads();
-  for (int stride = kSumThreads / 2; stride > 0; stride /= 2) {
-    if (threadIdx.x < stride) {
-      sa[threadIdx.x] += sa[threadIdx.x + stride];
-      sb[threadIdx.x] += sb[threadIdx.x + stride];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    target[slot] = (float)sa[0];
-    target[d.S + slot] = (float)sb[0];
-    m.sums[slot * 4 + which * 2] = sa[0];
-    m.sums[slot * 4 + which * 2 + 1] = sb[0];
+  // the planet's sums of what is left, as k_slot_sums takes them
+  const int half = threadIdx.x / kSumThreads, t = threadIdx.x % kSumThreads;
+  if (half < 2) s[half][t] = strided_sum((half ? F.fixpos : F.fixneg) + (size_t)slot * d.NHOR + t, d.NHOR / kSumThreads);
+  tree_sums(s, half, t, half < 2);
+  if (half < 2 && t == 0) {
+    F.fixsum[half * d.S + slot] = (float)s[half][0];
+    m.sums[slot * 4 + half] = s[half][0];
   }
 }
 
@@ -604,6 +599,7 @@ __global__ void __launch_bounds__(kBlock, 6)
   const float D2 = P.deltsec2;
   const float dp = F.dp[c];
   const float dt_surface = F.dt[NL * SN + c], dq_surface = F.dq[NL * SN + c];
+  if (h == 0) F.dca_skip[slot] = 0.f;  // raised again by mkdca's columns
   {
     // every load before the first store (the compiler cannot prove the
     // fields distinct)
@@ -863,33 +859,16 @@ __device__ __forceinline__ void b_mkdca(const Model& m, const PlanetConst* __res
     F.dca_dqdt[at] = (zqn[l] - zq[l]) / D2;
   }
   F.dca_limited[c] = limited;
+  // mkdca-limit (physics/precipitation/wgsl/mkdca-limit.wgsl): per slot, skip
+  // every adjustment when any column needed more than 2 NL passes. kuo cleared
+  // the slot's flag.
+  if (limited != 0.f) F.dca_skip[slot] = 1.f;
 }
 template <int NL>
 __global__ void __launch_bounds__(kBlock) k_mkdca(Model m, const PlanetConst* __restrict__ pcr, const float* __restrict__ tabr) {
   b_mkdca<NL>(m, pcr, tabr);
 }
 
-
-// mkdca-limit (physics/precipitation/wgsl/mkdca-limit.wgsl): per slot, skip
-// every adjustment when any column needed more than 2 NL passes.
-__global__ void __launch_bounds__(kSumThreads) k_mkdca_limit(Model m) {
-  pdl_wait();
-  pdl_release();
-  const Dims& d = m.d;
-  const int slot = blockIdx.x;
-  if (!m.params[slot].active) return;
-  __shared__ float part[kSumThreads];
-  float flag = 0.f;
-#pragma unroll 8
-  for (int h = threadIdx.x; h < d.NHOR; h += kSumThreads) flag = fmaxf(flag, m.f.dca_limited[slot * d.NHOR + h]);
-  part[threadIdx.x] = flag;
-  __syncthreads();
-  for (int stride = kSumThreads / 2; stride > 0; stride /= 2) {
-    if (threadIdx.x < stride) part[threadIdx.x] = fmaxf(part[threadIdx.x], part[threadIdx.x + stride]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) m.f.dca_skip[slot] = part[0];
-}
 
 // column.wgsl: mkdca's adjustment (unless skipped), mklsp, mkrain, mkclouds,
 // one thread per column. The level loops stay rolled: the condensation and
@@ -2035,18 +2014,17 @@ COLUMN_LAUNCHER(Carbon, k_carbon)
 COLUMN_LAUNCHER(Pack, k_pack)
 
 template <int NL>
-struct FixerRow {
+struct FixerRows {
   static void run(const Model& m, cudaStream_t st) {
-    step_launch(m.pdl, k_fixer_row<NL>, nblocks((size_t)m.d.S * m.d.NLAT, kRowWarps), 32 * kRowWarps, 0, st, m);
+    step_launch(m.pdl, k_fixer_rows<NL>, m.d.S, 32 * kRowWarps, 0, st, m);
   }
 };
 
 }  // namespace
 
 void phy_fixer(const Model& m, cudaStream_t st) {
-  by_levels<FixerColumn>(m.d.L, m, st);
-  by_levels<FixerRow>(m.d.L, m, st);
-  step_launch(m.pdl, k_slot_sums, m.d.S, kSumThreads, 0, st, m, m.f.fixneg, m.f.fixpos, m.f.fixsum, 0);
+  if (m.zero_gdt) by_levels<FixerColumn>(m.d.L, m, st);  // within a full step physics_in takes it
+  by_levels<FixerRows>(m.d.L, m, st);
   phy_fixer_apply(m, st);
 }
 
@@ -2060,7 +2038,6 @@ void phy_kuo(const Model& m, cudaStream_t st) { by_levels<Kuo>(m.d.L, m, st); }
 
 void phy_dca_rain(const Model& m, cudaStream_t st) {
   by_levels<Mkdca>(m.d.L, m, st);
-  step_launch(m.pdl, k_mkdca_limit, m.d.S, kSumThreads, 0, st, m);
   by_levels<RainColumn>(m.d.L, m, st);
 }
 
@@ -2069,7 +2046,7 @@ void phy_surface(const Model& m, cudaStream_t st) {
   step_launch(m.pdl, k_mkradv, nblocks((size_t)m.d.S * m.d.NHOR, kBlock), kBlock, 0, st, m);
   by_levels<LandSurface>(m.d.L, m, st);
   by_levels<SeaIce>(m.d.L, m, st);
-  step_launch(m.pdl, k_slot_sums, m.d.S, kSumThreads, 0, st, m, m.f.ice_part1, m.f.ice_part2, m.f.ice_sums, 1);
+  step_launch(m.pdl, k_slot_sums, m.d.S, 2 * kSumThreads, 0, st, m, m.f.ice_part1, m.f.ice_part2, m.f.ice_sums, 1);
   by_levels<Sea>(m.d.L, m, st);
 }
 
@@ -2091,7 +2068,7 @@ void phy_fused_surface_to_carbon(const Model& m, cudaStream_t st) {
   by_levels<Soil>(m.d.L, m, st);
   step_launch(m.pdl, k_mkradv, nblocks((size_t)m.d.S * m.d.NHOR, kBlock), kBlock, 0, st, m);
   by_levels<FusedLandSeaice>(m.d.L, m, st);
-  step_launch(m.pdl, k_slot_sums, m.d.S, kSumThreads, 0, st, m, m.f.ice_part1, m.f.ice_part2, m.f.ice_sums, 1);
+  step_launch(m.pdl, k_slot_sums, m.d.S, 2 * kSumThreads, 0, st, m, m.f.ice_part1, m.f.ice_part2, m.f.ice_sums, 1);
   by_levels<FusedSeaCarbon>(m.d.L, m, st);
 }
 

@@ -284,6 +284,7 @@ __global__ void __launch_bounds__(32 * NL)
   const float dqt_in = F.dqt[at], dq_in = F.dq[at], dqdt_in = F.dqdt[at], dt_in = F.dt[at], dtdt_in = F.dtdt[at];
   const float dsl = ds[l], sgl = sg[l];
   const float zdqt = dqt_in * K.PSURF * K.WW / dp;
+  if (l == 0 && c == slot * d.NHOR) F.dca_skip[slot] = 0.f;  // raised again by mkdca's columns
   F.dqt[at] = zdqt;
   const float zqe = dq_in + dqdt_in * D2, zte = dt_in + dtdt_in * D2;
   const float zacpe = K.ACPD * (1.f + K.ADV * dq_in);
