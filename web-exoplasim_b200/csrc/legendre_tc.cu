@@ -616,8 +616,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int a = S::fwd ? chunk % S::NA : gstep / ksb;
             const Term tm = term<KIND>(a, c_of_thread);
             const int p = p_of_thread;
+            // Rows of planes past the field's end are left as they are: a row
+            // of the accumulator depends on its own row of the operand alone,
+            // and theirs are not stored.
+            if (p >= np) continue;
             float x[4] = {0.f, 0.f, 0.f, 0.f};
-            if (p < np) {
+            {
               if (S::fwd) {
                 if (tm.field >= 0) {
                   // K indices 8 s + 4 kg + j of the unit's 32: half kk >> 4, pair kk & 15

@@ -9,14 +9,18 @@
 // copied in once (16-byte asynchronous copies of a slice laid out in HBM as
 // it sits in shared memory), pair-major ([pair][mode]): a row pitch of 4
 // (mod 32) banks and each
-// wavenumber's modes starting at a position of residue u (mod 4), for the
-// wavenumber pair u that reads them, put the 32 lanes of a warp (8 pairs x 4
-// wavenumber pairs) on 32 distinct banks. Per plane pair:
-//  1. Legendre: thread (wavenumber pair u, latitude pair jj) sums the modes of
-//     wavenumbers u and NTP1 - 1 - u for both planes: even-(n-m) and
-//     odd-(n-m) partial sums E, O in the order of the unfused latitude-pair
-//     kernel (legendre.cu), north = E + O, south = s (E - O). The Fourier
-//     coefficients go to the FFT's coefficient stage [plane][m][row].
+// wavenumber's modes starting at a position of residue m (mod 4) put the 32
+// lanes of a warp (8 pairs x 4 consecutive wavenumbers) on 32 distinct banks.
+// Per plane pair:
+//  1. Legendre: lane (wavenumber m, latitude pair jj) sums the modes of m for
+//     both planes: even-(n-m) and odd-(n-m) partial sums E, O in the order of
+//     the unfused latitude-pair kernel (legendre.cu), north = E + O, south =
+//     s (E - O). The Fourier coefficients go to the FFT's coefficient stage
+//     [plane][m][row]. The warps take the groups of four wavenumbers, which
+//     shorten with m, in snake order, so none sums much longer than another.
+//     (Threads taking wavenumber pairs (u, NTP1 - 1 - u), all of one length,
+//     did not divide evenly at T42: 704 pairs for 512 threads were two rounds,
+//     the second a third full.)
 //  2. FFT: the 32 rows of the pair, T threads per row, the four-step FFT of
 //     fft.cu; rows are written to the grid plane.
 // The next pair's spectral coefficients are fetched into registers during
@@ -57,14 +61,11 @@ __host__ __device__ constexpr int grid_table_pitch(int ntp1) {
   return ntp1 * (ntp1 + 1) / 2 + 3 * ntp1 + ((((4 - (ntp1 * (ntp1 + 1) / 2 + 3 * ntp1)) % 32) + 32) % 32);
 }
 
-// m is read by wavenumber pair u = m (m < (NTP1 + 1) / 2) or u = NTP1 - 1 - m,
-// and its modes start at a position of residue u (mod 4).
+// m's modes start at a position of residue m (mod 4).
 __host__ __device__ __forceinline__ void grid_table_positions(int ntp1, int* pos) {
-  const int groups = (ntp1 + 1) / 2;
   int at = 0;
   for (int m = 0; m < ntp1; ++m) {
-    const int u = m < groups ? m : ntp1 - 1 - m;
-    at += ((u - at) % 4 + 4) % 4;
+    at += ((m - at) % 4 + 4) % 4;
     pos[m] = at;
     at += ntp1 - m;
   }
@@ -100,8 +101,8 @@ struct GridShape {
   static constexpr int NPAIR = PP / 2;    // plane pairs per pass
   static constexpr int FROWS = PP * ROWS; // FFT rows per pass
   static constexpr int THREADS = FROWS * T;
-  static constexpr int GROUPS = (NTP1 + 1) / 2;
-  static constexpr int TASKS = GROUPS * JR * NPAIR;
+  static constexpr int GROUPS = (NTP1 + 3) / 4;              // groups of four wavenumbers
+  static constexpr int WARPS = THREADS / 32 / NPAIR;         // warps of a plane pair's Legendre sums
   static constexpr int TP = grid_table_pitch(NTP1);                // table row pitch, 4 (mod 32)
   static_assert((JR * TP) % 4 == 0, "a table slice is whole 16-byte chunks");
   static constexpr int PITCH = (ROWS + (((16 / T - ROWS) % 16) + 16) % 16);
@@ -210,13 +211,13 @@ __global__ void __launch_bounds__(GridShape<Q, PP>::THREADS)
     const int p = (pass - set.at[fi]) * G::PP, pend = set.f[fi].planes, opt = set.f[fi].opt;
     const bool dlambda = (opt & kTrDlambda) != 0;
     // 1. Legendre sums into the coefficient stage.
-    for (int task = threadIdx.x; task < G::TASKS; task += G::THREADS) {
-      const int pair = task / (G::GROUPS * JR), rest = task - pair * (G::GROUPS * JR);
-      const int u = rest / JR, jj = rest - u * JR;
+    {
+      const int warp = threadIdx.x / 32, pair = warp / G::WARPS, wi = warp - pair * G::WARPS;
+      const int mi = (threadIdx.x % 32) / JR, jj = threadIdx.x % JR;
 #pragma unroll 1
-      for (int side = 0; side < 2; ++side) {
-        const int m = side == 0 ? u : NTP1 - 1 - u;
-        if (side == 1 && m == u) break;
+      for (int round = 0; round * G::WARPS < G::GROUPS; ++round) {
+        const int m = 4 * (round * G::WARPS + ((round & 1) ? G::WARPS - 1 - wi : wi)) + mi;
+        if (m >= NTP1) continue;
         const int w0 = mode_start(m, NTP1), K = NTP1 - m;
         const float* qc = tab + jj * TP + tpos[m];
         const float4* sc = spec + pair * NCSP + w0;
