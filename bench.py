@@ -143,12 +143,13 @@ def make_planets(count, seed0=1000):
     return [planets.make_planet(seed0 + i, truncation=42, levels=10) for i in range(count)]
 
 
-# Launches of each timed kernel in one model step (engine.cu's step order),
-# counting a surface-pressure launch (one plane per slot) as 1/L of a
-# full-level launch; the timed launches are all full-level.
-PER_STEP = {"fourier_inverse": 10.2, "sp2gp": 8.2, "fourier_forward": 16.1, "legendre_inverse": 0.1, "dv2uv": 5,
-            "legendre_forward": 5.1, "uv2dv": 2, "qtend": 2, "swr": 1, "lwr_radstep": 1, "vdiff": 1, "kuo": 1,
-            "rain_column": 1, "calcgp": 1, "spectrala": 1, "mkdheat": 3, "physics_in": 1, "physics_out": 1}
+# Fields of each timed transform (launches of each other kernel) in one model
+# step on the optimized path (engine.cu), counting a surface-pressure field
+# (one plane per slot) as 1/L of a full-level one. A step's launch takes
+# several fields; a timed launch takes one full-level field.
+PER_STEP = {"fourier_inverse": 10, "sp2gp": 7.4, "fourier_forward": 16.1, "legendre_inverse": 0, "dv2uv": 5,
+            "legendre_forward": 4.1, "uv2dv": 2, "qtend": 2, "swr": 1, "lwr_radstep": 1, "vdiff": 1, "kuo": 1,
+            "rain_column": 1, "calcgp": 1, "spectrala": 1, "mkdheat": 1, "physics_in": 1, "physics_out": 1}
 
 
 # Kernels whose bound is HBM bandwidth (transforms and elementwise dynamics);

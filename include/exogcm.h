@@ -282,7 +282,7 @@ int exogcm_last_step_ms(exogcm_engine* engine, float* ms);
  * "legendre_inverse", "sp2gp" (the fused inverse Legendre transform and FFT
  * of the optimized path; "sp2gp_planes2" and "sp2gp_planes4" run it at 2
  * or 4 planes per pass whatever the tuning chose), "dv2uv", "uv2dv", "qtend", "calcgp", "spectrala",
- * "mkdheat" (its first stage), "physics_in", "physics_out", and the single
+ * "mkdheat" (its first two stages, one launch), "physics_in", "physics_out", and the single
  * column kernels "vdiff", "swr", "lwr_radstep", "kuo", "rain_column". The
  * launches change the state; use it for measurement only. */
 int exogcm_time_kernel(exogcm_engine* engine, const char* kernel, int reps, float* ms, double* bytes);

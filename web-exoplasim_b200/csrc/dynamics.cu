@@ -411,6 +411,9 @@ __global__ void __launch_bounds__(kBlock) k_mkdheat_winds(Model m) {
   };
   // IEEE divisions throughout mkdheat, as in spectrald's diffusion.
   auto friction = [&](float change, float ht) {
+    // friction acts on the top levels alone, and an IEEE division of zero takes
+    // the slow path of its routine: 128 T42 L10 planets 110 -> 72 us
+    if (change == 0.f && isfinite(ht) && ht != 0.f) return -change * ht;
     const float dtdt = __fdiv_rn(__fdiv_rn(__fdiv_rn(-change, P.deltsec2) * 0.5f, K.ACPD), ht);
     return __fdiv_rn(__fdiv_rn(dtdt, K.CT), K.WW);
   };

@@ -33,14 +33,14 @@
 // Pipeline (one CTA per SM, persistent over (m, plane tile) items; warp roles):
 //   warp 0  producer: TMA (cp.async.bulk.tensor) loads of the raw input rows
 //           into a double-buffered raw stage, and cp.async.bulk loads of the
-//           table chunks (4 K steps of hi and lo images) into a two-stage
-//           ring; every load completes on an mbarrier with a byte count.
-//   warps 1-4 converters and epilogue: build the data operand (gather,
+//           table chunks (4 K steps of hi and lo images) into a ring of up to
+//           eight stages; every load completes on an mbarrier with a byte count.
+//   warps 1-8 converters and epilogue: build the data operand (gather,
 //           sign, N +- S, hi/lo split) in the K-major no-swizzle layout for
 //           each chunk, then drain the previous item's accumulator
 //           (tcgen05.ld, a transpose through shared memory, coalesced
 //           stores) while the tensor cores run the current one.
-//   warp 5  MMA issuer: one thread issues the MMAs of a chunk as soon as its
+//   warp 9  MMA issuer: one thread issues the MMAs of a chunk as soon as its
 //           table and data stages are full, commits them to the stages'
 //           "empty" barriers and, after an item's last chunk, to the
 //           accumulator's "full" barrier; TMEM holds two accumulators.

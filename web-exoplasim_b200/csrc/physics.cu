@@ -1960,12 +1960,12 @@ __global__ void k_finite(Model m, int* fault_host) {
 
 
 // Fused column kernels (each thread takes its column through consecutive
-// routines in the reference's order, stepper/index.ts:148-161): kuo + mkdca,
-// rain + soil, land surface + sea ice, sea + carbon. A routine re-reads what
-// the one before it wrote or read for the same column from L1/L2 instead of
-// HBM. The full step uses the two that measured faster than their parts
-// (see phy_fused_precipitation_to_carbon); stage replay (exogcm_run_stage)
-// runs the separate kernels, and a full step equals its stages bit for bit.
+// routines in the reference's order, stepper/index.ts:148-161): land surface
+// + sea ice, sea + carbon. A routine re-reads what the one before it wrote or
+// read for the same column from L1/L2 instead of HBM. Fusing kuo with mkdca
+// and rain with soil measured slower than their parts. Stage replay
+// (exogcm_run_stage) runs the separate kernels, and a full step equals its
+// stages bit for bit.
 template <int NL>
 __global__ void __launch_bounds__(kBlock) k_fused_land_seaice(Model m, const PlanetConst* __restrict__ pcr,
                                                               const float* __restrict__ tabr) {

@@ -6,8 +6,8 @@
 // tendency left the reference's V3 tolerance than a sequential-f32 build's.
 // Arithmetic follows physics/fixer/wgsl/apply.wgsl, physics/surface-flux/
 // wgsl/{surflx,vdiff}.wgsl, physics/diffusion/wgsl/implicit.wgsl and
-// physics/radiation/wgsl/{solang,mko3}.wgsl; a full step runs the four as
-// one fused column kernel, stage replay as four launches.
+// physics/radiation/wgsl/{solang,mko3}.wgsl; each is a kernel of its own,
+// in a full step as in stage replay.
 #include "physics_common.cuh"
 
 namespace exogcm {
