@@ -219,6 +219,17 @@ struct Model {
   int storm;  // some slot runs the storm-climatology diagnostics (NSTORMDIAG > 0)
 };
 
+// x / d rounded to nearest where x is often zero: the division's routine takes
+// a slow path for a zero numerator, and the rest of the warp waits for it. So
+// a zero is replaced by 2^-23 (whose quotient overflows for no d but 0) and
+// the quotient times it is the answer: the signed zero, or NaN where d is 0
+// or NaN.
+__device__ __forceinline__ float quotient(float x, float d) {
+  const float q = __fdiv_rn(x == 0.f ? 0x1p-23f : x, d);
+  return x == 0.f ? x * q : q;
+}
+
+
 // physics/fixer/wgsl/column.wgsl: fix0d of one column, whose humidity dq and
 // surface pressure dp the caller holds. dq stays in registers for the stores
 // (a reload after each store would wait for it: the compiler cannot prove the

@@ -346,14 +346,15 @@ __global__ void __launch_bounds__(kBlock) k_spectrald_diffusion(Model m) {
     const float sqp = (k ? sqp0.y : sqp0.x) + D2 * (k ? sqt0.y : sqt0.x);
     // IEEE divisions (the file otherwise divides to 2 ulp): the diffusion
     // and friction increments feed mkdheat's heating through two more
-    // transforms, where 2-ulp quotients left V3's bound.
+    // transforms, where 2-ulp quotients left V3's bound. Most levels have no
+    // friction and most wavenumbers no diffusion: their numerators are zero.
     const float sk = sakpp[k];
-    const float stt = __fdiv_rn((-damp - tdisst * sk) * stp + damp * srp[k], 1.f + D2 * (damp + tdisst * sk));
-    const float sqt = __fdiv_rn(-tdissq * sk * sqp, 1.f + D2 * tdissq * sk);
-    const float zsdt1 = __fdiv_rn(-tfrc * sdp, 1.f + D2 * tfrc);
-    const float zsdt2 = __fdiv_rn(-tdissd * sk * sdp, 1.f + D2 * tdissd * sk);
-    float zszt1 = __fdiv_rn(-tfrc * szp, 1.f + D2 * tfrc);
-    float zszt2 = __fdiv_rn(-tdissz * sk * szp, 1.f + D2 * tdissz * sk);
+    const float stt = quotient((-damp - tdisst * sk) * stp + damp * srp[k], 1.f + D2 * (damp + tdisst * sk));
+    const float sqt = quotient(-tdissq * sk * sqp, 1.f + D2 * tdissq * sk);
+    const float zsdt1 = quotient(-tfrc * sdp, 1.f + D2 * tfrc);
+    const float zsdt2 = quotient(-tdissd * sk * sdp, 1.f + D2 * tdissd * sk);
+    float zszt1 = quotient(-tfrc * szp, 1.f + D2 * tfrc);
+    float zszt2 = quotient(-tdissz * sk * szp, 1.f + D2 * tdissz * sk);
     float szt = zszt1 + zszt2;
     if (s + k == 2) {
       zszt1 = zszt1 + __fdiv_rn(PLAVOR * tfrc, 1.f + D2 * tfrc);
@@ -412,7 +413,8 @@ __global__ void __launch_bounds__(kBlock) k_mkdheat_winds(Model m) {
   // IEEE divisions throughout mkdheat, as in spectrald's diffusion.
   auto friction = [&](float change, float ht) {
     // friction acts on the top levels alone, and an IEEE division of zero takes
-    // the slow path of its routine: 128 T42 L10 planets 110 -> 72 us
+    // the slow path of its routine: 128 T42 L10 planets 95 -> 58 us, as long as
+    // its loads and stores take
     if (change == 0.f && isfinite(ht) && ht != 0.f) return -change * ht;
     const float dtdt = __fdiv_rn(__fdiv_rn(__fdiv_rn(-change, P.deltsec2) * 0.5f, K.ACPD), ht);
     return __fdiv_rn(__fdiv_rn(dtdt, K.CT), K.WW);

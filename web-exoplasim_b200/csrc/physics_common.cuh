@@ -142,21 +142,23 @@ inline unsigned nblocks(size_t n, int b) { return (unsigned)((n + b - 1) / b); }
 // Implicit vertical diffusion (physics/diffusion/wgsl/implicit.wgsl): the
 // tridiagonal solve of one column, for a quantity and for potential
 // temperature, with IEEE divisions (the tendencies are small differences of
-// the diffused and the old profiles).
+// the diffused and the old profiles). Exchange coefficients and humidities
+// are often zero, hence quotient: vdiff 203 -> 193 us and kuo (mkshallow) 119
+// -> 112 at 128 T42 L10 planets, kuo 12.5 -> 7.6 at one T21 L10 planet.
 template <int NL>
 __device__ __forceinline__ void diffuse(const float* ds, float* x, const float* k) {
   float ebs[NL];
   const float ds0 = ds[0];
-  ebs[0] = __fdiv_rn(k[0], ds0 + k[0]);
-  x[0] = __fdiv_rn(ds0 * x[0], ds0 + k[0]);
+  ebs[0] = quotient(k[0], ds0 + k[0]);
+  x[0] = quotient(ds0 * x[0], ds0 + k[0]);
 #pragma unroll
   for (int l = 1; l < NL - 1; ++l) {
     const float den = ds[l] + k[l] + k[l - 1] * (1.f - ebs[l - 1]);
-    ebs[l] = __fdiv_rn(k[l], den);
-    x[l] = __fdiv_rn(x[l] * ds[l] + k[l - 1] * x[l - 1], den);
+    ebs[l] = quotient(k[l], den);
+    x[l] = quotient(x[l] * ds[l] + k[l - 1] * x[l - 1], den);
   }
   const float dsn = ds[NL - 1];
-  x[NL - 1] = __fdiv_rn(x[NL - 1] * dsn + k[NL - 2] * x[NL - 2], dsn + k[NL - 2] * (1.f - ebs[NL - 2]));
+  x[NL - 1] = quotient(x[NL - 1] * dsn + k[NL - 2] * x[NL - 2], dsn + k[NL - 2] * (1.f - ebs[NL - 2]));
 #pragma unroll
   for (int l = NL - 2; l >= 0; --l) x[l] = x[l] + ebs[l] * x[l + 1];
 }
@@ -165,20 +167,20 @@ template <int NL>
 __device__ __forceinline__ void diffuse_potential(const float* ds, float* x, const float* k, const float* skap) {
   float ebs[NL];
   const float ds0 = ds[0];
-  ebs[0] = __fdiv_rn(k[0], ds0 + __fdiv_rn(k[0], skap[0]));
-  x[0] = __fdiv_rn(ds0 * x[0], ds0 + __fdiv_rn(k[0], skap[0]));
+  ebs[0] = quotient(k[0], ds0 + quotient(k[0], skap[0]));
+  x[0] = quotient(ds0 * x[0], ds0 + quotient(k[0], skap[0]));
 #pragma unroll
   for (int l = 1; l < NL - 1; ++l) {
-    const float den = ds[l] + __fdiv_rn(k[l] + k[l - 1] * (1.f - __fdiv_rn(ebs[l - 1], skap[l - 1])), skap[l]);
-    ebs[l] = __fdiv_rn(k[l], den);
-    x[l] = __fdiv_rn(x[l] * ds[l] + __fdiv_rn(k[l - 1], skap[l - 1]) * x[l - 1], den);
+    const float den = ds[l] + quotient(k[l] + k[l - 1] * (1.f - quotient(ebs[l - 1], skap[l - 1])), skap[l]);
+    ebs[l] = quotient(k[l], den);
+    x[l] = quotient(x[l] * ds[l] + quotient(k[l - 1], skap[l - 1]) * x[l - 1], den);
   }
   const int last = NL - 1;
   const float dsn = ds[last];
-  x[last] = __fdiv_rn(x[last] * dsn + __fdiv_rn(k[NL - 2] * x[NL - 2], skap[NL - 2]),
-                      dsn + __fdiv_rn(k[NL - 2], skap[last]) * (1.f - __fdiv_rn(ebs[NL - 2], skap[NL - 2])));
+  x[last] = quotient(x[last] * dsn + quotient(k[NL - 2] * x[NL - 2], skap[NL - 2]),
+                      dsn + quotient(k[NL - 2], skap[last]) * (1.f - quotient(ebs[NL - 2], skap[NL - 2])));
 #pragma unroll
-  for (int l = NL - 2; l >= 0; --l) x[l] = x[l] + __fdiv_rn(ebs[l] * x[l + 1], skap[l + 1]);
+  for (int l = NL - 2; l >= 0; --l) x[l] = x[l] + quotient(ebs[l] * x[l + 1], skap[l + 1]);
 }
 
 
@@ -194,21 +196,21 @@ __device__ __forceinline__ float sum_products(float a, float b, float c, float d
 template <int NL, int STRIDE>
 __device__ __forceinline__ void diffuse_column(const float* __restrict__ ds, float* x, const float* k, float* ebs) {
   const float ds0 = ds[0], k0 = k[0];
-  float e = __fdiv_rn(k0, ds0 + k0), v = __fdiv_rn(ds0 * x[0], ds0 + k0), kp = k0;
+  float e = quotient(k0, ds0 + k0), v = quotient(ds0 * x[0], ds0 + k0), kp = k0;
   ebs[0] = e;
   x[0] = v;
 #pragma unroll 1
   for (int l = 1; l < NL - 1; ++l) {
     const float kl = k[l * STRIDE];
     const float den = ds[l] + kl + kp * (1.f - e);
-    e = __fdiv_rn(kl, den);
-    v = __fdiv_rn(sum_products(x[l * STRIDE], ds[l], kp, v), den);
+    e = quotient(kl, den);
+    v = quotient(sum_products(x[l * STRIDE], ds[l], kp, v), den);
     ebs[l * STRIDE] = e;
     x[l * STRIDE] = v;
     kp = kl;
   }
   const float dsn = ds[NL - 1];
-  v = __fdiv_rn(sum_products(x[(NL - 1) * STRIDE], dsn, kp, v), dsn + kp * (1.f - e));
+  v = quotient(sum_products(x[(NL - 1) * STRIDE], dsn, kp, v), dsn + kp * (1.f - e));
   x[(NL - 1) * STRIDE] = v;
 #pragma unroll 1
   for (int l = NL - 2; l >= 0; --l) {
@@ -221,28 +223,28 @@ template <int NL, int STRIDE>
 __device__ __forceinline__ void diffuse_potential_column(const float* __restrict__ ds, float* x, const float* k,
                                                          const float* __restrict__ skap, float* ebs) {
   const float ds0 = ds[0], k0 = k[0];
-  float e = __fdiv_rn(k0, ds0 + __fdiv_rn(k0, skap[0]));
-  float v = __fdiv_rn(ds0 * x[0], ds0 + __fdiv_rn(k0, skap[0]));
+  float e = quotient(k0, ds0 + quotient(k0, skap[0]));
+  float v = quotient(ds0 * x[0], ds0 + quotient(k0, skap[0]));
   float kp = k0;
   ebs[0] = e;
   x[0] = v;
 #pragma unroll 1
   for (int l = 1; l < NL - 1; ++l) {
     const float kl = k[l * STRIDE], sp = skap[l - 1];
-    const float den = ds[l] + __fdiv_rn(kl + kp * (1.f - __fdiv_rn(e, sp)), skap[l]);
-    e = __fdiv_rn(kl, den);
-    v = __fdiv_rn(sum_products(x[l * STRIDE], ds[l], __fdiv_rn(kp, sp), v), den);
+    const float den = ds[l] + quotient(kl + kp * (1.f - quotient(e, sp)), skap[l]);
+    e = quotient(kl, den);
+    v = quotient(sum_products(x[l * STRIDE], ds[l], quotient(kp, sp), v), den);
     ebs[l * STRIDE] = e;
     x[l * STRIDE] = v;
     kp = kl;
   }
   const int last = NL - 1;
   const float dsn = ds[last], sp = skap[NL - 2];
-  v = __fdiv_rn(x[last * STRIDE] * dsn + __fdiv_rn(kp * v, sp), dsn + __fdiv_rn(kp, skap[last]) * (1.f - __fdiv_rn(e, sp)));
+  v = quotient(x[last * STRIDE] * dsn + quotient(kp * v, sp), dsn + quotient(kp, skap[last]) * (1.f - quotient(e, sp)));
   x[last * STRIDE] = v;
 #pragma unroll 1
   for (int l = NL - 2; l >= 0; --l) {
-    v = x[l * STRIDE] + __fdiv_rn(ebs[l * STRIDE] * v, skap[l + 1]);
+    v = x[l * STRIDE] + quotient(ebs[l * STRIDE] * v, skap[l + 1]);
     x[l * STRIDE] = v;
   }
 }

@@ -217,7 +217,7 @@ __device__ __forceinline__ void b_vdiff(const Model& m, const PlanetConst* __res
 #pragma unroll
     for (int l = 0; l < NL; ++l) {
       const size_t at = l * SN + c;
-      F.dqdt[at] = tend(F.dqdt, l) + __fdiv_rn(zqn[l] - zq[l], D2);
+      F.dqdt[at] = tend(F.dqdt, l) + quotient(zqn[l] - zq[l], D2);
     }
   }
   // temperature: its diffusion increment, stored with the heating below
@@ -233,7 +233,7 @@ __device__ __forceinline__ void b_vdiff(const Model& m, const PlanetConst* __res
     for (int l = 0; l < NL - 1; ++l) kh[l] = kh[l] * skaph[l];
     diffuse_potential<NL>(ds, ztn, kh, zskap);
 #pragma unroll
-    for (int l = 0; l < NL; ++l) zdt[l] = __fdiv_rn(ztn[l] - zt[l], D2);
+    for (int l = 0; l < NL; ++l) zdt[l] = quotient(ztn[l] - zt[l], D2);
   }
   // winds and the dissipative heating
   float zu[NL], zv[NL], zun[NL], zvn[NL];
@@ -250,8 +250,8 @@ __device__ __forceinline__ void b_vdiff(const Model& m, const PlanetConst* __res
 #pragma unroll
   for (int l = 0; l < NL; ++l) {
     const size_t at = l * SN + c;
-    F.dudt[at] = tend(F.dudt, l) + __fdiv_rn(zun[l] - zu[l], D2);
-    F.dvdt[at] = tend(F.dvdt, l) + __fdiv_rn(zvn[l] - zv[l], D2);
+    F.dudt[at] = tend(F.dudt, l) + quotient(zun[l] - zu[l], D2);
+    F.dvdt[at] = tend(F.dvdt, l) + quotient(zvn[l] - zv[l], D2);
   }
   float heat[NL];
 #pragma unroll
