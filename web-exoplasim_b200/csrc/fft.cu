@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_fft_forward(const __grid_consta
 #pragma unroll
   for (int i = 0; i < Sh::QT; ++i)
 #pragma unroll
-    for (int p = 0; p < 8; ++p) a[i][p] = __ldg(in + Q * p + t + T * i);
+    for (int p = 0; p < 8; ++p) a[i][p] = in[Q * p + t + T * i];
   cp_async_wait_all();
   __syncthreads();
   float2* xr = xb + r * Sh::XP;
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_fft_inverse(const __grid_consta
     const float2* src = reinterpret_cast<const float2*>(set.f[fi].a) + plane * nlat * NTP1 + lat0 + lat;
 #pragma unroll 4
     for (int m = m0; m < NTP1; m += T) {
-      float2 v = __ldg(src + (size_t)m * nlat);
+      float2 v = src[(size_t)m * nlat];
       if (m == 0) v.y = 0.f;
       fc[m * pitch + lat] = v;
     }
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_fft_forward_persistent(const __
 #pragma unroll
     for (int i = 0; i < Sh::QT; ++i)
 #pragma unroll
-      for (int p = 0; p < 8; ++p) a[i][p] = __ldg(in + Q * p + t + T * i);
+      for (int p = 0; p < 8; ++p) a[i][p] = in[Q * p + t + T * i];
   };
   int item = blockIdx.x;
   copy_twiddles<Q>(twg, tw, twq);
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_fft_inverse_persistent(const __
 #pragma unroll
     for (int k = 0; k < KS; ++k) {
       const int m = m0 + T * k;
-      v[k] = m < NTP1 ? __ldg(src + (size_t)m * nlat) : make_float2(0.f, 0.f);
+      v[k] = m < NTP1 ? src[(size_t)m * nlat] : make_float2(0.f, 0.f);
     }
   };
   int item = blockIdx.x;

@@ -309,8 +309,8 @@ __global__ void __launch_bounds__(FwdShape<JH, TP>::THREADS)
       if (e < E && plane < pend && (mi == 0 || pair)) {
         const float* base = k == 0 ? in0 : k == 1 ? in1 : in2;
         const float2* row = reinterpret_cast<const float2*>(base + (size_t)plane * PLANE) + (mi ? mb : ma) * row_m;
-        a = __ldg(row + l * row_l);
-        b = __ldg(row + (NLAT - 1 - l) * row_l);
+        a = row[l * row_l];
+        b = row[(NLAT - 1 - l) * row_l];
       }
       rn[i] = a;
       rs[i] = b;

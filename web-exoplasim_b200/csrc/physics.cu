@@ -1864,75 +1864,88 @@ __global__ void __launch_bounds__(kBlock) k_pack(Model m, const PlanetConst* __r
     F.carbon_step[slot] = P.carbon;
   }
   if (snapflag == 0.f) return;
-  // Nothing below but the snapshot and its tracking is written here, so the
-  // fields are read as read-only data: the compiler may then hold many loads in
-  // flight past the stores, which it cannot prove distinct from the fields (33
-  // us for 7 T42 L5 planets when each of 76 loads waited for the store before it).
+  // Every value is read before the first store of its group (the compiler
+  // cannot prove the snapshot distinct from the fields): 33 us for 7 T42 L5
+  // planets when each of 76 loads waited for the store before it. Ordinary
+  // loads: the fields were written by the kernel this one may be resident beside.
   const int jet = (int)K.JET;
-  put(0, __ldg(F.dt + NL * SN + c));
-  put(1, __ldg(F.dtsa + c));
-  put(2, __ldg(F.du + (NL - 1) * SN + c));
-  put(3, __ldg(F.dv + (NL - 1) * SN + c));
-  put(4, __ldg(F.dcc + NL * SN + c));
-  put(5, __ldg(F.dprc + c) + __ldg(F.dprl + c));
-  put(6, __ldg(F.dp + c));
-  put(7, __ldg(F.dqvi + c));
-  put(8, __ldg(F.dicec + c));
-  put(9, __ldg(F.dsnow + c));
-  put(10, __ldg(F.dwatc + c));
-  put(11, __ldg(F.dalb + c));
-  put(12, __ldg(F.du + jet * SN + c));
-  put(13, __ldg(F.dv + jet * SN + c));
-  put(14, -__ldg(F.dlwfl + c));
-  put(15, __ldg(F.dls + c));
-  put(16, __ldg(F.dswfl + c) + __ldg(F.dlwfl + c));
-  put(17, __ldg(F.dsmelt + c) * -333700000.f + __ldg(F.dswfl + NL * SN + c) + __ldg(F.dlwfl + NL * SN + c) + __ldg(F.dshfl + c) + __ldg(F.dlhfl + c));
-  put(18, -__ldg(F.devap + c));
-  put(19, __ldg(F.drunoff + c));
-  put(20, __ldg(F.dforest + c));
-  put(21, __ldg(F.dlai + c));
-  put(22, __ldg(F.dprs + c));
-  put(23, __ldg(F.dsmelt + c));
-  put(24, __ldg(F.diced + c));
-  put(25, __ldg(F.dglac + c));
-  put(27, __ldg(F.dswfl + NL * SN + c));
-  put(28, __ldg(F.dlwfl + NL * SN + c));
-  put(29, __ldg(F.dshfl + c));
-  put(30, __ldg(F.dlhfl + c));
-  put(31, __ldg(F.dprc + c));
-  put(32, __ldg(F.dprl + c));
-  put(33, __ldg(F.dswfl + c));
-  put(34, __ldg(F.dlwfl + c));
+  float v[51];
+  v[0] = F.dt[NL * SN + c];
+  v[1] = F.dtsa[c];
+  v[2] = F.du[(NL - 1) * SN + c];
+  v[3] = F.dv[(NL - 1) * SN + c];
+  v[4] = F.dcc[NL * SN + c];
+  v[5] = F.dprc[c] + F.dprl[c];
+  v[6] = F.dp[c];
+  v[7] = F.dqvi[c];
+  v[8] = F.dicec[c];
+  v[9] = F.dsnow[c];
+  v[10] = F.dwatc[c];
+  v[11] = F.dalb[c];
+  v[12] = F.du[jet * SN + c];
+  v[13] = F.dv[jet * SN + c];
+  v[14] = -F.dlwfl[c];
+  v[15] = F.dls[c];
+  v[16] = F.dswfl[c] + F.dlwfl[c];
+  v[17] = F.dsmelt[c] * -333700000.f + F.dswfl[NL * SN + c] + F.dlwfl[NL * SN + c] + F.dshfl[c] + F.dlhfl[c];
+  v[18] = -F.devap[c];
+  v[19] = F.drunoff[c];
+  v[20] = F.dforest[c];
+  v[21] = F.dlai[c];
+  v[22] = F.dprs[c];
+  v[23] = F.dsmelt[c];
+  v[24] = F.diced[c];
+  v[25] = F.dglac[c];
+  v[27] = F.dswfl[NL * SN + c];
+  v[28] = F.dlwfl[NL * SN + c];
+  v[29] = F.dshfl[c];
+  v[30] = F.dlhfl[c];
+  v[31] = F.dprc[c];
+  v[32] = F.dprl[c];
+  v[33] = F.dswfl[c];
+  v[34] = F.dlwfl[c];
   const bool windowed = tr[8 * SN] != 0.f;
-  put(35, windowed ? tr[2 * SN] : tr[0]);
-  put(36, windowed ? tr[3 * SN] : tr[SN]);
-  put(37, windowed ? tr[4 * SN] : tr[SN] - tr[0]);
-  put(38, tr[5 * SN]);
-  put(39, tr[6 * SN]);
-  put(40, __ldg(F.dnpp + c));
-  put(41, __ldg(F.gmu0 + c));
+  v[35] = windowed ? tr[2 * SN] : tr[0];
+  v[36] = windowed ? tr[3 * SN] : tr[SN];
+  v[37] = windowed ? tr[4 * SN] : tr[SN] - tr[0];
+  v[38] = tr[5 * SN];
+  v[39] = tr[6 * SN];
+  v[40] = F.dnpp[c];
+  v[41] = F.gmu0[c];
+  v[42] = F.capen[c];
+  v[43] = F.lnb[c];
+  v[44] = F.mpoti[c];
+  v[45] = F.chim[c];
+  v[46] = F.laav[c];
+  v[47] = F.venti[c];
+  v[48] = F.vrmpi[c];
+  v[49] = F.gpi[c];
+  v[50] = F.shear[c];
+#pragma unroll
+  for (int i = 0; i < 51; ++i)
+    if (i != 26) put(i, v[i]);
   tr[5 * SN] = 0.f;
   tr[6 * SN] = 0.f;
+  const int lowest = NL - 1;
+  float lt[NL], lu[NL], lv[NL], lc[NL];
+#pragma unroll
+  for (int l = 0; l < NL; ++l) {
+    lt[l] = F.dt[l * SN + c];
+    lu[l] = F.du[l * SN + c];
+    lv[l] = F.dv[l * SN + c];
+    lc[l] = F.dcc[l * SN + c];
+  }
+  const float low_q = F.dq[lowest * SN + c];
 #pragma unroll
   for (int l = 0; l < NL; ++l) {
     const int f = 51 + 5 * l;
-    put(f, __ldg(F.dt + l * SN + c));
-    put(f + 1, __ldg(F.du + l * SN + c));
-    put(f + 2, __ldg(F.dv + l * SN + c));
-    put(f + 4, __ldg(F.dcc + l * SN + c));
+    put(f, lt[l]);
+    put(f + 1, lu[l]);
+    put(f + 2, lv[l]);
+    put(f + 4, lc[l]);
   }
-  put(42, __ldg(F.capen + c));
-  put(43, __ldg(F.lnb + c));
-  put(44, __ldg(F.mpoti + c));
-  put(45, __ldg(F.chim + c));
-  put(46, __ldg(F.laav + c));
-  put(47, __ldg(F.venti + c));
-  put(48, __ldg(F.vrmpi + c));
-  put(49, __ldg(F.gpi + c));
-  put(50, __ldg(F.shear + c));
-  const int lowest = NL - 1;
-  const float qsat = sat_divided(K, __ldg(F.dt + lowest * SN + c), __ldg(F.dp + c) * K.SIGMA_LOW);
-  put(51 + 5 * lowest + 3, fmaxf(0.f, __ldg(F.dq + lowest * SN + c)) / fmaxf(1.17549435e-38f, qsat));
+  const float qsat = sat_divided(K, lt[lowest], v[6] * K.SIGMA_LOW);
+  put(51 + 5 * lowest + 3, fmaxf(0.f, low_q) / fmaxf(1.17549435e-38f, qsat));
 }
 
 // Non-finite check per slot over the prognostic spectral state: sets

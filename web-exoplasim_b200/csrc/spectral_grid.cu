@@ -171,8 +171,8 @@ __global__ void __launch_bounds__(GridShape<Q, PP>::THREADS)
       const int pa = p + 2 * pair;
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
       if (e < G::SPEC && pa < pend) {
-        const float2 x = __ldg(reinterpret_cast<const float2*>(s + (size_t)pa * SPLANE) + w);
-        const float2 y = pa + 1 < pend ? __ldg(reinterpret_cast<const float2*>(s + (size_t)(pa + 1) * SPLANE) + w)
+        const float2 x = reinterpret_cast<const float2*>(s + (size_t)pa * SPLANE)[w];
+        const float2 y = pa + 1 < pend ? reinterpret_cast<const float2*>(s + (size_t)(pa + 1) * SPLANE)[w]
                                        : make_float2(0.f, 0.f);
         v = make_float4(x.x, x.y, y.x, y.y);
       }

@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(768) k_dft(const __grid_constant__ TrSet set, 
 }
 
 // gpmt: d/dlambda in Fourier space, (re, im) * i m (fourier/wgsl/dlambda.wgsl).
-__global__ void k_dlambda(const float* __restrict__ a, float* __restrict__ b, int n, int ntp1, int nfc) {
+__global__ void k_dlambda(const float* a, float* b, int n, int ntp1, int nfc) {
   pdl_wait();
   pdl_release();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -103,7 +103,7 @@ __global__ void k_dlambda(const float* __restrict__ a, float* __restrict__ b, in
 
 // The same on the optimized path's m-major Fourier planes (coefficient
 // (m, lat) at 2 * (m * NLAT + lat)).
-__global__ void k_dlambda_m_major(const float* __restrict__ a, float* __restrict__ b, int n, int nlat, int ntp1) {
+__global__ void k_dlambda_m_major(const float* a, float* b, int n, int nlat, int ntp1) {
   pdl_wait();
   pdl_release();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
