@@ -233,30 +233,48 @@ __device__ __forceinline__ float quotient(float x, float d) {
 // physics/fixer/wgsl/column.wgsl: fix0d of one column, whose humidity dq and
 // surface pressure dp the caller holds. dq stays in registers for the stores
 // (a reload after each store would wait for it: the compiler cannot prove the
-// fields distinct).
+// fields distinct). Its callers are built with and without -ftz, so the
+// operations that flush subnormals, as every physics routine's do, are
+// written out; the quotient is the physics files' (at most 2 ulp).
 #ifdef __CUDACC__
+__device__ __forceinline__ float mul_ftz(float a, float b) {
+  float r;
+  asm("mul.rn.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float fma_ftz(float a, float b, float c) {
+  float r;
+  asm("fma.rn.ftz.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float div_ftz(float a, float b) {
+  float r;
+  asm("div.full.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 template <int NL>
 __device__ __forceinline__ void fixer_column(const Model& m, const float* ds, size_t SN, int c, int h,
                                              const float (&dq)[NL], float dp) {
   float negative = 0.f, positive = 0.f;
 #pragma unroll
   for (int l = 0; l < NL; ++l) {
-    const float q = dq[l] * ds[l];
-    if (dq[l] < 0.f) negative = negative + q;
-    if (dq[l] > 0.f) positive = positive + q;
+    const float q = mul_ftz(dq[l], 1.f);  // a subnormal is zero
+    if (q < 0.f) negative = fma_ftz(q, ds[l], negative);
+    if (q > 0.f) positive = fma_ftz(q, ds[l], positive);
   }
   const float zgw = m.sh.zgw[h];
-  float zneg = -negative * dp * zgw;
-  float zpos = positive * dp * zgw;
+  float zneg = mul_ftz(mul_ftz(-negative, dp), zgw);
+  float zpos = mul_ftz(mul_ftz(positive, dp), zgw);
   float factor = 1.f;
   const bool fixed = zneg > 0.f && zpos >= zneg;
   if (fixed) {
-    factor = (zpos - zneg) / zpos;
+    factor = div_ftz(fma_ftz(zneg, -1.f, zpos), zpos);
     zneg = 0.f;
-    zpos = zpos * factor;
+    zpos = mul_ftz(zpos, factor);
   }
 #pragma unroll
-  for (int l = 0; l < NL; ++l) m.f.fixq[l * SN + c] = fixed ? fmaxf(dq[l] * factor, 0.f) : dq[l];
+  for (int l = 0; l < NL; ++l) m.f.fixq[l * SN + c] = fixed ? fmaxf(mul_ftz(dq[l], factor), 0.f) : dq[l];
   m.f.fixneg[c] = zneg;
   m.f.fixpos[c] = zpos;
 }

@@ -18,7 +18,7 @@ namespace {
 
 // ---------------------------------------------------------------- fixer
 // physics/fixer/wgsl/column.wgsl: fix0d per column (fixer_column in
-// physics_common.cuh). Stage replay's; within a full step physics_in takes it
+// common.cuh). Stage replay's; within a full step physics_in takes it
 // with the humidity it has just formed.
 template <int NL>
 __global__ void __launch_bounds__(kBlock) k_fixer_column(Model m, const PlanetConst* __restrict__ pcr, const float* __restrict__ tabr) {
