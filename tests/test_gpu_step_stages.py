@@ -41,7 +41,8 @@ def after_step_and_stages(mode, truncation, levels, slots, storm=False, change=N
 @pytest.mark.parametrize("mode,truncation,levels,slots,storm", [
     (0, 21, 5, 2, False), (0, 21, 10, 1, True), (1, 21, 5, 3, True), (1, 42, 10, 1, False),
     # more columns than the kernels with a thread per (column, level) take
-    (1, 21, 10, 11, False), (1, 42, 5, 3, True)])
+    (1, 21, 10, 11, False), (1, 42, 5, 3, True),
+    (2, 21, 10, 1, False), (2, 21, 5, 11, True), (2, 63, 5, 1, False)])
 def test_step_equals_its_stages(mode, truncation, levels, slots, storm):
     assert after_step_and_stages(mode, truncation, levels, slots, storm) == []
 

@@ -434,16 +434,17 @@ __global__ void __launch_bounds__(kBlock) k_mkdheat_winds(Model m) {
 // transform the kinetic energy to spectral space, keep mode (0, 0) alone
 // (dynamics/wgsl/mean-mode.wgsl) and transform that back. Only fc2sp's sum
 // of mode (0, 0) reaches the result, over the latitude pairs of the Fourier
-// rows' mean (fzdekin, m = 0), and back on the grid a latitude is the
-// constant q(0, 0)[lat] times it, exactly: every other term of sp2fc and
+// rows' mean (m = 0, in the scratch fzdv1), and back on the grid a latitude is
+// the constant q(0, 0)[lat] times it, exactly: every other term of sp2fc and
 // fc2gp is a sum with zeros. So each block takes that sum in the shaders'
 // order and no transform runs (fc2sp, the zeroing, sp2gp and this stage's
 // read of zdekin took 20 + 8 + 33 + 8 us at 128 T42 L10 planets, and three
 // of a single planet's launches). The slot's first block also writes the
-// spectral field. A block takes `chunks` runs of kCols4 columns of its plane,
-// so that the sum, a chain of NLAT / 2 multiply-adds in one warp, is taken
-// once for all of them.
-__global__ void __launch_bounds__(kBlock) k_mkdheat_mean(Model m, int chunks) {
+// spectral field, and with `fourier` the slot's blocks the Fourier field
+// between the two (a row's m = 0 is that constant, the rest zero). A block
+// takes `chunks` runs of kCols4 columns of its plane, so that the sum, a chain
+// of NLAT / 2 multiply-adds in one warp, is taken once for all of them.
+__global__ void __launch_bounds__(kBlock) k_mkdheat_mean(Model m, int chunks, int fourier) {
   constexpr int kMaxPairs = 48;
   __shared__ float pair_sum[kMaxPairs], pair_q[kMaxPairs];
   __shared__ float mean;
@@ -456,7 +457,7 @@ __global__ void __launch_bounds__(kBlock) k_mkdheat_mean(Model m, int chunks) {
   const FieldPtrs& F = m.f;
   const size_t plane = (size_t)l * d.S + slot;
   if (threadIdx.x < 32) {
-    const float* rows = F.fzdekin + plane * d.NLAT * d.NFC;
+    const float* rows = m.fzdv1 + plane * d.NLAT * d.NFC;
     const int step = m.mode >= 1 ? 2 : d.NFC;  // m-major or latitude-major
     const int half = d.NLAT / 2;
     for (int j = threadIdx.x; j < half; j += 32) {
@@ -478,6 +479,15 @@ __global__ void __launch_bounds__(kBlock) k_mkdheat_mean(Model m, int chunks) {
   if (first == slot * d.NHOR) {
     float* out = F.zsdef + plane * d.NRSP;
     for (int r = threadIdx.x; r < d.NRSP; r += kBlock) out[r] = r == 0 ? s00 : 0.f;
+  }
+  if (fourier) {
+    float* out = F.fzdekin + plane * d.NLAT * d.NFC;
+    const int block = (first - slot * d.NHOR) / (chunks * kCols4), blocks = d.NHOR / (chunks * kCols4);
+    for (int i = block * kBlock + threadIdx.x; i < d.NLAT * d.NFC; i += blocks * kBlock) {
+      const bool mean_part = m.mode >= 1 ? i < 2 * d.NLAT && i % 2 == 0 : i % d.NFC == 0;  // m-major or latitude-major
+      const int lat = m.mode >= 1 ? i / 2 : i / d.NFC;
+      out[i] = mean_part ? m.sh.qi[(size_t)lat * d.NCSP] * s00 : 0.f;
+    }
   }
   for (int k = 0; k < chunks; ++k) {
     const int c = first + k * kCols4 + 4 * threadIdx.x;
@@ -681,7 +691,9 @@ void dyn_mkdheat_mean(const Model& m, cudaStream_t st) {
   const size_t runs = (size_t)m.d.S * m.d.NHOR / kCols4;
   const int chunks = runs * m.d.NLEV >= 148 * 32 ? 4 : 1;
   const dim3 grid((unsigned)(runs / chunks), m.d.NLEV);
-  step_launch(m.pdl, k_mkdheat_mean, grid, kBlock, 0, st, m, chunks);
+  // mode 1 leaves the Fourier fields between fused transforms unwritten
+  const int fourier = m.mode != 1 || m.keep_fourier;
+  step_launch(m.pdl, k_mkdheat_mean, grid, kBlock, 0, st, m, chunks, fourier);
 }
 void dyn_spectrald_update(const Model& m, cudaStream_t st) {
   const dim3 grid(blocks((size_t)m.d.S * m.d.NRSP / 2, kBlock), m.d.NLEV);

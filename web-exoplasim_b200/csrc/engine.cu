@@ -603,16 +603,15 @@ void stage_spectrald(const Model& m, Lanes& on) {
                             fourier_field(F.fzdu, F.zdu, LP), fourier_field(F.fzdv, F.zdv, LP)),
                      st);
   dyn_mkdheat_winds(m, st);
-  // friction's heating goes through the scratch fzdu1, spent by now: its
-  // forward Legendre sums run beside the third stage's transforms
-  tr_fourier_forward(m, set_of(fourier_field(F.zdtdt, m.fzdu1, LP), fourier_field(F.zdekin, F.fzdekin, LP, 1)), st);
+  // friction's heating and the kinetic energy go through the scratch fzdu1 and
+  // fzdv1, spent by now: the heating's forward Legendre sums run beside the
+  // third stage's transforms, and fzdekin is the mean's
+  tr_fourier_forward(m, set_of(fourier_field(F.zdtdt, m.fzdu1, LP), fourier_field(F.zdekin, m.fzdv1, LP, 1)), st);
   on.fork(0);
   on.beside(0, [&](cudaStream_t side) {
     tr_legendre_forward(whole(m), set_of(fourier_field(m.fzdu1, F.zstt1, LP)), side);
   });
   dyn_mkdheat_mean(m, st);
-  // the mean's Fourier field, kept on the plain path and by stage replay
-  if (m.mode == 0 || m.keep_fourier) tr_legendre_inverse(m, set_of(fourier_field(F.zsdef, F.fzdekin, LP)), st);
   tr_fourier_forward(m, set_of(fourier_field(F.zdtdt, F.fzdtdt, LP)), st);
   tr_legendre_forward(m, set_of(fourier_field(F.fzdtdt, F.zstt2, LP)), st);
   on.join(0);
