@@ -144,8 +144,9 @@ int exogcm_release(exogcm_engine* engine, int slot);
 
 /* Runs `steps` model steps for every active slot (STEPPER.batch,
  * stepper/index.ts:203-276): per-step CPU values computed on the host,
- * uploaded once, then the whole batch as one CUDA graph. A slot whose step
- * number is a multiple of `publish_every` packs its snapshot on that step.
+ * uploaded once, then the whole batch as one CUDA graph (an engine's first
+ * batch of a length kernel by kernel). A slot whose step number is a multiple
+ * of `publish_every` packs its snapshot on that step.
  * `steps` must not exceed `publish_every` so a slot publishes at most once.
  * Returns when the batch is done (exogcm_step_async + exogcm_wait). */
 int exogcm_step(exogcm_engine* engine, int steps, int publish_every);
@@ -173,9 +174,10 @@ int exogcm_wait(exogcm_engine* engine);
  * CUDA graph whose nodes are the engines' captured batch graphs, so the
  * batches of a mixed-resolution ensemble (128 T21 L5 + 96 T42 L10 + 32 T63
  * L10 planets, say) run concurrently from one submission. Engines must be
- * distinct and on one device; the group graph is instantiated once per
- * (engines, steps) list and reused. Returns when every batch is done; *ms
- * (may be NULL) receives the device time of the launch. No counterpart in
+ * distinct and on one device; the group graph is instantiated at the second
+ * use of an (engines, steps) list and reused (the first launches each engine's
+ * kernels on its own stream). Returns when every batch is done; *ms
+ * (may be NULL) receives the device time of the batches. No counterpart in
  * the reference, whose worker steps one planet per device
  * (runner/webgpu/gcm.worker.ts:215-346). */
 int exogcm_group_step(exogcm_engine** engines, int count, const int* steps, int publish_every, float* ms);

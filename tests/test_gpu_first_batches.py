@@ -1,0 +1,71 @@
+"""A length's first batch is launched kernel by kernel and its later ones as a
+graph: the same kernels, so the same state bit for bit, and a new engine's
+first batch does not wait for a graph to be built."""
+import time
+
+import numpy as np
+import pytest
+
+from tests.helpers import oracle_field_list, pkg, planets
+
+pytestmark = pytest.mark.gpu
+
+
+def engine(truncation, levels, slots, mode):
+    e = pkg.Engine(truncation, levels, slots, mode=mode)
+    for s in range(slots):
+        e.configure(s, planets.make_planet(61 + s, truncation=truncation, levels=levels, stormclim=s == 1))
+    e.step(3)
+    return e
+
+
+def states_after_batches(engines, batch, count):
+    """The state after each of `count` batches from the same start."""
+    names = oracle_field_list()
+    start = [[e.checkpoint_save(s) for s in range(e.slots)] for e in engines]
+    states = []
+    for _ in range(count):
+        for e, saved in zip(engines, start):
+            for s, blob in enumerate(saved):
+                e.checkpoint_load(s, blob)
+        batch()
+        states.append({(i, s, n): e.read(s, n) for i, e in enumerate(engines) for s in range(e.slots) for n in names})
+    return states
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_first_and_later_batches_give_the_same_state(mode):
+    e = engine(21, 5, 2, mode)
+    try:
+        first, *later = states_after_batches([e], lambda: e.step(4, publish_every=4), 3)
+        for state in later:
+            assert [k for k in first if not np.array_equal(first[k], state[k], equal_nan=True)] == []
+    finally:
+        e.close()
+
+
+def test_first_and_later_group_batches_give_the_same_state():
+    engines = [engine(21, 5, 2, 1), engine(42, 10, 1, 1), engine(21, 10, 1, 2)]
+    try:
+        first, *later = states_after_batches(engines, lambda: pkg.group_step(engines, [3, 1, 2]), 3)
+        for state in later:
+            assert [k for k in first if not np.array_equal(first[k], state[k], equal_nan=True)] == []
+    finally:
+        for e in engines:
+            e.close()
+
+
+def test_a_new_engines_first_batch_waits_for_no_graph():
+    """Median over engines of the first batch's time against a repeated one's:
+    launched kernel by kernel about twice it, as a new graph about five times."""
+    ratios = []
+    for _ in range(7):
+        e = engine(21, 10, 1, 1)
+        times = []
+        for _ in range(12):
+            t = time.perf_counter()
+            e.step(32)
+            times.append(time.perf_counter() - t)
+        e.close()
+        ratios.append(times[0] / np.median(times[6:]))
+    assert np.median(ratios) < 3, ratios

@@ -202,9 +202,9 @@ def boundary_struct(planet, nhor: int, keep: dict) -> Boundary:
 
 
 def group_step(engines, steps, publish_every: int | None = None) -> float:
-    """Steps several engines (any resolutions) as one CUDA graph launch
-    (exogcm_group_step): engine i runs steps[i] model steps. Returns the
-    launch's device time in ms."""
+    """Steps several engines (any resolutions) together, as one CUDA graph
+    launch from the second use of a list on (exogcm_group_step): engine i runs
+    steps[i] model steps. Returns their device time in ms."""
     lib = load_library()
     n = len(engines)
     handles = (_VP * n)(*[e.h for e in engines])

@@ -9,7 +9,7 @@
 //   readback   -> LAYOUT.read (layout/index.ts:73-108)
 //   checkpoint -> RESTART.encode/decode (checkpoint/restart/index.ts:11-75)
 // for S planet slots at once. One device arena holds every field as
-// [plane][slot][points]; a batch of K steps is one CUDA graph whose step k
+// [plane][slot][points]; a repeated batch of K steps is one CUDA graph whose step k
 // reads its per-slot host values at params + k * S.
 #include <cuda_runtime.h>
 
@@ -134,6 +134,7 @@ struct exogcm_engine {
   std::vector<Slot> slots;
   std::map<int, cudaGraphExec_t> graphs;
   std::map<int, cudaGraph_t> graph_templates;  // the captured K-step graphs (child nodes of group graphs)
+  std::map<int, int> batches_of;  // batches of K steps submitted so far (kPlainBatches)
   Tuning tune{};
   SharedSetup shared_setup;  // host copy of the shared tables (set-up of later planets)
   // FP64 set-up loops on this device (setup_device.cu), created at the first
@@ -713,19 +714,41 @@ StepParams next_params(Slot& s, int publish_every, bool advance) {
   return p;
 }
 
-cudaGraphExec_t batch_graph(exogcm_engine* e, int K) {
-  auto it = e->graphs.find(K);
-  if (it != e->graphs.end()) return it->second;
+// The first batch of a length is launched kernel by kernel, the later ones as
+// a graph: to capture and instantiate one with a step's side chains takes
+// longer than such a batch, and a program may run a length once. us, a new
+// engine's first batch as a graph / kernel by kernel, a repeated one: four
+// steps of one T21 L10 planet 2,200-3,200 / 905, 484; two of one T42 L10
+// 1,790 / 519, 320; two of 37 T21 L10 2,060 / 852, 683.
+constexpr int kPlainBatches = 1;
+
+// K steps captured as a graph, kept for later batches and group graphs.
+cudaGraph_t captured_steps(exogcm_engine* e, int K) {
+  auto it = e->graph_templates.find(K);
+  if (it != e->graph_templates.end()) return it->second;
   cudaGraph_t graph;
   check(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed), "capture");
   Lanes on(e->stream, true);
   for (int k = 0; k < K; ++k) full_step(e->model(k), on);
   check(cudaStreamEndCapture(e->stream, &graph), "capture end");
-  cudaGraphExec_t exec;
-  check(cudaGraphInstantiate(&exec, graph, 0), "graph instantiate");
   e->graph_templates[K] = graph;
+  return graph;
+}
+
+cudaGraphExec_t batch_graph(exogcm_engine* e, int K) {
+  auto it = e->graphs.find(K);
+  if (it != e->graphs.end()) return it->second;
+  cudaGraphExec_t exec;
+  check(cudaGraphInstantiate(&exec, captured_steps(e, K), 0), "graph instantiate");
   e->graphs[K] = exec;
   return exec;
+}
+
+// Step k of a batch, launched on the engine's stream.
+void launch_step(exogcm_engine* e, int k) {
+  Lanes on(e->stream, false);
+  full_step(e->model(k), on);
+  check(cudaGetLastError(), "step launch");
 }
 
 // The slot's table block [to.stride] in float, into `block`.
@@ -981,7 +1004,11 @@ void autotune(exogcm_engine* e) {
 // (engine, steps), whose nodes are the engines' K-step batch graphs as
 // child graphs. Engines being destroyed drop the group graphs they are in.
 std::mutex g_group_mutex;
-std::map<std::vector<std::pair<const exogcm_engine*, int>>, cudaGraphExec_t> g_group_graphs;
+struct GroupGraph {
+  cudaGraphExec_t exec = nullptr;
+  int batches = 0;  // submitted so far (kPlainBatches)
+};
+std::map<std::vector<std::pair<const exogcm_engine*, int>>, GroupGraph> g_group_graphs;
 
 void drop_group_graphs(const exogcm_engine* e) {
   std::lock_guard<std::mutex> lock(g_group_mutex);
@@ -989,7 +1016,7 @@ void drop_group_graphs(const exogcm_engine* e) {
     bool has = false;
     for (const auto& m : it->first) has = has || m.first == e;
     if (has) {
-      cudaGraphExecDestroy(it->second);
+      if (it->second.exec) cudaGraphExecDestroy(it->second.exec);
       it = g_group_graphs.erase(it);
     } else {
       ++it;
@@ -1005,6 +1032,7 @@ void drop_graphs(exogcm_engine* e) {
   for (auto& g : e->graph_templates) cudaGraphDestroy(g.second);
   e->graphs.clear();
   e->graph_templates.clear();
+  e->batches_of.clear();
 }
 
 // Retires the oldest batch in flight once its stream has passed it:
@@ -1394,9 +1422,12 @@ int exogcm_step_async(exogcm_engine* e, int steps, int publish_every) {
     check(cudaMemcpyAsync(e->params, rows, (size_t)steps * S * sizeof(StepParams), cudaMemcpyHostToDevice,
                           e->stream),
           "params upload");
-    cudaGraphExec_t g = batch_graph(e, steps);
+    cudaGraphExec_t g = ++e->batches_of[steps] > kPlainBatches ? batch_graph(e, steps) : nullptr;
     check(cudaEventRecord(B.start, e->stream), "event");
-    check(cudaGraphLaunch(g, e->stream), "graph launch");
+    if (g)
+      check(cudaGraphLaunch(g, e->stream), "graph launch");
+    else
+      for (int k = 0; k < steps; ++k) launch_step(e, k);
     check(cudaEventRecord(B.end, e->stream), "event");
     phy_finite_check(e->model(steps - 1), B.fault_host, e->stream);
     // start/end bracket the graph alone (the step time); done marks the
@@ -1447,8 +1478,7 @@ int exogcm_group_step(exogcm_engine** engines, int count, const int* steps, int 
     }
     exogcm_engine* lead = engines[0];
     cudaStream_t st = lead->stream;
-    // Each engine's step values, uploaded to its own parameter block; its
-    // K-step graph (captured once) becomes a child node of the group graph.
+    // Each engine's step values, uploaded to its own parameter block.
     for (int i = 0; i < count; ++i) {
       exogcm_engine* e = engines[i];
       const int S = e->d.S;
@@ -1458,29 +1488,43 @@ int exogcm_group_step(exogcm_engine** engines, int count, const int* steps, int 
       check(cudaMemcpyAsync(e->params, e->hparams, (size_t)steps[i] * S * sizeof(StepParams),
                             cudaMemcpyHostToDevice, st),
             "params upload");
-      batch_graph(e, steps[i]);
     }
     cudaGraphExec_t exec = nullptr;
+    bool graph = false;
     {
       std::lock_guard<std::mutex> lock(g_group_mutex);
-      auto it = g_group_graphs.find(key);
-      if (it != g_group_graphs.end()) exec = it->second;
+      GroupGraph& group = g_group_graphs[key];
+      exec = group.exec;
+      graph = ++group.batches > kPlainBatches;
     }
-    if (!exec) {
+    if (graph && !exec) {
+      // each engine's K steps (captured once) are a child node of the group graph
       cudaGraph_t parent;
       check(cudaGraphCreate(&parent, 0), "group graph");
       for (int i = 0; i < count; ++i) {
         cudaGraphNode_t node;
-        check(cudaGraphAddChildGraphNode(&node, parent, nullptr, 0, engines[i]->graph_templates.at(steps[i])),
+        check(cudaGraphAddChildGraphNode(&node, parent, nullptr, 0, captured_steps(engines[i], steps[i])),
               "group graph child");
       }
       check(cudaGraphInstantiate(&exec, parent, 0), "group graph instantiate");
       cudaGraphDestroy(parent);
       std::lock_guard<std::mutex> lock(g_group_mutex);
-      g_group_graphs[key] = exec;
+      g_group_graphs[key].exec = exec;
     }
     check(cudaEventRecord(lead->ev0, st), "event");
-    check(cudaGraphLaunch(exec, st), "group graph launch");
+    if (graph) {
+      check(cudaGraphLaunch(exec, st), "group graph launch");
+    } else {
+      // every engine on its own stream, between the lead's two events
+      for (int i = 1; i < count; ++i) check(cudaStreamWaitEvent(engines[i]->stream, lead->ev0), "group fork");
+      for (int k = 0; k < *std::max_element(steps, steps + count); ++k)
+        for (int i = 0; i < count; ++i)
+          if (k < steps[i]) launch_step(engines[i], k);
+      for (int i = 1; i < count; ++i) {
+        check(cudaEventRecord(engines[i]->ev1, engines[i]->stream), "event");
+        check(cudaStreamWaitEvent(st, engines[i]->ev1), "group join");
+      }
+    }
     check(cudaEventRecord(lead->ev1, st), "event");
     for (int i = 0; i < count; ++i) phy_finite_check(engines[i]->model(steps[i] - 1), nullptr, st);
     check(cudaStreamSynchronize(st), "group step");
