@@ -241,6 +241,11 @@ int exogcm_set_stop(exogcm_engine* engine, int slot, long step);
 /* Per-slot model step counter and start-up steps still to run. */
 int exogcm_slot_info(exogcm_engine* engine, int slot, long* step, int* startup_left, int* active);
 
+/* Device bytes a slot of this engine holds: its state fields, the step's
+ * scratch, and its tables, constants and step values. What a server counts
+ * against its budget. */
+int exogcm_slot_bytes(exogcm_engine* engine, size_t* bytes);
+
 /* Field readback / write by the reference's state field names
  * (LAYOUT.read / LAYOUT.write), one slot at a time, f32. */
 int exogcm_field_size(exogcm_engine* engine, const char* name, size_t* count);
@@ -352,7 +357,7 @@ void* exogcm_stream(exogcm_engine* engine);
 typedef struct exogcm_server exogcm_server;
 
 typedef struct exogcm_server_options {
-  double budget_bytes; /* device bytes the blocks' state may take */
+  double budget_bytes; /* device bytes the blocks' slots may take (exogcm_slot_bytes) */
   int block_slots;     /* slots of a T21 L5 block; fewer at larger resolutions, by footprint */
   int chunk_steps;     /* model steps per batch of a block (1..64) */
   int mode;            /* engine mode of every block (exogcm_create) */

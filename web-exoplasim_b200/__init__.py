@@ -108,6 +108,7 @@ SIGNATURES = {
     "exogcm_set_stop": (ctypes.c_int, [_VP, ctypes.c_int, ctypes.c_long]),
     "exogcm_slot_info": (ctypes.c_int, [_VP, ctypes.c_int, ctypes.POINTER(ctypes.c_long),
                                         ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]),
+    "exogcm_slot_bytes": (ctypes.c_int, [_VP, ctypes.POINTER(ctypes.c_size_t)]),
     "exogcm_field_size": (ctypes.c_int, [_VP, ctypes.c_char_p, ctypes.POINTER(ctypes.c_size_t)]),
     "exogcm_read_field": (ctypes.c_int, [_VP, ctypes.c_int, ctypes.c_char_p, _FP, ctypes.c_size_t]),
     "exogcm_write_field": (ctypes.c_int, [_VP, ctypes.c_int, ctypes.c_char_p, _FP, ctypes.c_size_t]),
@@ -363,6 +364,12 @@ class Engine:
 
     def run_stage(self, stage: str) -> None:
         _check(_lib.exogcm_run_stage(self.h, stage.encode()))
+
+    def slot_bytes(self) -> int:
+        """Device bytes a slot of this engine holds."""
+        n = ctypes.c_size_t()
+        _check(_lib.exogcm_slot_bytes(self.h, ctypes.byref(n)))
+        return n.value
 
     def field_size(self, name: str) -> int:
         n = ctypes.c_size_t()

@@ -92,7 +92,6 @@ struct exogcm_engine {
   std::map<std::string, size_t> field_index;
   float* arena = nullptr;
   size_t arena_floats = 0;
-  size_t state_floats = 0;    // the fields'
   size_t scratch_offset = 0;  // mkdheat's scratch
   FieldPtrs fp{};
   // shared tables
@@ -217,7 +216,6 @@ void layout(exogcm_engine* e) {
     EXOGCM_FIELDS(EXOGCM_ADD_FIELD)
   }
 #undef EXOGCM_ADD_FIELD
-  e->state_floats = off;
   // mkdheat's scratch behind the state fields: two grid, two Fourier fields
   off = (off + 63) / 64 * 64;
   e->scratch_offset = off;
@@ -1703,6 +1701,14 @@ int exogcm_field_size(exogcm_engine* e, const char* name, size_t* count) {
     if (!e || !count) throw Error(EXOGCM_EINVAL, "null argument");
     const FieldInfo& fi = field(e, name);
     *count = fi.plane * fi.count;
+  });
+}
+
+int exogcm_slot_bytes(exogcm_engine* e, size_t* bytes) {
+  return guard([&] {
+    if (!e || !bytes) throw Error(EXOGCM_EINVAL, "null argument");
+    *bytes = (e->arena_floats + e->d.S - 1) / e->d.S * sizeof(float) + e->to.stride * sizeof(float) +
+             sizeof(PlanetConst) + kMaxBatch * sizeof(StepParams) + (kBudgetStride + 4) * sizeof(double) + sizeof(int);
   });
 }
 

@@ -26,7 +26,6 @@
 #include <vector>
 
 #include "../../include/exogcm.h"
-#include "fields.h"
 
 namespace exogcm {
 void set_error(const std::string& message);  // engine.cu
@@ -116,32 +115,20 @@ struct exogcm_server {
     }
   }
 
-  // Device bytes one slot of a (T, L) engine holds: every state field of
-  // the layout (fields.h), counted on a one-slot engine once, and its
-  // per-slot tables.
+  // Device bytes one slot of a (T, L) engine holds, asked of a one-slot
+  // engine once.
   double bytes_per_slot(int T, int L) {
     const auto key = std::make_pair(T, L);
     auto it = slot_bytes.find(key);
     if (it != slot_bytes.end()) return it->second;
     exogcm_engine* probe = nullptr;
     call(exogcm_create(T, L, 1, opt.mode, &probe), "server: engine");
-    size_t total = 0;
-#define EXOGCM_SERVER_FIELD(name, shape, count) #name,
-    static const char* const names[] = {EXOGCM_FIELDS(EXOGCM_SERVER_FIELD)};
-#undef EXOGCM_SERVER_FIELD
-    for (const char* name : names) {
-      size_t n = 0;
-      const int status = exogcm_field_size(probe, name, &n);
-      if (status != EXOGCM_OK) {
-        exogcm_destroy(probe);
-        call(status, "server: field size");
-      }
-      total += n;
-    }
+    size_t bytes = 0;
+    const int status = exogcm_slot_bytes(probe, &bytes);
     exogcm_destroy(probe);
-    const double bytes = (double)total * sizeof(float) + 64 * 1024;
-    slot_bytes[key] = bytes;
-    return bytes;
+    call(status, "server: slot bytes");
+    slot_bytes[key] = (double)bytes;
+    return (double)bytes;
   }
 
   // Slots of a new block: `block_slots` at T21 L5, fewer at larger

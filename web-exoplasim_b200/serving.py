@@ -58,23 +58,12 @@ class Request:
 
 
 def slot_bytes(truncation: int, levels: int) -> int:
-    """Device bytes one slot of a (T, L) engine holds (state plus tables)."""
+    """Device bytes one slot of a (T, L) engine holds."""
     e = pkg.Engine(truncation, levels, 1)
     try:
-        names = [n for n in FIELD_NAMES]
-        return sum(e.field_size(n) for n in names) * 4 + 64 * 1024
+        return e.slot_bytes()
     finally:
         e.close()
-
-
-FIELD_NAMES: list[str] = []
-
-
-def _field_names():
-    import os
-    import re
-    src = os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc", "fields.h")
-    return re.findall(r"X\((\w+),[SFGT],", open(src).read())
 
 
 class Group:
@@ -337,11 +326,8 @@ _SLOT_BYTES: dict = {}
 
 
 def slot_bytes_cached(truncation: int, levels: int) -> int:
-    global FIELD_NAMES
     key = (truncation, levels)
     if key not in _SLOT_BYTES:
-        if not FIELD_NAMES:
-            FIELD_NAMES = _field_names()
         _SLOT_BYTES[key] = slot_bytes(truncation, levels)
     return _SLOT_BYTES[key]
 
