@@ -29,7 +29,9 @@
 #include <vector>
 
 #include "../../include/exogcm.h"
+#include "capture.h"
 #include "common.cuh"
+#include "error.h"
 #include "launch.h"
 #include "setup.h"
 
@@ -46,15 +48,6 @@ void set_error(const std::string& message) { g_error = message; }
 }  // namespace exogcm
 
 namespace {
-
-struct Error : std::runtime_error {
-  int code;
-  Error(int c, const std::string& m) : std::runtime_error(m), code(c) {}
-};
-
-void check(cudaError_t e, const char* what) {
-  if (e != cudaSuccess) throw Error(EXOGCM_EDEVICE, std::string(what) + ": " + cudaGetErrorString(e));
-}
 
 struct FieldInfo {
   std::string name;
@@ -720,17 +713,21 @@ StepParams next_params(Slot& s, int publish_every, bool advance) {
 // 1,790 / 519, 320; two of 37 T21 L10 2,060 / 852, 683.
 constexpr int kPlainBatches = 1;
 
-// K steps captured as a graph, kept for later batches and group graphs.
+// K steps captured as a graph.
+void capture_steps(exogcm_engine* e, int K, Graph& graph) {
+  Capture capture(e->stream);
+  Lanes on(e->stream, true);
+  for (int k = 0; k < K; ++k) full_step(e->model(k), on);
+  capture.end(graph);
+}
+
+// The same, kept for later batches and group graphs.
 cudaGraph_t captured_steps(exogcm_engine* e, int K) {
   auto it = e->graph_templates.find(K);
   if (it != e->graph_templates.end()) return it->second;
-  cudaGraph_t graph;
-  check(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed), "capture");
-  Lanes on(e->stream, true);
-  for (int k = 0; k < K; ++k) full_step(e->model(k), on);
-  check(cudaStreamEndCapture(e->stream, &graph), "capture end");
-  e->graph_templates[K] = graph;
-  return graph;
+  Graph graph;
+  capture_steps(e, K, graph);
+  return e->graph_templates[K] = graph.release();
 }
 
 cudaGraphExec_t batch_graph(exogcm_engine* e, int K) {
@@ -1497,15 +1494,14 @@ int exogcm_group_step(exogcm_engine** engines, int count, const int* steps, int 
     }
     if (graph && !exec) {
       // each engine's K steps (captured once) are a child node of the group graph
-      cudaGraph_t parent;
-      check(cudaGraphCreate(&parent, 0), "group graph");
+      Graph parent;
+      check(cudaGraphCreate(parent.out(), 0), "group graph");
       for (int i = 0; i < count; ++i) {
         cudaGraphNode_t node;
-        check(cudaGraphAddChildGraphNode(&node, parent, nullptr, 0, captured_steps(engines[i], steps[i])),
+        check(cudaGraphAddChildGraphNode(&node, parent.get(), nullptr, 0, captured_steps(engines[i], steps[i])),
               "group graph child");
       }
-      check(cudaGraphInstantiate(&exec, parent, 0), "group graph instantiate");
-      cudaGraphDestroy(parent);
+      check(cudaGraphInstantiate(&exec, parent.get(), 0), "group graph instantiate");
       std::lock_guard<std::mutex> lock(g_group_mutex);
       g_group_graphs[key].exec = exec;
     }
@@ -2018,14 +2014,10 @@ int exogcm_tuning(exogcm_engine* e, int* values, int count) {
 int exogcm_graph_launches(exogcm_engine* e, int steps, size_t* launches) {
   return guard([&] {
     if (!e || !launches || steps < 1 || steps > kMaxBatch) throw Error(EXOGCM_EINVAL, "bad argument");
-    cudaGraph_t graph;
-    check(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed), "capture");
-    Lanes on(e->stream, true);
-    for (int k = 0; k < steps; ++k) full_step(e->model(k), on);
-    check(cudaStreamEndCapture(e->stream, &graph), "capture end");
+    Graph graph;
+    capture_steps(e, steps, graph);
     size_t n = 0;
-    check(cudaGraphGetNodes(graph, nullptr, &n), "graph nodes");
-    cudaGraphDestroy(graph);
+    check(cudaGraphGetNodes(graph.get(), nullptr, &n), "graph nodes");
     *launches = n;
   });
 }
