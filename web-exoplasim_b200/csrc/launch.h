@@ -7,49 +7,9 @@
 #include <vector>
 
 #include "common.cuh"
+#include "transform_set.h"
 
 namespace exogcm {
-
-// A set of fields one transform launch works through: independent planes of
-// several fields in one grid, so that a step pays one launch, one ramp and
-// one tail for all of them. What the pointers mean is each transform's own.
-struct TrField {
-  const float* a = nullptr;
-  const float* b = nullptr;
-  const float* c = nullptr;
-  float* x = nullptr;
-  float* y = nullptr;
-  int planes = 0;
-  int opt = 0;
-  float plavor = 0.f;
-};
-constexpr int kMaxTr = 12;
-struct TrSet {
-  int n = 0;
-  int at[kMaxTr + 1] = {};  // first tile of each field (tr_tiles)
-  TrField f[kMaxTr];
-  void add(const TrField& t) { f[n++] = t; }
-};
-// Numbers the tiles of `tile` planes of the set's fields one after another
-// (no tile spans two fields); returns their count.
-inline int tr_tiles(TrSet& s, int tile) {
-  s.at[0] = 0;
-  for (int i = 0; i < s.n; ++i) s.at[i + 1] = s.at[i] + (s.f[i].planes + tile - 1) / tile;
-  return s.at[s.n];
-}
-#ifdef __CUDACC__
-// The field of a tile; tile - s.at[field] is the tile's number in it.
-__device__ __forceinline__ int tr_find(const TrSet& s, int tile) {
-  int f = 0;
-  while (f + 1 < s.n && tile >= s.at[f + 1]) ++f;
-  return f;
-}
-#endif
-
-// Options of a spectral -> grid field (TrField::opt).
-constexpr int kTrDerivative = 1;  // sp2fcdmu: the d/dmu table
-constexpr int kTrDlambda = 2;     // d/dlambda of the Fourier coefficients before fc2gp
-constexpr int kTrKeep = 4;        // the Fourier field is written whatever Model::keep_fourier
 
 // transforms.cu
 void tr_init();

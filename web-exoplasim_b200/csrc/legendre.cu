@@ -545,7 +545,7 @@ void launch_inverse(const Model& m, TrSet set, const float* qa, const float* qb,
 
 // sp2fc of fields of one table (opt: kTrDerivative, the same for all).
 void leg_inverse(const Model& m, const TrSet& s, cudaStream_t st) {
-  const bool derivative = (s.f[0].opt & kTrDerivative) != 0;
+  const bool derivative = tr_every(s, [](const TrField& t) { return (t.opt & kTrDerivative) != 0; });
   launch_inverse<0>(m, s, derivative ? m.sh.qjT : m.sh.qiT, nullptr, derivative ? 1 : 0, st);
 }
 
@@ -594,7 +594,7 @@ Tuning default_tuning(const Dims& d) {
 void leg_forward(const Model& m, const TrSet& s, cudaStream_t st) { launch_sym_forward<0, 1>(m, s, st); }
 
 void leg_uv2dv(const Model& m, const TrSet& s, cudaStream_t st) {
-  if (s.f[0].c)
+  if (tr_every(s, [](const TrField& t) { return t.c != nullptr; }))
     launch_sym_forward<2, 3>(m, s, st);
   else
     launch_sym_forward<1, 2>(m, s, st);

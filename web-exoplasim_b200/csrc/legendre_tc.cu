@@ -908,7 +908,7 @@ void tc_dv2uv(const Model& m, const TrSet& s, cudaStream_t st) { launch<DV2UV>(m
 void tc_forward(const Model& m, const TrSet& s, cudaStream_t st) { launch<FWD>(m, s, SET_FC2SP, st); }
 
 void tc_uv2dv(const Model& m, const TrSet& s, cudaStream_t st) {
-  if (s.f[0].c)
+  if (tr_every(s, [](const TrField& t) { return t.c != nullptr; }))
     launch<MKTEND>(m, s, SET_MKTEND, st);
   else
     launch<UV2DV>(m, s, SET_UV2DV, st);

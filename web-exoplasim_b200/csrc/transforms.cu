@@ -301,6 +301,7 @@ void tr_spectral_part(const Model& m, const TrSet& s, cudaStream_t st) {
     const float* from = nullptr;
     for (int k = 0; k < s.n; ++k)
       if (s.f[k].a == s.f[i].a && !(s.f[k].opt & (kTrDlambda | kTrDerivative))) from = s.f[k].x;
+    if (!from) throw std::logic_error("transform launch: d/dlambda of a field not in the set");
     dlambda(m, from, s.f[i].x, s.f[i].planes, st);
   }
 }
