@@ -145,7 +145,8 @@ int exogcm_release(exogcm_engine* engine, int slot);
 /* Runs `steps` model steps for every active slot (STEPPER.batch,
  * stepper/index.ts:203-276): per-step CPU values computed on the host,
  * uploaded once, then the whole batch as one CUDA graph (an engine's first
- * batch of a length kernel by kernel). A slot whose step number is a multiple
+ * batch of a length kernel by kernel; exogcm_step_async's, above 16 steps, as
+ * a graph of steps in order). A slot whose step number is a multiple
  * of `publish_every` packs its snapshot on that step.
  * `steps` must not exceed `publish_every` so a slot publishes at most once.
  * Returns when the batch is done (exogcm_step_async + exogcm_wait). */

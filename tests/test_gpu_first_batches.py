@@ -69,3 +69,39 @@ def test_a_new_engines_first_batch_waits_for_no_graph():
         e.close()
         ratios.append(times[0] / np.median(times[6:]))
     assert np.median(ratios) < 3, ratios
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_first_and_later_long_batches_of_a_submitting_call_give_the_same_state(mode):
+    """Beyond what the launch queue takes, the first batch is a graph of steps in order."""
+    e = engine(21, 5, 2, mode)
+
+    def batch():
+        e.step_async(17, publish_every=17)
+        e.wait()
+
+    try:
+        first, *later = states_after_batches([e], batch, 2)
+        for state in later:
+            assert [k for k in first if not np.array_equal(first[k], state[k], equal_nan=True)] == []
+    finally:
+        e.close()
+
+
+@pytest.mark.parametrize("steps", [16, 64])
+def test_submitting_a_first_batch_does_not_wait_for_it(steps):
+    """The share of the batch's time the call takes: 0.13 and 0.2; launched
+    kernel by kernel 64 steps fill the launch queue, and the call takes 0.65."""
+    shares = []
+    for _ in range(3):
+        e = pkg.Engine(42, 10, 32, mode=1)
+        for s in range(32):
+            e.configure(s, planets.make_planet(61, truncation=42, levels=10))
+        e.step(3)
+        t = time.perf_counter()
+        e.step_async(steps)
+        submitted = time.perf_counter()
+        e.wait()
+        shares.append((submitted - t) / (time.perf_counter() - t))
+        e.close()
+    assert np.median(shares) < 0.4, shares

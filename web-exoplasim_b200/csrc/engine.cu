@@ -124,7 +124,7 @@ struct exogcm_engine {
   float* snap_stage = nullptr;  // device copy of the snapshot field
   bool copy_pending = false;
   std::vector<Slot> slots;
-  std::map<int, cudaGraphExec_t> graphs;
+  std::map<std::pair<int, bool>, cudaGraphExec_t> graphs;  // of K steps, with a step's side chains or without
   std::map<int, cudaGraph_t> graph_templates;  // the captured K-step graphs (child nodes of group graphs)
   std::map<int, int> batches_of;  // batches of K steps submitted so far (kPlainBatches)
   Tuning tune{};
@@ -713,10 +713,16 @@ StepParams next_params(Slot& s, int publish_every, bool advance) {
 // 1,790 / 519, 320; two of 37 T21 L10 2,060 / 852, 683.
 constexpr int kPlainBatches = 1;
 
+// Steps launched kernel by kernel that the device's launch queue takes while
+// it is busy, so that a call that only submits returns before they have run
+// (1,024 launches; a step is 45 to 47). A longer first batch of such a call is
+// a graph of steps in order, whose instantiation is cheap.
+constexpr int kQueuedSteps = 16;
+
 // K steps captured as a graph.
-void capture_steps(exogcm_engine* e, int K, Graph& graph) {
+void capture_steps(exogcm_engine* e, int K, bool sides, Graph& graph) {
   Capture capture(e->stream);
-  Lanes on(e->stream, true);
+  Lanes on(e->stream, sides);
   for (int k = 0; k < K; ++k) full_step(e->model(k), on);
   capture.end(graph);
 }
@@ -726,16 +732,18 @@ cudaGraph_t captured_steps(exogcm_engine* e, int K) {
   auto it = e->graph_templates.find(K);
   if (it != e->graph_templates.end()) return it->second;
   Graph graph;
-  capture_steps(e, K, graph);
+  capture_steps(e, K, true, graph);
   return e->graph_templates[K] = graph.release();
 }
 
-cudaGraphExec_t batch_graph(exogcm_engine* e, int K) {
-  auto it = e->graphs.find(K);
+cudaGraphExec_t batch_graph(exogcm_engine* e, int K, bool sides) {
+  auto it = e->graphs.find({K, sides});
   if (it != e->graphs.end()) return it->second;
+  Graph in_order;
+  if (!sides) capture_steps(e, K, false, in_order);
   cudaGraphExec_t exec;
-  check(cudaGraphInstantiate(&exec, captured_steps(e, K), 0), "graph instantiate");
-  e->graphs[K] = exec;
+  check(cudaGraphInstantiate(&exec, sides ? captured_steps(e, K) : in_order.get(), 0), "graph instantiate");
+  e->graphs[{K, sides}] = exec;
   return exec;
 }
 
@@ -1397,7 +1405,11 @@ int exogcm_release(exogcm_engine* e, int slot) {
   });
 }
 
-int exogcm_step_async(exogcm_engine* e, int steps, int publish_every) {
+}  // extern "C"
+
+namespace {
+// Submits a batch; `waits`: the call returns when it has run.
+int submit(exogcm_engine* e, int steps, int publish_every, bool waits) {
   return guard([&] {
     if (!e) throw Error(EXOGCM_EINVAL, "null engine");
     if (steps < 1 || steps > kMaxBatch) throw Error(EXOGCM_EINVAL, "steps must be 1..64");
@@ -1417,7 +1429,9 @@ int exogcm_step_async(exogcm_engine* e, int steps, int publish_every) {
     check(cudaMemcpyAsync(e->params, rows, (size_t)steps * S * sizeof(StepParams), cudaMemcpyHostToDevice,
                           e->stream),
           "params upload");
-    cudaGraphExec_t g = ++e->batches_of[steps] > kPlainBatches ? batch_graph(e, steps) : nullptr;
+    const bool first = ++e->batches_of[steps] <= kPlainBatches;
+    cudaGraphExec_t g = nullptr;
+    if (!first || (!waits && steps > kQueuedSteps)) g = batch_graph(e, steps, !first);
     check(cudaEventRecord(B.start, e->stream), "event");
     if (g)
       check(cudaGraphLaunch(g, e->stream), "graph launch");
@@ -1431,6 +1445,12 @@ int exogcm_step_async(exogcm_engine* e, int steps, int publish_every) {
     e->pending.push_back(b);
   });
 }
+
+}  // namespace
+
+extern "C" {
+
+int exogcm_step_async(exogcm_engine* e, int steps, int publish_every) { return submit(e, steps, publish_every, false); }
 
 int exogcm_poll(exogcm_engine* e, int* done) {
   return guard([&] {
@@ -1449,7 +1469,7 @@ int exogcm_wait(exogcm_engine* e) {
 }
 
 int exogcm_step(exogcm_engine* e, int steps, int publish_every) {
-  const int rc = exogcm_step_async(e, steps, publish_every);
+  const int rc = submit(e, steps, publish_every, true);
   if (rc != EXOGCM_OK) return rc;
   return exogcm_wait(e);
 }
@@ -2015,7 +2035,7 @@ int exogcm_graph_launches(exogcm_engine* e, int steps, size_t* launches) {
   return guard([&] {
     if (!e || !launches || steps < 1 || steps > kMaxBatch) throw Error(EXOGCM_EINVAL, "bad argument");
     Graph graph;
-    capture_steps(e, steps, graph);
+    capture_steps(e, steps, true, graph);
     size_t n = 0;
     check(cudaGraphGetNodes(graph.get(), nullptr, &n), "graph nodes");
     *launches = n;
