@@ -160,16 +160,22 @@ struct exogcm_engine {
     m.fzdu1 = m.zdv1 + grid;
     m.fzdv1 = m.fzdu1 + four;
     // Programmatic dependent launch. A dependent's waiting blocks are placed
-    // where there is room while its predecessor drains: that hides the launch,
-    // but packs a grid of one to three blocks per SM unevenly. us a step, column
-    // kernels without / with it, at columns: 8,192 (one T42 L10 planet)
-    // 150.5 / 149.3, 16,384 190 / 196, 18,432 288 / 299, 40,960 260 / 272,
-    // 49,152 266 / 276, 57,344 209 / 202, 131,072 487 / 483, 1,048,576 3109 /
-    // 3090. Everything else has it at every size (75,776 columns 342 -> 319,
+    // where there is room while its predecessor drains. That hides the launch,
+    // and gains where launches are most of a step (the smallest grids) and
+    // where grids run for several waves. Between, from a half to five blocks
+    // of 128 columns per SM, the step with it is the longer one, in most sizes by
+    // 2 to 7 %, so the column kernels there launch the ordinary way. us a step,
+    // column kernels without / with it, at columns (levels): 2,048 (10) 116 /
+    // 113, 4,096 (10) 118 / 116, 6,144 (10) 123 / 129, 8,192 (5) 111 / 114, 8,192
+    // (10) 143 / 142, 18,432 (10) 209 / 219, 53,248 (10) 244 / 255, 65,536 (10) 275
+    // / 293, 73,728 (10) 354 / 373, 98,304 (10) 389 / 397, 131,072 (5) 265 / 266,
+    // 131,072 (10) 473 / 469, 196,608 (10) 627 / 613, 589,824 (10) 1940 / 1906,
+    // 1,048,576 (10) 2969 / 2958; the lines are halfway between the sizes on their
+    // two sides. Everything else has it at every size (75,776 columns 342 -> 319,
     // 196,608 392 -> 372, 1,048,576 3108 -> 3090).
     const long columns = (long)d.S * d.NHOR;
     m.pdl = 1;
-    m.column_pdl = columns <= 8192 || columns > 53248 ? 1 : 0;
+    m.column_pdl = columns <= 5120 || columns > 114688 ? 1 : 0;
     m.storm = 0;
     for (const Slot& s : slots) m.storm |= s.storm ? 1 : 0;
     return m;
