@@ -689,7 +689,7 @@ void dyn_mkdheat_mean(const Model& m, cudaStream_t st) {
   // 4 kCols4 = 2,048 divides NHOR; four runs a block once that leaves several
   // blocks per SM
   const size_t runs = (size_t)m.d.S * m.d.NHOR / kCols4;
-  const int chunks = runs * m.d.NLEV >= 148 * 32 ? 4 : 1;
+  const int chunks = runs * m.d.NLEV >= (size_t)sm_count() * 32 ? 4 : 1;
   const dim3 grid((unsigned)(runs / chunks), m.d.NLEV);
   // mode 1 leaves the Fourier fields between fused transforms unwritten
   const int fourier = m.mode != 1 || m.keep_fourier;

@@ -91,7 +91,7 @@ struct exogcm_engine {
   bool shared_ready = false;
   int filter_kind = -1, filter_gp = -1, filter_sp = -1;
   float* shared_buf = nullptr;
-  int* mode_buf = nullptr;
+  int* tc_at_buf = nullptr;
   SharedTabs sh{};
   // per-slot tables and constants
   TabOffsets to{};
@@ -320,14 +320,10 @@ void upload_shared(exogcm_engine* e, const SharedSetup& s) {
     rcsq[h] = 1 / (1 - sn * sn);
   }
   for (int l = 0; l < d.NLAT; ++l) cola[l] = std::sqrt(1 - s.sines[l] * s.sines[l]);
-  std::vector<int> mm(d.NCSP), nn(d.NCSP);
   {
-    int w = 0, r = 0;
+    int r = 0;
     for (int m = 0; m <= d.T; ++m)
       for (int n = m; n <= d.T; ++n) {
-        mm[w] = m;
-        nn[w] = n;
-        ++w;
         nindex[r] = nindex[r + 1] = n;
         r += 2;
       }
@@ -355,7 +351,6 @@ void upload_shared(exogcm_engine* e, const SharedSetup& s) {
   // Tensor-core transforms (mode 2): hi/lo images of every table operand per m.
   std::vector<int> tc_at;
   const std::vector<float> img = e->mode == 2 ? tc_table_images(d, s.q, tc_at) : std::vector<float>();
-  if (tc_at.empty()) tc_at.assign(1, 0);
   auto put_floats = [&](const std::vector<float>& v) {
     while (buf.size() % 32) buf.push_back(0.f);
     const size_t at = buf.size();
@@ -366,11 +361,10 @@ void upload_shared(exogcm_engine* e, const SharedSetup& s) {
   const size_t igi = put_floats(grid_tables[0]), igj = put_floats(grid_tables[1]);
   check(cudaMalloc(&e->shared_buf, buf.size() * sizeof(float)), "shared tables");
   check(cudaMemcpy(e->shared_buf, buf.data(), buf.size() * sizeof(float), cudaMemcpyHostToDevice), "shared tables");
-  check(cudaMalloc(&e->mode_buf, (2 * d.NCSP + tc_at.size()) * sizeof(int)), "mode tables");
-  check(cudaMemcpy(e->mode_buf, mm.data(), d.NCSP * sizeof(int), cudaMemcpyHostToDevice), "mode tables");
-  check(cudaMemcpy(e->mode_buf + d.NCSP, nn.data(), d.NCSP * sizeof(int), cudaMemcpyHostToDevice), "mode tables");
-  check(cudaMemcpy(e->mode_buf + 2 * d.NCSP, tc_at.data(), tc_at.size() * sizeof(int), cudaMemcpyHostToDevice),
-        "mode tables");
+  if (!tc_at.empty()) {
+    check(cudaMalloc(&e->tc_at_buf, tc_at.size() * sizeof(int)), "table offsets");
+    check(cudaMemcpy(e->tc_at_buf, tc_at.data(), tc_at.size() * sizeof(int), cudaMemcpyHostToDevice), "table offsets");
+  }
   float* b = e->shared_buf;
   e->sh.fwd = b + fwd;
   e->sh.inv = b + inv;
@@ -398,9 +392,7 @@ void upload_shared(exogcm_engine* e, const SharedSetup& s) {
   e->sh.qiG = b + igi;
   e->sh.qjG = b + igj;
   e->sh.tc_img = b + itc;
-  e->sh.tc_at = e->mode_buf + 2 * d.NCSP;
-  e->sh.mode_m = e->mode_buf;
-  e->sh.mode_n = e->mode_buf + d.NCSP;
+  e->sh.tc_at = e->tc_at_buf;
   e->shared_ready = true;
 }
 
@@ -1154,7 +1146,7 @@ void exogcm_destroy(exogcm_engine* e) {
   for (auto& g : e->graph_templates) cudaGraphDestroy(g.second);
   cudaFree(e->arena);
   cudaFree(e->shared_buf);
-  cudaFree(e->mode_buf);
+  cudaFree(e->tc_at_buf);
   cudaFree(e->tabs);
   cudaFree(e->pc);
   cudaFree(e->params);

@@ -40,6 +40,7 @@ void tr_qtend(const Model& m, TrSet s, cudaStream_t st);
 constexpr size_t kLegSmemLimit = 200 * 1024;  // dynamic shared memory the transform kernels may ask
 void leg_init();
 // Resident blocks of `kernel` per SM for a launch shape, times the SM count.
+int sm_count();
 int persistent_grid(const void* kernel, int threads, size_t smem);
 size_t leg_inverse_smem(const Dims& d, int kind, int group, int tile);
 size_t leg_forward_smem(const Dims& d, int kind, int tile);
@@ -96,7 +97,6 @@ void lev_kuo(const Model& m, cudaStream_t st);
 // physics_flux.cu (IEEE division): fixer apply, surface fluxes, vdiff, solang/mko3
 void phy_fixer_apply(const Model& m, cudaStream_t st);
 void phy_solang_mko3(const Model& m, cudaStream_t st);
-void phy_fused_fixer_flux_solang(const Model& m, cudaStream_t st);
 bool phy_flux_launch_one(const Model& m, const std::string& kernel, cudaStream_t st);
 
 // physics.cu

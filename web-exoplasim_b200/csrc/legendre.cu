@@ -492,18 +492,22 @@ size_t forward_smem_for(const Dims& d, int tile) {
 
 }  // namespace
 
+int sm_count() {
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n;
+  }();
+  return sms;
+}
+
 // The persistent grid: resident blocks per SM for a launch shape, times
 // the SM count.
 int persistent_grid(const void* kernel, int threads, size_t smem) {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  }
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-  return sms * (per_sm > 0 ? per_sm : 1);
+  return sm_count() * (per_sm > 0 ? per_sm : 1);
 }
 
 template <int KIND, int NIN, int NB>

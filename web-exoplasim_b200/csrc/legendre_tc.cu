@@ -737,16 +737,6 @@ CUtensorMap map_2d(const float* field, int plane_floats, int planes, int box, in
   return map;
 }
 
-int sm_count() {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  }
-  return sms;
-}
-
 template <int KIND>
 TcGeom geometry(const Dims& d, int tiles) {
   using S = Shape<KIND>;

@@ -56,26 +56,24 @@ __device__ __forceinline__ void tree_sums(double (*s)[kSumThreads], int half, in
   }
 }
 
-// Per-slot global sums of two grid fields in FP64 with a fixed order (the
-// reference's reduction/wgsl/sum.wgsl, kept in double as the build asks of
-// global budget reductions), a half of the block each. Writes the sums as
-// floats to target[0|1 * S + slot] and as doubles to sums[slot * 4 + which * 2
-// + 0|1].
-__global__ void __launch_bounds__(2 * kSumThreads) k_slot_sums(Model m, const float* a, const float* b, float* target,
-                                                               int which) {
+// getiflx's global sums of two grid fields per slot, in FP64 with a fixed
+// order (the reference's reduction/wgsl/sum.wgsl, kept in double as the build
+// asks of global budget reductions), a half of the block each. Writes the sums
+// as floats to ice_sums[0|1 * S + slot] and as doubles to sums[slot * 4 + 2|3].
+__global__ void __launch_bounds__(2 * kSumThreads) k_slot_sums(Model m) {
   __shared__ double s[2][kSumThreads];
   pdl_wait();
   pdl_release();
   const Dims& d = m.d;
   const int slot = blockIdx.x;
   if (!m.params[slot].active) return;
-  if (which == 1 && m.params[slot].coupled == 0.f) return;  // getiflx runs with icestep only
+  if (m.params[slot].coupled == 0.f) return;  // getiflx runs with icestep only
   const int half = threadIdx.x / kSumThreads, t = threadIdx.x % kSumThreads;
-  s[half][t] = strided_sum((half ? b : a) + (size_t)slot * d.NHOR + t, d.NHOR / kSumThreads);
+  s[half][t] = strided_sum((half ? m.f.ice_part2 : m.f.ice_part1) + (size_t)slot * d.NHOR + t, d.NHOR / kSumThreads);
   tree_sums(s, half, t, true);
   if (t == 0) {
-    target[half * d.S + slot] = (float)s[half][0];
-    m.sums[slot * 4 + which * 2 + half] = s[half][0];
+    m.f.ice_sums[half * d.S + slot] = (float)s[half][0];
+    m.sums[slot * 4 + 2 + half] = s[half][0];
   }
 }
 
@@ -2059,7 +2057,7 @@ void phy_surface(const Model& m, cudaStream_t st) {
   step_launch(m.pdl, k_mkradv, nblocks((size_t)m.d.S * m.d.NHOR, kBlock), kBlock, 0, st, m);
   by_levels<LandSurface>(m.d.L, m, st);
   by_levels<SeaIce>(m.d.L, m, st);
-  step_launch(m.pdl, k_slot_sums, m.d.S, 2 * kSumThreads, 0, st, m, m.f.ice_part1, m.f.ice_part2, m.f.ice_sums, 1);
+  step_launch(m.pdl, k_slot_sums, m.d.S, 2 * kSumThreads, 0, st, m);
   by_levels<Sea>(m.d.L, m, st);
 }
 
@@ -2081,7 +2079,7 @@ void phy_fused_surface_to_carbon(const Model& m, cudaStream_t st) {
   by_levels<Soil>(m.d.L, m, st);
   step_launch(m.pdl, k_mkradv, nblocks((size_t)m.d.S * m.d.NHOR, kBlock), kBlock, 0, st, m);
   by_levels<FusedLandSeaice>(m.d.L, m, st);
-  step_launch(m.pdl, k_slot_sums, m.d.S, 2 * kSumThreads, 0, st, m, m.f.ice_part1, m.f.ice_part2, m.f.ice_sums, 1);
+  step_launch(m.pdl, k_slot_sums, m.d.S, 2 * kSumThreads, 0, st, m);
   by_levels<FusedSeaCarbon>(m.d.L, m, st);
 }
 

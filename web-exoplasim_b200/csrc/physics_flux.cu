@@ -142,10 +142,10 @@ __global__ void __launch_bounds__(kBlock) k_surflx(Model m, const PlanetConst* _
 // HOLD: which levels of the tendencies dtdt, dqdt, dudt, dvdt hold values on
 // entry: 1 every level (stage replay, Model::zero_gdt), 0 only the lowest
 // (within a full step, where physics_in's zeros are taken as values and
-// surflx raised the lowest level), -1 decided at run time from zero_gdt.
+// surflx raised the lowest level).
 // With HOLD = 0 the other levels' tendencies are the constant 0 and need no
 // registers.
-template <int NL, int HOLD = -1>
+template <int NL, int HOLD>
 __device__ __forceinline__ void b_vdiff(const Model& m, const PlanetConst* __restrict__ pcr, const float* __restrict__ tabr) {
   COLUMN_PROLOGUE
   const float* ds = tb + m.to.dsigma;
@@ -153,10 +153,9 @@ __device__ __forceinline__ void b_vdiff(const Model& m, const PlanetConst* __res
   const float* skap = tb + m.to.vdiff_skap;
   const float* skaph = tb + m.to.vdiff_skaph;
   const float D2 = P.deltsec2;
-  const bool all_held = HOLD < 0 ? m.zero_gdt != 0 : HOLD == 1;
   // An incoming tendency: every level in stage replay; within a full step
   // only the lowest holds more than physics_in's zeros (Model::zero_gdt).
-  auto tend = [&](const float* f, int l) { return all_held || l == NL - 1 ? f[l * SN + c] : 0.f; };
+  auto tend = [&](const float* f, int l) { return HOLD == 1 || l == NL - 1 ? f[l * SN + c] : 0.f; };
   // The routine runs in three phases so that few level columns are live at
   // once: the exchange coefficients, then humidity and temperature (whose
   // profiles are then dropped), then the winds and the dissipative heating,
@@ -322,19 +321,6 @@ __global__ void __launch_bounds__(kBlock) k_solang_mko3(Model m, const PlanetCon
   b_solang_mko3<NL>(m, pcr, tabr);
 }
 
-
-
-// The full step's fused kernel: fixer apply, surface fluxes, vertical
-// diffusion, solar angle and ozone for one column per thread.
-template <int NL>
-__global__ void __launch_bounds__(kBlock, 3) k_fused_fixer_flux_solang(Model m, const PlanetConst* __restrict__ pcr,
-                                                                       const float* __restrict__ tabr) {
-  b_fixer_apply<NL>(m, pcr, tabr);
-  b_surflx<NL>(m, pcr, tabr);
-  b_vdiff<NL>(m, pcr, tabr);
-  b_solang_mko3<NL>(m, pcr, tabr);
-}
-
 COLUMN_LAUNCHER(FixerApply, k_fixer_apply)
 COLUMN_LAUNCHER(Surflx, k_surflx)
 template <int NL>
@@ -348,7 +334,6 @@ struct Vdiff {
   }
 };
 COLUMN_LAUNCHER(SolangMko3, k_solang_mko3)
-COLUMN_LAUNCHER(FusedFixerFluxSolang, k_fused_fixer_flux_solang)
 
 }  // namespace
 
@@ -361,16 +346,16 @@ void phy_surface_flux(const Model& m, cudaStream_t st) {
 
 void phy_solang_mko3(const Model& m, cudaStream_t st) { by_levels<SolangMko3>(m.d.L, m, st); }
 
-void phy_fused_fixer_flux_solang(const Model& m, cudaStream_t st) {
-  by_levels<FusedFixerFluxSolang>(m.d.L, m, st);
-}
-
 bool phy_flux_launch_one(const Model& m, const std::string& kernel, cudaStream_t st) {
   if (kernel == "vdiff") by_levels<Vdiff>(m.d.L, m, st);
   else if (kernel == "surflx") by_levels<Surflx>(m.d.L, m, st);
   else if (kernel == "fixer_apply") by_levels<FixerApply>(m.d.L, m, st);
   else if (kernel == "solang_mko3") by_levels<SolangMko3>(m.d.L, m, st);
-  else if (kernel == "fused_fixer_flux_solang") by_levels<FusedFixerFluxSolang>(m.d.L, m, st);
+  else if (kernel == "fused_fixer_flux_solang") {  // the four as a step runs them
+    phy_fixer_apply(m, st);
+    phy_surface_flux(m, st);
+    phy_solang_mko3(m, st);
+  }
   else return false;
   return true;
 }

@@ -243,7 +243,7 @@ void allow_smem(K kernel) {
 // batch's many rows reuse a staged table pair 8 times.
 int dft_rows(const Dims& d, int planes) {
   for (int r : {32, 16})
-    if (planes * (d.NLAT / r) >= 148) return r;
+    if (planes * (d.NLAT / r) >= sm_count()) return r;
   return 8;
 }
 
