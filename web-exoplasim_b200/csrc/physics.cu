@@ -4,10 +4,13 @@
 // Arithmetic follows src/model/climate/gcm/physics/*/wgsl/*.wgsl and
 // snapshot/wgsl/pack.wgsl (ExoPlaSim's miscmod fixer, fluxmod, radmod,
 // rainmod, landmod, vegmod, glaciermod, icemod, oceanmod, seamod,
-// carbonmod). One thread owns one column c = slot * NHOR + h of the batch and
-// keeps its levels in registers (kernels are instantiated per level count).
-// The reference's per-planet global sums (fixer, getiflx) and the mkdca pass
-// limit run as one block per slot with a fixed summation order, in FP64.
+// carbonmod). One thread owns one column c = slot * NHOR + h of the batch
+// (swr: two threads, one per band; small batches' kuo and rain are in
+// physics_levels.cu) and keeps its levels in registers, or in its column of
+// shared memory where the level loops are rolled (swr, lwr, kuo, rain). Kernels
+// are instantiated per level count. The reference's per-planet global sums
+// (fixer, getiflx) run as one block per slot with a fixed summation order, in
+// FP64; the mkdca pass limit is raised by the columns that need it.
 // The fixer's apply step, the surface fluxes, vertical diffusion, solar
 // angle and ozone are in physics_flux.cu (IEEE division).
 #include "physics_common.cuh"
@@ -2063,14 +2066,13 @@ void phy_surface(const Model& m, cudaStream_t st) {
 
 void phy_carbon(const Model& m, cudaStream_t st) { by_levels<Carbon>(m.d.L, m, st); }
 
-// The full step's physics. Fusing
-// consecutive per-column routines into one kernel was measured per pair at
-// 128 T42 L10 planets (CUDA events): land surface + sea ice (86.5 against
-// 88.7 us) and sea + carbon (57.7 against 60.2 us) pay and run fused; fixer
-// apply + surflx + vdiff + solang/mko3 (375.6 against 354.1 us), kuo + mkdca
-// (199.7 against 180.6 us) and rain + soil (274.0 against 259.5 us) lost more
-// to the fused kernels' register pressure and lower occupancy than they saved
-// in re-reads, and run as separate kernels.
+// The full step's physics. Fusing consecutive per-column routines into one
+// kernel was measured per pair at 128 T42 L10 planets (CUDA events): land
+// surface + sea ice (85.2 against 85.6 us) and sea + carbon (54.9 against 59.9)
+// save a launch each and run fused. Kernels of fixer apply + surflx + vdiff +
+// solang/mko3, kuo + mkdca and rain + soil were 5 to 10 % slower than their parts,
+// in the forms these had before their level loops were rolled, by register
+// pressure and lower occupancy; the parts run by themselves (276, 152 and 199 us).
 void phy_swr(const Model& m, cudaStream_t st) { by_levels<Swr>(m.d.L, m, st); }
 
 void phy_lwr(const Model& m, cudaStream_t st) { by_levels<LwrRadstep>(m.d.L, m, st); }

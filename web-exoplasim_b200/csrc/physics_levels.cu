@@ -486,9 +486,12 @@ LEVEL_LAUNCHER(KuoLevels, k_kuo_levels)
 }  // namespace
 
 // us a launch, a thread per column against a thread per (column, level), at
-// columns x levels (CUDA events): rain 2,048 x 5 9.9 / 5.2, 8,192 x 10 17.1 /
-// 8.2, 18,432 x 10 16.2 / 12.4, 32,768 x 10 17.6 / 18.7, 65,536 x 10 24.4 /
-// 31.8; kuo 4.3 / 3.4, 8.2 / 3.9, 8.3 / 6.3, 17.1 / 17.3, 20.8 / 27.6.
+// columns x levels (CUDA events): rain 2,048 x 10 14.3 / 7.0, 8,192 x 10 14.6 /
+// 8.2, 18,432 x 10 16.5 / 14.5, 24,576 x 10 16.5 / 16.5, 32,768 x 10 16.5 / 22.2;
+// kuo 7.4 / 3.7, 7.4 / 4.0, 14.5 / 8.5, 10.4 / 10.4, 10.4 / 13.8. The line is ten
+// levels'. With five, whose blocks have half the warps, the second form still
+// wins somewhat above it: a step of T21 L5 planets 95 / 88 at 2,048 columns, 144 /
+// 136 at 20,480, 144 / 131 at 24,576, 154 / 141 at 32,768, 166 / 176 at 49,152.
 bool phy_levels(const Model& m) { return (long)m.d.S * m.d.NHOR <= 20480; }
 
 void lev_rain(const Model& m, cudaStream_t st) { by_levels<RainLevels>(m.d.L, m, st); }
