@@ -742,6 +742,8 @@ cudaGraphExec_t batch_graph(exogcm_engine* e, int K, bool sides) {
   cudaGraphExec_t exec;
   check(cudaGraphInstantiate(&exec, sides ? captured_steps(e, K) : in_order.get(), 0), "graph instantiate");
   e->graphs[{K, sides}] = exec;
+  // on the device before the batch's start event: its time is the steps' alone
+  check(cudaGraphUpload(exec, e->stream), "graph upload");
   return exec;
 }
 
@@ -1520,8 +1522,11 @@ int exogcm_group_step(exogcm_engine** engines, int count, const int* steps, int 
               "group graph child");
       }
       check(cudaGraphInstantiate(&exec, parent.get(), 0), "group graph instantiate");
-      std::lock_guard<std::mutex> lock(g_group_mutex);
-      g_group_graphs[key].exec = exec;
+      {
+        std::lock_guard<std::mutex> lock(g_group_mutex);
+        g_group_graphs[key].exec = exec;
+      }
+      check(cudaGraphUpload(exec, st), "group graph upload");
     }
     check(cudaEventRecord(lead->ev0, st), "event");
     if (graph) {
