@@ -162,20 +162,21 @@ struct exogcm_engine {
     // Programmatic dependent launch. A dependent's waiting blocks are placed
     // where there is room while its predecessor drains. That hides the launch,
     // and gains where launches are most of a step (the smallest grids) and
-    // where grids run for several waves. Between, from a half to five blocks
-    // of 128 columns per SM, the step with it is the longer one, in most sizes by
-    // 2 to 7 %, so the column kernels there launch the ordinary way. us a step,
+    // where grids run for several waves. Between, up to five blocks of 128
+    // columns per SM, the step with it is the longer one, in most sizes by 2 to 7
+    // %, so the column kernels there launch the ordinary way. us a step,
     // column kernels without / with it, at columns (levels): 2,048 (10) 116 /
     // 113, 4,096 (10) 118 / 116, 6,144 (10) 123 / 129, 8,192 (5) 111 / 114, 8,192
     // (10) 143 / 142, 18,432 (10) 209 / 219, 53,248 (10) 244 / 255, 65,536 (10) 275
     // / 293, 73,728 (10) 354 / 373, 98,304 (10) 389 / 397, 131,072 (5) 265 / 266,
     // 131,072 (10) 473 / 469, 196,608 (10) 627 / 613, 589,824 (10) 1940 / 1906,
-    // 1,048,576 (10) 2969 / 2958; the lines are halfway between the sizes on their
-    // two sides. Everything else has it at every size (75,776 columns 342 -> 319,
+    // 1,048,576 (10) 2969 / 2958. 6,144 columns are an exception below the lower
+    // line: a line at 5,120 gained 5 % there and lost 1 to 2 % at 8,192 (10). The
+    // upper one is halfway between 98,304 and 131,072. Everything else has it at every size (75,776 columns 342 -> 319,
     // 196,608 392 -> 372, 1,048,576 3108 -> 3090).
     const long columns = (long)d.S * d.NHOR;
     m.pdl = 1;
-    m.column_pdl = columns <= 5120 || columns > 114688 ? 1 : 0;
+    m.column_pdl = columns <= 8192 || columns > 114688 ? 1 : 0;
     m.storm = 0;
     for (const Slot& s : slots) m.storm |= s.storm ? 1 : 0;
     return m;
